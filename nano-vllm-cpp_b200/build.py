@@ -79,6 +79,31 @@ def build(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
+BINDING_SRC = os.path.join(HERE, "bindings", "nvk_torch.cpp")
+BINDING = os.path.join(HERE, "nvk_torch.so")
+
+
+def build_binding(force: bool = False) -> str:
+    """Builds the Python binding (``nvk_torch.so``) against ``libnvk.so`` and the installed torch."""
+    build()
+    header = os.path.join(os.path.dirname(HERE), "include", "nvk.h")
+    if not force and os.path.exists(BINDING) and os.path.getmtime(BINDING) >= max(os.path.getmtime(BINDING_SRC), os.path.getmtime(header)):
+        return BINDING
+    import sysconfig
+    import torch
+    from torch.utils.cpp_extension import include_paths
+    lib_dir = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd = [_gxx(), "-std=c++17", "-O2", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    for d in (sysconfig.get_paths()["include"], *include_paths(), os.path.join(CUDA_HOME, "include")):
+        cmd += ["-isystem", d]
+    cmd += ["-o", BINDING, BINDING_SRC, "-L", HERE, "-L", lib_dir, "-lnvk", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda",
+            "-Wl,-rpath,$ORIGIN"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"binding build failed:\n{res.stdout}\n{res.stderr}")
+    return BINDING
+
+
 HOST_DIR = os.path.join(HERE, "host")
 HOST_LIB = os.path.join(HERE, "libnvk_host.so")
 CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
@@ -123,4 +148,5 @@ def build_host(force: bool = False) -> str:
 
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose="-v" in sys.argv))
+    print(build_binding(force="--force" in sys.argv))
     print(build_host(force="--force" in sys.argv))
