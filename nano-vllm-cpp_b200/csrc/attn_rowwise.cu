@@ -2,8 +2,8 @@
 // head_dim <= 256, any block size, dense or paged keys, decode or bottom-right causal prefill.
 //
 // This is the shape-agnostic path behind nvk_decode_attention_paged and
-// nvk_prefill_attention_varlen for inputs the tensor-core kernels do not take (fp32 models,
-// the tiny shapes of the reference's own known-answer tests, odd head sizes).  It computes what
+// nvk_prefill_attention_varlen for inputs no other kernel takes (fp32 prefill, the tiny shapes of
+// the reference's own known-answer tests, odd head sizes).  It computes what
 // src/kernels/attention.cu:114-405 of the reference computes -- fp32 accumulation, natural
 // exponent, online softmax over keys in order -- with one code path instead of three kernels:
 // the per-row key range and addressing mode are resolved up front, and four keys are scored

@@ -118,6 +118,7 @@ int nvk_decode_attention_paged(const void* query, const void* k_cache, const voi
         }
         return launch_decode_mma(a);
     }
+    if (decode_simt_supported(a)) return launch_decode_simt(a);
     return launch_rowwise_decode(a);
 }
 

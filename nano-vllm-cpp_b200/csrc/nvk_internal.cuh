@@ -54,6 +54,8 @@ struct IndexArray {
 #endif
 };
 
+constexpr int kSmCount = 148;   // of a B200; grids are sized by it
+
 // ---- launchers (one per .cu file) -----------------------------------------------------------
 struct DecodeArgs {
     const void* q; const void* k_cache; const void* v_cache;
@@ -94,6 +96,9 @@ int launch_fused_prologue(const void* qkv, const int32_t* positions, const void*
 // General SIMT attention (any dtype of F16/BF16/F32, head_dim <= 256, any block size).
 int launch_rowwise_decode(const DecodeArgs& a);
 int launch_rowwise_prefill(const PrefillArgs& a);
+// fp32-arithmetic decode, head_dim 64 / 128 / 256 (decode_simt.cu).
+bool decode_simt_supported(const DecodeArgs& a);
+int launch_decode_simt(const DecodeArgs& a);
 // Tensor-core paths (F16/BF16, head_dim 128).
 bool decode_mma_supported(const DecodeArgs& a);
 size_t decode_mma_workspace_bytes(int64_t batch, int num_heads, int num_kv_heads, int head_dim,

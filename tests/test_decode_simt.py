@@ -1,0 +1,50 @@
+"""fp32-arithmetic paged decode (clusters of blocks over a sequence's keys) at the edges of its tiling: contexts around a
+warp's trip and a block's round of trips, every group remainder, cluster sizes 1 to 8, odd block sizes, ids outside the cache."""
+import math
+
+import numpy as np
+import pytest
+
+from util import nvk, to_dev, to_np, workloads
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def _reference(w, hkv, bs):
+    q, out = w["q"].astype(np.float64), np.zeros(w["q"].shape)
+    d = q.shape[2]
+    kc, vc = (np.concatenate([w[n].reshape(-1, hkv, d), np.zeros((1, hkv, d))]).astype(np.float64) for n in ("k_cache", "v_cache"))
+    for b, n in enumerate(w["context_lens"]):
+        pos = np.arange(max(int(n), 0))
+        if not len(pos):
+            continue
+        rows = w["block_tables"][b, pos // bs].astype(np.int64) * bs + pos % bs
+        rows[(rows < 0) | (rows >= len(kc) - 1)] = -1                    # ids outside the cache read as zeros
+        for h in range(q.shape[1]):
+            kv = h * hkv // q.shape[1]
+            s = kc[rows, kv] @ q[b, h] * w["scale"]
+            p = np.exp(s - s.max())
+            out[b, h] = p @ vc[rows, kv] / p.sum()
+    return out
+
+
+@pytest.mark.parametrize("dtype,head_dim,block_size", [("f32", 128, 256), ("f32", 64, 16), ("f32", 256, 7), ("bf16", 64, 16), ("f16", 256, 3)])
+@pytest.mark.parametrize("num_heads,num_kv_heads,batch", [(2, 2, 1), (6, 2, 5), (5, 1, 9), (8, 1, 3), (16, 8, 8), (4, 2, 160)])
+def test_decode_simt_matches_a_float64_reference(dtype, head_dim, block_size, num_heads, num_kv_heads, batch):
+    ctx = np.array(([0, 1, 7, 8, 9, 63, 64, 65, 127, 129, 300, 511, 513, 640] * 12)[:batch], np.int32)
+    ctx[-1] = 641
+    w = workloads().make_decode_workload(batch, num_heads, num_kv_heads, head_dim, block_size, 0, 0, seed=batch + head_dim, context_lens=ctx,
+                                         value_scale=0.5, rounded=dtype != "f32")
+    if dtype == "f16":
+        for n in ("q", "k_cache", "v_cache"):
+            w[n] = w[n].astype(np.float16).astype(np.float32)
+    w["block_tables"][-1, 1] = w["k_cache"].shape[0] + 5
+    td = {"f32": torch.float32, "bf16": torch.bfloat16, "f16": torch.float16}[dtype]
+    q = to_dev(w["q"], td)
+    out = torch.full_like(q, float("nan"))
+    nvk().launch_decode_attention_paged(q, to_dev(w["k_cache"], td), to_dev(w["v_cache"], td), to_dev(ctx), to_dev(w["block_tables"]), num_kv_heads,
+                                        head_dim, block_size, w["scale"], out)
+    err = np.abs(to_np(out) - _reference(w, num_kv_heads, block_size))
+    assert err.max() <= (2e-6 if dtype == "f32" else 1e-2), err.max()
+    assert math.isfinite(float(out.float().abs().max()))
