@@ -790,6 +790,8 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     const bool decode_first = MIXED && static_cast<int>(blockIdx.x) >= md.prefill_blocks;
     if (decode_first) {
         decode_half();
+        // the prefill half's bulk copies write the shared memory that the decode half has read and written
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         __syncthreads();
     }
     const uint32_t sm_q = smem_base + kOff4Q, sm_k = smem_base + kOff4K, sm_v = smem_base + kOff4V, sm_p = smem_base + kOff4P;
@@ -1059,10 +1061,14 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             tc_fence_after();
             {
                 // The last P.V is complete, so the P buffer is free: stage this warp's 32 output rows there (16-byte
-                // chunks XOR-swizzled by row) and write them out as whole 256-byte rows.  The next item's Q is
-                // already being loaded into the Q buffer meanwhile.
+                // chunks XOR-swizzled by row) and write them out as whole 256-byte rows.  A row is staged where the same row
+                // of P lies in the two panels: a warp that is ahead may already write the next item's P rows, and those must
+                // not be where a slower warp's output still waits to be read.  The next item's Q is already being loaded into
+                // the Q buffer meanwhile.
                 const float inv = l_run > 0.0f ? 1.0f / l_run : 0.0f;
-                unsigned char* stage = p_panels;
+                auto staged = [&](int r, int chunk) {
+                    return reinterpret_cast<uint4*>(p_panels + (chunk >> 3) * kPanelBytes + r * 128 + (((chunk & 7) ^ (r & 7)) << 4));
+                };
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     uint32_t r[32];
@@ -1076,7 +1082,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                         v.z = ElemTraits<T>::pack2(__uint_as_float(r[q4 * 8 + 4]) * inv, __uint_as_float(r[q4 * 8 + 5]) * inv);
                         v.w = ElemTraits<T>::pack2(__uint_as_float(r[q4 * 8 + 6]) * inv, __uint_as_float(r[q4 * 8 + 7]) * inv);
                         const int chunk = c * 4 + q4;
-                        *reinterpret_cast<uint4*>(stage + row * 256 + ((chunk ^ (row & 15)) << 4)) = v;
+                        *staged(row, chunk) = v;
                     }
                 }
                 // O has left TMEM: the arrive on p_full in the next item's first round tells the issuer so
@@ -1086,7 +1092,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 for (int i = 0; i < 16; ++i) {
                     const int r = wq * 32 + 2 * i + (lane >> 4), chunk = lane & 15;
                     if (r < g.rows_here) {
-                        const uint4 v = *reinterpret_cast<const uint4*>(stage + r * 256 + ((chunk ^ (r & 15)) << 4));
+                        const uint4 v = *staged(r, chunk);
                         *reinterpret_cast<uint4*>(o0 + r * out_stride + chunk * 8) = v;
                     }
                 }
