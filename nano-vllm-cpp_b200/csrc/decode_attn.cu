@@ -33,28 +33,6 @@ namespace {
 
 using namespace dec;   // constants, DecodeParams and decode_split_body: decode_body.cuh
 
-// The decode kernels are launched with the programmatic-stream-serialization attribute: a kernel's blocks may be
-// scheduled while its predecessor in the stream still runs, wait here until that predecessor has completed and its
-// writes are visible (the first thing every block does, so nothing is read early), and at once allow their own
-// successor the same head start.  In a decode graph of several hundred short kernels this hides launch latency.
-__device__ __forceinline__ void pdl_wait_then_release() {
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-}
-
-// <<<grid, block, smem, stream>>> with that attribute.
-template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
-}
-
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 2) decode_split_kernel(const DecodeParams p) {
     extern __shared__ __align__(128) unsigned char smem[];

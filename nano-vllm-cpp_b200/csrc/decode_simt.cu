@@ -75,8 +75,7 @@ __global__ void __launch_bounds__(kThreads, HG <= 2 ? 2 : 1) decode_simt_kernel(
     __shared__ float s_m[kWarps][HG], s_l[kWarps][HG];
     __shared__ float s_po[HG][D];                         // this block's merged partial result, read by the whole cluster
     __shared__ float s_pm[HG], s_pl[HG];
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    pdl_wait_then_release();
     cg::cluster_group cluster = cg::this_cluster();
     const int csize = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;

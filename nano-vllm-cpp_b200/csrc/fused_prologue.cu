@@ -19,9 +19,6 @@
 //   * about 64 registers per thread, so four 256-thread blocks (32 warps) are resident per SM -- the first
 //     version of this kernel kept three heads and a prefetched row per thread in 122 registers and was
 //     latency-bound at 16 warps per SM.
-// The launch carries the programmatic-stream-serialization attribute: the kernel waits for its predecessor
-// in the stream with griddepcontrol.wait as its first action, so its launch latency overlaps the predecessor's
-// tail, and it releases its own dependents at once (they wait the same way).
 #include "nvk_internal.cuh"
 
 namespace nvk {
@@ -83,8 +80,7 @@ template <typename T, int D>   // D = head_dim: 64, 128 or 256
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) fused_prologue_kernel(const PrologueParams p) {
     constexpr int LANES = D / 16;                           // lanes per head
     constexpr int GROUPS = 32 / LANES;                      // heads a warp handles at once
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");    // the packed rows come from the kernel before this one
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    pdl_wait_then_release();                                // the packed rows come from the kernel before this one
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sub = lane % LANES, group = lane / LANES;
     const int heads = p.hq + 2 * p.hkv;
@@ -191,36 +187,15 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) fused_prologue_kernel(
     }
 }
 
-int prologue_sm_count() {
-    static int sms[64] = {};
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return 148;
-    if (sms[device] == 0) {
-        int n = 0;
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || n <= 0) n = 148;
-        sms[device] = n;
-    }
-    return sms[device];
-}
-
 template <typename T, int D>
 int launch_dim(const PrologueParams& p, cudaStream_t stream) {
     constexpr int GROUPS = 32 / (D / 16);
     const int heads = p.hq + 2 * p.hkv;
     const int64_t units = p.rows * ((heads + GROUPS * kSteps - 1) / (GROUPS * kSteps));
-    const int64_t resident = static_cast<int64_t>(prologue_sm_count()) * 4;   // four blocks per SM
+    const int64_t resident = static_cast<int64_t>(kSmCount) * 4;   // four blocks per SM
     int64_t blocks = (units + kWarpsPerBlock - 1) / kWarpsPerBlock;
     if (blocks > resident) blocks = resident;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(static_cast<unsigned>(blocks));
-    cfg.blockDim = dim3(kWarpsPerBlock * 32);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, fused_prologue_kernel<T, D>, p);
+    const cudaError_t e = launch_pdl(fused_prologue_kernel<T, D>, dim3(static_cast<unsigned>(blocks)), dim3(kWarpsPerBlock * 32), 0, stream, p);
     if (e != cudaSuccess) return fail(NVK_ERR_CUDA, "fused_split_norm_rope_store kernel launch: %s", cudaGetErrorString(e));
     return check_launch("fused_split_norm_rope_store kernel launch");
 }

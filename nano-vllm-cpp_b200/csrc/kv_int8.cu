@@ -47,6 +47,7 @@ store_int8_kernel(const T* __restrict__ key, const T* __restrict__ value, int8_t
                   const int32_t* __restrict__ slot_mapping, int64_t num_tokens, int num_kv_heads, int64_t cache_rows) {
     constexpr int D = V * LANES;
     constexpr int kPerWarp = 32 / LANES;
+    pdl_wait_then_release();
     const int lane = threadIdx.x & 31;
     const int sub = lane % LANES;
     const int64_t total = num_tokens * num_kv_heads;
@@ -145,6 +146,7 @@ store_int8_packed_kernel(const T* __restrict__ key, const T* __restrict__ value,
     using P = typename Pair16<T>::type;
     constexpr int D = 8 * LANES;
     constexpr int kPerWarp = 32 / LANES;
+    pdl_wait_then_release();
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t sub = lane % LANES;
     uint32_t work = (blockIdx.x * kStoreWarps + (threadIdx.x >> 5)) * kPerWarp + lane / LANES;   // (token, head)
@@ -199,6 +201,7 @@ store_fp8_packed_kernel(const T* __restrict__ key, const T* __restrict__ value, 
     using P = typename Pair16<T>::type;
     constexpr int D = 8 * LANES;
     constexpr int kPerWarp = 32 / LANES;
+    pdl_wait_then_release();
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t sub = lane % LANES;
     uint32_t work = (blockIdx.x * kStoreWarps + (threadIdx.x >> 5)) * kPerWarp + lane / LANES;   // (token, head)
@@ -239,8 +242,9 @@ int launch_store_fp8_typed(const void* key, const void* value, void* k_cache, vo
     if (work >= 0x7fffffffLL) return fail(NVK_ERR_INVALID_ARGUMENT, "store_kvcache_fp8: too many tokens");
     const int64_t per_block = static_cast<int64_t>(kStoreWarps) * (32 / lanes);
     const int64_t blocks = (work + per_block - 1) / per_block;
+    cudaError_t e = cudaSuccess;
 #define NVK_LAUNCH_FP8(L)                                                                                           \
-    store_fp8_packed_kernel<T, L><<<static_cast<unsigned>(blocks), kStoreWarps * 32, 0, stream>>>(                   \
+    e = launch_pdl(store_fp8_packed_kernel<T, L>, dim3(static_cast<unsigned>(blocks)), dim3(kStoreWarps * 32), 0, stream,\
         static_cast<const T*>(key), static_cast<const T*>(value), static_cast<uint8_t*>(k_cache),                  \
         static_cast<uint8_t*>(v_cache), static_cast<__half*>(k_scale), static_cast<__half*>(v_scale), slot_mapping, \
         static_cast<uint32_t>(work), static_cast<uint32_t>(num_kv_heads), cache_rows)
@@ -250,6 +254,7 @@ int launch_store_fp8_typed(const void* key, const void* value, void* k_cache, vo
         default: NVK_LAUNCH_FP8(32); break;
     }
 #undef NVK_LAUNCH_FP8
+    if (e != cudaSuccess) return fail(NVK_ERR_CUDA, "store_kvcache_fp8 kernel launch: %s", cudaGetErrorString(e));
     return check_launch("store_kvcache_fp8 kernel launch");
 }
 
@@ -316,10 +321,11 @@ int launch_store_typed(const void* key, const void* value, void* k_cache, void* 
     const int64_t per_block = static_cast<int64_t>(kStoreWarps) * (32 / lanes);
     const int64_t blocks = (work + per_block - 1) / per_block;
     if (blocks > 0x7fffffffLL) return fail(NVK_ERR_INVALID_ARGUMENT, "store_kvcache_int8: too many tokens");
+    cudaError_t e = cudaSuccess;
     if constexpr (sizeof(T) == 2) {
         if (work > 0 && work < 0x7fffffffLL) {
 #define NVK_LAUNCH_PACKED(L)                                                                                        \
-    store_int8_packed_kernel<T, L><<<static_cast<unsigned>(blocks), kStoreWarps * 32, 0, stream>>>(                  \
+    e = launch_pdl(store_int8_packed_kernel<T, L>, dim3(static_cast<unsigned>(blocks)), dim3(kStoreWarps * 32), 0, stream,\
         static_cast<const T*>(key), static_cast<const T*>(value), static_cast<int8_t*>(k_cache),                   \
         static_cast<int8_t*>(v_cache), static_cast<__half*>(k_scale), static_cast<__half*>(v_scale), slot_mapping, \
         static_cast<uint32_t>(work), static_cast<uint32_t>(num_kv_heads), cache_rows)
@@ -329,11 +335,12 @@ int launch_store_typed(const void* key, const void* value, void* k_cache, void* 
                 default: NVK_LAUNCH_PACKED(32); break;
             }
 #undef NVK_LAUNCH_PACKED
+            if (e != cudaSuccess) return fail(NVK_ERR_CUDA, "store_kvcache_int8 kernel launch: %s", cudaGetErrorString(e));
             return check_launch("store_kvcache_int8 kernel launch");
         }
     }
 #define NVK_LAUNCH(L)                                                                                               \
-    store_int8_kernel<T, V, L><<<static_cast<unsigned>(blocks), kStoreWarps * 32, 0, stream>>>(                      \
+    e = launch_pdl(store_int8_kernel<T, V, L>, dim3(static_cast<unsigned>(blocks)), dim3(kStoreWarps * 32), 0, stream,\
         static_cast<const T*>(key), static_cast<const T*>(value), static_cast<int8_t*>(k_cache),                   \
         static_cast<int8_t*>(v_cache), static_cast<__half*>(k_scale), static_cast<__half*>(v_scale), slot_mapping, \
         num_tokens, num_kv_heads, cache_rows)
@@ -343,6 +350,7 @@ int launch_store_typed(const void* key, const void* value, void* k_cache, void* 
         default: NVK_LAUNCH(32); break;
     }
 #undef NVK_LAUNCH
+    if (e != cudaSuccess) return fail(NVK_ERR_CUDA, "store_kvcache_int8 kernel launch: %s", cudaGetErrorString(e));
     return check_launch("store_kvcache_int8 kernel launch");
 }
 

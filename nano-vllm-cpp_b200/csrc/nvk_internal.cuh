@@ -10,6 +10,7 @@
 #include <cstddef>
 #include <cstdint>
 #include <cstdio>
+#include <utility>
 
 #include "../../include/nvk.h"
 
@@ -209,6 +210,28 @@ __device__ __forceinline__ float fast_exp2(float x) {
 }
 
 constexpr float kLog2e = 1.4426950408889634f;
+
+// The kernels are launched with the programmatic-stream-serialization attribute: a kernel's blocks may be scheduled while
+// its predecessor in the stream still runs, wait here until that predecessor has completed and its writes are visible
+// (before anything is read or written), and at once allow their own successor the same head start.  In a step of many short
+// kernels this hides launch latency.
+__device__ __forceinline__ void pdl_wait_then_release() {
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
+// <<<grid, block, smem, stream>>> with that attribute.
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
 
 #endif  // __CUDACC__
 

@@ -279,6 +279,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const int tid = threadIdx.x, warp = tid >> 5;
     const int head = blockIdx.x;
     const int kvh = head * p.num_kv_heads / p.num_heads;
+    pdl_wait_then_release();
 
     // (reversed) tile index -> (sequence, first query row): later tiles of a sequence see more keys
     if (tid == 0) {
@@ -788,6 +789,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         }
     };
     const bool decode_first = MIXED && static_cast<int>(blockIdx.x) >= md.prefill_blocks;
+    if (MIXED) pdl_wait_then_release();
     if (decode_first) {
         decode_half();
         // the prefill half's bulk copies write the shared memory that the decode half has read and written
@@ -823,6 +825,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&s_tmem_base)), "r"(kTmemCols2) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
+    if (!MIXED) pdl_wait_then_release();   // barriers and TMEM are set up under the predecessor's tail
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -1235,12 +1238,14 @@ int launch_typed(const PrefillArgs& a, bool bf16) {
         pp.total = static_cast<unsigned int>(pp.pairs) * static_cast<unsigned int>(tiles);
         pp.slot = static_cast<int>(g_launch_seq.fetch_add(1u) % kTicketSlots);
         const unsigned int blocks = pp.total < static_cast<unsigned int>(sms) ? pp.total : static_cast<unsigned int>(sms);
-        prefill_tc5_kernel<T, false><<<blocks, kThreads5, kSmemBytes4, a.stream>>>(tq, tk, tv, pp, MixedDecode{});
+        const cudaError_t e = launch_pdl(prefill_tc5_kernel<T, false>, dim3(blocks), dim3(kThreads5), kSmemBytes4, a.stream, tq, tk, tv, pp, MixedDecode{});
+        if (e != cudaSuccess) return fail(NVK_ERR_CUDA, "prefill_tc5_kernel launch: %s", cudaGetErrorString(e));
         return check_launch("prefill_tc5_kernel launch");
     }
     // odd group sizes: one block per (query tile, head)
     const dim3 grid(a.num_heads, static_cast<unsigned>(tiles));
-    prefill_tc_kernel<T><<<grid, kThreads, kSmemBytes, a.stream>>>(tq, tk, tv, p);
+    const cudaError_t e = launch_pdl(prefill_tc_kernel<T>, grid, dim3(kThreads), kSmemBytes, a.stream, tq, tk, tv, p);
+    if (e != cudaSuccess) return fail(NVK_ERR_CUDA, "prefill_tc_kernel launch: %s", cudaGetErrorString(e));
     return check_launch("prefill_tc_kernel launch");
 }
 
@@ -1298,7 +1303,9 @@ int launch_mixed_typed(const PrefillArgs& a, const DecodeArgs& d, int prefill_bl
     if (prefill_blocks < 1) prefill_blocks = 1;
     if (prefill_blocks > sms) prefill_blocks = sms;
     md.prefill_blocks = prefill_blocks;
-    prefill_tc5_kernel<T, true><<<static_cast<unsigned int>(sms), kThreads5, kSmemBytes4, a.stream>>>(L.tq, L.tk, L.tv, pp, md);
+    const cudaError_t e = launch_pdl(prefill_tc5_kernel<T, true>, dim3(static_cast<unsigned int>(sms)), dim3(kThreads5), kSmemBytes4, a.stream, L.tq, L.tk,
+                                     L.tv, pp, md);
+    if (e != cudaSuccess) return fail(NVK_ERR_CUDA, "mixed prefill + decode kernel launch: %s", cudaGetErrorString(e));
     rc = check_launch("mixed prefill + decode kernel launch");
     if (rc != NVK_OK) return rc;
     return launch_decode_merge(md.dp, d.batch, d.dtype, d.stream);

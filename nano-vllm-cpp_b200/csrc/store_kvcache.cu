@@ -21,6 +21,7 @@ store_rows_kernel(const VecT* __restrict__ key, const VecT* __restrict__ value,
                   VecT* __restrict__ k_cache, VecT* __restrict__ v_cache,
                   const SlotT* __restrict__ slot_mapping, int64_t num_tokens, int64_t row_vecs,
                   int64_t cache_rows) {
+    pdl_wait_then_release();
     const int64_t per_tensor = num_tokens * row_vecs;
     const int64_t total = 2 * per_tensor;
     const int64_t stride = static_cast<int64_t>(gridDim.x) * kThreads * kUnroll;
@@ -60,23 +61,19 @@ int launch_typed(const void* key, const void* value, void* k_cache, void* v_cach
                  bool slot_i64, int64_t num_tokens, int64_t row_bytes, int64_t cache_rows, cudaStream_t stream) {
     const int64_t row_vecs = row_bytes / static_cast<int64_t>(sizeof(VecT));
     const int64_t total = 2 * num_tokens * row_vecs;
-    int device = 0, sms = 148;
-    cudaGetDevice(&device);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const int64_t per_block = static_cast<int64_t>(kThreads) * kUnroll;
     int64_t blocks = (total + per_block - 1) / per_block;
-    const int64_t cap = static_cast<int64_t>(sms) * 8;  // 8 resident 256-thread blocks per SM
+    const int64_t cap = static_cast<int64_t>(kSmCount) * 8;  // 8 resident 256-thread blocks per SM
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
-    if (slot_i64) {
-        store_rows_kernel<VecT, int64_t><<<static_cast<unsigned>(blocks), kThreads, 0, stream>>>(
-            static_cast<const VecT*>(key), static_cast<const VecT*>(value), static_cast<VecT*>(k_cache),
-            static_cast<VecT*>(v_cache), static_cast<const int64_t*>(slot_mapping), num_tokens, row_vecs, cache_rows);
-    } else {
-        store_rows_kernel<VecT, int32_t><<<static_cast<unsigned>(blocks), kThreads, 0, stream>>>(
-            static_cast<const VecT*>(key), static_cast<const VecT*>(value), static_cast<VecT*>(k_cache),
-            static_cast<VecT*>(v_cache), static_cast<const int32_t*>(slot_mapping), num_tokens, row_vecs, cache_rows);
-    }
+    auto launch = [&](auto* slots, auto kernel) {
+        return launch_pdl(kernel, dim3(static_cast<unsigned>(blocks)), dim3(kThreads), 0, stream, static_cast<const VecT*>(key),
+                          static_cast<const VecT*>(value), static_cast<VecT*>(k_cache), static_cast<VecT*>(v_cache), slots, num_tokens, row_vecs,
+                          cache_rows);
+    };
+    const cudaError_t e = slot_i64 ? launch(static_cast<const int64_t*>(slot_mapping), store_rows_kernel<VecT, int64_t>)
+                                   : launch(static_cast<const int32_t*>(slot_mapping), store_rows_kernel<VecT, int32_t>);
+    if (e != cudaSuccess) return fail(NVK_ERR_CUDA, "store_kvcache kernel launch: %s", cudaGetErrorString(e));
     return check_launch("store_kvcache kernel launch");
 }
 
