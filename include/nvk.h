@@ -106,7 +106,7 @@ size_t nvk_decode_attention_workspace_bytes(int64_t batch, int num_heads, int nu
  *   sequence b lives in cache row block_tables[b][k / block_size] * block_size + k % block_size.
  *   context_lens[b] <= 0 gives a zero row; a value beyond max_blocks * block_size (more keys than the table row
  *   can address) is treated as max_blocks * block_size.
- * workspace may be NULL (then every sequence is processed by one thread block per KV head);
+ * workspace may be NULL (then every sequence is processed by at most eight thread blocks per KV head);
  * otherwise it must hold nvk_decode_attention_workspace_bytes(...) bytes, 16-byte aligned.
  * dtype F16/BF16 with head_dim 128 take the tensor-core path; other shapes and F32 take the
  * general SIMT path.

@@ -1,6 +1,21 @@
-// Device code of the split-K paged decode step, shared by decode_split_kernel (decode_attn.cu) and the mixed
-// prefill + decode kernel (prefill_attn_tc.cu): one group of four warps works on one (KV head, split, sequence) item.
-// The group synchronises on a named barrier, so several groups can live in one thread block.
+// Device code of paged decode attention on tensor cores (F16 / BF16 queries, head_dim 128; 16-bit, int8 or e4m3 cache), shared
+// by the decode kernels (decode_attn.cu) and the mixed prefill + decode kernel (prefill_attn_tc.cu).
+//
+// The op is HBM-bound: every K and V row of every context is read once.  A group of four warps takes a range of the keys of one
+// (sequence, KV head); the G = Hq / Hkv <= 8 query heads of the KV head are the rows of the MMA tile, so a K / V row is read once
+// per KV head.  Each warp streams every fourth tile of 16 keys through a private ring of cp.async stages (no barrier in the main
+// loop); at the end the four warps merge through shared memory.
+//
+// Two ways to share a sequence out, by the sizes the host knows:
+//   chunks     ranges of `chunk_tokens` keys; where a context is longer than one, the ranges leave partial results (maximum, sum,
+//              unnormalised output) in the workspace and a second kernel merges them;
+//   per_seq    num_splits equal ranges of every sequence in one thread-block cluster, merged through distributed shared memory in
+//              the same launch, without a workspace: for small steps.
+//
+// Cutting the whole batch's keys into equal runs that ignore sequence boundaries (each block sums up the contexts, warps or groups
+// walk on from one sequence to the next with their rings full, a quarter of the work handed out dynamically) was built and measured:
+// the main loop gains 2 to 15 %, but the pass over the contexts, the look-ups and three to eight partial results per sequence
+// cost more: 48 us against 37 at 37 sequences of 100 to 2048 keys, 700 against 697 at 256 of 1024 to 8192.
 #pragma once
 
 #include "nvk_internal.cuh"
@@ -9,218 +24,508 @@ namespace nvk {
 namespace dec {
 
 constexpr int kHeadDim = 128;
-constexpr int kWarps = 4;
-constexpr int kThreads = kWarps * 32;
-constexpr int kTileTokens = 16;                       // tokens per warp tile
-constexpr int kRowBytes = kHeadDim * 2;               // one head row of K or V
-constexpr int kTileBytes = kTileTokens * kRowBytes;   // 4 KiB (K) ; V follows
-constexpr int kStageBytes = 2 * kTileBytes;           // K + V
-constexpr int kStages = 3;
-constexpr int kMaxGroup = 8;                          // query heads per KV head
-constexpr int kMaxChunkBlocks = 128;                  // block-table entries cached per block
-constexpr int kSmemBytes = kWarps * kStages * kStageBytes;  // 96 KiB -> two blocks per SM
+constexpr int kTileTokens = 16;
+constexpr int kMaxGroup = 8;           // query heads per KV head
+constexpr int kGroupWarps = 4;
+constexpr int kGroupThreads = kGroupWarps * 32;
+constexpr int kMergeWarps = 8;         // warps that merge the parts of one (sequence, head) where there are many
 
 struct DecodeParams {
     const void* q; const void* k_cache; const void* v_cache;
+    const __half* k_scale; const __half* v_scale;      // 8-bit caches
     IndexArray context_lens; IndexArray block_tables;
-    void* out; float* ws_o; float* ws_lse;
+    void* out; float* ws_o; float2* ws_ml;             // partial results: [sequence][KV head][split][group][128] and (maximum, sum)
     int64_t max_blocks, num_cache_blocks;
-    int num_heads, num_kv_heads, group, block_size, chunk_tokens, num_splits;
+    int batch, num_heads, num_kv_heads, group, block_size;
+    int chunk_tokens, num_splits;
+    int per_seq;                                       // 1: num_splits equal ranges per sequence instead of chunks
     float scale_log2;
 };
 
-// context_lens[b], limited to what the block table can address (max_blocks * block_size): a longer value would make
-// the split kernels read block_tables past the row and the merge kernel read partial results of the next row.
-__device__ __forceinline__ int clamped_context(const DecodeParams& p, int64_t b) {
+// context_lens[b], limited to what the block table can address (max_blocks * block_size), and not negative.
+__device__ __forceinline__ int clamped_context(const DecodeParams& p, int b) {
     const int64_t ctx = p.context_lens[b];
     const int64_t cap = p.max_blocks * p.block_size;
-    return static_cast<int>(ctx < cap ? ctx : cap);
+    return static_cast<int>(ctx < 0 ? 0 : ctx < cap ? ctx : cap);
+}
+// Keys of range `split` of a context: [t0, t1), empty where t0 >= t1; returns how many ranges have keys.
+__device__ __forceinline__ int split_range(const DecodeParams& p, int ctx, int split, int& t0, int& t1) {
+    const int len = p.per_seq ? ((ctx + p.num_splits - 1) / p.num_splits + kTileTokens - 1) / kTileTokens * kTileTokens : p.chunk_tokens;
+    t0 = split * len;
+    t1 = min(ctx, t0 + len);
+    return ctx > 0 ? (ctx + len - 1) / len : 0;
 }
 
-// Barrier over the 128 threads of one group (id 1..15; a block of exactly one group may as well use __syncthreads()).
-__device__ __forceinline__ void group_sync(int bar_id) { asm volatile("bar.sync %0, 128;\n" ::"r"(bar_id) : "memory"); }
+__device__ __forceinline__ void group_sync(int bar_id, int threads) { asm volatile("bar.sync %0, %1;\n" ::"r"(bar_id), "r"(threads) : "memory"); }
 
-// One (KV head, split, sequence) item.  `smem`: kSmemBytes of shared memory owned by this group (128-byte aligned),
-// `s_blocks`: kMaxChunkBlocks ints of shared memory, `tid`: 0..127 inside the group.  All 128 threads call it.
-template <typename T>
-__device__ __forceinline__ void decode_split_body(const DecodeParams& p, int kvh, int split, int64_t b, unsigned char* smem,
-                                                  int* s_blocks, int tid, int bar_id) {
-    const int warp = tid >> 5, lane = tid & 31;
-    const int g = lane >> 2, t = lane & 3;
-    const int G = p.group;
+// ---- cache formats: how a tile is fetched and what a warp does with it ---------------------------------------------------
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, int src_bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
+}
+__device__ __forceinline__ void lds32x4(uint32_t addr, uint32_t (&w)[4]) {
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(addr));
+}
 
-    const int ctx = clamped_context(p, b);
-    const int t0 = split * p.chunk_tokens;
-    T* out = static_cast<T*>(p.out);
-    if (ctx <= 0) {
-        if (split == 0) {  // empty context: zero rows for the whole group
-            for (int i = tid; i < G * kHeadDim; i += kThreads)
-                out[(b * p.num_heads + kvh * G) * kHeadDim + i] = ElemTraits<T>::from_float(0.0f);
+// Online-softmax state of a warp: accumulator columns of lane (g, t) = (lane / 4, lane % 4) are heads 2t and 2t + 1; maximum and
+// sum are those of head g.
+struct SoftmaxState {
+    float o[8][4];
+    float m, l;
+    __device__ __forceinline__ void reset() {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f; }
+        m = -INFINITY; l = 0.0f;
+    }
+    // New tile maximum: rescale where it moves (a handful of tiles of a sequence; the branch is warp-uniform).  `extra`: further
+    // columns that are scaled along.
+    __device__ __forceinline__ void raise_max(float m_tile, int t, float* extra) {
+        m_tile = fmaxf(m_tile, __shfl_xor_sync(0xffffffffu, m_tile, 1));
+        m_tile = fmaxf(m_tile, __shfl_xor_sync(0xffffffffu, m_tile, 2));
+        if (__any_sync(0xffffffffu, m_tile > m)) {
+            const float m_new = fmaxf(m, m_tile);   // finite: the tile's first key is always valid
+            const float corr = fast_exp2(m - m_new);
+            l *= corr;
+            m = m_new;
+            const float c0 = __shfl_sync(0xffffffffu, corr, 8 * t), c1 = __shfl_sync(0xffffffffu, corr, 8 * t + 4);
+#pragma unroll
+            for (int mt = 0; mt < 8; ++mt) { o[mt][0] *= c0; o[mt][1] *= c1; o[mt][2] *= c0; o[mt][3] *= c1; }
+            if (extra != nullptr) { extra[0] *= c0; extra[1] *= c1; extra[2] *= c0; extra[3] *= c1; }
         }
-        return;
     }
-    if (t0 >= ctx) return;
-    const int t1 = min(ctx, t0 + p.chunk_tokens);
-    const int live_splits = (ctx + p.chunk_tokens - 1) / p.chunk_tokens;
+};
 
-    // Physical block ids of this chunk (-1 = outside the cache: reads as zeros).
-    const int blk0 = t0 / p.block_size;
-    const int nblk = (t1 - 1) / p.block_size - blk0 + 1;
-    for (int i = tid; i < nblk; i += kThreads) {
-        const int64_t id = p.block_tables[b * p.max_blocks + blk0 + i];
-        s_blocks[i] = (id >= 0 && id < p.num_cache_blocks) ? static_cast<int>(id) : -1;
+// Keys past `valid` of a tile get no weight; only a sequence's last tile has any (warp-uniform branch).
+__device__ __forceinline__ void mask_scores(float (&sc)[4], int t, int valid) {
+    if (valid < kTileTokens) {
+        const int tk = 2 * t;
+        if (tk >= valid) sc[0] = -INFINITY;
+        if (tk + 1 >= valid) sc[1] = -INFINITY;
+        if (tk + 8 >= valid) sc[2] = -INFINITY;
+        if (tk + 9 >= valid) sc[3] = -INFINITY;
     }
-    group_sync(bar_id);
+}
 
-    // Query fragments: rows g < G of the 16-row A tile, rows 8..15 are zero.
-    uint32_t qa[8][2];
-    {
-        const uint32_t* qrow = reinterpret_cast<const uint32_t*>(
-            static_cast<const T*>(p.q) + (b * p.num_heads + kvh * G + (g < G ? g : 0)) * kHeadDim);
+// 16-bit cache.  K and V tiles of 16 x 256 bytes, XOR-swizzled by row; S = Q K^T as mma.sync m16n8k16 with the (zero padded)
+// query heads as the 16 rows; O^T = V^T P^T with V^T taken straight from the row-major V tile by ldmatrix.trans, so that the
+// probability fragment of S is already in the layout the second MMA wants.
+// 8 warps per SM x 3 stages of 8 KiB: 128 KiB in flight.
+template <typename T>
+struct Cache16 {
+    static constexpr int kGroups = 2;   // resident per SM
+    static constexpr int kRowBytes = kHeadDim * 2;
+    static constexpr int kTileBytes = kTileTokens * kRowBytes;
+    static constexpr int kStageBytes = 2 * kTileBytes;
+    static constexpr int kStages = 3;
+
+    SoftmaxState s;
+    uint32_t qa[8][2];   // rows g < G of the 16-row A tile; rows 8..15 are zero
+
+    __device__ __forceinline__ void start(const DecodeParams& p, int b, int kvh, int lane) {
+        const int g = lane >> 2, t = lane & 3;
+        const bool live = g < p.group;
+        const uint32_t* row = reinterpret_cast<const uint32_t*>(
+            static_cast<const T*>(p.q) + (static_cast<int64_t>(b) * p.num_heads + kvh * p.group + (live ? g : 0)) * kHeadDim);
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
-            qa[ks][0] = g < G ? qrow[ks * 8 + t] : 0u;
-            qa[ks][1] = g < G ? qrow[ks * 8 + 4 + t] : 0u;
+            qa[ks][0] = live ? row[ks * 8 + t] : 0u;
+            qa[ks][1] = live ? row[ks * 8 + 4 + t] : 0u;
+        }
+        s.reset();
+    }
+    // Rows row0 .. row0 + valid - 1 of the cache into a stage; the rest of the tile is zero-filled (stale cache contents, even NaN,
+    // never reach the arithmetic).
+    static __device__ __forceinline__ void issue(const DecodeParams& p, int kvh, int64_t row0, int valid, uint32_t stage, int lane) {
+        const size_t stride = static_cast<size_t>(p.num_kv_heads) * kRowBytes;
+        const int c = lane & 15, rhalf = lane >> 4;   // 16-byte piece c of rows 2 i + rhalf
+        const size_t base = static_cast<size_t>(row0) * stride + static_cast<size_t>(kvh) * kRowBytes + c * 16;
+        const unsigned char* kc = static_cast<const unsigned char*>(p.k_cache) + base;
+        const unsigned char* vc = static_cast<const unsigned char*>(p.v_cache) + base;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int r = 2 * i + rhalf;
+            const int bytes = r < valid ? 16 : 0;
+            const size_t src = bytes ? r * stride : 0;
+            const uint32_t dst = stage + r * kRowBytes + ((c ^ (r & 7)) << 4);
+            cp_async16(dst, kc + src, bytes);
+            cp_async16(dst + kTileBytes, vc + src, bytes);
         }
     }
-
-    unsigned char* ring = smem + warp * (kStages * kStageBytes);
-    const uint32_t ring_u32 = smem_u32(ring);
-    const int num_tiles = (t1 - t0 + kTileTokens - 1) / kTileTokens;
-    const int my_tiles = num_tiles > warp ? (num_tiles - warp + kWarps - 1) / kWarps : 0;
-    const size_t row_stride = static_cast<size_t>(p.num_kv_heads) * kRowBytes;  // bytes between tokens
-    const unsigned char* kc = static_cast<const unsigned char*>(p.k_cache) + static_cast<size_t>(kvh) * kRowBytes;
-    const unsigned char* vc = static_cast<const unsigned char*>(p.v_cache) + static_cast<size_t>(kvh) * kRowBytes;
-
-    // Lane's piece of a tile: 16-byte column c of rows r = 2 * i + (lane >> 4), i = 0..7.
-    const int c = lane & 15, rhalf = lane >> 4;
-
-    auto issue = [&](int j) {  // load this warp's j-th tile into stage j % kStages
-        if (j < my_tiles) {
-            const int tok0 = t0 + (warp + j * kWarps) * kTileTokens;
-            const int blk = tok0 / p.block_size;
-            const int phys = s_blocks[blk - blk0];
-            const int off = tok0 - blk * p.block_size;
-            const size_t base = (static_cast<size_t>(phys < 0 ? 0 : phys) * p.block_size + off) * row_stride + c * 16;
-            const uint32_t stage = ring_u32 + (j % kStages) * kStageBytes;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int r = 2 * i + rhalf;
-                const int bytes = (phys >= 0 && tok0 + r < t1) ? 16 : 0;
-                const size_t src = base + (bytes ? r * row_stride : 0);
-                const uint32_t dst = stage + r * kRowBytes + ((c ^ (r & 7)) << 4);
-                cp_async16(dst, kc + src, bytes);
-                cp_async16(dst + kTileBytes, vc + src, bytes);
-            }
-        }
-        cp_async_commit();
-    };
-
-    float o[8][4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f; }
-    float m_run = -INFINITY, l_run = 0.0f;  // per head g (replicated over the 4 lanes of a row)
-
-#pragma unroll
-    for (int s = 0; s < kStages - 1; ++s) issue(s);
-
-    // ldmatrix lane addressing.  K (non-transposed): matrices (tok 0-7, d lo), (tok 0-7, d hi),
-    // (tok 8-15, d lo), (tok 8-15, d hi) of one 16-wide k-step.  V (transposed): matrices
-    // (tok 0-7, d lo), (tok 0-7, d hi), (tok 8-15, d lo), (tok 8-15, d hi) of one 16-wide d-tile.
-    const int k_row = ((lane >> 4) << 3) + (lane & 7);
-    const int k_sel = (lane >> 3) & 1;
-    const int v_row = (((lane >> 3) >> 1) << 3) + (lane & 7);
-    const int v_sel = (lane >> 3) & 1;
-
-    for (int j = 0; j < my_tiles; ++j) {
-        issue(j + kStages - 1);
-        cp_async_wait<kStages - 1>();
-        __syncwarp();
-        const uint32_t stage = ring_u32 + (j % kStages) * kStageBytes;
-        const int tok0 = t0 + (warp + j * kWarps) * kTileTokens;
-
+    __device__ __forceinline__ void step(const DecodeParams& p, uint32_t stage, int valid, int /*kvh*/, int lane) {
+        const int t = lane & 3;
+        // ldmatrix lane addressing.  K: matrices (tok 0-7, d lo), (tok 0-7, d hi), (tok 8-15, d lo), (tok 8-15, d hi) of one
+        // 16-wide k-step.  V (transposed): the same of one 16-wide d-tile.
+        const int row = ((lane >> 4) << 3) + (lane & 7), sel = (lane >> 3) & 1;
         float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
             uint32_t b0, b1, b2, b3;
-            const int chunk = 2 * ks + k_sel;
-            ldmatrix_x4(b0, b1, b2, b3, stage + k_row * kRowBytes + ((chunk ^ (k_row & 7)) << 4));
+            ldmatrix_x4(b0, b1, b2, b3, stage + row * kRowBytes + (((2 * ks + sel) ^ (row & 7)) << 4));
             mma_16816<T>(s0, qa[ks][0], 0u, qa[ks][1], 0u, b0, b1);
             mma_16816<T>(s1, qa[ks][0], 0u, qa[ks][1], 0u, b2, b3);
         }
-        // scores of head g: tokens tok0 + {2t, 2t+1, 8+2t, 9+2t}
-        float sc[4];
-        sc[0] = s0[0] * p.scale_log2; sc[1] = s0[1] * p.scale_log2;
-        sc[2] = s1[0] * p.scale_log2; sc[3] = s1[1] * p.scale_log2;
-        const int tk = tok0 + 2 * t;
-        if (tk >= t1) sc[0] = -INFINITY;
-        if (tk + 1 >= t1) sc[1] = -INFINITY;
-        if (tk + 8 >= t1) sc[2] = -INFINITY;
-        if (tk + 9 >= t1) sc[3] = -INFINITY;
-        float m_tile = fmaxf(fmaxf(sc[0], sc[1]), fmaxf(sc[2], sc[3]));
-        m_tile = fmaxf(m_tile, __shfl_xor_sync(0xffffffffu, m_tile, 1));
-        m_tile = fmaxf(m_tile, __shfl_xor_sync(0xffffffffu, m_tile, 2));
-        const float m_new = fmaxf(m_run, m_tile);   // finite: token tok0 is always valid
-        const float corr = fast_exp2(m_run - m_new);
-        const float p0 = fast_exp2(sc[0] - m_new), p1 = fast_exp2(sc[1] - m_new);
-        const float p2 = fast_exp2(sc[2] - m_new), p3 = fast_exp2(sc[3] - m_new);
-        l_run = l_run * corr + ((p0 + p1) + (p2 + p3));
-        m_run = m_new;
-        const uint32_t pb0 = ElemTraits<T>::pack2(p0, p1);
-        const uint32_t pb1 = ElemTraits<T>::pack2(p2, p3);
-        // accumulator columns of this lane are heads 2t and 2t+1
-        const float c0 = __shfl_sync(0xffffffffu, corr, 8 * t);
-        const float c1 = __shfl_sync(0xffffffffu, corr, 8 * t + 4);
+        float sc[4] = {s0[0] * p.scale_log2, s0[1] * p.scale_log2, s1[0] * p.scale_log2, s1[1] * p.scale_log2};   // keys 2t, 2t+1, 8+2t, 9+2t
+        mask_scores(sc, t, valid);
+        s.raise_max(fmaxf(fmaxf(sc[0], sc[1]), fmaxf(sc[2], sc[3])), t, nullptr);
+        const float p0 = fast_exp2(sc[0] - s.m), p1 = fast_exp2(sc[1] - s.m), p2 = fast_exp2(sc[2] - s.m), p3 = fast_exp2(sc[3] - s.m);
+        s.l += (p0 + p1) + (p2 + p3);
+        const uint32_t pb0 = ElemTraits<T>::pack2(p0, p1), pb1 = ElemTraits<T>::pack2(p2, p3);
 #pragma unroll
         for (int mt = 0; mt < 8; ++mt) {
             uint32_t a0, a1, a2, a3;
-            const int chunk = 2 * mt + v_sel;
-            ldmatrix_x4_trans(a0, a1, a2, a3, stage + kTileBytes + v_row * kRowBytes + ((chunk ^ (v_row & 7)) << 4));
-            o[mt][0] *= c0; o[mt][1] *= c1; o[mt][2] *= c0; o[mt][3] *= c1;
-            mma_16816<T>(o[mt], a0, a1, a2, a3, pb0, pb1);
+            ldmatrix_x4_trans(a0, a1, a2, a3, stage + kTileBytes + row * kRowBytes + (((2 * mt + sel) ^ (row & 7)) << 4));
+            mma_16816<T>(s.o[mt], a0, a1, a2, a3, pb0, pb1);
         }
+    }
+    // Position i = 0..15 of lane group g holds d = dim(g, i) of head 2t + h.
+    __device__ __forceinline__ float value(int h, int i) const { return s.o[i >> 1][(i & 1) * 2 + h]; }
+    static __device__ __forceinline__ int dim(int g, int i) { return (i >> 1) * 16 + (i & 1) * 8 + g; }
+};
+
+// Two 8-bit cache elements -> two f16 (MMA operand halves).  int8: the byte glued under the exponent byte of 1024 (the word has
+// had its sign bits flipped: value + 1152, taken out algebraically afterwards); e4m3: the hardware conversion, exact.
+template <bool FP8> __device__ __forceinline__ uint32_t widen_pair_lo(uint32_t x) {   // bytes 0, 1
+    if constexpr (FP8) {
+        uint32_t d;
+        asm("cvt.rn.f16x2.e4m3x2 %0, %1;\n" : "=r"(d) : "h"(static_cast<unsigned short>(x & 0xffffu)));
+        return d;
+    } else {
+        return __byte_perm(x, 0x64646464u, 0x4140);
+    }
+}
+template <bool FP8> __device__ __forceinline__ uint32_t widen_pair_hi(uint32_t x) {   // bytes 2, 3
+    if constexpr (FP8) {
+        uint32_t d;
+        asm("cvt.rn.f16x2.e4m3x2 %0, %1;\n" : "=r"(d) : "h"(static_cast<unsigned short>(x >> 16)));
+        return d;
+    } else {
+        return __byte_perm(x, 0x64646464u, 0x4342);
+    }
+}
+
+// 8-bit cache (int8, the reference's format: src/kernels/attention.cu:746-842; or e4m3 of the same layout): per token and KV head
+// 128 bytes of K, 128 of V and two fp16 scales.  The MMA fragments are built from the bytes in registers -- no widened copy in
+// shared memory, no ldmatrix:
+//   * an int8 x becomes the fp16 number 1024 + (x + 128) by gluing the byte (x ^ 0x80) under the exponent byte 0x64 (one PRMT per
+//     pair); the constant 1152 is taken out afterwards: q . (k' - 1152) = q . k' - 1152 * sum(q), and P (v' - 1152) = P v' - 1152 *
+//     sum(P), where sum(P) comes from one extra MMA per tile against a row of ones, i.e. from exactly the rounded probabilities the
+//     other MMAs used;
+//   * the MMAs contract over d (scores) and over keys (output); a contraction does not care in which order its index runs, and
+//     neither does the output care which accumulator row holds which d, so every lane takes whole 16-byte pieces: for K, piece 4q + t
+//     of key row g supplies its k-steps 4q .. 4q + 3 (the query fragment is loaded with the same permutation); for V, piece g of key
+//     rows 2t, 2t+1, 2t+8, 2t+9 supplies all eight d-tiles after a byte interleave of row pairs (two PRMTs), and accumulator row g /
+//     g + 8 of d-tile 2a + e holds d = 16 g + 4 a + 2 e (+ 1);
+//   * pieces are XOR-swizzled in the ring so that those 16-byte reads are conflict free.
+// The scales never touch the tiles: k_scale multiplies the score of its key after the first MMA, v_scale the probability of its key
+// before the second (the row sum uses the unscaled probability).  MMAs run as f16 whatever the query type: the query is converted
+// once, probabilities are <= 1.  12 warps per SM x 4 stages of 4.1 KiB: 148 KiB in flight.
+template <typename T, bool FP8>
+struct Cache8 {
+    static constexpr int kGroups = 3;
+    static constexpr int kRowBytes = kHeadDim;
+    static constexpr int kTileBytes = kTileTokens * kRowBytes;
+    static constexpr int kScaleBytes = 2 * kTileTokens * 4;   // one 32-bit word per (K | V, token): the word that holds its fp16 scale
+    static constexpr int kStageBytes = 2 * kTileBytes + kScaleBytes;
+    static constexpr int kStages = 4;
+    static constexpr float kOffset = FP8 ? 0.0f : 1152.0f;    // 1024 (exponent glue) + 128 (sign flip)
+    static constexpr uint32_t kFlip = FP8 ? 0u : 0x80808080u; // int8: sign bits flipped before the glue
+
+    SoftmaxState s;
+    float osum[4];       // sum of the (scaled, rounded) probabilities per head, from the ones-row MMA
+    float q_off;
+    uint32_t qa[8][2];   // k-step ks = 4 q + w, positions {2t, 2t+1 | 2t+8, 2t+9} <- d = 64 q + 16 t + 4 w + {0, 1 | 2, 3}
+
+    __device__ __forceinline__ void start(const DecodeParams& p, int b, int kvh, int lane) {
+        const int g = lane >> 2, t = lane & 3;
+        const bool live = g < p.group;
+        const T* row = static_cast<const T*>(p.q) + (static_cast<int64_t>(b) * p.num_heads + kvh * p.group + (live ? g : 0)) * kHeadDim;
+        float qsum = 0.0f;   // of the f16-rounded query row g
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks) {
+            const int d0 = 64 * (ks >> 2) + 16 * t + 4 * (ks & 3);
+#pragma unroll
+            for (int hlf = 0; hlf < 2; ++hlf) {
+                const __half2 h2 = __floats2half2_rn(ElemTraits<T>::to_float(row[d0 + 2 * hlf]), ElemTraits<T>::to_float(row[d0 + 2 * hlf + 1]));
+                qa[ks][hlf] = live ? *reinterpret_cast<const uint32_t*>(&h2) : 0u;
+                if (live) qsum += __low2float(h2) + __high2float(h2);
+            }
+        }
+        qsum += __shfl_xor_sync(0xffffffffu, qsum, 1);
+        qsum += __shfl_xor_sync(0xffffffffu, qsum, 2);
+        q_off = kOffset * qsum;
+        osum[0] = osum[1] = osum[2] = osum[3] = 0.0f;
+        s.reset();
+    }
+    static __device__ __forceinline__ void issue(const DecodeParams& p, int kvh, int64_t row0, int valid, uint32_t stage, int lane) {
+        const size_t stride = static_cast<size_t>(p.num_kv_heads) * kRowBytes;
+        const int c = lane & 7, rq = lane >> 3;   // 16-byte piece c of rows 4 i + rq; ring swizzles: K piece c ^ ((r & 1) << 2), V piece c ^ (r & 6)
+        const size_t base = static_cast<size_t>(row0) * stride + static_cast<size_t>(kvh) * kRowBytes + c * 16;
+        const unsigned char* kc = static_cast<const unsigned char*>(p.k_cache) + base;
+        const unsigned char* vc = static_cast<const unsigned char*>(p.v_cache) + base;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = 4 * i + rq;
+            const int bytes = r < valid ? 16 : 0;
+            const size_t src = bytes ? r * stride : 0;
+            cp_async16(stage + r * kRowBytes + ((c ^ ((r & 1) << 2)) << 4), kc + src, bytes);
+            cp_async16(stage + kTileBytes + r * kRowBytes + ((c ^ (r & 6)) << 4), vc + src, bytes);
+        }
+        // the scale of token (lane & 15): lanes 0-15 K, lanes 16-31 V; copied as the aligned 32-bit word around it
+        const int tr = lane & 15;
+        const int sbytes = tr < valid ? 4 : 0;
+        const size_t sidx = sbytes ? (static_cast<size_t>(row0) + tr) * p.num_kv_heads + kvh : 0;
+        cp_async4(stage + 2 * kTileBytes + lane * 4, (lane < 16 ? p.k_scale : p.v_scale) + (sidx & ~static_cast<size_t>(1)), sbytes);
+    }
+    __device__ __forceinline__ void step(const DecodeParams& p, uint32_t stage, int valid, int kvh, int lane) {
+        const int g = lane >> 2, t = lane & 3;
+        // which half of the copied word is this lane's scale: cache rows of a tile start at an even row, so the parity of row * Hkv +
+        // kvh is that of (token & Hkv & 1) + kvh
+        float scale;
+        {
+            uint32_t word;
+            asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(word) : "r"(stage + 2 * kTileBytes + lane * 4));
+            const __half2 pair = *reinterpret_cast<const __half2*>(&word);
+            scale = ((((lane & p.num_kv_heads) ^ kvh) & 1) != 0 ? __high2float(pair) : __low2float(pair)) * (lane < 16 ? p.scale_log2 : 1.0f);
+        }
+        // scores: keys g (n-tile 0) and g + 8 (n-tile 1)
+        float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            uint32_t w0[4], w1[4];
+            lds32x4(stage + g * kRowBytes + (((4 * q + t) ^ ((g & 1) << 2)) << 4), w0);
+            lds32x4(stage + (g + 8) * kRowBytes + (((4 * q + t) ^ ((g & 1) << 2)) << 4), w1);
+#pragma unroll
+            for (int wi = 0; wi < 4; ++wi) {
+                const int ks = 4 * q + wi;
+                const uint32_t x0 = w0[wi] ^ kFlip, x1 = w1[wi] ^ kFlip;
+                mma_16816<__half>(s0, qa[ks][0], 0u, qa[ks][1], 0u, widen_pair_lo<FP8>(x0), widen_pair_hi<FP8>(x0));
+                mma_16816<__half>(s1, qa[ks][0], 0u, qa[ks][1], 0u, widen_pair_lo<FP8>(x1), widen_pair_hi<FP8>(x1));
+            }
+        }
+        const float ks0 = __shfl_sync(0xffffffffu, scale, 2 * t), ks1 = __shfl_sync(0xffffffffu, scale, 2 * t + 1);
+        const float ks2 = __shfl_sync(0xffffffffu, scale, 8 + 2 * t), ks3 = __shfl_sync(0xffffffffu, scale, 9 + 2 * t);
+        const float vs0 = __shfl_sync(0xffffffffu, scale, 16 + 2 * t), vs1 = __shfl_sync(0xffffffffu, scale, 17 + 2 * t);
+        const float vs2 = __shfl_sync(0xffffffffu, scale, 24 + 2 * t), vs3 = __shfl_sync(0xffffffffu, scale, 25 + 2 * t);
+        float sc[4] = {(s0[0] - q_off) * ks0, (s0[1] - q_off) * ks1, (s1[0] - q_off) * ks2, (s1[1] - q_off) * ks3};   // keys 2t, 2t+1, 8+2t, 9+2t
+        mask_scores(sc, t, valid);
+        s.raise_max(fmaxf(fmaxf(sc[0], sc[1]), fmaxf(sc[2], sc[3])), t, FP8 ? nullptr : osum);
+        const float p0 = fast_exp2(sc[0] - s.m), p1 = fast_exp2(sc[1] - s.m), p2 = fast_exp2(sc[2] - s.m), p3 = fast_exp2(sc[3] - s.m);
+        s.l += (p0 + p1) + (p2 + p3);
+        const uint32_t pb0 = ElemTraits<__half>::pack2(p0 * vs0, p1 * vs1), pb1 = ElemTraits<__half>::pack2(p2 * vs2, p3 * vs3);
+        // output: V rows 2t, 2t+1, 2t+8, 2t+9, piece g (d = 16 g .. 16 g + 15)
+        uint32_t v0[4], v1[4], v2[4], v3[4];
+        const uint32_t vbase = stage + kTileBytes;
+        lds32x4(vbase + (2 * t) * kRowBytes + ((g ^ ((2 * t) & 6)) << 4), v0);
+        lds32x4(vbase + (2 * t + 1) * kRowBytes + ((g ^ ((2 * t + 1) & 6)) << 4), v1);
+        lds32x4(vbase + (2 * t + 8) * kRowBytes + ((g ^ ((2 * t + 8) & 6)) << 4), v2);
+        lds32x4(vbase + (2 * t + 9) * kRowBytes + ((g ^ ((2 * t + 9) & 6)) << 4), v3);
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            const uint32_t x0 = v0[a] ^ kFlip, x1 = v1[a] ^ kFlip, x2 = v2[a] ^ kFlip, x3 = v3[a] ^ kFlip;
+            // bytes of one d from two consecutive keys, side by side
+            const uint32_t lo01 = __byte_perm(x0, x1, 0x5140), hi01 = __byte_perm(x0, x1, 0x7362);
+            const uint32_t lo23 = __byte_perm(x2, x3, 0x5140), hi23 = __byte_perm(x2, x3, 0x7362);
+            mma_16816<__half>(s.o[2 * a], widen_pair_lo<FP8>(lo01), widen_pair_hi<FP8>(lo01), widen_pair_lo<FP8>(lo23), widen_pair_hi<FP8>(lo23), pb0, pb1);
+            mma_16816<__half>(s.o[2 * a + 1], widen_pair_lo<FP8>(hi01), widen_pair_hi<FP8>(hi01), widen_pair_lo<FP8>(hi23), widen_pair_hi<FP8>(hi23), pb0, pb1);
+        }
+        constexpr uint32_t kOnes = 0x3C003C00u;   // {1.0, 1.0}
+        if (!FP8) mma_16816<__half>(osum, kOnes, kOnes, kOnes, kOnes, pb0, pb1);
+    }
+    __device__ __forceinline__ float value(int h, int i) const { return s.o[i >> 1][(i & 1) * 2 + h] - kOffset * osum[h]; }
+    static __device__ __forceinline__ int dim(int g, int i) { return 16 * g + i; }
+};
+
+// ---- a group's range of keys ---------------------------------------------------------------------------------------------
+template <class F>
+struct alignas(128) GroupSmem {
+    union {
+        unsigned char ring[kGroupWarps][F::kStages * F::kStageBytes];
+        struct {                                       // the merge, when the rings are idle
+            float o[kGroupWarps][kMaxGroup][kHeadDim];
+            float2 ml[kGroupWarps][kMaxGroup];
+        } m;
+    };
+};
+
+__device__ __forceinline__ float quad_sum(float v) {
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    return v + __shfl_xor_sync(0xffffffffu, v, 2);
+}
+
+// Keys [t0, t1) of sequence b (t0 < t1), one KV head.  sink(h, d, o, m, l) takes element d = this thread of head h: unnormalised
+// output, maximum and sum.  `tid`: 0..127 inside the group, `bar_id`: its named barrier; all its threads call it.
+template <class F, class Sink>
+__device__ __forceinline__ void attend_range(const DecodeParams& p, int b, int kvh, int t0, int t1, GroupSmem<F>& sm, int tid, int bar_id, Sink sink) {
+    const int bs = p.block_size, warp = tid >> 5, lane = tid & 31;
+    const uint32_t ring = smem_u32(sm.ring[warp]);
+    const int num_tiles = (t1 - t0 + kTileTokens - 1) / kTileTokens;
+    const int my_tiles = num_tiles > warp ? (num_tiles - warp + kGroupWarps - 1) / kGroupWarps : 0;
+    const int blocks = (t1 + bs - 1) / bs;
+    // The issuing end: this warp's next tile begins at row `off` of table entry `blk`.  Lane i holds the cache block of entry
+    // id_base + i (-1: outside the cache, reads as zeros).
+    int tok = t0 + warp * kTileTokens;
+    int blk = tok / bs, off = tok - blk * bs, id_base = 0, ids = -1;
+    auto load_ids = [&]() {
+        id_base = blk;
+        int64_t id = -1;
+        if (blk + lane < blocks) id = p.block_tables[b * p.max_blocks + blk + lane];
+        ids = (id >= 0 && id < p.num_cache_blocks) ? static_cast<int>(id) : -1;
+    };
+    load_ids();
+    uint32_t istage = ring;
+    auto issue = [&]() {
+        if (tok < t1) {
+            const int phys = __shfl_sync(0xffffffffu, ids, blk - id_base);
+            F::issue(p, kvh, phys < 0 ? 0 : static_cast<int64_t>(phys) * bs + off, phys < 0 ? 0 : t1 - tok, istage, lane);
+            istage = istage == ring + (F::kStages - 1) * F::kStageBytes ? ring : istage + F::kStageBytes;
+            tok += kGroupWarps * kTileTokens;
+            for (off += kGroupWarps * kTileTokens; off >= bs; off -= bs) ++blk;
+            if (blk - id_base >= 32 && tok < t1) load_ids();
+        }
+        cp_async_commit();
+    };
+#pragma unroll
+    for (int s = 0; s < F::kStages - 1; ++s) issue();
+
+    F st;
+    st.start(p, b, kvh, lane);
+    uint32_t cstage = ring;
+    int left = t1 - t0 - warp * kTileTokens;   // keys from this warp's tile on
+    for (int j = 0; j < my_tiles; ++j) {
+        issue();
+        cp_async_wait<F::kStages - 1>();
         __syncwarp();
+        st.step(p, cstage, left, kvh, lane);
+        __syncwarp();   // the stage is refilled by other lanes' copies
+        cstage = cstage == ring + (F::kStages - 1) * F::kStageBytes ? ring : cstage + F::kStageBytes;
+        left -= kGroupWarps * kTileTokens;
     }
     cp_async_wait<0>();
-    group_sync(bar_id);  // every ring is idle from here on: reuse it for the cross-warp merge
-
-    l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
-    l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
-
-    float* sm_o = reinterpret_cast<float*>(smem);                    // [warp][head][128]
-    float* sm_m = sm_o + kWarps * kMaxGroup * kHeadDim;              // [warp][head]
-    float* sm_l = sm_m + kWarps * kMaxGroup;
-    if (t == 0) { sm_m[warp * kMaxGroup + g] = m_run; sm_l[warp * kMaxGroup + g] = l_run; }
+    group_sync(bar_id, kGroupThreads);   // every ring is idle from here on
+    const int g = lane >> 2, t = lane & 3;
+    const float l = quad_sum(st.s.l);
+    if (t == 0) sm.m.ml[warp][g] = make_float2(st.s.m, l);
 #pragma unroll
-    for (int mt = 0; mt < 8; ++mt) {
-        const int d = mt * 16 + g;
-        float* dst = sm_o + (warp * kMaxGroup + 2 * t) * kHeadDim + d;
-        dst[0] = o[mt][0]; dst[kHeadDim] = o[mt][1]; dst[8] = o[mt][2]; dst[kHeadDim + 8] = o[mt][3];
+    for (int h = 0; h < 2; ++h) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) sm.m.o[warp][2 * t + h][F::dim(g, i)] = st.value(h, i);
     }
-    group_sync(bar_id);
-
-    // thread d merges column d of every head of the group over the four warps
-    const int d = tid;
-    for (int h = 0; h < G; ++h) {
-        float mx = -INFINITY;
+    group_sync(bar_id, kGroupThreads);
+    for (int h = 0; h < p.group; ++h) {
+        float mx = -INFINITY, o = 0.0f, sum = 0.0f;
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) mx = fmaxf(mx, sm_m[w * kMaxGroup + h]);
-        float acc = 0.0f, lsum = 0.0f;
+        for (int w = 0; w < kGroupWarps; ++w) mx = fmaxf(mx, sm.m.ml[w][h].x);
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
-            const float f = fast_exp2(sm_m[w * kMaxGroup + h] - mx);
-            acc += f * sm_o[(w * kMaxGroup + h) * kHeadDim + d];
-            lsum += f * sm_l[w * kMaxGroup + h];
+        for (int w = 0; w < kGroupWarps; ++w) {
+            const float f = fast_exp2(sm.m.ml[w][h].x - mx);   // 0 for a warp without a tile
+            o += f * sm.m.o[w][h][tid];
+            sum += f * sm.m.ml[w][h].y;
         }
-        const float val = acc / lsum;
-        const int64_t head = b * p.num_heads + kvh * G + h;
-        if (live_splits == 1) {
-            out[head * kHeadDim + d] = ElemTraits<T>::from_float(val);
-        } else {
-            p.ws_o[(head * p.num_splits + split) * kHeadDim + d] = val;
-            if (d == 0) p.ws_lse[head * p.num_splits + split] = mx + log2f(lsum);
+        sink(h, tid, o, mx, sum);
+    }
+}
+
+__device__ __forceinline__ void write_part(float* po, float2* pml, int h, int d, float o, float m, float l) {   // [group][128], [group]
+    po[h * kHeadDim + d] = o;
+    if (d == 0) pml[h] = make_float2(m, l);
+}
+
+// Range `split` of (b, kvh): the result if it is all of the context, else a part in the workspace.
+template <class F, typename T>
+__device__ __forceinline__ void run_split(const DecodeParams& p, int b, int kvh, int split, GroupSmem<F>& sm, int tid, int bar_id) {
+    const int ctx = clamped_context(p, b);
+    int t0, t1;
+    const int live = split_range(p, ctx, split, t0, t1);
+    T* out = static_cast<T*>(p.out) + (static_cast<int64_t>(b) * p.num_heads + kvh * p.group) * kHeadDim;
+    if (t0 >= t1) {
+        if (ctx == 0 && split == 0) {
+            for (int i = tid; i < p.group * kHeadDim; i += kGroupThreads) out[i] = ElemTraits<T>::from_float(0.0f);
+        }
+        return;
+    }
+    const size_t part = (static_cast<size_t>(b) * p.num_kv_heads + kvh) * p.num_splits + split;
+    attend_range<F>(p, b, kvh, t0, t1, sm, tid, bar_id, [&](int h, int d, float o, float m, float l) {
+        if (live == 1) out[h * kHeadDim + d] = ElemTraits<T>::from_float(o * (1.0f / l));   // (rounded as write_merged does)
+        else write_part(p.ws_o + part * p.group * kHeadDim, p.ws_ml + part * p.group, h, d, o, m, l);
+    });
+}
+
+// ---- merging the parts of a sequence -------------------------------------------------------------------------------------
+// HG heads of one (sequence, KV head) at a time.  Where there can be few parts one warp takes them in order, otherwise they are
+// dealt over kMergeWarps warps.
+struct PartRef { const float* o; const float2* ml; };   // head 0 of a part
+struct Merged {                                         // elements 4 lane .. 4 lane + 3 of a head's output, maximum and row sum
+    float4 o;
+    float m, l;
+    __device__ __forceinline__ void add(const float4& v, float vm, float vl) {
+        const float mx = fmaxf(m, vm), f = fast_exp2(m - mx), w = fast_exp2(vm - mx);
+        o.x = o.x * f + w * v.x; o.y = o.y * f + w * v.y; o.z = o.z * f + w * v.z; o.w = o.w * f + w * v.w;
+        l = l * f + w * vl;
+        m = mx;
+    }
+};
+
+// Heads h0 .. h0 + HG - 1 (clamped to the group) over parts first, first + stride, ...
+template <int HG, class Get>
+__device__ __forceinline__ void sum_parts(Get get, int n, int first, int stride, int h0, int group, int lane, Merged (&acc)[HG]) {
+    constexpr int U = HG == 4 ? 4 : 8;   // parts in flight
+#pragma unroll
+    for (int h = 0; h < HG; ++h) acc[h] = Merged{make_float4(0.f, 0.f, 0.f, 0.f), -INFINITY, 0.0f};
+    for (int i0 = first; i0 < n; i0 += U * stride) {
+        float2 ml[U][HG];
+        float4 v[U][HG];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const PartRef r = get(min(i0 + u * stride, n - 1));   // (loads without branches, so that all are in flight at once)
+#pragma unroll
+            for (int h = 0; h < HG; ++h) {
+                const int hh = min(h0 + h, group - 1);
+                ml[u][h] = r.ml[hh];
+                v[u][h] = *reinterpret_cast<const float4*>(r.o + hh * kHeadDim + 4 * lane);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (i0 + u * stride < n) {
+#pragma unroll
+                for (int h = 0; h < HG; ++h) acc[h].add(v[u][h], ml[u][h].x, ml[u][h].y);
+            }
         }
     }
+}
+template <typename T>
+__device__ __forceinline__ void write_merged(T* row, const Merged& a, int lane) {
+    const float inv = a.l > 0.0f ? 1.0f / a.l : 0.0f;
+    reinterpret_cast<uint2*>(row)[lane] = make_uint2(ElemTraits<T>::pack2(a.o.x * inv, a.o.y * inv), ElemTraits<T>::pack2(a.o.z * inv, a.o.w * inv));
+}
+// All heads of the group, rows of `out`, by one warp.
+template <typename T, int HG, class Get>
+__device__ __forceinline__ void merge_by_warp(Get get, int n, int group, T* out, int lane) {
+    for (int h0 = 0; h0 < group; h0 += HG) {
+        Merged acc[HG];
+        sum_parts<HG>(get, n, 0, 1, h0, group, lane, acc);
+#pragma unroll
+        for (int h = 0; h < HG; ++h)
+            if (h0 + h < group) write_merged<T>(out + (h0 + h) * kHeadDim, acc[h], lane);
+    }
+}
+// One head, by the whole block; the first kMergeWarps warps work.
+struct MergeScratch { float4 o[kMergeWarps][32]; float2 ml[kMergeWarps]; };
+template <typename T, class Get>
+__device__ __forceinline__ void merge_by_block(Get get, int n, int head, int group, T* row, MergeScratch& sm, int warp, int lane) {
+    if (warp < kMergeWarps) {
+        Merged acc[1];
+        sum_parts<1>(get, n, warp, kMergeWarps, head, group, lane, acc);
+        sm.o[warp][lane] = acc[0].o;
+        if (lane == 0) sm.ml[warp] = make_float2(acc[0].m, acc[0].l);
+    }
+    __syncthreads();
+    if (warp == 0) {
+        Merged a{make_float4(0.f, 0.f, 0.f, 0.f), -INFINITY, 0.0f};
+#pragma unroll
+        for (int w = 0; w < kMergeWarps; ++w) a.add(sm.o[w][lane], sm.ml[w].x, sm.ml[w].y);
+        write_merged<T>(row, a, lane);
+    }
+    __syncthreads();
 }
 
 }  // namespace dec

@@ -212,7 +212,7 @@ int nvk_decode_attention_paged_fp8(const void* query, const void* k_cache, const
                      k_scale, v_scale, true};
     if (!decode_int8_mma_supported(a))
         return fail(NVK_ERR_UNSUPPORTED, "decode attention (fp8): F16 / BF16 queries, head_dim 128, at most 8 query heads per KV head, "
-                                         "block_size a multiple of 16 (and a workspace beyond 8 cache blocks per sequence)");
+                                         "block_size a multiple of 16");
     if (workspace != nullptr) {
         const size_t need = decode_mma_workspace_bytes(batch, num_heads, num_kv_heads, head_dim, max_blocks, block_size);
         if (workspace_bytes < need)

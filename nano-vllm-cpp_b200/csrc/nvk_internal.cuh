@@ -106,8 +106,8 @@ size_t decode_mma_workspace_bytes(int64_t batch, int num_heads, int num_kv_heads
                                   int64_t max_blocks, int block_size);
 int launch_decode_mma(const DecodeArgs& a);
 namespace dec { struct DecodeParams; }
-int decode_plan(const DecodeArgs& a, dec::DecodeParams* out);
-int launch_decode_merge(const dec::DecodeParams& p, int64_t batch, int dtype, cudaStream_t stream);
+int decode_plan(const DecodeArgs& a, int groups, dec::DecodeParams* out, int* cluster);
+int launch_decode_merge(const dec::DecodeParams& p, int dtype, cudaStream_t stream);
 // Fused all-reduce launchers (tp_allreduce.cu); `pushed`: the other ranks' slices were already pushed by the GEMM
 // that produced the addend (gemm_fused.cu), the kernel starts with the reduction.
 void set_multimem_wait_cycles(long long cycles);   // tp_allreduce_mm.cu: the wait limit of the multimem kernels

@@ -742,15 +742,14 @@ __device__ __forceinline__ bool tc5_locate(const TcParams& p, int64_t want, int&
     return false;
 }
 
-// The decode half of a mixed step (prefill_tc5_kernel<T, true>): the split-K decode items of decode_split_kernel, taken
-// from a second ticket counter by the same persistent blocks.  A block runs the two halves one after the other --
-// blocks [0, prefill_blocks) the prefill items first, the others the decode items first -- so while some SMs are busy
-// on the tensor pipe the rest stream the KV cache, and no SM idles between the two parts of the step as it does at the
-// boundary of two launches.  In the decode half the eight softmax warps form two groups of four warps, each with its
-// own 96 KiB of the block's shared memory, i.e. what two resident blocks of decode_split_kernel have per SM.
+// The decode half of a mixed step (prefill_tc5_kernel<T, true>): the (KV head, split, sequence) items of the decode kernels, taken
+// from a second ticket counter by the same persistent blocks.  A block runs the two halves one after the other -- blocks
+// [0, prefill_blocks) the prefill items first, the others the decode items first -- so while some SMs are busy on the tensor pipe
+// the rest stream the KV cache, and no SM idles between the two parts of the step as it does at the boundary of two launches.  In
+// the decode half the eight softmax warps form two groups of four warps, each with its own part of the block's shared memory: what
+// two resident blocks of decode_split_kernel have per SM.
 struct MixedDecode {
     dec::DecodeParams dp;
-    unsigned int items;       // KV heads x splits x sequences
     int prefill_blocks;
 };
 __device__ unsigned int g_decode_ticket[kTicketSlots];
@@ -758,33 +757,37 @@ __device__ unsigned int g_decode_ticket[kTicketSlots];
 template <typename T, bool MIXED>
 __global__ void __launch_bounds__(kThreads5, 1)
 prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                   const __grid_constant__ CUtensorMap tm_v, const Tc5Params pp, const MixedDecode md) {
+                   const __grid_constant__ CUtensorMap tm_v, const Tc5Params pp, const __grid_constant__ MixedDecode md) {
+    using Decode16 = dec::Cache16<T>;
+    struct MixedGroup {
+        dec::GroupSmem<Decode16> g;
+        unsigned int item;
+    };
+    static_assert(Decode16::kGroups * sizeof(MixedGroup) <= kOff4Bar, "the decode half's shared memory");
     const TcParams& p = pp.base;
     extern __shared__ unsigned char smem_raw[];
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
     __shared__ Tc5Item s_ring[4];
-    __shared__ int s_dec_blocks[MIXED ? 2 : 1][MIXED ? dec::kMaxChunkBlocks : 1];
-    __shared__ unsigned int s_dec_item[2];
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     unsigned char* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-    // decode half: warps 0-3 and 4-7 are two independent groups, each taking (KV head, split, sequence) items
     auto decode_half = [&]() {
-        if (MIXED && warp < 8) {
-            const int group = warp >> 2, gtid = tid & 127, bar = 1 + group;
-            unsigned char* gsmem = smem_gen + group * dec::kSmemBytes;
-            const unsigned int hkv = static_cast<unsigned int>(md.dp.num_kv_heads), splits = static_cast<unsigned int>(md.dp.num_splits);
+        if (MIXED && warp < Decode16::kGroups * dec::kGroupWarps) {
+            const dec::DecodeParams& dp = md.dp;
+            MixedGroup& sm = reinterpret_cast<MixedGroup*>(smem_gen)[warp / dec::kGroupWarps];
+            const int gtid = tid % dec::kGroupThreads, bar = 1 + warp / dec::kGroupWarps;
+            const unsigned int hkv = static_cast<unsigned int>(dp.num_kv_heads), splits = static_cast<unsigned int>(dp.num_splits);
             while (true) {
-                if (gtid == 0) s_dec_item[group] = atomicAdd(&g_decode_ticket[pp.slot], 1u);
-                dec::group_sync(bar);
-                const unsigned int item = s_dec_item[group];
-                dec::group_sync(bar);   // everyone holds the item before the next ticket overwrites it
-                if (item >= md.items) break;
-                dec::decode_split_body<T>(md.dp, static_cast<int>(item % hkv), static_cast<int>((item / hkv) % splits),
-                                          static_cast<int64_t>(item / (hkv * splits)), gsmem, s_dec_blocks[MIXED ? group : 0], gtid, bar);
-                dec::group_sync(bar);   // the group's shared memory is free for its next item
+                if (gtid == 0) sm.item = atomicAdd(&g_decode_ticket[pp.slot], 1u);
+                dec::group_sync(bar, dec::kGroupThreads);
+                const unsigned int item = sm.item;
+                dec::group_sync(bar, dec::kGroupThreads);   // everyone holds the item before the next ticket overwrites it
+                if (item >= hkv * splits * static_cast<unsigned int>(dp.batch)) break;
+                dec::run_split<Decode16, T>(dp, static_cast<int>(item / (hkv * splits)), static_cast<int>(item % hkv), static_cast<int>((item / hkv) % splits),
+                                            sm.g, gtid, bar);
+                dec::group_sync(bar, dec::kGroupThreads);   // the group's shared memory is free for its next item
             }
         }
     };
@@ -1282,9 +1285,9 @@ int launch_mixed_typed(const PrefillArgs& a, const DecodeArgs& d, int prefill_bl
     rc = prepare_tc5<T, true>(&sms);
     if (rc != NVK_OK) return rc;
     MixedDecode md{};
-    rc = decode_plan(d, &md.dp);
+    int cluster = 0;   // the ranges of the cluster kernel are taken one by one here and merged through the workspace
+    rc = decode_plan(d, dec::Cache16<T>::kGroups, &md.dp, &cluster);
     if (rc != NVK_OK) return rc;
-    md.items = static_cast<unsigned int>(d.num_kv_heads) * static_cast<unsigned int>(md.dp.num_splits) * static_cast<unsigned int>(d.batch);
     Tc5Params pp{};
     pp.base = L.p;
     pp.pairs = a.num_heads / 2;
@@ -1308,7 +1311,7 @@ int launch_mixed_typed(const PrefillArgs& a, const DecodeArgs& d, int prefill_bl
     if (e != cudaSuccess) return fail(NVK_ERR_CUDA, "mixed prefill + decode kernel launch: %s", cudaGetErrorString(e));
     rc = check_launch("mixed prefill + decode kernel launch");
     if (rc != NVK_OK) return rc;
-    return launch_decode_merge(md.dp, d.batch, d.dtype, d.stream);
+    return launch_decode_merge(md.dp, d.dtype, d.stream);
 }
 
 }  // namespace

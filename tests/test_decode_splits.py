@@ -1,0 +1,59 @@
+"""Tensor-core paged decode at the edges of how a sequence is shared out: clusters of 1 to 8 blocks, chunks with few and with many
+partial results, no workspace, contexts around a tile, a round of the four warps' tiles, a chunk and a part, empty ones among them."""
+import numpy as np
+import pytest
+
+import oracle
+from util import assert_attention_close, nvk, to_dev, to_np, workloads
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+EDGES = [0, 1, 15, 16, 17, 63, 64, 65, 127, 129, 255, 256, 257, 511, 513]
+
+
+def _workspace(batch, hq, hkv, blocks, bs):
+    return torch.empty(max(16, nvk().decode_attention_workspace_bytes(batch, hq, hkv, 128, blocks, bs)), dtype=torch.uint8, device="cuda")
+
+
+@pytest.mark.parametrize("hq,hkv,bs,lens,table_blocks", [
+    (8, 2, 256, [300], 2),                                  # eight blocks per (sequence, KV head)
+    (32, 8, 256, [700, 0, 33], 4),
+    (16, 8, 16, EDGES[:9], 9),                              # four, two and one
+    (4, 4, 256, EDGES, 3),
+    (8, 8, 32, EDGES * 3, 17),
+    (8, 1, 256, [2047, 2048, 2049, 1, 9000], 80),           # chunks: up to 36 parts of one context
+    (16, 8, 256, EDGES * 3 + [4096, 2500, 2048], 16),       # whole contexts, 4096-key tables
+    (16, 8, 256, [4097, 8192, 5000] + EDGES * 3, 33),       # chunks: up to 5 parts
+])
+def test_every_way_to_share_out_a_context_matches_the_oracle(hq, hkv, bs, lens, table_blocks):
+    w = workloads().make_decode_workload(len(lens), hq, hkv, 128, bs, 0, 0, seed=len(lens) + hq, context_lens=np.array(lens, np.int32),
+                                         pad_blocks_to=table_blocks)
+    bf = torch.bfloat16
+    q, kc, vc, ctx, bt = to_dev(w["q"], bf), to_dev(w["k_cache"], bf), to_dev(w["v_cache"], bf), to_dev(w["context_lens"]), to_dev(w["block_tables"])
+    ref = oracle.decode_attention_paged(w["q"], w["k_cache"], w["v_cache"], w["context_lens"], w["block_tables"], hkv, 128, bs, w["scale"])
+    for ws in (_workspace(len(lens), hq, hkv, bt.shape[1], bs), None):
+        out = torch.full_like(q, float("nan"))
+        nvk().launch_decode_attention_paged(q, kc, vc, ctx, bt, hkv, 128, bs, w["scale"], out, ws)
+        assert_attention_close(to_np(out), ref)
+
+
+@pytest.mark.parametrize("fmt", ["int8", "fp8"])
+@pytest.mark.parametrize("hq,hkv,lens,table_blocks", [(8, 2, [300, 17], 2), (16, 8, EDGES * 2, 3), (8, 1, [5000, 1, 2049], 40)])
+def test_8_bit_caches_do_not_depend_on_how_a_context_is_shared_out(fmt, hq, hkv, lens, table_blocks):
+    w = workloads().make_decode_workload(len(lens), hq, hkv, 128, 256, 0, 0, seed=5, context_lens=np.array(lens, np.int32), pad_blocks_to=table_blocks)
+    bf, lib = torch.bfloat16, nvk()
+    store, decode = ((lib.store_kvcache_int8, lib.launch_decode_attention_paged_int8) if fmt == "int8" else
+                     (lib.store_kvcache_fp8, lib.launch_decode_attention_paged_fp8))
+    k16, v16 = to_dev(w["k_cache"], bf), to_dev(w["v_cache"], bf)
+    kc, vc = (torch.empty(k16.shape, dtype=torch.int8 if fmt == "int8" else torch.uint8, device="cuda") for _ in range(2))
+    ks, vs = (torch.empty(k16.shape[:-1], dtype=torch.float16, device="cuda") for _ in range(2))
+    rows = torch.arange(ks.numel() // hkv, dtype=torch.int32, device="cuda")
+    store(k16.view(-1, hkv, 128), v16.view(-1, hkv, 128), kc, vc, ks, vs, rows)
+    q, ctx, bt = to_dev(w["q"], bf), to_dev(w["context_lens"]), to_dev(w["block_tables"])
+    a, b = torch.full_like(q, float("nan")), torch.full_like(q, float("nan"))
+    decode(q, kc, vc, ks, vs, ctx, bt, hkv, 128, 256, w["scale"], a, _workspace(len(lens), hq, hkv, bt.shape[1], 256))
+    decode(q, kc, vc, ks, vs, ctx, bt, hkv, 128, 256, w["scale"], b, None)
+    ref = oracle.decode_attention_paged(w["q"], w["k_cache"], w["v_cache"], w["context_lens"], w["block_tables"], hkv, 128, 256, w["scale"])
+    assert float((a.float() - b.float()).abs().max()) <= 1e-2
+    assert np.abs(to_np(a) - ref).max() <= (5e-2 if fmt == "int8" else 2.5e-1) and not torch.isnan(b.float()).any()
