@@ -30,11 +30,36 @@ constexpr int kMaxCluster = 8;          // portable cluster size
 // pass (alone, from call to result: 17) where split and merge took 9.4 (41).
 constexpr int kClusterTokens = 512;
 
+// The sequence with the rank-th longest context (ties in index order), found by every block for itself; `keys`: kMaxSorted ints.  In
+// index order the last blocks to start can be the longest: 100 sequences of 500 to 4096 keys, int8, left half the SMs idle for the
+// last 40 of 106 us; in this order the pass takes 103 us instead of 115.  64 sequences of 100 to 2048 keys, 16-bit: 6 us less.
+constexpr int kMaxSorted = 512;
+__device__ __forceinline__ int sequence_of_rank(const DecodeParams& p, int rank, int* keys) {
+    __shared__ int found;
+    const int padded = (p.batch + 3) & ~3;
+    for (int i = threadIdx.x; i < padded; i += kGroupThreads) keys[i] = i < p.batch ? clamped_context(p, i) : -1;
+    __syncthreads();
+    for (int i = threadIdx.x; i < p.batch; i += kGroupThreads) {
+        const int mine = keys[i];
+        int longer = 0;
+        for (int j = 0; j < padded; j += 4) {
+            const int4 k = *reinterpret_cast<const int4*>(keys + j);
+            longer += (k.x > mine || (k.x == mine && j < i)) + (k.y > mine || (k.y == mine && j + 1 < i)) +
+                      (k.z > mine || (k.z == mine && j + 2 < i)) + (k.w > mine || (k.w == mine && j + 3 < i));
+        }
+        if (longer == rank) found = i;
+    }
+    __syncthreads();
+    return found;
+}
+
 template <class F, typename T>
 __global__ void __launch_bounds__(kGroupThreads, F::kGroups) decode_split_kernel(const __grid_constant__ DecodeParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
     pdl_wait_then_release();
-    run_split<F, T>(p, blockIdx.z, blockIdx.x, blockIdx.y, *reinterpret_cast<GroupSmem<F>*>(smem), threadIdx.x, 1);
+    const int b = p.longest_first ? sequence_of_rank(p, blockIdx.z, reinterpret_cast<int*>(smem)) : blockIdx.z;
+    if (p.longest_first) __syncthreads();   // (the ring takes the keys' place)
+    run_split<F, T>(p, b, blockIdx.x, blockIdx.y, *reinterpret_cast<GroupSmem<F>*>(smem), threadIdx.x, 1);
 }
 
 // HG > 0: one warp per (sequence, KV head), HG heads at a time, in blocks of kMergeBlockWarps warps, small enough to be resident
@@ -109,10 +134,10 @@ int cluster_size(int64_t batch, int num_kv_heads, int64_t max_blocks, int block_
     return pairs <= resident && max_blocks * block_size <= static_cast<int64_t>(kClusterTokens) * c ? c : 0;
 }
 
-// Chunk length in keys (whole cache blocks).  2048 where that gives every resident group a block -- a chunk more costs a second pass
-// over its partial result --, else shorter, down to 256.  Tables of up to 4096 keys are not cut at all once there is a sequence and
-// KV head for every resident group: 37 sequences of up to 2048 keys, 8 KV heads, 4096-key tables take 34.6 us a pass without the
-// merge kernel and 36.6 with it.
+// Chunk length in keys (whole cache blocks).  Contexts of tables of up to 4096 keys stay whole once there is one per resident group:
+// no merge (2 us of 37 at 37 sequences of 100 to 2048 keys, 8 KV heads), and taken longest first they balance each other.  Otherwise
+// 2048, or less, down to 256, where that leaves resident groups without a block.  (Whole contexts of 8192-key tables, 256 sequences:
+// 694 us a pass, 689 with chunks.)
 int chunk_tokens(int64_t batch, int num_kv_heads, int64_t max_blocks, int block_size, int groups) {
     const int64_t max_tokens = max_blocks * block_size, pairs = batch * num_kv_heads, resident = static_cast<int64_t>(kSmCount) * groups;
     if (max_tokens <= 4096 && pairs >= resident) return static_cast<int>(max_tokens);
@@ -170,6 +195,8 @@ int decode_plan(const DecodeArgs& a, int groups, dec::DecodeParams* out, int* cl
     p.per_seq = s.cluster > 0 ? 1 : 0;
     p.chunk_tokens = s.chunk;
     p.num_splits = s.count;
+    // whole contexts in more than one wave of blocks: the long ones first, so that the last blocks to start are short
+    p.longest_first = s.cluster == 0 && s.count == 1 && a.batch * a.num_kv_heads > static_cast<int64_t>(kSmCount) * groups && a.batch <= kMaxSorted;
     if (a.workspace != nullptr) {
         p.ws_o = static_cast<float*>(a.workspace);
         p.ws_ml = reinterpret_cast<float2*>(p.ws_o + part_count(s, a.batch, a.num_kv_heads) * p.group * kHeadDim);

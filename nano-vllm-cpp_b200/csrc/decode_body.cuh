@@ -39,6 +39,7 @@ struct DecodeParams {
     int batch, num_heads, num_kv_heads, group, block_size;
     int chunk_tokens, num_splits;
     int per_seq;                                       // 1: num_splits equal ranges per sequence instead of chunks
+    int longest_first;                                 // blocks take the sequences in order of falling context length
     float scale_log2;
 };
 

@@ -1,5 +1,6 @@
 """Tensor-core paged decode at the edges of how a sequence is shared out: clusters of 1 to 8 blocks, chunks with few and with many
-partial results, no workspace, contexts around a tile, a round of the four warps' tiles, a chunk and a part, empty ones among them."""
+partial results, no workspace, whole contexts taken
+longest first, contexts around a tile, a round of the four warps' tiles, a chunk and a part, equal and empty ones among them."""
 import numpy as np
 import pytest
 
@@ -39,7 +40,7 @@ def test_every_way_to_share_out_a_context_matches_the_oracle(hq, hkv, bs, lens, 
 
 
 @pytest.mark.parametrize("fmt", ["int8", "fp8"])
-@pytest.mark.parametrize("hq,hkv,lens,table_blocks", [(8, 2, [300, 17], 2), (16, 8, EDGES * 2, 3), (8, 1, [5000, 1, 2049], 40)])
+@pytest.mark.parametrize("hq,hkv,lens,table_blocks", [(8, 2, [300, 17], 2), (16, 8, EDGES * 4, 3), (8, 1, [5000, 1, 2049], 40)])
 def test_8_bit_caches_do_not_depend_on_how_a_context_is_shared_out(fmt, hq, hkv, lens, table_blocks):
     w = workloads().make_decode_workload(len(lens), hq, hkv, 128, 256, 0, 0, seed=5, context_lens=np.array(lens, np.int32), pad_blocks_to=table_blocks)
     bf, lib = torch.bfloat16, nvk()
