@@ -13,17 +13,22 @@
 //     by the GEMM, tile by tile, while the other tiles still compute.  The all-reduce kernel that follows is told to
 //     skip its push.
 //
-// GEMM core: C[M, N] = A[M, K] * B[N, K]^T, both operands K-major as torch linears keep them.  One block per 128 x 128
-// tile of C; a TMA warp streams 128 x 64 panels of A and B (128-byte swizzle) through a ring of shared-memory stages,
-// one thread issues tcgen05.mma (M 128, N 128, K 16) into a 128-column TMEM accumulator, four warps read it back
-// (thread = row) for the epilogue.  At decode sizes (M = a few hundred rows) the GEMM streams the weight once and is
-// HBM-bound; what the fusion removes is the round trip of the result and one or two launches per layer.
+// GEMM core: C[M, N] = A[M, K] * B[N, K]^T, both operands K-major as torch linears keep them; TMA (128-byte swizzle) into a ring of
+// shared-memory stages, tcgen05.mma into TMEM.  Two kernels, chosen by size (choose_gemm):
+//   gemm_split_kernel   few rows.  The GEMM streams the weight once and is HBM-bound, so every SM has to stream: a block takes 128 or
+//                       256 rows x 128 columns of C over a part of K, the blocks of a cluster the parts of one tile; they add up
+//                       through distributed shared memory, each for its share of the rows, and run the epilogue on that share.
+//   gemm_pair_kernel    many rows, bound by the tensor pipe.  Persistent pairs of blocks (cta_group::2): 256 x 256 tiles, each block
+//                       loads half of A and half of B, so an SM moves half the operand bytes of a 128 x 256 tile of its own.  The
+//                       accumulator is double buffered in TMEM: the epilogue of a tile runs under the next tile's MMAs.
+// Before, one block per 128 x 128 tile whatever the size (microseconds in a loop over weights larger than L2; K 4096):
+//   64 x 6144  22 -> 16      64 x 4096  21 -> 12     7440 x 4096  295 -> 175 (1430 TFLOP/s)     7440 x 6144 with QKV epilogue  597 -> 277
+// What the fusion removes is the round trip of the result and one or two launches per layer.
 // Every mbarrier wait is bounded; a wait that runs out raises an error word (nvk_gemm_status) and the block leaves.
 #include "nvk_internal.cuh"
 
 #include <cuda.h>
 
-#include <atomic>
 #include <mutex>
 
 namespace nvk {
@@ -31,12 +36,12 @@ namespace {
 
 constexpr int kBM = 128, kBN = 128, kBK = 64;
 constexpr int kPanelBytes = kBM * kBK * 2;            // 16 KiB: 128 rows x 128 bytes
-constexpr int kStageBytes = 2 * kPanelBytes;          // A panel + B panel
-constexpr int kStages = 6;
-constexpr int kBarOffset = kStages * kStageBytes;     // 192 KiB
-constexpr int kSmemBytes = kBarOffset + 256 + 1024;
-constexpr int kThreads = 192;                         // warp 0 TMA, warp 1 MMA + TMEM, warps 2-5 epilogue
-constexpr int kTmemCols = 128;
+constexpr int kRingBytes = 12 * kPanelBytes;          // 192 KiB: 6 stages of 2 panels or 4 of 3
+constexpr int kStageOffset = kRingBytes + 256;        // after the barriers: 4 KiB per epilogue warp of gemm_pair_kernel
+constexpr int kSmemBytes = kStageOffset + 8 * 4096 + 1024;   // + slack for 1024-byte alignment
+constexpr int kThreads = 192;                         // warp 0 TMA, warp 1 MMA + TMEM, warps 2-5 TMEM readers
+constexpr int kPairThreads = 320;                     // the same with warps 2-9 for the epilogue
+constexpr int kMaxSplits = 8;                         // portable cluster size
 constexpr long long kWaitCycles = 4000000000LL;       // ~2 s
 constexpr int kMaxRanks = NVK_TP_MAX_RANKS;
 
@@ -48,6 +53,8 @@ struct GemmParams {
     void* out;                 // kPlain: C [M, N]
     int64_t m, n, k;
     uint32_t idesc;
+    int tiles_m, tiles_n;      // gemm_pair_kernel
+    int a_rows;                // gemm_split_kernel: rows of A that a load brings in (a multiple of 8; the tile's other rows stay undefined)
     // kQkvPrologue
     const int32_t* positions; const void* q_weight; const void* k_weight; const float* cos_sin; const int32_t* slot_mapping;
     void* q_out; void* k_cache; void* v_cache;
@@ -98,6 +105,33 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
+// The same from a block of a pair: the barrier may be the other block's (`bar`: a shared::cluster address).
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(bar) : "memory");
+}
+__device__ __forceinline__ uint32_t in_block(uint32_t addr, uint32_t rank) {   // the same place in block `rank` of the cluster
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm("mov.u32 %0, %cluster_ctarank;\n" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ float4 ld_cluster(uint32_t addr) {                  // shared::cluster address
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+    return v;
+}
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
 }
@@ -105,6 +139,16 @@ __device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t a_desc, uint64
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc) : "memory");
+}
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {                  // arrives in both blocks of the pair
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
+                 ::"r"(bar), "h"(static_cast<uint16_t>(3)) : "memory");
+}
+__device__ __forceinline__ void umma_ss_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc) : "memory");
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t addr, uint32_t (&r)[32]) {
@@ -147,35 +191,294 @@ __device__ __forceinline__ void load_rounded(uint32_t taddr, float (&v)[32]) {
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = ElemTraits<T>::to_float(ElemTraits<T>::from_float(__uint_as_float(r[i])));
 }
+template <typename T> __device__ __forceinline__ uint4 pack8(const float* v) {
+    return make_uint4(ElemTraits<T>::pack2(v[0], v[1]), ElemTraits<T>::pack2(v[2], v[3]), ElemTraits<T>::pack2(v[4], v[5]), ElemTraits<T>::pack2(v[6], v[7]));
+}
+// Every lane has a row: 32 elements for dst + off0 and 32 for dst + off1 (dst == nullptr: nothing).  Through 4 KiB of shared memory, so
+// that four lanes write 64 contiguous bytes of a row where one lane each would write 16-byte pieces of 32 rows: with short K the tile's
+// epilogue is the bound (7000 x 4096, K 512: 53 -> 38 us).
 template <typename T>
-__device__ __forceinline__ void store32(T* dst, const float (&v)[32]) {   // 64 bytes, 16-byte aligned
+__device__ __forceinline__ void store_rows(T* dst, int off0, int off1, const float (&v0)[32], const float (&v1)[32], unsigned char* stage, int lane) {
+    uint4* row = reinterpret_cast<uint4*>(stage + lane * 128);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        uint4 w;
-        w.x = ElemTraits<T>::pack2(v[q * 8 + 0], v[q * 8 + 1]); w.y = ElemTraits<T>::pack2(v[q * 8 + 2], v[q * 8 + 3]);
-        w.z = ElemTraits<T>::pack2(v[q * 8 + 4], v[q * 8 + 5]); w.w = ElemTraits<T>::pack2(v[q * 8 + 6], v[q * 8 + 7]);
-        reinterpret_cast<uint4*>(dst)[q] = w;
+        row[q ^ (lane & 7)] = pack8<T>(v0 + 8 * q);
+        row[(4 + q) ^ (lane & 7)] = pack8<T>(v1 + 8 * q);
+    }
+    __syncwarp();
+    const unsigned long long addr = reinterpret_cast<unsigned long long>(dst);
+    const int c = lane & 7, off = (c < 4 ? off0 : off1) + (c & 3) * 8;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int r = i * 4 + (lane >> 3);
+        T* to = reinterpret_cast<T*>(__shfl_sync(0xffffffffu, addr, r));
+        const uint4 w = reinterpret_cast<const uint4*>(stage + r * 128)[c ^ (r & 7)];
+        if (to != nullptr) *reinterpret_cast<uint4*>(to + off) = w;
+    }
+    __syncwarp();
+}
+
+// ---- epilogues of one 128-column tile (with head_dim 128: of one head) -------------------------------------------------------
+// What a row of tile `nt` turns into: where it goes, and for q and k heads how it is normalised and rotated.
+template <typename T>
+struct QkvRow {
+    T* dst;
+    const T* weight;      // nullptr: no norm
+    const float* table;   // nullptr: no rotation
+    bool is_v;
+};
+template <typename T>
+__device__ __forceinline__ QkvRow<T> qkv_row(const GemmParams& p, int head, int64_t row, bool live) {
+    const bool is_q = head < p.hq, is_k = !is_q && head < p.hq + p.hkv;
+    const int pos = live ? __ldg(p.positions + row) : 0;
+    const int64_t slot = live ? (p.slot_mapping != nullptr ? static_cast<int64_t>(__ldg(p.slot_mapping + row)) : row) : -1;
+    QkvRow<T> x{nullptr, nullptr, nullptr, !is_q && !is_k};
+    if (live) {
+        if (is_q) x.dst = static_cast<T*>(p.q_out) + (row * p.hq + head) * kBN;
+        else if (slot >= 0 && slot < p.cache_rows)
+            x.dst = static_cast<T*>(is_k ? p.k_cache : p.v_cache) + (slot * p.hkv + (is_k ? head - p.hq : head - p.hq - p.hkv)) * kBN;
+    }
+    if (p.q_weight != nullptr) x.weight = static_cast<const T*>(is_q ? p.q_weight : p.k_weight);
+    if (pos >= 0 && pos < p.max_positions) x.table = p.cos_sin + static_cast<int64_t>(pos) * kBN;
+    return x;
+}
+// Where a row of a partial sum is reduced: `addend` (this rank) or a tagged slot of the owner's staging area.
+template <typename T>
+struct PushRow {
+    T* addend;
+    uint4* slot;
+    uint32_t epoch;
+};
+template <typename T>
+__device__ __forceinline__ PushRow<T> push_row(const GemmParams& p, int64_t row, bool live, int n0) {
+    const uint32_t last = *reinterpret_cast<const volatile uint32_t*>(p.flags);
+    PushRow<T> x{nullptr, nullptr, last + 1u == 0u ? 1u : last + 1u};      // the epoch the all-reduce launch after this GEMM will use
+    if (!live || *reinterpret_cast<const volatile uint32_t*>(p.flags + 2) != 0u) return x;
+    const int64_t rows_per_rank = p.m / p.world, row_vecs = p.n / 8, chunk_vecs = rows_per_rank * row_vecs;
+    const int owner = static_cast<int>(row / rows_per_rank);
+    if (owner == p.rank) x.addend = static_cast<T*>(p.addend) + row * p.n + n0;
+    else x.slot = p.stage[owner] + 2 * (p.rank * chunk_vecs + (row - owner * rows_per_rank) * row_vecs + n0 / 8);
+    return x;
+}
+
+// One thread holds the whole row in TMEM columns t_row .. t_row + 127 (warp-collective: every lane runs all of it).  `stage`: 4 KiB of
+// shared memory of this warp.
+template <typename T, int EPI>
+__device__ __forceinline__ void epilogue_row(const GemmParams& p, uint32_t t_row, int64_t row, int nt, unsigned char* stage, int lane) {
+    const bool live = row < p.m;
+    const int n0 = nt * kBN;
+    if (EPI == kAllReducePush) {
+        const PushRow<T> x = push_row<T>(p, row, live, n0);
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+            float v[32];
+            load_rounded<T>(t_row + c * 32, v);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint4 w = pack8<T>(v + 8 * q);
+                if (x.addend != nullptr) reinterpret_cast<uint4*>(x.addend + c * 32)[q] = w;
+                else if (x.slot != nullptr) st_tagged(x.slot + 2 * (c * 4 + q), w, x.epoch);
+            }
+        }
+        return;
+    }
+    QkvRow<T> x{};
+    if (EPI == kQkvPrologue) x = qkv_row<T>(p, nt, row, live);
+    if (EPI == kPlain || x.is_v) {             // the rounded GEMM output as it is
+        T* dst = EPI == kQkvPrologue ? x.dst : live ? static_cast<T*>(p.out) + row * p.n + n0 : nullptr;
+#pragma unroll 1
+        for (int c = 0; c < 2; ++c) {
+            float v0[32], v1[32];
+            load_rounded<T>(t_row + c * 64, v0);
+            load_rounded<T>(t_row + c * 64 + 32, v1);
+            store_rows<T>(dst, c * 64, c * 64 + 32, v0, v1, stage, lane);
+        }
+        return;
+    }
+    float inv_rms = 1.0f;
+    if (x.weight != nullptr) {                 // pass 1 over the accumulator: the head's sum of squares
+        float ss = 0.0f;
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+            float v[32];
+            load_rounded<T>(t_row + c * 32, v);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) ss += v[i] * v[i];
+        }
+        inv_rms = rsqrtf(ss / static_cast<float>(kBN) + p.eps);
+    }
+#pragma unroll 1
+    for (int c = 0; c < 2; ++c) {              // pass 2: columns [32 c, 32 c + 32) rotate with [64 + 32 c, 64 + 32 c + 32)
+        float lo[32], hi[32];
+        load_rounded<T>(t_row + c * 32, lo);
+        load_rounded<T>(t_row + 64 + c * 32, hi);
+        if (x.weight != nullptr) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+                lo[i] = lo[i] * inv_rms * ElemTraits<T>::to_float(x.weight[c * 32 + i]);
+                hi[i] = hi[i] * inv_rms * ElemTraits<T>::to_float(x.weight[64 + c * 32 + i]);
+            }
+        }
+        if (x.table != nullptr) {              // first half: x cos - partner sin; second half: x cos + partner sin
+            // 16-byte loads: every lane reads its own table row, so an instruction costs 32 cache lines whatever its width
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+                const float4 c4 = __ldg(reinterpret_cast<const float4*>(x.table + c * 32 + i)), s4 = __ldg(reinterpret_cast<const float4*>(x.table + 64 + c * 32 + i));
+                const float cs[4] = {c4.x, c4.y, c4.z, c4.w}, sn[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const float a = lo[i + u], b = hi[i + u];
+                    lo[i + u] = fmaf(a, cs[u], b * -sn[u]);
+                    hi[i + u] = fmaf(b, cs[u], a * sn[u]);
+                }
+            }
+        }
+        store_rows<T>(x.dst, c * 32, 64 + c * 32, lo, hi, stage, lane);
     }
 }
 
+// Eight lanes hold a row: lane `sub` elements 32 q + 4 sub .. + 3, q = 0 .. 3 (v[q]), so that the eight read 128 contiguous bytes of the
+// sums at a time -- from another block's shared memory 32-byte pieces 32 bytes apart come in at a quarter of the rate -- and rotation pairs
+// (d, d + 64) meet in a lane.  octet_row fetches what the epilogue of a row needs besides the sums (positions, then table rows: two
+// dependent trips to memory), so that this can be under way before the sums are there.
+template <typename T>
+struct OctetRow {
+    T* dst;               // kPlain, kQkvPrologue, kAllReducePush (own rows); nullptr: nothing to write there
+    uint4* slot;          // kAllReducePush
+    uint32_t epoch;
+    bool rotate;
+    float4 cs[2], sn[2];
+};
 template <typename T, int EPI>
+__device__ __forceinline__ OctetRow<T> octet_row(const GemmParams& p, int64_t row, int nt, int sub) {
+    const bool live = row < p.m;
+    OctetRow<T> x{};
+    if (EPI == kPlain) {
+        x.dst = live ? static_cast<T*>(p.out) + row * p.n + nt * kBN : nullptr;
+    } else if (EPI == kQkvPrologue) {
+        const QkvRow<T> q = qkv_row<T>(p, nt, row, live);
+        x.dst = q.dst;
+        x.rotate = !q.is_v && q.table != nullptr;
+        if (x.rotate) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                x.cs[i] = __ldg(reinterpret_cast<const float4*>(q.table + 32 * i + 4 * sub));
+                x.sn[i] = __ldg(reinterpret_cast<const float4*>(q.table + 64 + 32 * i + 4 * sub));
+            }
+        }
+    } else {
+        const PushRow<T> q = push_row<T>(p, row, live, nt * kBN);
+        x.dst = q.addend; x.slot = q.slot; x.epoch = q.epoch;
+    }
+    return x;
+}
+// Every lane of the warp runs it (shuffles).
+template <typename T, int EPI>
+__device__ __forceinline__ void epilogue_octet(const GemmParams& p, const OctetRow<T>& x, float4 (&v)[4], int nt, int sub) {
+    float e[4][4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        e[q][0] = v[q].x; e[q][1] = v[q].y; e[q][2] = v[q].z; e[q][3] = v[q].w;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) e[q][i] = ElemTraits<T>::to_float(ElemTraits<T>::from_float(e[q][i]));
+    }
+    if (EPI == kQkvPrologue && nt < p.hq + p.hkv) {   // a q or k head (the same for the whole block)
+        if (p.q_weight != nullptr) {
+            const T* weight = static_cast<const T*>(nt < p.hq ? p.q_weight : p.k_weight) + 4 * sub;
+            float ss = 0.0f;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) ss += e[q][i] * e[q][i];
+            }
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            const float inv_rms = rsqrtf(ss / static_cast<float>(kBN) + p.eps);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) e[q][i] = e[q][i] * inv_rms * ElemTraits<T>::to_float(weight[32 * q + i]);
+            }
+        }
+        if (x.rotate) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const float cs[4] = {x.cs[q].x, x.cs[q].y, x.cs[q].z, x.cs[q].w}, sn[4] = {x.sn[q].x, x.sn[q].y, x.sn[q].z, x.sn[q].w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float a = e[q][i], b = e[q + 2][i];
+                    e[q][i] = fmaf(a, cs[i], b * -sn[i]);
+                    e[q + 2][i] = fmaf(b, cs[i], a * sn[i]);
+                }
+            }
+        }
+    }
+    // neighbours exchange pieces: an even lane ends up with eight elements of quarter 0 (and 2), an odd one with eight of quarter 1 (and 3)
+    const bool odd = (sub & 1) != 0;
+    const int at = (odd ? 32 : 0) + 4 * (sub & ~1);
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const uint2 a = make_uint2(ElemTraits<T>::pack2(e[2 * half][0], e[2 * half][1]), ElemTraits<T>::pack2(e[2 * half][2], e[2 * half][3]));
+        const uint2 b = make_uint2(ElemTraits<T>::pack2(e[2 * half + 1][0], e[2 * half + 1][1]), ElemTraits<T>::pack2(e[2 * half + 1][2], e[2 * half + 1][3]));
+        const uint2 give = odd ? a : b;
+        uint2 got;
+        got.x = __shfl_xor_sync(0xffffffffu, give.x, 1);
+        got.y = __shfl_xor_sync(0xffffffffu, give.y, 1);
+        const uint4 w = odd ? make_uint4(got.x, got.y, b.x, b.y) : make_uint4(a.x, a.y, got.x, got.y);
+        if (x.dst != nullptr) *reinterpret_cast<uint4*>(x.dst + 64 * half + at) = w;
+        else if (EPI == kAllReducePush && x.slot != nullptr) st_tagged(x.slot + 2 * (8 * half + at / 8), w, x.epoch);
+    }
+}
+
+// Sum of one row over the blocks of a cluster, U blocks at a time (loads without branches, so that all of a trip's are in flight).
+template <int U>
+__device__ __forceinline__ void sum_over_cluster(uint32_t at, int splits, float4 (&sum)[4]) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) sum[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int r0 = 0; r0 < splits; r0 += U) {
+        float4 v[U][4];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint32_t src = in_block(at, static_cast<uint32_t>(min(r0 + u, splits - 1)));
+#pragma unroll
+            for (int q = 0; q < 4; ++q) v[u][q] = ld_cluster(src + 128 * q);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (r0 + u < splits) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) { sum[q].x += v[u][q].x; sum[q].y += v[u][q].y; sum[q].z += v[u][q].z; sum[q].w += v[u][q].w; }
+            }
+        }
+    }
+}
+
+// ---- few rows: blocks of a cluster share K ------------------------------------------------------------------------------------
+// blockIdx.x = tile column * splits + part of K (= rank in the cluster), blockIdx.y = tile row of MT * 128 rows.  The partial sums go to
+// shared memory as fp32 rows of 132 words (no bank conflicts for the writing threads, each of which has a row); block r adds up and
+// finishes rows r, r + splits, ... of the tile, eight lanes a row.
+constexpr int kRowWords = kBN + 4;
+template <typename T, int EPI, int MT>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const GemmParams p) {
+gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ GemmParams p, int splits) {
+    constexpr int kStageBytes = (MT + 1) * kPanelBytes, kStages = kRingBytes / kStageBytes, kTmemCols = MT * kBN;
+    static_assert(MT * kBM * kRowWords * 4 <= kRingBytes, "the partial sums take the ring's place");
     extern __shared__ unsigned char smem_raw[];
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t bars = smem_base + kBarOffset;
+    const uint32_t bars = smem_base + kRingBytes;
     auto bar_full = [&](int s) { return bars + 8 * s; };
     auto bar_empty = [&](int s) { return bars + 64 + 8 * s; };
     const uint32_t bar_acc = bars + 128;
     volatile int* abort_flag = &s_abort;
-    const int n0 = blockIdx.x * kBN, m0 = blockIdx.y * kBM;
-    const int kb_count = static_cast<int>((p.k + kBK - 1) / kBK);
+    const int rank = static_cast<int>(blockIdx.x) % splits, nt = static_cast<int>(blockIdx.x) / splits;
+    const int n0 = nt * kBN, m0 = blockIdx.y * (MT * kBM);
+    const int rows = static_cast<int>(min(static_cast<int64_t>(MT * kBM), p.m - m0));   // of the tile that are in C
+    const int kb_all = static_cast<int>((p.k + kBK - 1) / kBK);
+    const int kb0 = kb_all * rank / splits, kb_count = kb_all * (rank + 1) / splits - kb0;
 
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");             // A comes from the kernel before this one
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     if (tid == 0) {
         s_abort = 0;
         for (int s = 0; s < kStages; ++s) { mbar_init(bar_full(s), 1); mbar_init(bar_empty(s), 1); }
@@ -187,6 +490,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&s_tmem_base)), "r"(kTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
+    pdl_wait_then_release();   // A comes from the kernel before this one; barriers and TMEM were set up under its tail
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -195,141 +499,58 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
         if (lane == 0) {
-            for (int kb = 0; kb < kb_count; ++kb) {
-                const int s = kb % kStages;
-                if (kb >= kStages && !mbar_wait(bar_empty(s), ((kb / kStages) & 1) ^ 1, abort_flag, 1)) break;
-                mbar_expect_tx(bar_full(s), kStageBytes);
-                tma_load_2d(smem_base + s * kStageBytes, &tm_a, kb * kBK, m0, bar_full(s));
-                tma_load_2d(smem_base + s * kStageBytes + kPanelBytes, &tm_b, kb * kBK, n0, bar_full(s));
+            for (int i = 0; i < kb_count; ++i) {
+                const int s = i % kStages;
+                if (i >= kStages && !mbar_wait(bar_empty(s), ((i / kStages) & 1) ^ 1, abort_flag, 1)) break;
+                mbar_expect_tx(bar_full(s), kPanelBytes + (MT == 1 ? p.a_rows * kBK * 2 : 2 * kPanelBytes));
+                const uint32_t at = smem_base + s * kStageBytes;
+                tma_load_2d(at + MT * kPanelBytes, &tm_b, (kb0 + i) * kBK, n0, bar_full(s));
+#pragma unroll
+                for (int t = 0; t < MT; ++t) tma_load_2d(at + t * kPanelBytes, &tm_a, (kb0 + i) * kBK, m0 + t * kBM, bar_full(s));
             }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
         if (lane == 0) {
             bool ok = true;
-            for (int kb = 0; kb < kb_count && ok; ++kb) {
-                const int s = kb % kStages;
-                ok = mbar_wait(bar_full(s), (kb / kStages) & 1, abort_flag, 2);
+            for (int i = 0; i < kb_count && ok; ++i) {
+                const int s = i % kStages;
+                ok = mbar_wait(bar_full(s), (i / kStages) & 1, abort_flag, 2);
                 if (!ok) break;
                 tc_fence_after();
-                const uint64_t da = make_smem_desc(smem_base + s * kStageBytes), db = make_smem_desc(smem_base + s * kStageBytes + kPanelBytes);
+                const uint32_t at = smem_base + s * kStageBytes;
+                const uint64_t db = make_smem_desc(at + MT * kPanelBytes);
 #pragma unroll
-                for (int ks = 0; ks < kBK / 16; ++ks)   // 32 bytes further along the 128-byte row per K step: +2 in the address field
-                    umma_ss(tmem_base, da + 2 * ks, db + 2 * ks, p.idesc, (kb > 0 || ks > 0) ? 1u : 0u);
+                for (int t = 0; t < MT; ++t) {
+                    const uint64_t da = make_smem_desc(at + t * kPanelBytes);
+#pragma unroll
+                    for (int ks = 0; ks < kBK / 16; ++ks)   // 32 bytes further along the 128-byte row per K step: +2 in the address field
+                        umma_ss(tmem_base + t * kBN, da + 2 * ks, db + 2 * ks, p.idesc, (i > 0 || ks > 0) ? 1u : 0u);
+                }
                 tc_commit(bar_empty(s));
             }
             if (ok) tc_commit(bar_acc);
         }
     } else {
-        // ------------------------------------------------------------------ epilogue: thread = row of the tile
+        // ------------------------------------------------------------------ TMEM -> shared memory: thread = row of the tile
         const int wq = warp & 3;                       // TMEM lanes 32 wq .. 32 wq + 31 belong to this warp
-        const int row_in_tile = wq * 32 + lane;
-        const int64_t row = m0 + row_in_tile;
-        const uint32_t t_row = tmem_base + (static_cast<uint32_t>(wq * 32) << 16);
         bool ok = true;
         if (lane == 0) ok = mbar_wait(bar_acc, 0, abort_flag, 3);
         ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
         tc_fence_after();
         if (ok) {
-            if (EPI == kPlain) {
 #pragma unroll 1
-                for (int c = 0; c < 4; ++c) {
-                    float v[32];
-                    load_rounded<T>(t_row + c * 32, v);
-                    if (row < p.m) store32<T>(static_cast<T*>(p.out) + row * p.n + n0 + c * 32, v);
-                }
-            } else if (EPI == kQkvPrologue) {
-                // this tile is head `blockIdx.x` of the packed qkv row: q heads, then k heads, then v heads
-                const int head = blockIdx.x;
-                const bool is_q = head < p.hq, is_k = !is_q && head < p.hq + p.hkv;
-                const bool live = row < p.m;
-                const int pos = live ? __ldg(p.positions + row) : 0;
-                const int64_t slot = live ? (p.slot_mapping != nullptr ? static_cast<int64_t>(__ldg(p.slot_mapping + row)) : row) : -1;
-                T* dst = nullptr;
-                if (live) {
-                    if (is_q) dst = static_cast<T*>(p.q_out) + (row * p.hq + head) * kBN;
-                    else if (slot >= 0 && slot < p.cache_rows)
-                        dst = static_cast<T*>(is_k ? p.k_cache : p.v_cache) + (slot * p.hkv + (is_k ? head - p.hq : head - p.hq - p.hkv)) * kBN;
-                }
-                if (!is_q && !is_k) {                  // v heads: the rounded GEMM output as it is
-#pragma unroll 1
-                    for (int c = 0; c < 4; ++c) {
-                        float v[32];
-                        load_rounded<T>(t_row + c * 32, v);
-                        if (dst != nullptr) store32<T>(dst + c * 32, v);
-                    }
-                } else {
-                    const bool normed = p.q_weight != nullptr;
-                    float inv_rms = 1.0f;
-                    if (normed) {                      // pass 1 over the accumulator: the head's sum of squares
-                        float ss = 0.0f;
-#pragma unroll 1
-                        for (int c = 0; c < 4; ++c) {
-                            float v[32];
-                            load_rounded<T>(t_row + c * 32, v);
+            for (int c = 0; c < MT * 4; ++c) {
+                if ((c >> 2) * kBM + wq * 32 >= rows) break;   // (warp-uniform: no row of this warp is in C)
+                const int row_in_tile = (c >> 2) * kBM + wq * 32 + lane;
+                uint32_t r[32];
+                tmem_ld32(tmem_base + (static_cast<uint32_t>(wq * 32) << 16) + c * 32, r);
+                tc_wait_ld();
+                reg_fence32(r);
+                const uint32_t dst = smem_base + (row_in_tile * kRowWords + (c & 3) * 32) * 4;
 #pragma unroll
-                            for (int i = 0; i < 32; ++i) ss += v[i] * v[i];
-                        }
-                        inv_rms = rsqrtf(ss / static_cast<float>(kBN) + p.eps);
-                    }
-                    const bool rotate = pos >= 0 && pos < p.max_positions;
-                    const float* table = p.cos_sin + static_cast<int64_t>(rotate ? pos : 0) * kBN;
-                    const T* weight = static_cast<const T*>(is_q ? p.q_weight : p.k_weight);
-#pragma unroll 1
-                    for (int c = 0; c < 2; ++c) {      // pass 2: columns [32 c, 32 c + 32) rotate with [64 + 32 c, 64 + 32 c + 32)
-                        float lo[32], hi[32];
-                        load_rounded<T>(t_row + c * 32, lo);
-                        load_rounded<T>(t_row + 64 + c * 32, hi);
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) {
-                            float a = lo[i], b = hi[i];
-                            if (normed) {
-                                a = a * inv_rms * ElemTraits<T>::to_float(weight[c * 32 + i]);
-                                b = b * inv_rms * ElemTraits<T>::to_float(weight[64 + c * 32 + i]);
-                            }
-                            if (rotate) {              // first half: x cos - partner sin; second half: x cos + partner sin
-                                const float cs = __ldg(table + c * 32 + i), sn = __ldg(table + 64 + c * 32 + i);
-                                lo[i] = fmaf(a, cs, b * -sn);
-                                hi[i] = fmaf(b, cs, a * sn);
-                            } else {
-                                lo[i] = a; hi[i] = b;
-                            }
-                        }
-                        if (dst != nullptr) {
-                            store32<T>(dst + c * 32, lo);
-                            store32<T>(dst + 64 + c * 32, hi);
-                        }
-                    }
-                }
-            } else {   // kAllReducePush: every row of the partial sum goes to the rank that reduces it
-                const uint32_t last = *reinterpret_cast<const volatile uint32_t*>(p.flags);
-                const uint32_t epoch = last + 1u == 0u ? 1u : last + 1u;      // the epoch the all-reduce launch after this GEMM will use
-                const bool poisoned = *reinterpret_cast<const volatile uint32_t*>(p.flags + 2) != 0u;
-                const int64_t rows_per_rank = p.m / p.world;
-                const int64_t row_vecs = p.n / 8, chunk_vecs = rows_per_rank * row_vecs;
-                // (the TMEM loads are warp-collective: every lane runs them, only the stores depend on the row)
-                const bool live = row < p.m && !poisoned;
-                const int owner = live ? static_cast<int>(row / rows_per_rank) : p.rank;
-                {
-#pragma unroll 1
-                    for (int c = 0; c < 4; ++c) {
-                        float v[32];
-                        load_rounded<T>(t_row + c * 32, v);
-                        if (!live) continue;
-                        if (owner == p.rank) {
-                            store32<T>(static_cast<T*>(p.addend) + row * p.n + n0 + c * 32, v);
-                        } else {
-                            uint4* slot = p.stage[owner] + 2 * (p.rank * chunk_vecs + (row - owner * rows_per_rank) * row_vecs + (n0 + c * 32) / 8);
-#pragma unroll
-                            for (int q = 0; q < 4; ++q) {
-                                uint4 w;
-                                w.x = ElemTraits<T>::pack2(v[q * 8 + 0], v[q * 8 + 1]); w.y = ElemTraits<T>::pack2(v[q * 8 + 2], v[q * 8 + 3]);
-                                w.z = ElemTraits<T>::pack2(v[q * 8 + 4], v[q * 8 + 5]); w.w = ElemTraits<T>::pack2(v[q * 8 + 6], v[q * 8 + 7]);
-                                st_tagged(slot + 2 * q, w, epoch);
-                            }
-                        }
-                    }
-                }
+                for (int q = 0; q < 8; ++q)
+                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(dst + q * 16), "r"(r[4 * q]), "r"(r[4 * q + 1]), "r"(r[4 * q + 2]), "r"(r[4 * q + 3]) : "memory");
             }
         }
     }
@@ -337,6 +558,146 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     __syncthreads();
     if (warp == 1) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
+    }
+    // ---------------------------------------------------------------------- sum over the cluster and epilogue
+    const int sub = lane & 7;
+    int q = warp * 4;                      // four rows per warp and trip
+    auto row_of = [&](int first) { return (first + (lane >> 3)) * splits + rank; };
+    OctetRow<T> x = octet_row<T, EPI>(p, row_of(q) < rows ? m0 + row_of(q) : p.m, nt, sub);
+    if (splits > 1) cluster_sync_all();
+    bool arrived = false;
+    if (!*abort_flag) {
+        for (; q * splits + rank < rows; q += kThreads / 8) {
+            const uint32_t at = smem_base + min(row_of(q), rows - 1) * (kRowWords * 4) + sub * 16;
+            float4 sum[4];
+            if (splits > 2) sum_over_cluster<4>(at, splits, sum);
+            else sum_over_cluster<2>(at, splits, sum);
+            const int next = q + kThreads / 8;
+            if (splits > 1 && next * splits + rank >= rows) {   // this warp's last trip: its peers' memory is not needed any more
+                asm volatile("barrier.cluster.arrive;\n" ::: "memory");
+                arrived = true;
+            }
+            epilogue_octet<T, EPI>(p, x, sum, nt, sub);
+            if (next * splits + rank < rows) x = octet_row<T, EPI>(p, row_of(next) < rows ? m0 + row_of(next) : p.m, nt, sub);
+        }
+    }
+    if (splits > 1) {                      // no block leaves while a peer still reads its shared memory
+        if (!arrived) asm volatile("barrier.cluster.arrive;\n" ::: "memory");
+        asm volatile("barrier.cluster.wait;\n" ::: "memory");
+    }
+}
+
+// ---- many rows: persistent pairs of blocks ---------------------------------------------------------------------------------------
+constexpr int kPairStages = 6;
+constexpr int kPairStageBytes = 2 * kPanelBytes;      // this block's halves of A (128 of 256 rows) and B (128 of 256 columns)
+constexpr int kPairCols = 256;                        // accumulator columns of a tile; two of them fill TMEM
+template <typename T, int EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ GemmParams p) {
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ uint32_t s_tmem_base;
+    __shared__ int s_abort;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const uint32_t bars = smem_base + kRingBytes;
+    auto bar_full = [&](int s) { return bars + 8 * s; };         // used in the leader: both blocks' loads of a stage
+    auto bar_empty = [&](int s) { return bars + 64 + 8 * s; };   // in each block: the pair's MMAs have read the stage
+    auto bar_acc = [&](int b) { return bars + 128 + 8 * b; };    // in each block: accumulator b is complete
+    auto bar_free = [&](int b) { return bars + 144 + 8 * b; };   // in the leader: both blocks have read accumulator b
+    volatile int* abort_flag = &s_abort;
+    const uint32_t rank = cluster_rank();
+    const int kb_count = static_cast<int>((p.k + kBK - 1) / kBK);
+    const int tiles = p.tiles_m * p.tiles_n, first = blockIdx.x >> 1, step = gridDim.x >> 1;
+    // tiles in column-major order: a wave of pairs shares a few column panels of the weight
+    auto row0_of = [&](int tile) { return (tile % p.tiles_m) * 256 + static_cast<int>(rank) * kBM; };
+    auto col0_of = [&](int tile) { return (tile / p.tiles_m) * 256; };
+
+    if (tid == 0) {
+        s_abort = 0;
+        for (int s = 0; s < kPairStages; ++s) { mbar_init(bar_full(s), 1); mbar_init(bar_empty(s), 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(bar_acc(b), 1); mbar_init(bar_free(b), 16); }   // eight reading warps in each block
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    __syncwarp();
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&s_tmem_base)), "r"(2 * kPairCols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
+    }
+    pdl_wait_then_release();
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();   // the other block's barriers are set up
+    tc_fence_after();
+    const uint32_t tmem_base = s_tmem_base;
+
+    if (warp == 0) {
+        // ------------------------------------------------------------------ TMA producer of this block's halves
+        if (lane == 0) {
+            bool ok = true;
+            int it = 0;
+            for (int tile = first; tile < tiles && ok; tile += step) {
+                const int m0 = row0_of(tile), n0 = col0_of(tile) + static_cast<int>(rank) * kBN;
+                for (int kb = 0; kb < kb_count && ok; ++kb, ++it) {
+                    const int s = it % kPairStages;
+                    if (it >= kPairStages) ok = mbar_wait(bar_empty(s), ((it / kPairStages) & 1) ^ 1, abort_flag, 1);
+                    if (!ok) break;
+                    if (rank == 0) mbar_expect_tx(bar_full(s), 2 * kPairStageBytes);
+                    const uint32_t at = smem_base + s * kPairStageBytes, full = in_block(bar_full(s), 0);
+                    tma_load_2d_pair(at, &tm_a, kb * kBK, m0, full);
+                    tma_load_2d_pair(at + kPanelBytes, &tm_b, kb * kBK, n0, full);
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ------------------------------------------------------------------ MMA issuer, for both blocks
+        if (lane == 0 && rank == 0) {
+            bool ok = true;
+            int it = 0, n = 0;
+            for (int tile = first; tile < tiles && ok; tile += step, ++n) {
+                const int b = n & 1;
+                if (n >= 2) ok = mbar_wait(bar_free(b), ((n >> 1) & 1) ^ 1, abort_flag, 4);
+                if (!ok) break;
+                tc_fence_after();
+                for (int kb = 0; kb < kb_count; ++kb, ++it) {
+                    const int s = it % kPairStages;
+                    ok = mbar_wait(bar_full(s), (it / kPairStages) & 1, abort_flag, 2);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint64_t da = make_smem_desc(smem_base + s * kPairStageBytes), db = make_smem_desc(smem_base + s * kPairStageBytes + kPanelBytes);
+#pragma unroll
+                    for (int ks = 0; ks < kBK / 16; ++ks)
+                        umma_ss_pair(tmem_base + b * kPairCols, da + 2 * ks, db + 2 * ks, p.idesc, (kb > 0 || ks > 0) ? 1u : 0u);
+                    tc_commit_pair(bar_empty(s));
+                }
+                if (ok) tc_commit_pair(bar_acc(b));
+            }
+        }
+    } else {
+        // ------------------------------------------------------------------ epilogue: thread = row, warps 2-5 the first 128 columns of
+        // the tile, 6-9 the second (with one tile per pair nothing hides it: 500 rows of QKV took 10 us longer than the plain product)
+        const int wq = warp & 3, half = warp >= 6 ? 1 : 0;
+        int n = 0;
+        for (int tile = first; tile < tiles; tile += step, ++n) {
+            const int b = n & 1;
+            bool ok = true;
+            if (lane == 0) ok = mbar_wait(bar_acc(b), (n >> 1) & 1, abort_flag, 3);
+            if (__shfl_sync(0xffffffffu, ok ? 1 : 0, 0) == 0) break;
+            tc_fence_after();
+            const int64_t row = row0_of(tile) + wq * 32 + lane;
+            const uint32_t t_row = tmem_base + b * kPairCols + (static_cast<uint32_t>(wq * 32) << 16);
+            const int nt = col0_of(tile) / kBN + half;
+            unsigned char* stage = smem_raw + (smem_base - smem_u32(smem_raw)) + kStageOffset + (warp - 2) * 4096;
+            if (nt * kBN < p.n) epilogue_row<T, EPI>(p, t_row + half * kBN, row, nt, stage, lane);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(in_block(bar_free(b), 0));
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();   // neither block leaves while the other may still signal its barriers or read its operands
+    if (warp == 1) {
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(2 * kPairCols) : "memory");
     }
 }
 
@@ -356,50 +717,94 @@ EncodeFn encode_fn() {
     });
     return fn;
 }
-// [rows, k] 16-bit row-major -> boxes of 128 rows x 64 elements, 128-byte swizzle; rows past the end read as zeros
-bool make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t k, bool bf16) {
+// [rows, k] 16-bit row-major -> boxes of `box_rows` rows x 64 elements, 128-byte swizzle; rows past the end read as zeros
+bool make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t k, bool bf16, int box_rows = kBM) {
     EncodeFn fn = encode_fn();
     if (fn == nullptr) return false;
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(k), static_cast<cuuint64_t>(rows)};
     const cuuint64_t strides[1] = {static_cast<cuuint64_t>(k) * 2};
-    const cuuint32_t box[2] = {kBK, kBM};
+    const cuuint32_t box[2] = {kBK, static_cast<cuuint32_t>(box_rows)};
     const cuuint32_t elem[2] = {1, 1};
     return fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims,
               strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-uint32_t make_idesc(bool bf16) {   // kind::f16: D = F32, A / B = F16 or BF16 (both K-major), M 128, N 128
+uint32_t make_idesc(bool bf16, int m, int n) {   // kind::f16: D = F32, A / B = F16 or BF16 (both K-major)
     const uint32_t fmt = bf16 ? 1u : 0u;
-    return (1u << 4) | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>(kBN >> 3) << 17) | (static_cast<uint32_t>(kBM >> 4) << 24);
+    return (1u << 4) | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
+}
+
+// Kernel and shape for a size, by what the slowest SM does: waves of blocks times steps of 64 along K, plus a fixed part.  The
+// microseconds are measured (1 to 7440 rows, 768 to 6144 columns, K 4096).  A step of a 128 x 128 tile takes 0.30 us, of a 256 x 128
+// one 0.43: 32 and 48 KiB out of L2, the bound here, not the tensor pipe; a 256 x 256 tile of a pair, with 32 KiB per SM, 0.37.
+// The launch, the first loads and the epilogue take 5 us, the sum over a cluster 1 to 2 more, 4 to 6 with twice the rows.
+struct GemmShape { int mt, splits; };   // mt 1 or 2: gemm_split_kernel; 0: gemm_pair_kernel
+GemmShape choose_gemm(int64_t m, int64_t n, int64_t k) {
+    // clusters of such blocks that a B200 holds at once (its GPCs have 16 to 20 SMs)
+    struct { int splits, clusters; double fixed[2]; } constexpr kWays[] = {{1, 148, {5.0, 5.0}}, {2, 74, {6.0, 9.0}}, {4, 33, {7.0, 11.0}}, {8, 15, {7.0, 11.0}}};
+    const int64_t kb = (k + kBK - 1) / kBK, tiles_n = n / kBN;
+    const int64_t pair_tiles = ((m + 255) / 256) * ((n + 255) / 256);
+    GemmShape best{0, 1};
+    double best_time = m > kBM ? static_cast<double>((pair_tiles + 73) / 74 * kb) * 0.37 + 6.0 : 1e30;
+    for (int mt = 1; mt <= 2; ++mt) {
+        if (mt == 2 && m <= kBM) break;
+        const int64_t tiles = (m + mt * kBM - 1) / (mt * kBM) * tiles_n;
+        for (const auto& w : kWays) {
+            if (w.splits > 1 && (kb / w.splits < 4 || tiles > w.clusters)) break;
+            const double time = static_cast<double>((tiles + w.clusters - 1) / w.clusters * ((kb + w.splits - 1) / w.splits)) * (mt == 1 ? 0.30 : 0.43) + w.fixed[mt - 1];
+            if (time < best_time) { best_time = time; best = GemmShape{mt, w.splits}; }
+        }
+    }
+    return best;
+}
+
+template <typename... KArgs>
+int launch_kernel(void (*kernel)(KArgs...), bool* attr_done, dim3 grid, int threads, int cluster, cudaStream_t stream, const char* what,
+                  KArgs... args) {
+    int device = 0;
+    cudaGetDevice(&device);
+    if (device >= 0 && device < 64 && !attr_done[device]) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+        if (e != cudaSuccess) return fail(NVK_ERR_CUDA, "%s: cudaFuncSetAttribute: %s", what, cudaGetErrorString(e));
+        attr_done[device] = true;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = kSmemBytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 0 ? 2 : 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+    if (e != cudaSuccess) return fail(NVK_ERR_CUDA, "%s launch: %s", what, cudaGetErrorString(e));
+    return check_launch(what);
 }
 
 template <typename T, int EPI>
 int launch(const void* a, const void* b, GemmParams& p, bool bf16, cudaStream_t stream, const char* what) {
-    static bool attr_done[64] = {};
-    int device = 0;
-    cudaGetDevice(&device);
-    if (device >= 0 && device < 64 && !attr_done[device]) {
-        const cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<T, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-        if (e != cudaSuccess) return fail(NVK_ERR_CUDA, "%s: cudaFuncSetAttribute: %s", what, cudaGetErrorString(e));
-        attr_done[device] = true;
-    }
+    static bool done[3][64] = {};
     CUtensorMap ta, tb;
-    if (!make_map(&ta, a, p.m, p.k, bf16) || !make_map(&tb, b, p.n, p.k, bf16))
+    const GemmShape g = choose_gemm(p.m, p.n, p.k);
+    p.a_rows = g.mt == 1 && p.m < kBM ? static_cast<int>((p.m + 7) / 8 * 8) : kBM;
+    if (!make_map(&ta, a, p.m, p.k, bf16, p.a_rows) || !make_map(&tb, b, p.n, p.k, bf16))
         return fail(NVK_ERR_CUDA, "%s: cuTensorMapEncodeTiled failed", what);
-    p.idesc = make_idesc(bf16);
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(static_cast<unsigned>(p.n / kBN), static_cast<unsigned>((p.m + kBM - 1) / kBM));
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = kSmemBytes;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<T, EPI>, ta, tb, p);
-    if (e != cudaSuccess) return fail(NVK_ERR_CUDA, "%s launch: %s", what, cudaGetErrorString(e));
-    return check_launch(what);
+    if (g.mt == 0) {
+        p.idesc = make_idesc(bf16, 256, 256);
+        p.tiles_m = static_cast<int>((p.m + 255) / 256);
+        p.tiles_n = static_cast<int>((p.n + 255) / 256);
+        const int64_t pairs = static_cast<int64_t>(p.tiles_m) * p.tiles_n;
+        return launch_kernel(gemm_pair_kernel<T, EPI>, done[0], dim3(static_cast<unsigned>(2 * (pairs < kSmCount / 2 ? pairs : kSmCount / 2))), kPairThreads, 0,
+                             stream, what, ta, tb, p);
+    }
+    p.idesc = make_idesc(bf16, kBM, kBN);
+    const dim3 grid(static_cast<unsigned>(p.n / kBN * g.splits), static_cast<unsigned>((p.m + g.mt * kBM - 1) / (g.mt * kBM)));
+    return g.mt == 1 ? launch_kernel(gemm_split_kernel<T, EPI, 1>, done[1], grid, kThreads, g.splits, stream, what, ta, tb, p, g.splits)
+                     : launch_kernel(gemm_split_kernel<T, EPI, 2>, done[2], grid, kThreads, g.splits, stream, what, ta, tb, p, g.splits);
 }
 
 int check_gemm(const char* what, const void* a, const void* b, int64_t m, int64_t n, int64_t k, int dtype) {

@@ -1,0 +1,57 @@
+"""The linears at the edges of their two kernels' tilings: parts of K in clusters of 1, 2, 4 and 8 blocks, one and two row tiles, pairs of
+blocks with one and with several tiles, a last column tile of half width, remainders of rows and of K."""
+import numpy as np
+import pytest
+
+import oracle
+from util import nvk, to_dev, to_np, workloads
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,out_features,in_features", [
+    (1, 128, 8), (8, 768, 4096), (9, 768, 1032), (64, 4096, 1024), (128, 6144, 520), (129, 768, 4096), (200, 6144, 512), (256, 2048, 2048),
+    (257, 4096, 512), (500, 6144, 512), (513, 9472, 128), (1030, 1408, 264), (3000, 384, 2048), (5000, 4096, 72),
+])
+def test_linear_at_tile_edges(dtype, rows, out_features, in_features):
+    gen = torch.Generator(device="cuda").manual_seed(rows + out_features)
+    x = torch.randn((rows, in_features), generator=gen, device="cuda").to(dtype)
+    w = (torch.randn((out_features, in_features), generator=gen, device="cuda") / in_features ** 0.5).to(dtype)
+    guard = torch.full((rows + 1, out_features), float("nan"), device="cuda", dtype=dtype)
+    nvk().linear(x, w, guard[:rows])
+    torch.cuda.synchronize()
+    assert nvk().gemm_status() == 0
+    want = x.float() @ w.float().t()
+    err = (guard[:rows].float() - want).abs()
+    ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    assert bool((err <= want.abs().clamp_min(0.05) * 2 * ulp + 1e-3).all()), float(err.max())
+    assert bool(torch.isnan(guard[rows].float()).all())          # nothing past the last row
+
+
+@pytest.mark.parametrize("num_q_heads,num_kv_heads,rows,hidden", [(4, 1, 3, 2048), (32, 8, 200, 512), (16, 8, 700, 1024), (6, 3, 2100, 256), (32, 8, 1500, 128)])
+def test_qkv_prologue_at_tile_edges(num_q_heads, num_kv_heads, rows, hidden):
+    bf, d, max_pos, heads = torch.bfloat16, 128, 400, num_q_heads + 2 * num_kv_heads
+    gen = torch.Generator(device="cuda").manual_seed(heads + rows)
+    x = torch.randn((rows, hidden), generator=gen, device="cuda").to(bf)
+    w = (torch.randn((heads * d, hidden), generator=gen, device="cuda") / hidden ** 0.5).to(bf)
+    cache_rows = rows + 100
+    pw = workloads().make_prologue_workload(rows, num_q_heads, num_kv_heads, d, cache_rows, max_pos, seed=rows)
+    pw["slot_mapping"][rows // 2] = -1
+    pw["positions"][0] = max_pos
+    table = oracle.build_cos_sin_cache(max_pos, d, pw["rope_base"])
+    kc = torch.zeros(cache_rows, num_kv_heads, d, dtype=bf, device="cuda")
+    vc, q_out = torch.zeros_like(kc), torch.full((rows, num_q_heads, d), float("nan"), dtype=bf, device="cuda")
+    nvk().qkv_linear_norm_rope_store(x, w, to_dev(pw["positions"]), to_dev(pw["q_norm_weight"], bf), to_dev(pw["k_norm_weight"], bf), pw["eps"],
+                                     to_dev(table), to_dev(pw["slot_mapping"]), kc, vc, num_q_heads, num_kv_heads, d, q_out)
+    qkv = torch.empty((rows, heads * d), dtype=bf, device="cuda")
+    nvk().linear(x, w, qkv)
+    torch.cuda.synchronize()
+    assert nvk().gemm_status() == 0
+    kc_ref, vc_ref = np.zeros((cache_rows, num_kv_heads, d), np.float32), np.zeros((cache_rows, num_kv_heads, d), np.float32)
+    q_ref = oracle.fused_split_norm_rope_store(to_np(qkv), pw["positions"], pw["q_norm_weight"], pw["k_norm_weight"], pw["eps"], table,
+                                               pw["slot_mapping"], kc_ref, vc_ref, num_q_heads, num_kv_heads, d)
+    assert np.array_equal(to_np(vc), vc_ref)                      # V: the rounded product, copied
+    for got, ref in ((to_np(q_out), q_ref), (to_np(kc), kc_ref)):
+        assert (np.abs(got - ref) <= np.maximum(np.abs(ref), 1e-3) * 2.0 ** -7).all()
