@@ -754,47 +754,77 @@ struct Tc5Params {
     int slot;             // ticket counter of this launch
 };
 
-struct Tc5Item {          // one (query tile, head pair), published by the producer warp
+// One (query tile, head pair), with all that the roles need to know of it, so that none of them reads the sequence bounds again.
+struct Tc5Item {
     int kind;             // 1 = work, 0 = no more work
-    int seq, q0, pair;
+    int seq, pair;
+    int q_row, rows;      // first query row and the rows there are
+    int lim0, k_len;      // query row r sees keys [0, min(lim0 + r, k_len))
+    int num_kt, last_partial;
+    int k_row;            // row of the sequence's first key (keys without a block table)
+    int row0, row1;       // rows of its first two key tiles
 };
 
-// Geometry of an item, derived identically by every role from (seq, q0).
-struct Tc5Geom {
-    int64_t qb, kb;
-    int q_len, k_len, rows_here, shift, num_kt, last_partial;
-};
-__device__ __forceinline__ Tc5Geom tc5_geometry(const TcParams& p, int seq, int q0) {
-    Tc5Geom g;
-    if (p.cu_q == nullptr) { g.qb = 0; g.kb = 0; g.q_len = static_cast<int>(p.total_q); g.k_len = static_cast<int>(p.total_k); }
-    else {
-        g.qb = p.cu_q[seq]; g.kb = p.cu_k[seq];
-        g.q_len = p.cu_q[seq + 1] - static_cast<int>(g.qb); g.k_len = p.cu_k[seq + 1] - static_cast<int>(g.kb);
-    }
-    g.rows_here = min(kBM, g.q_len - q0);
-    g.shift = g.k_len - g.q_len;
-    int k_hi = g.shift + q0 + g.rows_here;
-    if (k_hi > g.k_len) k_hi = g.k_len;
-    g.num_kt = k_hi > 0 ? (k_hi + kBN - 1) / kBN : 0;
-    g.last_partial = (g.num_kt * kBN > g.k_len) ? g.num_kt - 1 : -1;
-    return g;
+// Row of key `key0` of a sequence in the K / V tensors; key_rows (past the end: the copy fills zeros) for an invalid block.
+__device__ __forceinline__ int tc5_key_row(const TcParams& p, int seq, int k_row, int key0) {
+    if (!p.block_tables) return k_row + key0;
+    const int64_t id = p.block_tables[static_cast<int64_t>(seq) * p.max_blocks + key0 / p.block_size];
+    if (id < 0 || id >= p.num_cache_blocks) return static_cast<int>(p.key_rows);
+    return static_cast<int>(id) * p.block_size + key0 % p.block_size;
 }
 
-// Query tile number `want` (0 = first tile of the first sequence) -> (seq, q0); false when past the end.
-__device__ __forceinline__ bool tc5_locate(const TcParams& p, int64_t want, int& seq, int& q0) {
-    if (p.cu_q == nullptr) {
-        if (want * kBM >= p.total_q) return false;
-        seq = 0; q0 = static_cast<int>(want * kBM);
-        return true;
+// Finds the sequence of a query tile.  One warp holds a window of 32 sequences, one per lane, and moves it as the tiles it is asked
+// for descend: a look-up is one ballot, and the bounds are loaded once per window.  (One lane walking the sequences one dependent
+// load after the other took 5 to 7 thousand clocks an item with 16 to 32 sequences, more than an item of short sequences lasts:
+// 64 x 256 tokens 191 -> 130 us, 32 x 512 182 -> 169, 16 x 2048 620 -> 605.)
+struct Tc5Finder {
+    int base, before, sum;     // first sequence of the window, tiles before it, tiles in it
+    int mine;                  // tiles of the window before this lane's sequence
+    int tiles, qb, qe, kb, ke; // of this lane's sequence
+
+    __device__ __forceinline__ void load(const TcParams& p, int lane) {
+        qb = 0; qe = 0; kb = 0; ke = 0;
+        if (p.cu_q == nullptr) {
+            if (lane == 0) { qe = static_cast<int>(p.total_q); ke = static_cast<int>(p.total_k); }
+        } else if (base + lane < p.num_seqs) {
+            qb = static_cast<int>(p.cu_q[base + lane]); qe = static_cast<int>(p.cu_q[base + lane + 1]);
+            kb = static_cast<int>(p.cu_k[base + lane]); ke = static_cast<int>(p.cu_k[base + lane + 1]);
+        }
+        tiles = max((qe - qb + kBM - 1) / kBM, 0);
+        int inc = tiles;
+#pragma unroll
+        for (int d = 1; d < 32; d *= 2) {
+            const int up = __shfl_up_sync(0xffffffffu, inc, d);
+            if (lane >= d) inc += up;
+        }
+        mine = inc - tiles;
+        sum = __shfl_sync(0xffffffffu, inc, 31);
     }
-    int64_t acc = 0;
-    for (int64_t s = 0; s < p.num_seqs; ++s) {
-        const int64_t tiles = (static_cast<int64_t>(p.cu_q[s + 1]) - p.cu_q[s] + kBM - 1) / kBM;
-        if (want < acc + tiles) { seq = static_cast<int>(s); q0 = static_cast<int>((want - acc) * kBM); return true; }
-        acc += tiles;
+    // Opens on the last window (the first tile asked for is the last one) and returns the number of tiles of all sequences.
+    __device__ __forceinline__ int open(const TcParams& p, int lane) {
+        base = 0; before = 0;
+        load(p, lane);
+        while (p.cu_q != nullptr && base + 32 < p.num_seqs) { before += sum; base += 32; load(p, lane); }
+        return before + sum;
     }
-    return false;
-}
+    // Tile number `want`, in [0, open()): its item, without the pair.
+    __device__ __forceinline__ void find(const TcParams& p, int lane, int want, Tc5Item& it) {
+        while (want < before) { base -= 32; load(p, lane); before -= sum; }
+        const int at = 31 - __clz(__ballot_sync(0xffffffffu, before + mine <= want && tiles > 0));
+        const int q0 = (want - before - __shfl_sync(0xffffffffu, mine, at)) * kBM;
+        const int q_begin = __shfl_sync(0xffffffffu, qb, at), q_len = __shfl_sync(0xffffffffu, qe, at) - q_begin;
+        it.seq = base + at;
+        it.q_row = q_begin + q0;
+        it.rows = min(kBM, q_len - q0);
+        it.k_row = __shfl_sync(0xffffffffu, kb, at);
+        it.k_len = __shfl_sync(0xffffffffu, ke, at) - it.k_row;
+        it.lim0 = it.k_len - q_len + q0 + 1;
+        const int k_hi = min(it.lim0 + it.rows - 1, it.k_len);
+        it.num_kt = k_hi > 0 ? (k_hi + kBN - 1) / kBN : 0;
+        it.last_partial = it.num_kt * kBN > it.k_len ? it.num_kt - 1 : -1;
+    }
+};
+
 
 // The decode half of a mixed step (prefill_tc5_kernel<T, true>): the (KV head, split, sequence) items of the decode kernels, taken
 // from a second ticket counter by the same persistent blocks.  A block runs the two halves one after the other -- blocks
@@ -901,65 +931,46 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         int n = 0;            // items published so far (all of them carry work)
         int gk = 0, gv = 0;   // K / V tiles loaded so far, over all items
         bool ok = true;
-        // Next item that carries work (whole warp; lane 0 takes the tickets).  Tiles past the last sequence are
-        // skipped, tiles whose rows see no key are zero-filled right here and never published.
-        auto take_item = [&](int& kind, int& seq, int& q0, int& pair, Tc5Geom& g) {
+        Tc5Finder find;
+        const int tiles = min(find.open(p, lane), pp.tiles);
+        const unsigned int total = static_cast<unsigned int>(tiles) * static_cast<unsigned int>(pp.pairs);
+        // Next item that carries work (whole warp).  Tiles whose rows see no key are zero-filled right here and never published.
+        auto take_item = [&]() -> Tc5Item {
+            Tc5Item it{};
             while (true) {
-                kind = 0; seq = 0; q0 = 0; pair = 0;
-                if (lane == 0) {
-                    while (true) {
-                        const unsigned int ticket = atomicAdd(&g_prefill_ticket[pp.slot], 1u);
-                        if (ticket >= pp.total) break;
-                        pair = static_cast<int>(ticket % static_cast<unsigned int>(pp.pairs));
-                        const int64_t want = static_cast<int64_t>(pp.tiles) - 1 - static_cast<int64_t>(ticket / static_cast<unsigned int>(pp.pairs));
-                        if (tc5_locate(p, want, seq, q0)) { kind = 1; break; }
-                    }
-                }
-                kind = __shfl_sync(0xffffffffu, kind, 0);
-                seq = __shfl_sync(0xffffffffu, seq, 0);
-                q0 = __shfl_sync(0xffffffffu, q0, 0);
-                pair = __shfl_sync(0xffffffffu, pair, 0);
-                if (!kind) return;
-                g = tc5_geometry(p, seq, q0);
-                if (g.num_kt > 0) return;
+                unsigned int ticket = 0;
+                if (lane == 0) ticket = atomicAdd(&g_prefill_ticket[pp.slot], 1u);
+                ticket = __shfl_sync(0xffffffffu, ticket, 0);
+                if (ticket >= total) return it;
+                it.pair = static_cast<int>(ticket % static_cast<unsigned int>(pp.pairs));
+                find.find(p, lane, tiles - 1 - static_cast<int>(ticket / static_cast<unsigned int>(pp.pairs)), it);
+                if (it.num_kt > 0) break;
                 for (int t = 0; t < 2; ++t) {
-                    T* o0 = static_cast<T*>(p.out) + (static_cast<size_t>(g.qb + q0) * p.num_heads + 2 * pair + t) * kHeadDim;
-                    for (int i = lane; i < g.rows_here * (kHeadDim / 8); i += 32) {
+                    T* o0 = static_cast<T*>(p.out) + (static_cast<size_t>(it.q_row) * p.num_heads + 2 * it.pair + t) * kHeadDim;
+                    for (int i = lane; i < it.rows * (kHeadDim / 8); i += 32) {
                         const int r = i / (kHeadDim / 8), c = i % (kHeadDim / 8);
                         *reinterpret_cast<uint4*>(o0 + r * out_stride + c * 8) = make_uint4(0u, 0u, 0u, 0u);
                     }
                 }
             }
+            it.kind = 1;
+            it.row0 = tc5_key_row(p, it.seq, it.k_row, 0);
+            it.row1 = it.num_kt > 1 ? tc5_key_row(p, it.seq, it.k_row, kBN) : 0;
+            return it;
         };
-        int kind = 0, seq = 0, q0 = 0, pair = 0;
-        Tc5Geom g{};
-        int nkind = 0, nseq = 0, nq0 = 0, npair = 0;
-        Tc5Geom ng{};
-        take_item(nkind, nseq, nq0, npair, ng);
+        Tc5Item next = take_item();
         while (ok) {
-            kind = nkind; seq = nseq; q0 = nq0; pair = npair; g = ng;
+            const Tc5Item it = next;
             if (lane == 0) {
-                Tc5Item it;
-                it.kind = kind; it.seq = seq; it.q0 = q0; it.pair = pair;
                 s_ring[n & 3] = it;
                 mbar_arrive(bar_item(n & 3));   // release: the entry is visible to whoever waits on the barrier
             }
-            if (!kind) break;
-            const int head0 = 2 * pair;
+            if (!it.kind) break;
+            const int head0 = 2 * it.pair;
             const int kvh = head0 * p.num_kv_heads / p.num_heads;
-            const IndexArray table = p.block_tables ? p.block_tables + static_cast<int64_t>(seq) * p.max_blocks : IndexArray();
-            auto key_row = [&](int key0) -> int {
-                if (table) {
-                    const int64_t id = table[key0 / p.block_size];
-                    if (id < 0 || id >= p.num_cache_blocks) return static_cast<int>(p.key_rows);
-                    return static_cast<int>(id) * p.block_size + key0 % p.block_size;
-                }
-                return static_cast<int>(g.kb) + key0;
-            };
-            auto load_k = [&](int j) -> bool {   // lane 0 only
+            auto load_k = [&](int j, int r) -> bool {   // lane 0 only
                 const int c = gk + j, s = c & 1;
                 if (c >= 2 && !mbar_wait(bar_kempty(s), ((c >> 1) & 1) ^ 1, abort_flag, 11)) return false;
-                const int r = key_row(j * kBN);
                 mbar_expect_tx(bar_kfull(s), kTileBytes);
                 tma_load_3d(sm_k + s * kTileBytes, &tm_k, 0, kvh, r, bar_kfull(s));
                 tma_load_3d(sm_k + s * kTileBytes + kPanelBytes, &tm_k, 64, kvh, r, bar_kfull(s));
@@ -970,33 +981,33 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 if (ok) {
                     mbar_expect_tx(bar_qfull, 2 * kTileBytes);
                     for (int t = 0; t < 2; ++t) {
-                        tma_load_3d(sm_q + t * kTileBytes, &tm_q, 0, head0 + t, static_cast<int>(g.qb) + q0, bar_qfull);
-                        tma_load_3d(sm_q + t * kTileBytes + kPanelBytes, &tm_q, 64, head0 + t, static_cast<int>(g.qb) + q0, bar_qfull);
+                        tma_load_3d(sm_q + t * kTileBytes, &tm_q, 0, head0 + t, it.q_row, bar_qfull);
+                        tma_load_3d(sm_q + t * kTileBytes + kPanelBytes, &tm_q, 64, head0 + t, it.q_row, bar_qfull);
                     }
-                    ok = load_k(0);
+                    ok = load_k(0, it.row0);
                 }
             }
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-            // the next ticket, its sequence look-up and geometry are fetched now, under this item's rounds
-            if (ok) take_item(nkind, nseq, nq0, npair, ng);
-            for (int j = 0; j < g.num_kt && ok; ++j) {
+            int row = it.row0, next_row = it.row1;   // (a block's id is read a round before its copy)
+            for (int j = 0; j < it.num_kt && ok; ++j) {
                 const int cv = gv + j;
                 if (lane == 0) {
-                    if (j + 1 < g.num_kt) ok = load_k(j + 1);            // K runs one tile ahead of V
+                    if (j + 1 < it.num_kt) ok = load_k(j + 1, next_row);            // K runs one tile ahead of V
                     if (ok && cv >= 1) ok = mbar_wait(bar_vempty, (cv - 1) & 1, abort_flag, 12);
                     if (ok) {
-                        const int r = key_row(j * kBN);
                         mbar_expect_tx(bar_vfull, kTileBytes);
-                        tma_load_3d(sm_v, &tm_v, 0, kvh, r, bar_vfull);
-                        tma_load_3d(sm_v + kPanelBytes, &tm_v, 64, kvh, r, bar_vfull);
+                        tma_load_3d(sm_v, &tm_v, 0, kvh, row, bar_vfull);
+                        tma_load_3d(sm_v + kPanelBytes, &tm_v, 64, kvh, row, bar_vfull);
                     }
+                    row = next_row;
+                    if (j + 2 < it.num_kt) next_row = tc5_key_row(p, it.seq, it.k_row, (j + 2) * kBN);
                 }
                 ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-                if (ok && j == g.last_partial) {
+                if (ok && j == it.last_partial) {
                     // rows of V past the sequence may hold anything (0 * NaN = NaN): zero them once landed
                     ok = warp_mbar_wait(bar_vfull, cv & 1, abort_flag, 13);
                     if (ok) {
-                        const int first_bad = g.k_len - j * kBN;   // in (0, 128)
+                        const int first_bad = it.k_len - j * kBN;   // in (0, 128)
                         for (int i = lane; i < (kBN - first_bad) * 16; i += 32) {
                             const int r = first_bad + i / 16, c16 = i % 16;
                             *reinterpret_cast<uint4*>(smem_gen + kOff4V + (c16 >> 3) * kPanelBytes + r * 128 + (c16 & 7) * 16) =
@@ -1007,8 +1018,9 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                         if (lane == 0) mbar_arrive(bar_vfix);
                     }
                 }
+                if (ok && j == 0) next = take_item();   // under this item's rounds
             }
-            gk += g.num_kt; gv += g.num_kt; ++n;
+            gk += it.num_kt; gv += it.num_kt; ++n;
         }
     } else if (warp == 8 || warp == 8 + 2 * (kIssuers5 - 1)) {
         // ------------------------------------------------------------------ MMA issuer(s): with two, warp 8 drives
@@ -1030,7 +1042,6 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 if (!ok) break;
                 const Tc5Item it = s_ring[n & 3];
                 if (it.kind == 0) break;
-                const Tc5Geom g = tc5_geometry(p, it.seq, it.q0);
                 auto issue_s = [&](int t, int j) {
                     const int s = (gk + j) & 1;
                     umma_scores(std::make_integer_sequence<int, 8>{}, tmem_base + t * 128, dq[t], dk[s], p.idesc_s);
@@ -1046,9 +1057,9 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 }
                 if (!ok) break;
                 tc_commit(bar_kempty(gk & 1));              // (every issuer arrives)
-                if (g.num_kt == 1) tc_commit(bar_qempty);   // every score MMA of the item has been issued
-                for (int j = 0; j < g.num_kt && ok; ++j) {
-                    if (j + 1 < g.num_kt) {   // next scores as soon as this step's scores have been read
+                if (it.num_kt == 1) tc_commit(bar_qempty);   // every score MMA of the item has been issued
+                for (int j = 0; j < it.num_kt && ok; ++j) {
+                    if (j + 1 < it.num_kt) {   // next scores as soon as this step's scores have been read
                         const int c = gk + j + 1;
                         ok = mbar_wait(bar_kfull(c & 1), (c >> 1) & 1, abort_flag, 26);
                         for (int t = t_lo; t < t_hi && ok; ++t) {
@@ -1059,10 +1070,10 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                         }
                         if (!ok) break;
                         tc_commit(bar_kempty(c & 1));
-                        if (j + 2 == g.num_kt) tc_commit(bar_qempty);
+                        if (j + 2 == it.num_kt) tc_commit(bar_qempty);
                     }
                     ok = mbar_wait(bar_vfull, (gv + j) & 1, abort_flag, 23);
-                    if (ok && j == g.last_partial) ok = mbar_wait(bar_vfix, nf & 1, abort_flag, 24);
+                    if (ok && j == it.last_partial) ok = mbar_wait(bar_vfix, nf & 1, abort_flag, 24);
                     for (int t = t_lo; t < t_hi && ok; ++t) {
                         // p_full of an item's first round also says that the previous item's output has left TMEM
                         ok = mbar_wait(bar_pfull(t), (G + j) & 1, abort_flag, 25);
@@ -1070,12 +1081,12 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                         tc_fence_after();
                         umma_pv(std::make_integer_sequence<int, 8>{}, tmem_base + 256 + t * 128, dp[t], dv, p.idesc_pv, j > 0 ? 1u : 0u);
                         tc_commit(bar_odone(t));
-                        if (j == g.num_kt - 1) tc_commit(bar_ofinal(t));
+                        if (j == it.num_kt - 1) tc_commit(bar_ofinal(t));
                     }
                     if (ok) tc_commit(bar_vempty);
                 }
-                G += g.num_kt; gk += g.num_kt; gv += g.num_kt; ++n;
-                if (g.last_partial >= 0) ++nf;
+                G += it.num_kt; gk += it.num_kt; gv += it.num_kt; ++n;
+                if (it.last_partial >= 0) ++nf;
             }
         }
     }
@@ -1096,16 +1107,14 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             if (!alive) break;
             const Tc5Item it = s_ring[n & 3];
             if (it.kind == 0) break;
-            const Tc5Geom g = tc5_geometry(p, it.seq, it.q0);
-            const int q0 = it.q0;
-            const int lim = min(g.shift + q0 + row + 1, g.k_len);
+            const int lim = min(it.lim0 + row, it.k_len);
             float m_ref = -INFINITY, l_run = 0.0f;
-            for (int j = 0; j < g.num_kt; ++j) {
+            for (int j = 0; j < it.num_kt; ++j) {
                 alive = warp_mbar_wait(bar_sfull(t), (G + j) & 1, abort_flag, 31);
                 if (!alive) break;
                 tc_fence_after();
                 const int key0 = j * kBN;
-                const bool need_mask = key0 + kBN > min(g.shift + q0 + 1, g.k_len);
+                const bool need_mask = key0 + kBN > min(it.lim0, it.k_len);
                 alive = softmax_row_to_smem<T>(t_s, t_o, p_panels, row, need_mask, key0, lim, p.scale_log2, j == 0, m_ref, l_run,
                                                bar_odone(t), (G + j - 1) & 1, abort_flag, [&] {
                                                    tc_fence_before();
@@ -1147,18 +1156,18 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 }
                 // O has left TMEM: the arrive on p_full in the next item's first round tells the issuer so
                 __syncwarp();
-                T* o0 = static_cast<T*>(p.out) + (static_cast<size_t>(g.qb + q0) * p.num_heads + 2 * it.pair + t) * kHeadDim;
+                T* o0 = static_cast<T*>(p.out) + (static_cast<size_t>(it.q_row) * p.num_heads + 2 * it.pair + t) * kHeadDim;
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
                     const int r = wq * 32 + 2 * i + (lane >> 4), chunk = lane & 15;
-                    if (r < g.rows_here) {
+                    if (r < it.rows) {
                         const uint4 v = *staged(r, chunk);
                         *reinterpret_cast<uint4*>(o0 + r * out_stride + chunk * 8) = v;
                     }
                 }
                 __syncwarp();   // the staging rows are read before the next item's probabilities overwrite them
             }
-            G += g.num_kt; ++n;
+            G += it.num_kt; ++n;
         }
     }
     tc_fence_before();
