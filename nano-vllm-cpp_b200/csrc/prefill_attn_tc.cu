@@ -1138,11 +1138,14 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 auto staged = [&](int r, int chunk) {
                     return reinterpret_cast<uint4*>(p_panels + (chunk >> 3) * kPanelBytes + r * 128 + (((chunk & 7) ^ (r & 7)) << 4));
                 };
+                uint32_t o[4][32];   // the whole row at once: one TMEM latency instead of four
+#pragma unroll
+                for (int c = 0; c < 4; ++c) tmem_ld32(t_o + c * 32, o[c]);
+                tc_wait_ld();
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    uint32_t r[32];
-                    tmem_ld32(t_o + c * 32, r);
-                    tc_wait_ld(); reg_fence32(r);
+                    reg_fence32(o[c]);
+                    const uint32_t (&r)[32] = o[c];
 #pragma unroll
                     for (int q4 = 0; q4 < 4; ++q4) {
                         uint4 v;
@@ -1157,13 +1160,13 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 // O has left TMEM: the arrive on p_full in the next item's first round tells the issuer so
                 __syncwarp();
                 T* o0 = static_cast<T*>(p.out) + (static_cast<size_t>(it.q_row) * p.num_heads + 2 * it.pair + t) * kHeadDim;
+                uint4 v[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] = *staged(wq * 32 + 2 * i + (lane >> 4), lane & 15);
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                    const int r = wq * 32 + 2 * i + (lane >> 4), chunk = lane & 15;
-                    if (r < it.rows) {
-                        const uint4 v = *staged(r, chunk);
-                        *reinterpret_cast<uint4*>(o0 + r * out_stride + chunk * 8) = v;
-                    }
+                    const int r = wq * 32 + 2 * i + (lane >> 4);
+                    if (r < it.rows) *reinterpret_cast<uint4*>(o0 + r * out_stride + (lane & 15) * 8) = v[i];
                 }
                 __syncwarp();   // the staging rows are read before the next item's probabilities overwrite them
             }
