@@ -2,7 +2,7 @@
 // by the decode kernels (decode_attn.cu) and the mixed prefill + decode kernel (prefill_attn_tc.cu).
 //
 // The op is HBM-bound: every K and V row of every context is read once.  A group of four warps takes a range of the keys of one
-// (sequence, KV head); the G = Hq / Hkv <= 8 query heads of the KV head are the rows of the MMA tile, so a K / V row is read once
+// (sequence, KV head); the G = Hq / Hkv <= 8 query heads of the KV head are the columns of the MMA tile, so a K / V row is read once
 // per KV head.  Each warp streams every fourth tile of 16 keys through a private ring of cp.async stages (no barrier in the main
 // loop); at the end the four warps merge through shared memory.
 //
@@ -67,48 +67,59 @@ __device__ __forceinline__ void lds32x4(uint32_t addr, uint32_t (&w)[4]) {
     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(addr));
 }
 
-// Online-softmax state of a warp: accumulator columns of lane (g, t) = (lane / 4, lane % 4) are heads 2t and 2t + 1; maximum and
-// sum are those of head g.
+// 8 x 8 matrix of 16-bit elements over a warp (lane (g, t): row g, columns 2t, 2t + 1), transposed.
+__device__ __forceinline__ uint32_t transpose_8x8(uint32_t a) {
+    uint32_t d;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(d) : "r"(a));
+    return d;
+}
+
+// Online-softmax state of a warp.  Lane (g, t) = (lane / 4, lane % 4) holds heads 2t and 2t + 1: columns of the accumulators, the
+// maxima (equal over g) and, over the keys that the lane has seen, the sums.
 struct SoftmaxState {
     float o[8][4];
-    float m, l;
+    float m[2], l[2];
     __device__ __forceinline__ void reset() {
 #pragma unroll
         for (int i = 0; i < 8; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f; }
-        m = -INFINITY; l = 0.0f;
+        m[0] = m[1] = -INFINITY; l[0] = l[1] = 0.0f;
     }
-    // New tile maximum: rescale where it moves (a handful of tiles of a sequence; the branch is warp-uniform).  `extra`: further
+    // Scores of a tile: rescale where a maximum moves (a handful of tiles of a sequence; the branch is warp-uniform).  `extra`: further
     // columns that are scaled along.
-    __device__ __forceinline__ void raise_max(float m_tile, int t, float* extra) {
-        m_tile = fmaxf(m_tile, __shfl_xor_sync(0xffffffffu, m_tile, 1));
-        m_tile = fmaxf(m_tile, __shfl_xor_sync(0xffffffffu, m_tile, 2));
-        if (__any_sync(0xffffffffu, m_tile > m)) {
-            const float m_new = fmaxf(m, m_tile);   // finite: the tile's first key is always valid
-            const float corr = fast_exp2(m - m_new);
-            l *= corr;
-            m = m_new;
-            const float c0 = __shfl_sync(0xffffffffu, corr, 8 * t), c1 = __shfl_sync(0xffffffffu, corr, 8 * t + 4);
+    __device__ __forceinline__ void raise_max(const float (&sc)[4], float* extra) {
+        float top[2] = {fmaxf(sc[0], sc[2]), fmaxf(sc[1], sc[3])};
+        if (__any_sync(0xffffffffu, top[0] > m[0] || top[1] > m[1])) {
+            float c[2];
 #pragma unroll
-            for (int mt = 0; mt < 8; ++mt) { o[mt][0] *= c0; o[mt][1] *= c1; o[mt][2] *= c0; o[mt][3] *= c1; }
-            if (extra != nullptr) { extra[0] *= c0; extra[1] *= c1; extra[2] *= c0; extra[3] *= c1; }
+            for (int h = 0; h < 2; ++h) {
+#pragma unroll
+                for (int x = 4; x < 32; x *= 2) top[h] = fmaxf(top[h], __shfl_xor_sync(0xffffffffu, top[h], x));
+                const float m_new = fmaxf(m[h], top[h]);   // finite: the tile's first key is always valid
+                c[h] = fast_exp2(m[h] - m_new);
+                l[h] *= c[h];
+                m[h] = m_new;
+            }
+#pragma unroll
+            for (int mt = 0; mt < 8; ++mt) { o[mt][0] *= c[0]; o[mt][1] *= c[1]; o[mt][2] *= c[0]; o[mt][3] *= c[1]; }
+            if (extra != nullptr) { extra[0] *= c[0]; extra[1] *= c[1]; extra[2] *= c[0]; extra[3] *= c[1]; }
         }
     }
 };
 
-// Keys past `valid` of a tile get no weight; only a sequence's last tile has any (warp-uniform branch).
-__device__ __forceinline__ void mask_scores(float (&sc)[4], int t, int valid) {
+// Scores of lane (g, t): keys g (sc[0], sc[1]) and g + 8 (sc[2], sc[3]), heads 2t and 2t + 1 of each.  Keys past `valid` of a tile get no
+// weight; only a sequence's last tile has any (warp-uniform branch).
+__device__ __forceinline__ void mask_scores(float (&sc)[4], int g, int valid) {
     if (valid < kTileTokens) {
-        const int tk = 2 * t;
-        if (tk >= valid) sc[0] = -INFINITY;
-        if (tk + 1 >= valid) sc[1] = -INFINITY;
-        if (tk + 8 >= valid) sc[2] = -INFINITY;
-        if (tk + 9 >= valid) sc[3] = -INFINITY;
+        if (g >= valid) sc[0] = sc[1] = -INFINITY;
+        if (g + 8 >= valid) sc[2] = sc[3] = -INFINITY;
     }
 }
 
-// 16-bit cache.  K and V tiles of 16 x 256 bytes, XOR-swizzled by row; S = Q K^T as mma.sync m16n8k16 with the (zero padded)
-// query heads as the 16 rows; O^T = V^T P^T with V^T taken straight from the row-major V tile by ldmatrix.trans, so that the
-// probability fragment of S is already in the layout the second MMA wants.
+// 16-bit cache.  K and V tiles of 16 x 256 bytes, XOR-swizzled by row; S^T = K Q^T as mma.sync m16n8k16: the 16 keys are the rows,
+// the (zero padded) query heads the 8 columns; O^T = V^T P^T with V^T taken straight from the row-major V tile by ldmatrix.trans and
+// P^T from S^T by two 8 x 8 transposes.  (Heads as the 16 rows need no transpose but twice the MMAs, half of them on padding, in a
+// chain twice as long.)  Even and odd k-steps have accumulators of their own: a step is a serial chain that few warps hide.
+// Measured: 37 sequences of up to 2048 keys 34.8 -> 33.7 us; 100 int8 ones of up to 4096, where the step is closer to the bound, 97 -> 89.
 // 8 warps per SM x 3 stages of 8 KiB: 128 KiB in flight.
 template <typename T>
 struct Cache16 {
@@ -119,7 +130,7 @@ struct Cache16 {
     static constexpr int kStages = 3;
 
     SoftmaxState s;
-    uint32_t qa[8][2];   // rows g < G of the 16-row A tile; rows 8..15 are zero
+    uint32_t qa[8][2];   // head g of the 8-column B tile; zero from head G on
 
     __device__ __forceinline__ void start(const DecodeParams& p, int b, int kvh, int lane) {
         const int g = lane >> 2, t = lane & 3;
@@ -152,24 +163,25 @@ struct Cache16 {
         }
     }
     __device__ __forceinline__ void step(const DecodeParams& p, uint32_t stage, int valid, int /*kvh*/, int lane) {
-        const int t = lane & 3;
         // ldmatrix lane addressing.  K: matrices (tok 0-7, d lo), (tok 0-7, d hi), (tok 8-15, d lo), (tok 8-15, d hi) of one
         // 16-wide k-step.  V (transposed): the same of one 16-wide d-tile.
         const int row = ((lane >> 4) << 3) + (lane & 7), sel = (lane >> 3) & 1;
         float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
-            uint32_t b0, b1, b2, b3;
-            ldmatrix_x4(b0, b1, b2, b3, stage + row * kRowBytes + (((2 * ks + sel) ^ (row & 7)) << 4));
-            mma_16816<T>(s0, qa[ks][0], 0u, qa[ks][1], 0u, b0, b1);
-            mma_16816<T>(s1, qa[ks][0], 0u, qa[ks][1], 0u, b2, b3);
+            uint32_t k0, k1, k2, k3;
+            ldmatrix_x4(k0, k1, k2, k3, stage + row * kRowBytes + (((2 * ks + sel) ^ (row & 7)) << 4));
+            mma_16816<T>(ks & 1 ? s1 : s0, k0, k2, k1, k3, qa[ks][0], qa[ks][1]);
         }
-        float sc[4] = {s0[0] * p.scale_log2, s0[1] * p.scale_log2, s1[0] * p.scale_log2, s1[1] * p.scale_log2};   // keys 2t, 2t+1, 8+2t, 9+2t
-        mask_scores(sc, t, valid);
-        s.raise_max(fmaxf(fmaxf(sc[0], sc[1]), fmaxf(sc[2], sc[3])), t, nullptr);
-        const float p0 = fast_exp2(sc[0] - s.m), p1 = fast_exp2(sc[1] - s.m), p2 = fast_exp2(sc[2] - s.m), p3 = fast_exp2(sc[3] - s.m);
-        s.l += (p0 + p1) + (p2 + p3);
-        const uint32_t pb0 = ElemTraits<T>::pack2(p0, p1), pb1 = ElemTraits<T>::pack2(p2, p3);
+        float sc[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sc[i] = (s0[i] + s1[i]) * p.scale_log2;
+        mask_scores(sc, lane >> 2, valid);
+        s.raise_max(sc, nullptr);
+        const float p0 = fast_exp2(sc[0] - s.m[0]), p1 = fast_exp2(sc[1] - s.m[1]), p2 = fast_exp2(sc[2] - s.m[0]), p3 = fast_exp2(sc[3] - s.m[1]);
+        s.l[0] += p0 + p2;
+        s.l[1] += p1 + p3;
+        const uint32_t pb0 = transpose_8x8(ElemTraits<T>::pack2(p0, p1)), pb1 = transpose_8x8(ElemTraits<T>::pack2(p2, p3));
 #pragma unroll
         for (int mt = 0; mt < 8; ++mt) {
             uint32_t a0, a1, a2, a3;
@@ -232,7 +244,7 @@ struct Cache8 {
 
     SoftmaxState s;
     float osum[4];       // sum of the (scaled, rounded) probabilities per head, from the ones-row MMA
-    float q_off;
+    float q_off[2];
     uint32_t qa[8][2];   // k-step ks = 4 q + w, positions {2t, 2t+1 | 2t+8, 2t+9} <- d = 64 q + 16 t + 4 w + {0, 1 | 2, 3}
 
     __device__ __forceinline__ void start(const DecodeParams& p, int b, int kvh, int lane) {
@@ -252,7 +264,8 @@ struct Cache8 {
         }
         qsum += __shfl_xor_sync(0xffffffffu, qsum, 1);
         qsum += __shfl_xor_sync(0xffffffffu, qsum, 2);
-        q_off = kOffset * qsum;
+        q_off[0] = kOffset * __shfl_sync(0xffffffffu, qsum, 8 * t);
+        q_off[1] = kOffset * __shfl_sync(0xffffffffu, qsum, 8 * t + 4);
         osum[0] = osum[1] = osum[2] = osum[3] = 0.0f;
         s.reset();
     }
@@ -278,16 +291,21 @@ struct Cache8 {
     }
     __device__ __forceinline__ void step(const DecodeParams& p, uint32_t stage, int valid, int kvh, int lane) {
         const int g = lane >> 2, t = lane & 3;
-        // which half of the copied word is this lane's scale: cache rows of a tile start at an even row, so the parity of row * Hkv +
-        // kvh is that of (token & Hkv & 1) + kvh
-        float scale;
+        // Scales of keys g and g + 8.  Which half of a copied word is the scale: cache rows of a tile start at an even row, so the parity of
+        // row * Hkv + kvh is that of (token & Hkv & 1) + kvh.
+        float2 kscale, vscale;
         {
-            uint32_t word;
-            asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(word) : "r"(stage + 2 * kTileBytes + lane * 4));
-            const __half2 pair = *reinterpret_cast<const __half2*>(&word);
-            scale = ((((lane & p.num_kv_heads) ^ kvh) & 1) != 0 ? __high2float(pair) : __low2float(pair)) * (lane < 16 ? p.scale_log2 : 1.0f);
+            uint32_t w[4];
+            const uint32_t at = stage + 2 * kTileBytes + g * 4;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(w[i]) : "r"(at + i * 32));
+            const uint32_t pick = (((g & p.num_kv_heads) ^ kvh) & 1) != 0 ? 0x7632u : 0x5410u;
+            const uint32_t k2 = __byte_perm(w[0], w[1], pick), v2 = __byte_perm(w[2], w[3], pick);
+            kscale = __half22float2(*reinterpret_cast<const __half2*>(&k2));
+            vscale = __half22float2(*reinterpret_cast<const __half2*>(&v2));
+            kscale.x *= p.scale_log2;
+            kscale.y *= p.scale_log2;
         }
-        // scores: keys g (n-tile 0) and g + 8 (n-tile 1)
         float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
@@ -298,20 +316,19 @@ struct Cache8 {
             for (int wi = 0; wi < 4; ++wi) {
                 const int ks = 4 * q + wi;
                 const uint32_t x0 = w0[wi] ^ kFlip, x1 = w1[wi] ^ kFlip;
-                mma_16816<__half>(s0, qa[ks][0], 0u, qa[ks][1], 0u, widen_pair_lo<FP8>(x0), widen_pair_hi<FP8>(x0));
-                mma_16816<__half>(s1, qa[ks][0], 0u, qa[ks][1], 0u, widen_pair_lo<FP8>(x1), widen_pair_hi<FP8>(x1));
+                mma_16816<__half>(ks & 1 ? s1 : s0, widen_pair_lo<FP8>(x0), widen_pair_lo<FP8>(x1), widen_pair_hi<FP8>(x0), widen_pair_hi<FP8>(x1), qa[ks][0],
+                                  qa[ks][1]);
             }
         }
-        const float ks0 = __shfl_sync(0xffffffffu, scale, 2 * t), ks1 = __shfl_sync(0xffffffffu, scale, 2 * t + 1);
-        const float ks2 = __shfl_sync(0xffffffffu, scale, 8 + 2 * t), ks3 = __shfl_sync(0xffffffffu, scale, 9 + 2 * t);
-        const float vs0 = __shfl_sync(0xffffffffu, scale, 16 + 2 * t), vs1 = __shfl_sync(0xffffffffu, scale, 17 + 2 * t);
-        const float vs2 = __shfl_sync(0xffffffffu, scale, 24 + 2 * t), vs3 = __shfl_sync(0xffffffffu, scale, 25 + 2 * t);
-        float sc[4] = {(s0[0] - q_off) * ks0, (s0[1] - q_off) * ks1, (s1[0] - q_off) * ks2, (s1[1] - q_off) * ks3};   // keys 2t, 2t+1, 8+2t, 9+2t
-        mask_scores(sc, t, valid);
-        s.raise_max(fmaxf(fmaxf(sc[0], sc[1]), fmaxf(sc[2], sc[3])), t, FP8 ? nullptr : osum);
-        const float p0 = fast_exp2(sc[0] - s.m), p1 = fast_exp2(sc[1] - s.m), p2 = fast_exp2(sc[2] - s.m), p3 = fast_exp2(sc[3] - s.m);
-        s.l += (p0 + p1) + (p2 + p3);
-        const uint32_t pb0 = ElemTraits<__half>::pack2(p0 * vs0, p1 * vs1), pb1 = ElemTraits<__half>::pack2(p2 * vs2, p3 * vs3);
+        float sc[4] = {(s0[0] + s1[0] - q_off[0]) * kscale.x, (s0[1] + s1[1] - q_off[1]) * kscale.x, (s0[2] + s1[2] - q_off[0]) * kscale.y,
+                       (s0[3] + s1[3] - q_off[1]) * kscale.y};
+        mask_scores(sc, g, valid);
+        s.raise_max(sc, FP8 ? nullptr : osum);
+        const float p0 = fast_exp2(sc[0] - s.m[0]), p1 = fast_exp2(sc[1] - s.m[1]), p2 = fast_exp2(sc[2] - s.m[0]), p3 = fast_exp2(sc[3] - s.m[1]);
+        s.l[0] += p0 + p2;
+        s.l[1] += p1 + p3;
+        const uint32_t pb0 = transpose_8x8(ElemTraits<__half>::pack2(p0 * vscale.x, p1 * vscale.x));
+        const uint32_t pb1 = transpose_8x8(ElemTraits<__half>::pack2(p2 * vscale.y, p3 * vscale.y));
         // output: V rows 2t, 2t+1, 2t+8, 2t+9, piece g (d = 16 g .. 16 g + 15)
         uint32_t v0[4], v1[4], v2[4], v3[4];
         const uint32_t vbase = stage + kTileBytes;
@@ -346,11 +363,6 @@ struct alignas(128) GroupSmem {
         } m;
     };
 };
-
-__device__ __forceinline__ float quad_sum(float v) {
-    v += __shfl_xor_sync(0xffffffffu, v, 1);
-    return v + __shfl_xor_sync(0xffffffffu, v, 2);
-}
 
 // Keys [t0, t1) of sequence b (t0 < t1), one KV head.  sink(h, d, o, m, l) takes element d = this thread of head h: unnormalised
 // output, maximum and sum.  `tid`: 0..127 inside the group, `bar_id`: its named barrier; all its threads call it.
@@ -403,10 +415,12 @@ __device__ __forceinline__ void attend_range(const DecodeParams& p, int b, int k
     cp_async_wait<0>();
     group_sync(bar_id, kGroupThreads);   // every ring is idle from here on
     const int g = lane >> 2, t = lane & 3;
-    const float l = quad_sum(st.s.l);
-    if (t == 0) sm.m.ml[warp][g] = make_float2(st.s.m, l);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
+        float l = st.s.l[h];
+#pragma unroll
+        for (int x = 4; x < 32; x *= 2) l += __shfl_xor_sync(0xffffffffu, l, x);
+        if (g == 0) sm.m.ml[warp][2 * t + h] = make_float2(st.s.m[h], l);
 #pragma unroll
         for (int i = 0; i < 16; ++i) sm.m.o[warp][2 * t + h][F::dim(g, i)] = st.value(h, i);
     }
