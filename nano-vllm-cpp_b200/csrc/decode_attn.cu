@@ -30,35 +30,61 @@ constexpr int kMaxCluster = 8;          // portable cluster size
 // pass (alone, from call to result: 17) where split and merge took 9.4 (41).
 constexpr int kClusterTokens = 512;
 
-// The sequence with the rank-th longest context (ties in index order), found by every block for itself; `keys`: kMaxSorted ints.  In
-// index order the last blocks to start can be the longest: 100 sequences of 500 to 4096 keys, int8, left half the SMs idle for the
-// last 40 of 106 us; in this order the pass takes 103 us instead of 115.  64 sequences of 100 to 2048 keys, 16-bit: 6 us less.
+// Sequence number `rank` in order of falling context length, found by every block for itself.  In index order the last blocks to start
+// can be the longest: 100 sequences of 500 to 4096 keys, int8, left half the SMs idle for the last 40 of 106 us; in this order the pass
+// takes 103 us instead of 115.  64 sequences of 100 to 2048 keys, 16-bit: 6 us less.  The order is that of 128 classes of length, and of
+// the index inside a class: a histogram, one scan and a search through the class.  (Comparing every context with every other one took
+// each block 5 us at 254 sequences: with 4 KV heads and contexts of up to 157 keys 39 us a pass.)
 constexpr int kMaxSorted = 512;
-__device__ __forceinline__ int sequence_of_rank(const DecodeParams& p, int rank, int* keys) {
-    __shared__ int found;
-    const int padded = (p.batch + 3) & ~3;
-    for (int i = threadIdx.x; i < padded; i += kGroupThreads) keys[i] = i < p.batch ? clamped_context(p, i) : -1;
+constexpr int kMinSortedTokens = 1024;   // tables of fewer keys: a block lasts hardly longer than the 1 us that this takes
+struct SortScratch { int count[128]; unsigned char cls[kMaxSorted]; };
+__device__ __forceinline__ int sequence_of_rank(const DecodeParams& p, int rank, SortScratch& sm) {
+    static_assert(kGroupThreads == 128, "one thread per class");
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int shift = max(0, 25 - __clz(static_cast<int>(p.max_blocks * p.block_size)));   // the longest context there can be is in class 127 at most
+    sm.count[tid] = 0;
     __syncthreads();
-    for (int i = threadIdx.x; i < p.batch; i += kGroupThreads) {
-        const int mine = keys[i];
-        int longer = 0;
-        for (int j = 0; j < padded; j += 4) {
-            const int4 k = *reinterpret_cast<const int4*>(keys + j);
-            longer += (k.x > mine || (k.x == mine && j < i)) + (k.y > mine || (k.y == mine && j + 1 < i)) +
-                      (k.z > mine || (k.z == mine && j + 2 < i)) + (k.w > mine || (k.w == mine && j + 3 < i));
-        }
-        if (longer == rank) found = i;
+    for (int i = tid; i < p.batch; i += kGroupThreads) {
+        const int c = 127 - (clamped_context(p, i) >> shift);
+        sm.cls[i] = static_cast<unsigned char>(c);
+        atomicAdd(&sm.count[c], 1);
     }
     __syncthreads();
-    return found;
+    // every warp finds the class (four per lane), then the sequence
+    const int4 n = reinterpret_cast<const int4*>(sm.count)[lane];
+    const int mine = n.x + n.y + n.z + n.w;
+    int upto = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d *= 2) {
+        const int up = __shfl_up_sync(0xffffffffu, upto, d);
+        if (lane >= d) upto += up;
+    }
+    const int owner = __ffs(__ballot_sync(0xffffffffu, upto > rank)) - 1;
+    int c = 4 * lane, left = rank - (upto - mine);   // (the owner's values are used)
+    if (left >= n.x) {
+        left -= n.x; ++c;
+        if (left >= n.y) {
+            left -= n.y; ++c;
+            if (left >= n.z) { left -= n.z; ++c; }
+        }
+    }
+    c = __shfl_sync(0xffffffffu, c, owner);
+    left = __shfl_sync(0xffffffffu, left, owner);
+    for (int i0 = 0;; i0 += 32) {
+        const bool in = i0 + lane < p.batch && sm.cls[i0 + lane] == c;
+        const unsigned int all = __ballot_sync(0xffffffffu, in);
+        const unsigned int hit = __ballot_sync(0xffffffffu, in && __popc(all & ((1u << lane) - 1u)) == left);
+        if (hit != 0 || i0 + 32 >= p.batch) return i0 + max(0, __ffs(hit) - 1);
+        left -= __popc(all);
+    }
 }
 
 template <class F, typename T>
 __global__ void __launch_bounds__(kGroupThreads, F::kGroups) decode_split_kernel(const __grid_constant__ DecodeParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
     pdl_wait_then_release();
-    const int b = p.longest_first ? sequence_of_rank(p, blockIdx.z, reinterpret_cast<int*>(smem)) : blockIdx.z;
-    if (p.longest_first) __syncthreads();   // (the ring takes the keys' place)
+    const int b = p.longest_first ? sequence_of_rank(p, blockIdx.z, *reinterpret_cast<SortScratch*>(smem)) : blockIdx.z;
+    if (p.longest_first) __syncthreads();   // (the ring takes the scratch's place)
     run_split<F, T>(p, b, blockIdx.x, blockIdx.y, *reinterpret_cast<GroupSmem<F>*>(smem), threadIdx.x, 1);
 }
 
@@ -196,7 +222,8 @@ int decode_plan(const DecodeArgs& a, int groups, dec::DecodeParams* out, int* cl
     p.chunk_tokens = s.chunk;
     p.num_splits = s.count;
     // whole contexts in more than one wave of blocks: the long ones first, so that the last blocks to start are short
-    p.longest_first = s.cluster == 0 && s.count == 1 && a.batch * a.num_kv_heads > static_cast<int64_t>(kSmCount) * groups && a.batch <= kMaxSorted;
+    p.longest_first = s.cluster == 0 && s.count == 1 && a.batch * a.num_kv_heads > static_cast<int64_t>(kSmCount) * groups && a.batch <= kMaxSorted &&
+                      a.max_blocks * a.block_size >= kMinSortedTokens;
     if (a.workspace != nullptr) {
         p.ws_o = static_cast<float*>(a.workspace);
         p.ws_ml = reinterpret_cast<float2*>(p.ws_o + part_count(s, a.batch, a.num_kv_heads) * p.group * kHeadDim);

@@ -25,6 +25,7 @@ def _workspace(batch, hq, hkv, blocks, bs):
     (8, 8, 32, EDGES * 3, 17),
     (8, 1, 256, [2047, 2048, 2049, 1, 9000], 80),           # chunks: up to 36 parts of one context
     (16, 8, 256, EDGES * 3 + [4096, 2500, 2048], 16),       # whole contexts, 4096-key tables
+    (8, 2, 256, [300] * 170 + EDGES * 3 + [1024], 4),       # longest first with most in one class of length
     (16, 8, 256, [4097, 8192, 5000] + EDGES * 3, 33),       # chunks: up to 5 parts
 ])
 def test_every_way_to_share_out_a_context_matches_the_oracle(hq, hkv, bs, lens, table_blocks):
