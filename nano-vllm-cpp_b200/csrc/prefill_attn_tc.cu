@@ -98,6 +98,9 @@ __device__ __forceinline__ bool warp_mbar_wait(uint32_t bar, uint32_t parity, vo
     if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, abort_flag, code) ? 1 : 0;
     return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
+    asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+}
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
     asm volatile(
         "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n"
@@ -743,8 +746,9 @@ constexpr int kIssuers5 = 2;        // issuing warps, one per query tile
 constexpr int kThreads5 = 384;      // three warpgroups (register reallocation works on whole warpgroups)
 constexpr int kRegsLow5 = 56;       // registers per thread of the third warpgroup after setmaxnreg.dec
 constexpr int kRegsHigh5 = 224;     // registers per thread of the two softmax warpgroups after setmaxnreg.inc
+// Ticket counters, zero between launches: every block takes tickets up to its first one past the end, so the launch's last ticket is known,
+// and who holds it sets the counter back.  (A counter of finished blocks is a trip to memory at the end that everything waits for: 1 us.)
 __device__ unsigned int g_prefill_ticket[kTicketSlots];
-__device__ unsigned int g_prefill_done[kTicketSlots];
 
 struct Tc5Params {
     TcParams base;
@@ -868,7 +872,11 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 dec::group_sync(bar, dec::kGroupThreads);
                 const unsigned int item = sm.item;
                 dec::group_sync(bar, dec::kGroupThreads);   // everyone holds the item before the next ticket overwrites it
-                if (item >= hkv * splits * static_cast<unsigned int>(dp.batch)) break;
+                const unsigned int total = hkv * splits * static_cast<unsigned int>(dp.batch);
+                if (item >= total) {
+                    if (gtid == 0 && item == total + Decode16::kGroups * gridDim.x - 1) g_decode_ticket[pp.slot] = 0u;
+                    break;
+                }
                 dec::run_split<Decode16, T>(dp, static_cast<int>(item / (hkv * splits)), static_cast<int>(item % hkv), static_cast<int>((item / hkv) % splits),
                                             sm.g, gtid, bar);
                 dec::group_sync(bar, dec::kGroupThreads);   // the group's shared memory is free for its next item
@@ -912,7 +920,8 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&s_tmem_base)), "r"(kTmemCols2) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
-    if (!MIXED) pdl_wait_then_release();   // barriers and TMEM are set up under the predecessor's tail
+    if (tid == 0) { prefetch_map(&tm_q); prefetch_map(&tm_k); prefetch_map(&tm_v); }
+    if (!MIXED) pdl_wait_then_release();   // barriers, TMEM and tensor maps are set up under the predecessor's tail
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -931,6 +940,10 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         int n = 0;            // items published so far (all of them carry work)
         int gk = 0, gv = 0;   // K / V tiles loaded so far, over all items
         bool ok = true;
+        // The first ticket is taken under the look at the sequence bounds.
+        unsigned int ticket = 0;
+        bool have_ticket = true;
+        if (lane == 0) ticket = atomicAdd(&g_prefill_ticket[pp.slot], 1u);
         Tc5Finder find;
         const int tiles = min(find.open(p, lane), pp.tiles);
         const unsigned int total = static_cast<unsigned int>(tiles) * static_cast<unsigned int>(pp.pairs);
@@ -938,10 +951,13 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         auto take_item = [&]() -> Tc5Item {
             Tc5Item it{};
             while (true) {
-                unsigned int ticket = 0;
-                if (lane == 0) ticket = atomicAdd(&g_prefill_ticket[pp.slot], 1u);
+                if (!have_ticket && lane == 0) ticket = atomicAdd(&g_prefill_ticket[pp.slot], 1u);
+                have_ticket = false;
                 ticket = __shfl_sync(0xffffffffu, ticket, 0);
-                if (ticket >= total) return it;
+                if (ticket >= total) {
+                    if (lane == 0 && ticket == total + gridDim.x - 1) g_prefill_ticket[pp.slot] = 0u;
+                    return it;
+                }
                 it.pair = static_cast<int>(ticket % static_cast<unsigned int>(pp.pairs));
                 find.find(p, lane, tiles - 1 - static_cast<int>(ticket / static_cast<unsigned int>(pp.pairs)), it);
                 if (it.num_kt > 0) break;
@@ -954,8 +970,9 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 }
             }
             it.kind = 1;
-            it.row0 = tc5_key_row(p, it.seq, it.k_row, 0);
-            it.row1 = it.num_kt > 1 ? tc5_key_row(p, it.seq, it.k_row, kBN) : 0;
+            const int row = lane < 2 && lane < it.num_kt ? tc5_key_row(p, it.seq, it.k_row, lane * kBN) : 0;   // (both trips at once)
+            it.row0 = __shfl_sync(0xffffffffu, row, 0);
+            it.row1 = __shfl_sync(0xffffffffu, row, 1);
             return it;
         };
         Tc5Item next = take_item();
@@ -1022,6 +1039,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             }
             gk += it.num_kt; gv += it.num_kt; ++n;
         }
+        while (!ok && next.kind) next = take_item();   // a wait gave up: the tickets are still taken to the end
     } else if (warp == 8 || warp == 8 + 2 * (kIssuers5 - 1)) {
         // ------------------------------------------------------------------ MMA issuer(s): with two, warp 8 drives
         // tile 0 and warp 10 tile 1 (one thread sustains about one MMA per 100 clocks here, the tensor pipe one per 64)
@@ -1179,16 +1197,9 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kTmemCols2) : "memory");
     }
     if (MIXED && !decode_first) decode_half();
-    if (MIXED) __syncthreads();
-    if (tid == 0) {   // the last block to finish re-arms the ticket counters for the next launch that uses this slot
-        __threadfence();
-        if (atomicAdd(&g_prefill_done[pp.slot], 1u) == gridDim.x - 1) {
-            g_prefill_ticket[pp.slot] = 0u;
-            g_decode_ticket[pp.slot] = 0u;
-            g_prefill_done[pp.slot] = 0u;
-            __threadfence();
-        }
-    }
+    // Nothing needs this fence, but grids of several items per block measure faster with it (16 x 2048 tokens 618 -> 603 us, 2 x 8192
+    // 953 -> 946, on every box; the compiled loops are others).  For one item a block it would only add 0.5 us.
+    if (tid == 0 && pp.total > gridDim.x) __threadfence();
 }
 
 // ---- host side ------------------------------------------------------------------------------------------
