@@ -83,9 +83,10 @@ template <class F, typename T>
 __global__ void __launch_bounds__(kGroupThreads, F::kGroups) decode_split_kernel(const __grid_constant__ DecodeParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
     pdl_wait_then_release();
-    const int b = p.longest_first ? sequence_of_rank(p, blockIdx.z, *reinterpret_cast<SortScratch*>(smem)) : blockIdx.z;
+    const int rank = p.chunk_major ? blockIdx.y : blockIdx.z, split = p.chunk_major ? blockIdx.z : blockIdx.y;
+    const int b = p.longest_first ? sequence_of_rank(p, rank, *reinterpret_cast<SortScratch*>(smem)) : rank;
     if (p.longest_first) __syncthreads();   // (the ring takes the scratch's place)
-    run_split<F, T>(p, b, blockIdx.x, blockIdx.y, *reinterpret_cast<GroupSmem<F>*>(smem), threadIdx.x, 1);
+    run_split<F, T>(p, b, blockIdx.x, split, *reinterpret_cast<GroupSmem<F>*>(smem), threadIdx.x, 1);
 }
 
 // HG > 0: one warp per (sequence, KV head), HG heads at a time, in blocks of kMergeBlockWarps warps, small enough to be resident
@@ -224,6 +225,12 @@ int decode_plan(const DecodeArgs& a, int groups, dec::DecodeParams* out, int* cl
     // whole contexts in more than one wave of blocks: the long ones first, so that the last blocks to start are short
     p.longest_first = s.cluster == 0 && s.count == 1 && a.batch * a.num_kv_heads > static_cast<int64_t>(kSmCount) * groups && a.batch <= kMaxSorted &&
                       a.max_blocks * a.block_size >= kMinSortedTokens;
+    // Contexts shorter than the table leave chunks without keys, whose blocks exit at once.  With sequence after sequence they lie between
+    // the blocks with work, and these pile up on the SMs where the empty ones were quickest gone; chunk after chunk the ones with
+    // work come first and spread evenly (us a call: 2 int8 sequences of 3000 keys, 8 KV heads, 32768-key tables, 21.4 -> 14.4; 37 of 1000
+    // keys 31.2 -> 23.6; 64 of 9000 keys, 10240-key tables, 200.8 -> 190.2; 24 16-bit ones of 300 keys 15.3 -> 10.4).  From two waves of 16-bit
+    // blocks on HBM is the bound and the empty ones cost least among the others (128 of 1000 keys: 82.5, chunk after chunk 92.8).
+    p.chunk_major = groups == 3 || a.batch * a.num_kv_heads < 2 * static_cast<int64_t>(kSmCount) * groups;
     if (a.workspace != nullptr) {
         p.ws_o = static_cast<float*>(a.workspace);
         p.ws_ml = reinterpret_cast<float2*>(p.ws_o + part_count(s, a.batch, a.num_kv_heads) * p.group * kHeadDim);
@@ -285,7 +292,8 @@ int launch_typed(const DecodeArgs& a, const void* k_scale, const void* v_scale) 
         return check_launch("decode_cluster_kernel launch");
     }
     if (a.batch > 65535 || p.num_splits > 65535) return fail(NVK_ERR_UNSUPPORTED, "decode attention: batch or split count exceeds grid limits");
-    const dim3 grid(a.num_kv_heads, p.num_splits, static_cast<unsigned>(a.batch));
+    const unsigned batch = static_cast<unsigned>(a.batch), splits = static_cast<unsigned>(p.num_splits);
+    const dim3 grid = p.chunk_major ? dim3(a.num_kv_heads, batch, splits) : dim3(a.num_kv_heads, splits, batch);
     const cudaError_t e = launch_pdl(decode_split_kernel<F, T>, grid, dim3(kGroupThreads), kSmem, a.stream, p);
     if (e != cudaSuccess) return fail(NVK_ERR_CUDA, "decode_split_kernel launch: %s", cudaGetErrorString(e));
     const int rc2 = check_launch("decode_split_kernel launch");

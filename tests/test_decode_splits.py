@@ -27,6 +27,8 @@ def _workspace(batch, hq, hkv, blocks, bs):
     (16, 8, 256, EDGES * 3 + [4096, 2500, 2048], 16),       # whole contexts, 4096-key tables
     (8, 2, 256, [300] * 170 + EDGES * 3 + [1024], 4),       # longest first with most in one class of length
     (16, 8, 256, [4097, 8192, 5000] + EDGES * 3, 33),       # chunks: up to 5 parts
+    (16, 8, 256, [300, 0, 2500, 17], 128),                  # most chunks empty, chunk after chunk
+    (8, 8, 256, EDGES * 5, 20),                             # most chunks empty, sequence after sequence
 ])
 def test_every_way_to_share_out_a_context_matches_the_oracle(hq, hkv, bs, lens, table_blocks):
     w = workloads().make_decode_workload(len(lens), hq, hkv, 128, bs, 0, 0, seed=len(lens) + hq, context_lens=np.array(lens, np.int32),
@@ -41,7 +43,7 @@ def test_every_way_to_share_out_a_context_matches_the_oracle(hq, hkv, bs, lens, 
 
 
 @pytest.mark.parametrize("fmt", ["int8", "fp8"])
-@pytest.mark.parametrize("hq,hkv,lens,table_blocks", [(8, 2, [300, 17], 2), (16, 8, EDGES * 4, 3), (8, 1, [5000, 1, 2049], 40)])
+@pytest.mark.parametrize("hq,hkv,lens,table_blocks", [(8, 2, [300, 17], 2), (16, 8, EDGES * 4, 3), (8, 1, [5000, 1, 2049], 40), (8, 8, EDGES * 4, 20)])
 def test_8_bit_caches_do_not_depend_on_how_a_context_is_shared_out(fmt, hq, hkv, lens, table_blocks):
     w = workloads().make_decode_workload(len(lens), hq, hkv, 128, 256, 0, 0, seed=5, context_lens=np.array(lens, np.int32), pad_blocks_to=table_blocks)
     bf, lib = torch.bfloat16, nvk()
