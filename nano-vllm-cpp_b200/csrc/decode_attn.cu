@@ -91,7 +91,11 @@ __global__ void __launch_bounds__(kGroupThreads, F::kGroups) decode_split_kernel
 
 // HG > 0: one warp per (sequence, KV head), HG heads at a time, in blocks of kMergeBlockWarps warps, small enough to be resident
 // beside the blocks of decode_split_kernel.  HG == 0: one block per (sequence, head), where there can be more parts than one warp
-// should add up: 3 sequences of up to 40000 keys left 12 blocks adding up 20 parts each one after the other, 10 us.
+// should add up: 3 sequences of up to 40000 keys left 12 blocks adding up 20 parts each one after the other, 10 us.  These blocks do not
+// fit beside those of decode_split_kernel, so that many of them only queue up behind it.  By warps -> by blocks, us a call: 32 rows of 75
+// parts 18.3 -> 14.3, 128 rows of 64 157.1 -> 155.4, 256 of 64 160.4 -> 157.1; but 512 rows of which none has a second part 10.5 -> 11.2,
+// 4096 such rows 45.0 -> 50.8, 4096 rows of 2 parts in 32768-key tables 230 -> 244.
+constexpr int kMergeBlockRows = 2 * kSmCount;
 constexpr int kMergeBlockWarps = 2;
 template <typename T, int HG>
 __global__ void __launch_bounds__((HG > 0 ? kMergeBlockWarps : kMergeWarps) * 32) decode_merge_kernel(const __grid_constant__ DecodeParams p) {
@@ -245,7 +249,7 @@ template <typename T>
 int launch_merge_typed(const dec::DecodeParams& p, cudaStream_t stream) {
     if (p.num_splits <= 1) return NVK_OK;
     cudaError_t e;
-    if (p.num_splits > kMergeWarps) {
+    if (p.num_splits > kMergeWarps && p.batch * p.num_heads <= kMergeBlockRows) {
         e = launch_pdl(decode_merge_kernel<T, 0>, dim3(p.batch * p.num_heads), dim3(kMergeWarps * 32), 0, stream, p);
     } else {
         const dim3 grid((p.batch * p.num_kv_heads + kMergeBlockWarps - 1) / kMergeBlockWarps), block(kMergeBlockWarps * 32);

@@ -28,6 +28,8 @@ def _workspace(batch, hq, hkv, blocks, bs):
     (8, 2, 256, [300] * 170 + EDGES * 3 + [1024], 4),       # longest first with most in one class of length
     (16, 8, 256, [4097, 8192, 5000] + EDGES * 3, 33),       # chunks: up to 5 parts
     (16, 8, 256, [300, 0, 2500, 17], 128),                  # most chunks empty, chunk after chunk
+    (8, 1, 256, [300, 17, 9000] + [40] * 34, 80),           # merged by a block per head, 296 rows
+    (8, 1, 256, [300, 17, 9000] + [40] * 35, 80),           # and by warps, 304
     (8, 8, 256, EDGES * 5, 20),                             # most chunks empty, sequence after sequence
 ])
 def test_every_way_to_share_out_a_context_matches_the_oracle(hq, hkv, bs, lens, table_blocks):
