@@ -155,14 +155,21 @@ __global__ void __launch_bounds__(kGroupThreads, F::kGroups) decode_cluster_kern
 
 // ---- host side -----------------------------------------------------------------------------------------------------------
 
-// Blocks per (sequence, KV head) of the cluster kernel, or 0: chunks.  As many as are resident at once; without a workspace there is
-// nothing else.  `groups`: resident groups per SM.
+// Blocks per (sequence, KV head) of the cluster kernel, or 0: chunks.  Only clusters that are all resident at once: a cluster has to fit
+// into one GPC, so that these are fewer than the places for single blocks (the driver's occupancy query for these kernels at two and
+// three blocks per SM).  With one more a second wave follows: clusters of 4, 1024 keys, 70 -> 72 pairs 11.0 -> 15.6 us a call, clusters of
+// 8, 300 keys, 32 -> 34 pairs 5.8 -> 9.4 (in one block each 5.7).  Clusters of 2 gain nothing on whole contexts in one block each (80 pairs of
+// 300 / 1024 keys 8.5 / 12.2 us, 6.6 / 11.8), nor do clusters of 4 in tables of up to 512 keys (64 pairs of 300 / 512 keys 7.6 / 8.7, 6.4 / 7.8).
+// Without a workspace there is nothing else, and any cluster that fits is taken.
 int cluster_size(int64_t batch, int num_kv_heads, int64_t max_blocks, int block_size, int groups, bool have_workspace) {
-    const int64_t pairs = batch * num_kv_heads, resident = static_cast<int64_t>(kSmCount) * groups;
-    int c = 1;
-    while (c < kMaxCluster && pairs * c * 2 <= resident) c *= 2;
-    if (!have_workspace) return c;
-    return pairs <= resident && max_blocks * block_size <= static_cast<int64_t>(kClusterTokens) * c ? c : 0;
+    struct { int size, resident[2]; } constexpr kWays[] = {{8, {33, 48}}, {4, {71, 104}}, {2, {148, 222}}};
+    const int64_t pairs = batch * num_kv_heads, max_tokens = max_blocks * block_size;
+    for (const auto& w : kWays) {
+        if (pairs > w.resident[groups == 3]) continue;
+        if (!have_workspace) return w.size;
+        return w.size > 2 && max_tokens <= static_cast<int64_t>(kClusterTokens) * w.size && (w.size == 8 || max_tokens > kClusterTokens) ? w.size : 0;
+    }
+    return have_workspace ? 0 : 1;
 }
 
 // Chunk length in keys (whole cache blocks).  Contexts of tables of up to 4096 keys stay whole once there is one per resident group:

@@ -23,6 +23,11 @@ def _workspace(batch, hq, hkv, blocks, bs):
     (16, 8, 16, EDGES[:9], 9),                              # four, two and one
     (4, 4, 256, EDGES, 3),
     (8, 8, 32, EDGES * 3, 17),
+    (4, 1, 256, (EDGES * 3)[:33], 3),                       # as many clusters of eight as are resident, and one more
+    (4, 1, 256, (EDGES * 3)[:34], 3),
+    (4, 1, 256, (EDGES * 5)[:71], 4),                       # the same for clusters of four
+    (4, 1, 256, (EDGES * 5)[:72], 4),
+    (4, 1, 256, (EDGES[:12] * 4)[:40], 2),                  # tables of 512 keys in one block each
     (8, 1, 256, [2047, 2048, 2049, 1, 9000], 80),           # chunks: up to 36 parts of one context
     (16, 8, 256, EDGES * 3 + [4096, 2500, 2048], 16),       # whole contexts, 4096-key tables
     (8, 2, 256, [300] * 170 + EDGES * 3 + [1024], 4),       # longest first with most in one class of length
