@@ -172,15 +172,33 @@ int cluster_size(int64_t batch, int num_kv_heads, int64_t max_blocks, int block_
     return have_workspace ? 0 : 1;
 }
 
-// Chunk length in keys (whole cache blocks).  Contexts of tables of up to 4096 keys stay whole once there is one per resident group:
-// no merge (2 us of 37 at 37 sequences of 100 to 2048 keys, 8 KV heads), and taken longest first they balance each other.  Otherwise
-// 2048, or less, down to 256, where that leaves resident groups without a block.  (Whole contexts of 8192-key tables, 256 sequences:
-// 694 us a pass, 689 with chunks.)
+// A grid just past a full wave of resident groups: its last blocks run almost alone, and nothing balances equal ones.
+bool just_past_a_wave(int64_t pairs, int groups) { return pairs > kSmCount * groups && 3 * pairs < 4 * kSmCount * groups; }
+
+// Chunk length in keys (whole cache blocks), from the number of (sequence, KV head) pairs and the table's width; us a call below.
+// Whole contexts: no merge, no second launch.
+//   * Tables of up to 1024 keys: 176 pairs of 1024 keys 19.3, as two chunks 23.7; 264 24.6, 29.1; 432 int8 ones 24.3, 30.5.  But 8-bit
+//     caches with 1.5 to 2 pairs per SM, 264 int8 ones of 1024 keys / of 100 to 1024: 22.3 / 19.6, in two chunks 22.9 / 17.6.
+//   * Tables of up to 4096 keys with a pair for every resident group: 37 sequences of 100 to 2048 keys, 8 KV heads, 2 of 37; but not just past
+//     a wave: 304 / 352 pairs of 4096 keys 116.8 / 123.7, in chunks of 2048 106.1 / 113.5 (384 pairs 126.2, 121.9; 448 137.0, 145.8).
+// Chunks of 2048 otherwise, halved down to 256 while they leave resident groups without a block.
+//   * A table that 2048 keys cover is cut only below 1.5 (8-bit: 2.5) pairs per SM: 264 pairs of 2048 keys 44.7 whole, 48.5 cut; 432 int8 ones
+//     43.8, 47.5; but 328 int8 ones of 100 to 2048 keys 35.1, 28.7.  What is cut is cut no finer than it takes to have 1.5 blocks per SM
+//     (8-bit: 2.25 of 512 keys): 72 pairs of 2048 keys 4 parts 18.2, 8 21.4; 144 2 parts 29.8, 4 32.2; 106 e4m3 ones 4 parts 17.8, 8 22.6.
+//   * Longer ones need every place filled, since contexts are often shorter than the table (64 pairs of 1000 keys, 4096-key tables: 512-key
+//     chunks 12.0, 1024-key ones 14.9), but 512 keys are not cut for the last few (36 pairs of 4096 keys 19.0, as chunks of 256 21.0).
+// (Whole contexts of 8192-key tables, 256 sequences: 694 us a pass, 689 with chunks.)
 int chunk_tokens(int64_t batch, int num_kv_heads, int64_t max_blocks, int block_size, int groups) {
     const int64_t max_tokens = max_blocks * block_size, pairs = batch * num_kv_heads, resident = static_cast<int64_t>(kSmCount) * groups;
-    if (max_tokens <= 4096 && pairs >= resident) return static_cast<int>(max_tokens);
+    if (max_tokens <= 1024 && (groups == 2 || 2 * pairs <= 3 * kSmCount || pairs >= 2 * kSmCount)) return static_cast<int>(max_tokens);
+    if (max_tokens <= 4096 && pairs >= resident && !just_past_a_wave(pairs, groups)) return static_cast<int>(max_tokens);
     int64_t chunk = 2048;
-    while (chunk > 256 && pairs * ((max_tokens + chunk - 1) / chunk) < resident) chunk >>= 1;
+    for (; chunk > 256; chunk >>= 1) {
+        const int64_t parts = (max_tokens + chunk - 1) / chunk;
+        const double blocks_per_sm = groups == 2 ? (max_tokens <= 2048 ? 1.5 : chunk <= 512 ? 1.8 : 2.0)
+                                                 : (parts == 1 ? 2.5 : max_tokens <= 2048 && chunk <= 512 ? 2.25 : 3.0);
+        if (static_cast<double>(pairs * parts) >= blocks_per_sm * kSmCount) break;
+    }
     chunk = (chunk + block_size - 1) / block_size * block_size;
     return static_cast<int>(chunk < max_tokens ? chunk : max_tokens);
 }
@@ -233,9 +251,10 @@ int decode_plan(const DecodeArgs& a, int groups, dec::DecodeParams* out, int* cl
     p.per_seq = s.cluster > 0 ? 1 : 0;
     p.chunk_tokens = s.chunk;
     p.num_splits = s.count;
-    // whole contexts in more than one wave of blocks: the long ones first, so that the last blocks to start are short
-    p.longest_first = s.cluster == 0 && s.count == 1 && a.batch * a.num_kv_heads > static_cast<int64_t>(kSmCount) * groups && a.batch <= kMaxSorted &&
-                      a.max_blocks * a.block_size >= kMinSortedTokens;
+    // More than one wave of blocks: the long contexts first, so that the last blocks to start are short.  Contexts in a few chunks as well:
+    // 38 / 48 sequences of 500 / 2000 to 4096 keys, 8 KV heads, 65.4 / 96.6 -> 58.7 / 92.7 us a call (whole 59.8 / 90.4).
+    p.longest_first = s.cluster == 0 && (s.count == 1 || a.max_blocks * a.block_size <= 4096) && a.batch * a.num_kv_heads > static_cast<int64_t>(kSmCount) * groups &&
+                      a.batch <= kMaxSorted && a.max_blocks * a.block_size >= kMinSortedTokens;
     // Contexts shorter than the table leave chunks without keys, whose blocks exit at once.  With sequence after sequence they lie between
     // the blocks with work, and these pile up on the SMs where the empty ones were quickest gone; chunk after chunk the ones with
     // work come first and spread evenly (us a call: 2 int8 sequences of 3000 keys, 8 KV heads, 32768-key tables, 21.4 -> 14.4; 37 of 1000

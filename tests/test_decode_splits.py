@@ -29,7 +29,10 @@ def _workspace(batch, hq, hkv, blocks, bs):
     (4, 1, 256, (EDGES * 5)[:72], 4),
     (4, 1, 256, (EDGES[:12] * 4)[:40], 2),                  # tables of 512 keys in one block each
     (8, 1, 256, [2047, 2048, 2049, 1, 9000], 80),           # chunks: up to 36 parts of one context
-    (16, 8, 256, EDGES * 3 + [4096, 2500, 2048], 16),       # whole contexts, 4096-key tables
+    (16, 8, 256, EDGES * 3 + [4096, 2500, 2048], 16),       # 4096-key tables just past a wave: chunks, longest first
+    (16, 8, 256, EDGES * 3 + [4096, 2500, 2048, 9, 99], 16),   # and whole contexts
+    (4, 1, 256, (EDGES * 15)[:221] + [2048], 8),            # 2048-key tables, whole
+    (4, 1, 256, (EDGES * 15)[:220] + [2048], 8),            # and in two chunks
     (8, 2, 256, [300] * 170 + EDGES * 3 + [1024], 4),       # longest first with most in one class of length
     (16, 8, 256, [4097, 8192, 5000] + EDGES * 3, 33),       # chunks: up to 5 parts
     (16, 8, 256, [300, 0, 2500, 17], 128),                  # most chunks empty, chunk after chunk
@@ -50,7 +53,8 @@ def test_every_way_to_share_out_a_context_matches_the_oracle(hq, hkv, bs, lens, 
 
 
 @pytest.mark.parametrize("fmt", ["int8", "fp8"])
-@pytest.mark.parametrize("hq,hkv,lens,table_blocks", [(8, 2, [300, 17], 2), (16, 8, EDGES * 4, 3), (8, 1, [5000, 1, 2049], 40), (8, 8, EDGES * 4, 20)])
+@pytest.mark.parametrize("hq,hkv,lens,table_blocks", [(8, 2, [300, 17], 2), (16, 8, EDGES * 4, 3), (8, 1, [5000, 1, 2049], 40), (8, 8, EDGES * 4, 20),
+                                                     (4, 1, (EDGES * 18)[:263] + [1024], 4), (4, 1, (EDGES * 25)[:369] + [2048], 8)])
 def test_8_bit_caches_do_not_depend_on_how_a_context_is_shared_out(fmt, hq, hkv, lens, table_blocks):
     w = workloads().make_decode_workload(len(lens), hq, hkv, 128, 256, 0, 0, seed=5, context_lens=np.array(lens, np.int32), pad_blocks_to=table_blocks)
     bf, lib = torch.bfloat16, nvk()
