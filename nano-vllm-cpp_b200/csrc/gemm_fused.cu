@@ -476,6 +476,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     const int rank = static_cast<int>(blockIdx.x) % splits, nt = static_cast<int>(blockIdx.x) / splits;
     const int n0 = nt * kBN, m0 = blockIdx.y * (MT * kBM);
     const int rows = static_cast<int>(min(static_cast<int64_t>(MT * kBM), p.m - m0));   // of the tile that are in C
+    // A block with all of K has nothing to add up: TMEM straight to the result, unless a tile of few rows would leave three of four epilogue
+    // warps idle (us: 4096 columns, K 128, 128 rows 5.5 -> 4.0, 8 rows 3.2 -> 3.7).
+    const bool direct = splits == 1 && rows > 32;
     const int kb_all = static_cast<int>((p.k + kBK - 1) / kBK);
     const int kb0 = kb_all * rank / splits, kb_count = kb_all * (rank + 1) / splits - kb0;
 
@@ -538,7 +541,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         if (lane == 0) ok = mbar_wait(bar_acc, 0, abort_flag, 3);
         ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
         tc_fence_after();
-        if (ok) {
+        if (ok && direct) {
+            unsigned char* stage = smem_raw + (smem_base - smem_u32(smem_raw)) + kStageOffset + (warp - 2) * 4096;
+#pragma unroll 1
+            for (int t = 0; t < MT; ++t)
+                if (t * kBM + wq * 32 < rows)
+                    epilogue_row<T, EPI>(p, tmem_base + (static_cast<uint32_t>(wq * 32) << 16) + t * kBN, m0 + t * kBM + wq * 32 + lane, nt, stage, lane);
+        } else if (ok) {
 #pragma unroll 1
             for (int c = 0; c < MT * 4; ++c) {
                 if ((c >> 2) * kBM + wq * 32 >= rows) break;   // (warp-uniform: no row of this warp is in C)
@@ -559,6 +568,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     if (warp == 1) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
     }
+    if (direct) return;
     // ---------------------------------------------------------------------- sum over the cluster and epilogue
     const int sub = lane & 7;
     int q = warp * 4;                      // four rows per warp and trip
@@ -734,26 +744,29 @@ uint32_t make_idesc(bool bf16, int m, int n) {   // kind::f16: D = F32, A / B = 
     return (1u << 4) | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
 }
 
-// Kernel and shape for a size, by what the slowest SM does: waves of blocks times steps of 64 along K, plus a fixed part.  The
-// microseconds are measured (1 to 7440 rows, 768 to 6144 columns, K 4096).  A step of a 128 x 128 tile takes 0.30 us, of a 256 x 128
-// one 0.43: 32 and 48 KiB out of L2, the bound here, not the tensor pipe; a 256 x 256 tile of a pair, with 32 KiB per SM, 0.37.
-// The launch, the first loads and the epilogue take 5 us, the sum over a cluster 1 to 2 more, 4 to 6 with twice the rows.
+// Kernel and shape for a size, by what the slowest SM does: waves of blocks times (steps of 64 along K and a fixed part).  The microseconds
+// are fitted to all nine ways at 8 to 7440 rows x 768 to 12288 columns, K 128 to 4096 (replayed graphs over weights larger than L2).  A step
+// costs 32 or 48 KiB out of L2, the bound here, not the tensor pipe (32 KiB per SM for a pair's 256 x 256 tile).  The fixed part (launch, first
+// loads, epilogue; with the sum over the cluster also in proportion to the tile's rows) comes with every wave of blocks, that of a
+// pair's tile is hidden but for the epilogue.  (One fixed part whatever the waves, measured at K 4096 only, took 256-row blocks for
+// 1500 x 4096, K 512: 21.6 us, pairs 12.3.)  One rule for all epilogues, so that they round the same sums: its constants lie between
+// the plain ones (choice within 1 % of the fastest on average, 12 % at most) and those of the slower QKV epilogue (2 %, but 30 % where K is 512).
 struct GemmShape { int mt, splits; };   // mt 1 or 2: gemm_split_kernel; 0: gemm_pair_kernel
 GemmShape choose_gemm(int64_t m, int64_t n, int64_t k) {
-    // clusters of such blocks that a B200 holds at once (its GPCs have 16 to 20 SMs)
-    struct { int splits, clusters; double fixed[2]; } constexpr kWays[] = {{1, 148, {5.0, 5.0}}, {2, 74, {6.0, 9.0}}, {4, 33, {7.0, 11.0}}, {8, 15, {7.0, 11.0}}};
-    const int64_t kb = (k + kBK - 1) / kBK, tiles_n = n / kBN;
-    const int64_t pair_tiles = ((m + 255) / 256) * ((n + 255) / 256);
+    // clusters: what a B200 holds at once (its GPCs have 16 to 20 SMs); rows: per 128 rows of a tile
+    struct { int mt, splits, clusters; double step, fixed, rows; } constexpr kWays[] = {
+        {1, 1, 148, 0.286, 4.1, 0.6}, {1, 2, 74, 0.307, 3.7, 2.5}, {1, 4, 33, 0.35, 3.7, 3.4}, {1, 8, 15, 0.46, 3.3, 4.4},
+        {2, 1, 148, 0.387, 6.1, 0.7}, {2, 2, 74, 0.395, 5.4, 1.9}, {2, 4, 33, 0.42, 7.0, 1.5}, {2, 8, 15, 0.457, 8.0, 2.3}};
+    const int64_t kb = (k + kBK - 1) / kBK, tiles_n = n / kBN, pair_tiles = ((m + 255) / 256) * ((n + 255) / 256);
     GemmShape best{0, 1};
-    double best_time = m > kBM ? static_cast<double>((pair_tiles + 73) / 74 * kb) * 0.37 + 6.0 : 1e30;
-    for (int mt = 1; mt <= 2; ++mt) {
-        if (mt == 2 && m <= kBM) break;
-        const int64_t tiles = (m + mt * kBM - 1) / (mt * kBM) * tiles_n;
-        for (const auto& w : kWays) {
-            if (w.splits > 1 && (kb / w.splits < 4 || tiles > w.clusters)) break;
-            const double time = static_cast<double>((tiles + w.clusters - 1) / w.clusters * ((kb + w.splits - 1) / w.splits)) * (mt == 1 ? 0.30 : 0.43) + w.fixed[mt - 1];
-            if (time < best_time) { best_time = time; best = GemmShape{mt, w.splits}; }
-        }
+    double best_time = m > kBM ? static_cast<double>((pair_tiles + 73) / 74) * (static_cast<double>(kb) * 0.31 + 3.0) + 4.7 : 1e30;
+    for (const auto& w : kWays) {
+        const int64_t tile_rows = w.mt * kBM, tiles = (m + tile_rows - 1) / tile_rows * tiles_n;
+        if ((w.mt == 2 && m <= kBM) || (w.splits > 1 && (kb / w.splits < 2 || tiles > w.clusters))) continue;
+        const double rows = static_cast<double>(m < tile_rows ? m : tile_rows) / kBM;
+        const double time = static_cast<double>((tiles + w.clusters - 1) / w.clusters) *
+                            (static_cast<double>((kb + w.splits - 1) / w.splits) * w.step + w.fixed + w.rows * rows);
+        if (time < best_time) { best_time = time; best = GemmShape{w.mt, w.splits}; }
     }
     return best;
 }

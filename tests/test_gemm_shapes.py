@@ -14,6 +14,7 @@ torch = pytest.importorskip("torch")
 @pytest.mark.parametrize("rows,out_features,in_features", [
     (1, 128, 8), (8, 768, 4096), (9, 768, 1032), (64, 4096, 1024), (128, 6144, 520), (129, 768, 4096), (200, 6144, 512), (256, 2048, 2048),
     (257, 4096, 512), (500, 6144, 512), (513, 9472, 128), (1030, 1408, 264), (3000, 384, 2048), (5000, 4096, 72),
+    (32, 4096, 128), (33, 4096, 128), (97, 12288, 256), (161, 6144, 256), (700, 512, 64),          # blocks with all of K, few rows and many
 ])
 def test_linear_at_tile_edges(dtype, rows, out_features, in_features):
     gen = torch.Generator(device="cuda").manual_seed(rows + out_features)
