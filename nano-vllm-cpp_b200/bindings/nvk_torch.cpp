@@ -32,6 +32,17 @@ void check(int rc) {
     throw Raised{};
 }
 
+// One call of the library, with the interpreter free for other threads meanwhile: a launch blocks while the queue is full, and in a process
+// with a thread per rank the one that would launch what the GPU is waiting for must not wait for this one.  (The arguments are
+// evaluated before.)
+template <typename... P, typename... A> void launch(int (*function)(P...), A... args) {
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = function(args...);
+    Py_END_ALLOW_THREADS
+    check(rc);
+}
+
 int code(const at::Tensor& t) {
     switch (t.scalar_type()) {
         case at::kHalf: return NVK_F16;
@@ -116,7 +127,7 @@ long store_kvcache(PyObject* const* a) {
     const int64_t row = key.numel() / n;
     const int64_t cache_rows = rows_of(kc, row);
     if (kc.numel() % row != 0 || kc.numel() != vc.numel()) raise(PyExc_ValueError, "%s", "k_cache does not contain an integer number of cache rows");
-    check(nvk_store_kvcache(ptr(key), ptr(value), ptr(kc), ptr(vc), ptr(slots), code(slots), n, row, cache_rows, code(key), stream()));
+    launch(nvk_store_kvcache, ptr(key), ptr(value), ptr(kc), ptr(vc), ptr(slots), code(slots), n, row, cache_rows, code(key), stream());
     return 1;
 }
 
@@ -127,10 +138,10 @@ long fused_split_norm_rope_store(PyObject* const* a) {
                      &vc = cuda("v_cache", a[8]), &q_out = cuda("q_out", a[12]);
     const at::Tensor *qw = optional_cuda("q_norm_weight", a[2]), *kw = optional_cuda("k_norm_weight", a[3]), *slots = optional_cuda("slot_mapping", a[6]);
     const int64_t hq = integer(a[9]), hkv = integer(a[10]), d = integer(a[11]);
-    check(nvk_fused_split_norm_rope_store(ptr(qkv), static_cast<const int32_t*>(ptr(pos)), ptr(qw), ptr(kw), real(a[4]),
-                                          static_cast<const float*>(ptr(table)), size(table, 0, "cos_sin_cache"), static_cast<const int32_t*>(ptr(slots)),
-                                          ptr(kc), ptr(vc), rows_of(kc, hkv * d), size(qkv, 0, "qkv"), static_cast<int>(hq), static_cast<int>(hkv),
-                                          static_cast<int>(d), ptr(q_out), code(qkv), stream()));
+    launch(nvk_fused_split_norm_rope_store, ptr(qkv), static_cast<const int32_t*>(ptr(pos)), ptr(qw), ptr(kw), real(a[4]),
+                                            static_cast<const float*>(ptr(table)), size(table, 0, "cos_sin_cache"), static_cast<const int32_t*>(ptr(slots)),
+                                            ptr(kc), ptr(vc), rows_of(kc, hkv * d), size(qkv, 0, "qkv"), static_cast<int>(hq), static_cast<int>(hkv),
+                                            static_cast<int>(d), ptr(q_out), code(qkv), stream());
     return 1;
 }
 
@@ -156,18 +167,18 @@ struct Decode {
 long decode(PyObject* const* a) {
     const Decode x(a[0], a[1], a[2], a[3], a[4], a[9], a[5], a[6], a[7], a[8]);
     const at::Tensor* ws = optional("workspace", a[10]);
-    check(nvk_decode_attention_paged(ptr(x.q), ptr(x.kc), ptr(x.vc), x.lens.p, x.lens.dtype, x.tables.p, x.tables.dtype, x.batch, x.max_blocks,
-                                     x.blocks, static_cast<int>(x.heads), static_cast<int>(x.hkv), static_cast<int>(x.d), static_cast<int>(x.bs),
-                                     x.scale, ptr(x.out), code(x.q), ptr(ws), bytes(ws), stream()));
+    launch(nvk_decode_attention_paged, ptr(x.q), ptr(x.kc), ptr(x.vc), x.lens.p, x.lens.dtype, x.tables.p, x.tables.dtype, x.batch, x.max_blocks,
+                                       x.blocks, static_cast<int>(x.heads), static_cast<int>(x.hkv), static_cast<int>(x.d), static_cast<int>(x.bs),
+                                       x.scale, ptr(x.out), code(x.q), ptr(ws), bytes(ws), stream());
     return x.launches(ws);
 }
 
 // the same without a workspace
 long decode_static(PyObject* const* a) {
     const Decode x(a[0], a[1], a[2], a[3], a[4], a[9], a[5], a[6], a[7], a[8]);
-    check(nvk_decode_attention_paged_static(ptr(x.q), ptr(x.kc), ptr(x.vc), x.lens.p, x.lens.dtype, x.tables.p, x.tables.dtype, x.batch, x.max_blocks,
-                                            x.blocks, static_cast<int>(x.heads), static_cast<int>(x.hkv), static_cast<int>(x.d),
-                                            static_cast<int>(x.bs), x.scale, ptr(x.out), code(x.q), stream()));
+    launch(nvk_decode_attention_paged_static, ptr(x.q), ptr(x.kc), ptr(x.vc), x.lens.p, x.lens.dtype, x.tables.p, x.tables.dtype, x.batch, x.max_blocks,
+                                              x.blocks, static_cast<int>(x.heads), static_cast<int>(x.hkv), static_cast<int>(x.d),
+                                              static_cast<int>(x.bs), x.scale, ptr(x.out), code(x.q), stream());
     return 2;
 }
 
@@ -176,10 +187,10 @@ template <bool FP8> long decode8(PyObject* const* a) {
     const Decode x(a[0], a[1], a[2], a[5], a[6], a[11], a[7], a[8], a[9], a[10]);
     const at::Tensor &ks = cuda("k_scale", a[3]), &vs = cuda("v_scale", a[4]);
     const at::Tensor* ws = optional("workspace", a[12]);
-    check((FP8 ? nvk_decode_attention_paged_fp8 : nvk_decode_attention_paged_int8)(
+    launch(FP8 ? nvk_decode_attention_paged_fp8 : nvk_decode_attention_paged_int8,
         ptr(x.q), ptr(x.kc), ptr(x.vc), ptr(ks), ptr(vs), x.lens.p, x.lens.dtype, x.tables.p, x.tables.dtype, x.batch, x.max_blocks, x.blocks,
         static_cast<int>(x.heads), static_cast<int>(x.hkv), static_cast<int>(x.d), static_cast<int>(x.bs), x.scale, ptr(x.out), code(x.q), ptr(ws),
-        bytes(ws), stream()));
+        bytes(ws), stream());
     return x.launches(ws);
 }
 
@@ -197,9 +208,9 @@ template <bool FP8> long store8(PyObject* const* a) {
     if (key.dim() != 3) raise(PyExc_ValueError, "key must be rank-3 for %s store", FP8 ? "the fp8" : "int8");
     if (slots.element_size() != 4) raise(PyExc_ValueError, "%s", "slot_mapping must be int32");
     const int64_t hkv = key.size(1), d = key.size(2);
-    check((FP8 ? nvk_store_kvcache_fp8 : nvk_store_kvcache_int8)(ptr(key), ptr(value), ptr(kc), ptr(vc), ptr(ks), ptr(vs),
-                                                                 static_cast<const int32_t*>(ptr(slots)), slots.numel(), static_cast<int>(hkv),
-                                                                 static_cast<int>(d), rows_of(kc, hkv * d), code(key), stream()));
+    launch(FP8 ? nvk_store_kvcache_fp8 : nvk_store_kvcache_int8, ptr(key), ptr(value), ptr(kc), ptr(vc), ptr(ks), ptr(vs),
+                                                                   static_cast<const int32_t*>(ptr(slots)), slots.numel(), static_cast<int>(hkv),
+                                                                   static_cast<int>(d), rows_of(kc, hkv * d), code(key), stream());
     return 1;
 }
 
@@ -215,11 +226,11 @@ long prefill(PyObject* const* a) {
     }
     const Index iq("cu_seqlens_q", cu_q), ik("cu_seqlens_k", cu_k), it("block_tables", bt);
     const int64_t hkv = integer(a[8]), d = integer(a[9]), bs = integer(a[10]);
-    check(nvk_prefill_attention_varlen(ptr(q), ptr(k), ptr(v), ptr(kc), ptr(vc), iq.p, iq.dtype, ik.p, ik.dtype, it.p, it.dtype,
-                                       cu_q != nullptr ? cu_q->numel() - 1 : 1, size(q, 0, "query"), k != nullptr ? size(*k, 0, "key") : 0,
-                                       bt != nullptr ? size(*bt, 1, "block_tables") : 0, kc != nullptr ? cache_blocks(*kc, bs, hkv, d) : 0,
-                                       static_cast<int>(integer(a[13])), static_cast<int>(size(q, 1, "query")), static_cast<int>(hkv),
-                                       static_cast<int>(d), static_cast<int>(bs), real(a[11]), ptr(out), code(q), stream()));
+    launch(nvk_prefill_attention_varlen, ptr(q), ptr(k), ptr(v), ptr(kc), ptr(vc), iq.p, iq.dtype, ik.p, ik.dtype, it.p, it.dtype,
+                                         cu_q != nullptr ? cu_q->numel() - 1 : 1, size(q, 0, "query"), k != nullptr ? size(*k, 0, "key") : 0,
+                                         bt != nullptr ? size(*bt, 1, "block_tables") : 0, kc != nullptr ? cache_blocks(*kc, bs, hkv, d) : 0,
+                                         static_cast<int>(integer(a[13])), static_cast<int>(size(q, 1, "query")), static_cast<int>(hkv),
+                                         static_cast<int>(d), static_cast<int>(bs), real(a[11]), ptr(out), code(q), stream());
     return 1;
 }
 
@@ -231,19 +242,19 @@ long mixed_step(PyObject* const* a) {
     const at::Tensor *cu_q = optional("cu_seqlens_q", a[1]), *pk = optional("p_key", a[2]), *pv = optional("p_value", a[3]),
                      *cu_k = optional("cu_seqlens_k", a[4]), *pt = optional("p_block_tables", a[5]);
     const Index iq("cu_seqlens_q", cu_q), ik("cu_seqlens_k", cu_k), it("p_block_tables", pt);
-    check(nvk_attention_mixed_step(ptr(pq), ptr(pk), ptr(pv), ptr(x.kc), ptr(x.vc), iq.p, iq.dtype, ik.p, ik.dtype, it.p, it.dtype,
-                                   cu_q != nullptr ? cu_q->numel() - 1 : 1, size(pq, 0, "p_query"), pk != nullptr ? size(*pk, 0, "p_key") : 0,
-                                   pt != nullptr ? size(*pt, 1, "p_block_tables") : 0, 0, ptr(po), ptr(x.q), x.lens.p, x.lens.dtype, x.tables.p,
-                                   x.tables.dtype, x.batch, x.max_blocks, ptr(x.out), x.blocks, static_cast<int>(size(pq, 1, "p_query")),
-                                   static_cast<int>(x.hkv), static_cast<int>(x.d), static_cast<int>(x.bs), x.scale, code(pq), ptr(ws), ws.nbytes(),
-                                   static_cast<int>(integer(a[18])), stream()));
+    launch(nvk_attention_mixed_step, ptr(pq), ptr(pk), ptr(pv), ptr(x.kc), ptr(x.vc), iq.p, iq.dtype, ik.p, ik.dtype, it.p, it.dtype,
+                                     cu_q != nullptr ? cu_q->numel() - 1 : 1, size(pq, 0, "p_query"), pk != nullptr ? size(*pk, 0, "p_key") : 0,
+                                     pt != nullptr ? size(*pt, 1, "p_block_tables") : 0, 0, ptr(po), ptr(x.q), x.lens.p, x.lens.dtype, x.tables.p,
+                                     x.tables.dtype, x.batch, x.max_blocks, ptr(x.out), x.blocks, static_cast<int>(size(pq, 1, "p_query")),
+                                     static_cast<int>(x.hkv), static_cast<int>(x.d), static_cast<int>(x.bs), x.scale, code(pq), ptr(ws), ws.nbytes(),
+                                     static_cast<int>(integer(a[18])), stream());
     return 2;
 }
 
 // (x, weight, out)
 long linear(PyObject* const* a) {
     const at::Tensor &x = cuda("x", a[0]), &w = cuda("weight", a[1]), &out = cuda("out", a[2]);
-    check(nvk_linear(ptr(x), ptr(w), ptr(out), size(x, 0, "x"), size(w, 0, "weight"), size(w, 1, "weight"), code(x), stream()));
+    launch(nvk_linear, ptr(x), ptr(w), ptr(out), size(x, 0, "x"), size(w, 0, "weight"), size(w, 1, "weight"), code(x), stream());
     return 1;
 }
 
@@ -254,10 +265,10 @@ long qkv_linear(PyObject* const* a) {
                      &kc = cuda("k_cache", a[8]), &vc = cuda("v_cache", a[9]), &q_out = cuda("q_out", a[13]);
     const at::Tensor *qw = optional("q_norm_weight", a[3]), *kw = optional("k_norm_weight", a[4]), *slots = optional("slot_mapping", a[7]);
     const int64_t hq = integer(a[10]), hkv = integer(a[11]), d = integer(a[12]);
-    check(nvk_qkv_linear_norm_rope_store(ptr(x), ptr(w), size(x, 0, "x"), size(x, 1, "x"), static_cast<const int32_t*>(ptr(pos)), ptr(qw), ptr(kw),
-                                         real(a[5]), static_cast<const float*>(ptr(table)), size(table, 0, "cos_sin_cache"),
-                                         static_cast<const int32_t*>(ptr(slots)), ptr(kc), ptr(vc), rows_of(kc, hkv * d), static_cast<int>(hq),
-                                         static_cast<int>(hkv), static_cast<int>(d), ptr(q_out), code(x), stream()));
+    launch(nvk_qkv_linear_norm_rope_store, ptr(x), ptr(w), size(x, 0, "x"), size(x, 1, "x"), static_cast<const int32_t*>(ptr(pos)), ptr(qw), ptr(kw),
+                                           real(a[5]), static_cast<const float*>(ptr(table)), size(table, 0, "cos_sin_cache"),
+                                           static_cast<const int32_t*>(ptr(slots)), ptr(kc), ptr(vc), rows_of(kc, hkv * d), static_cast<int>(hq),
+                                           static_cast<int>(hkv), static_cast<int>(d), ptr(q_out), code(x), stream());
     return 1;
 }
 
