@@ -290,7 +290,7 @@ int launch_merge_typed(const dec::DecodeParams& p, cudaStream_t stream) {
 template <class F, typename T>
 int launch_typed(const DecodeArgs& a, const void* k_scale, const void* v_scale) {
     constexpr int kSmem = static_cast<int>(sizeof(GroupSmem<F>));
-    static bool attr_done[64] = {};  // per device; the attribute calls are idempotent
+    static std::atomic<bool> attr_done[64] = {};  // per device; the attribute calls are idempotent
     int device = 0;
     cudaGetDevice(&device);
     if (device >= 0 && device < 64 && !attr_done[device]) {

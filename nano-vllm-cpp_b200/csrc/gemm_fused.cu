@@ -29,6 +29,7 @@
 
 #include <cuda.h>
 
+#include <atomic>
 #include <mutex>
 
 namespace nvk {
@@ -772,7 +773,7 @@ GemmShape choose_gemm(int64_t m, int64_t n, int64_t k) {
 }
 
 template <typename... KArgs>
-int launch_kernel(void (*kernel)(KArgs...), bool* attr_done, dim3 grid, int threads, int cluster, cudaStream_t stream, const char* what,
+int launch_kernel(void (*kernel)(KArgs...), std::atomic<bool>* attr_done, dim3 grid, int threads, int cluster, cudaStream_t stream, const char* what,
                   KArgs... args) {
     int device = 0;
     cudaGetDevice(&device);
@@ -800,7 +801,7 @@ int launch_kernel(void (*kernel)(KArgs...), bool* attr_done, dim3 grid, int thre
 
 template <typename T, int EPI>
 int launch(const void* a, const void* b, GemmParams& p, bool bf16, cudaStream_t stream, const char* what) {
-    static bool done[3][64] = {};
+    static std::atomic<bool> done[3][64] = {};
     CUtensorMap ta, tb;
     const GemmShape g = choose_gemm(p.m, p.n, p.k);
     p.a_rows = g.mt == 1 && p.m < kBM ? static_cast<int>((p.m + 7) / 8 * 8) : kBM;

@@ -15,6 +15,7 @@
 // tile is masked per element.  Heavier (later) query tiles are scheduled first.
 #include "nvk_internal.cuh"
 
+#include <atomic>
 #include <cmath>
 
 namespace nvk {
@@ -267,7 +268,7 @@ __global__ void __launch_bounds__(kThreads, 2) prefill_tile_kernel(const Prefill
 
 template <typename T>
 int launch_typed(const PrefillArgs& a) {
-    static bool attr_done[64] = {};
+    static std::atomic<bool> attr_done[64] = {};
     int device = 0;
     cudaGetDevice(&device);
     if (device >= 0 && device < 64 && !attr_done[device]) {

@@ -1274,17 +1274,16 @@ int prepare_tc_launch(const PrefillArgs& a, bool bf16, TcLaunch* out) {
 // Shared-memory attribute and SM count of the persistent head-pair kernel, once per device.
 template <typename T, bool MIXED>
 int prepare_tc5(int* sms_out) {
-    static bool done[64] = {};
-    static int sm_count[64] = {};
-    int device = 0;
+    static std::atomic<int> sm_count[64] = {};   // 0 until the attribute is set
+    int device = 0, sms = 0;
     cudaGetDevice(&device);
     if (device < 0 || device >= 64) return fail(NVK_ERR_UNSUPPORTED, "prefill attention: device index %d not supported", device);
-    if (!done[device]) {
+    if (sm_count[device] == 0) {
         const cudaError_t e = cudaFuncSetAttribute(prefill_tc5_kernel<T, MIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes4);
         if (e != cudaSuccess) return fail(NVK_ERR_CUDA, "prefill attention (head pairs): cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-        if (cudaDeviceGetAttribute(&sm_count[device], cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sm_count[device] <= 0)
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0)
             return fail(NVK_ERR_CUDA, "prefill attention (head pairs): cannot read the SM count");
-        done[device] = true;
+        sm_count[device] = sms;
     }
     *sms_out = sm_count[device];
     return NVK_OK;
@@ -1292,7 +1291,7 @@ int prepare_tc5(int* sms_out) {
 
 template <typename T>
 int launch_typed(const PrefillArgs& a, bool bf16) {
-    static bool attr_done[64] = {};
+    static std::atomic<bool> attr_done[64] = {};
     int device = 0;
     cudaGetDevice(&device);
     if (device >= 0 && device < 64 && !attr_done[device]) {

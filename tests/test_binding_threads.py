@@ -1,11 +1,13 @@
-"""The torch binding and several Python threads: a call leaves the interpreter to the others while it is inside the library."""
+"""The torch binding and several Python threads: a call leaves the interpreter to the others while it is inside the library, and
+first calls from several threads at once, each on its own stream, give what one thread gets."""
+import os
 import shutil
 import subprocess
 import sys
 
 import pytest
 
-from util import nvk
+from util import ROOT, nvk
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -54,3 +56,45 @@ def test_a_call_does_not_hold_the_interpreter(tmp_path):
     subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(tmp_path / "libnvk.so"), str(tmp_path / "stand_in.c")], check=True)
     shutil.copy(nvk().BINDING_PATH, tmp_path / "nvk_torch.so")   # finds the library beside it
     subprocess.run([sys.executable, "-c", CALLER, str(tmp_path)], check=True, timeout=120)
+
+THREADS = """
+import threading
+import torch
+from util import nvk, to_dev, workloads
+bf, lib = torch.bfloat16, nvk()
+d = workloads().make_decode_workload(5, 8, 2, 128, 256, 1, 3000, seed=1)
+p = workloads().make_prefill_workload([300, 70], [256, 0], 8, 2, 128, 256, seed=2)
+dev = {n: to_dev(d[n], bf) for n in ("q", "k_cache", "v_cache")}
+pre = {n: to_dev(p[n], bf) for n in ("q", "k_cache", "v_cache")}
+ctx, bt, cu_q, cu_k, pt = (to_dev(a) for a in (d["context_lens"], d["block_tables"], p["cu_q"], p["cu_k"], p["block_tables"]))
+x, w = torch.randn(200, 512, device="cuda").to(bf), torch.randn(768, 512, device="cuda").to(bf)
+torch.cuda.synchronize()
+def work():
+    ws = torch.empty(lib.decode_attention_workspace_bytes(5, 8, 2, 128, bt.shape[1], 256), dtype=torch.uint8, device="cuda")
+    o = [torch.empty_like(dev["q"]), torch.empty_like(pre["q"]), torch.empty(200, 768, device="cuda", dtype=bf)]
+    for _ in range(30):
+        lib.launch_decode_attention_paged(dev["q"], dev["k_cache"], dev["v_cache"], ctx, bt, 2, 128, 256, d["scale"], o[0], ws)
+        lib.launch_prefill_attention_paged(pre["q"], cu_q, pre["k_cache"], pre["v_cache"], cu_k, pt, 2, 128, 256, p["scale"], o[1])
+        lib.linear(x, w, o[2])
+    return o
+got = [None] * 4
+start = threading.Barrier(4)
+def thread(i):
+    with torch.cuda.stream(torch.cuda.Stream()):
+        start.wait()
+        got[i] = work()
+        torch.cuda.current_stream().synchronize()
+ts = [threading.Thread(target=thread, args=(i,)) for i in range(4)]
+[t.start() for t in ts]
+[t.join() for t in ts]
+want = work()
+torch.cuda.synchronize()
+assert lib.prefill_status() == 0 and lib.gemm_status() == 0
+for o in got:
+    assert all(torch.equal(a, b) for a, b in zip(o, want))
+"""
+
+
+def test_first_calls_from_several_threads():
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([os.path.join(ROOT, "tests"), ROOT]))
+    subprocess.run([sys.executable, "-c", THREADS], check=True, timeout=300, env=env, cwd=ROOT)
