@@ -61,6 +61,7 @@ struct GemmParams {
     void* q_out; void* k_cache; void* v_cache;
     int64_t cache_rows;
     int max_positions, hq, hkv;
+    int table_vec;             // cos_sin starts on a 16-byte boundary
     float eps;
     // kAllReducePush
     void* addend;              // this rank's addend buffer [M, N]: rows it reduces itself
@@ -220,6 +221,11 @@ __device__ __forceinline__ void store_rows(T* dst, int off0, int off1, const flo
 }
 
 // ---- epilogues of one 128-column tile (with head_dim 128: of one head) -------------------------------------------------------
+// Four elements of a row of the rotary table, which callers may have at any float's address.
+__device__ __forceinline__ float4 ld_table(const GemmParams& p, const float* at) {
+    if (p.table_vec) return __ldg(reinterpret_cast<const float4*>(at));
+    return make_float4(__ldg(at), __ldg(at + 1), __ldg(at + 2), __ldg(at + 3));
+}
 // What a row of tile `nt` turns into: where it goes, and for q and k heads how it is normalised and rotated.
 template <typename T>
 struct QkvRow {
@@ -324,7 +330,7 @@ __device__ __forceinline__ void epilogue_row(const GemmParams& p, uint32_t t_row
             // 16-byte loads: every lane reads its own table row, so an instruction costs 32 cache lines whatever its width
 #pragma unroll
             for (int i = 0; i < 32; i += 4) {
-                const float4 c4 = __ldg(reinterpret_cast<const float4*>(x.table + c * 32 + i)), s4 = __ldg(reinterpret_cast<const float4*>(x.table + 64 + c * 32 + i));
+                const float4 c4 = ld_table(p, x.table + c * 32 + i), s4 = ld_table(p, x.table + 64 + c * 32 + i);
                 const float cs[4] = {c4.x, c4.y, c4.z, c4.w}, sn[4] = {s4.x, s4.y, s4.z, s4.w};
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
@@ -363,8 +369,8 @@ __device__ __forceinline__ OctetRow<T> octet_row(const GemmParams& p, int64_t ro
         if (x.rotate) {
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                x.cs[i] = __ldg(reinterpret_cast<const float4*>(q.table + 32 * i + 4 * sub));
-                x.sn[i] = __ldg(reinterpret_cast<const float4*>(q.table + 64 + 32 * i + 4 * sub));
+                x.cs[i] = ld_table(p, q.table + 32 * i + 4 * sub);
+                x.sn[i] = ld_table(p, q.table + 64 + 32 * i + 4 * sub);
             }
         }
     } else {
@@ -870,7 +876,7 @@ extern "C" int nvk_qkv_linear_norm_rope_store(const void* x, const void* qkv_wei
         return fail(NVK_ERR_INVALID_ARGUMENT, "%s: q_out and the caches must be 16-byte aligned", what);
     GemmParams p{};
     p.m = rows; p.n = n; p.k = in_features;
-    p.positions = positions; p.q_weight = q_norm_weight; p.k_weight = k_norm_weight; p.cos_sin = cos_sin_cache;
+    p.positions = positions; p.q_weight = q_norm_weight; p.k_weight = k_norm_weight; p.cos_sin = cos_sin_cache; p.table_vec = aligned_to(cos_sin_cache, 16);
     p.slot_mapping = slot_mapping; p.q_out = q_out; p.k_cache = k_cache; p.v_cache = v_cache; p.cache_rows = cache_rows;
     p.max_positions = static_cast<int>(max_positions); p.hq = num_q_heads; p.hkv = num_kv_heads; p.eps = norm_eps;
     return dtype == NVK_BF16 ? launch<__nv_bfloat16, kQkvPrologue>(x, qkv_weight, p, true, static_cast<cudaStream_t>(stream), what)

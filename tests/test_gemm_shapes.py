@@ -56,3 +56,25 @@ def test_qkv_prologue_at_tile_edges(num_q_heads, num_kv_heads, rows, hidden):
     assert np.array_equal(to_np(vc), vc_ref)                      # V: the rounded product, copied
     for got, ref in ((to_np(q_out), q_ref), (to_np(kc), kc_ref)):
         assert (np.abs(got - ref) <= np.maximum(np.abs(ref), 1e-3) * 2.0 ** -7).all()
+
+
+@pytest.mark.parametrize("rows,hidden", [(37, 2048), (200, 512), (700, 1024)])     # summed over a cluster, a block each, pairs
+def test_qkv_prologue_takes_a_rotary_table_at_any_address(rows, hidden):
+    bf, d, hq, hkv = torch.bfloat16, 128, 16, 8
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn((rows, hidden), generator=gen, device="cuda").to(bf)
+    w = (torch.randn(((hq + 2 * hkv) * d, hidden), generator=gen, device="cuda") / hidden ** 0.5).to(bf)
+    table, norm = to_dev(oracle.build_cos_sin_cache(rows, d, 1e6)), torch.ones(d, dtype=bf, device="cuda")
+    pos = torch.arange(rows, dtype=torch.int32, device="cuda")
+    flat = torch.zeros(table.numel() + 4, device="cuda")
+    got = []
+    for offset in (0, 1, 2):
+        t = flat[offset:offset + table.numel()].view(rows, d)
+        t.copy_(table)
+        out = [torch.full((rows, h, d), float("nan"), dtype=bf, device="cuda") for h in (hq, hkv, hkv)]
+        nvk().qkv_linear_norm_rope_store(x, w, pos, norm, norm, 1e-6, t, pos, out[1], out[2], hq, hkv, d, out[0])
+        got.append(out)
+    torch.cuda.synchronize()
+    assert nvk().gemm_status() == 0
+    for o in got[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(o, got[0])) and not any(torch.isnan(a.float()).any() for a in o)
