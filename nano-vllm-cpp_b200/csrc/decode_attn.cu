@@ -203,19 +203,6 @@ int chunk_tokens(int64_t batch, int num_kv_heads, int64_t max_blocks, int block_
     return static_cast<int>(chunk < max_tokens ? chunk : max_tokens);
 }
 
-struct Splits { int cluster, chunk, count; };
-Splits choose_splits(int64_t batch, int num_kv_heads, int64_t max_blocks, int block_size, int groups, bool have_workspace) {
-    Splits s{cluster_size(batch, num_kv_heads, max_blocks, block_size, groups, have_workspace), 0, 0};
-    if (s.cluster > 0) { s.count = s.cluster; return s; }
-    s.chunk = chunk_tokens(batch, num_kv_heads, max_blocks, block_size, groups);
-    s.count = static_cast<int>((max_blocks * block_size + s.chunk - 1) / s.chunk);
-    return s;
-}
-size_t part_bytes(size_t parts, int group) { return parts * group * (kHeadDim * sizeof(float) + sizeof(float2)); }
-size_t part_count(const Splits& s, int64_t batch, int num_kv_heads) {   // (the cluster kernel itself needs none: the mixed step does)
-    return s.count > 1 ? static_cast<size_t>(batch) * num_kv_heads * s.count : 0;
-}
-
 // Split-K scratch of the chunked split that earlier versions of this library used (chunks of 256 to 2048 keys).  The public
 // workspace size never falls below it, because the limit of nvk_decode_attention_paged_static and what counts as a problem that
 // needs no scratch at all are stated in terms of it.
@@ -232,6 +219,27 @@ size_t chunk_scratch_bytes(int64_t batch, int num_heads, int num_kv_heads, int h
     return (rows * sizeof(float) + 15) / 16 * 16 + rows * static_cast<size_t>(head_dim) * sizeof(float);
 }
 
+struct Splits { int cluster, chunk, count; };
+size_t part_bytes(size_t parts, int group) { return parts * group * (kHeadDim * sizeof(float) + sizeof(float2)); }
+size_t part_count(const Splits& s, int64_t batch, int num_kv_heads) {   // (the cluster kernel itself needs none: the mixed step does)
+    return s.count > 1 ? static_cast<size_t>(batch) * num_kv_heads * s.count : 0;
+}
+Splits choose_splits(int64_t batch, int num_heads, int num_kv_heads, int64_t max_blocks, int block_size, int groups, bool have_workspace) {
+    Splits s{cluster_size(batch, num_kv_heads, max_blocks, block_size, groups, have_workspace), 0, 0};
+    if (s.cluster > 0) { s.count = s.cluster; return s; }
+    const int64_t max_tokens = max_blocks * block_size;
+    s.chunk = chunk_tokens(batch, num_kv_heads, max_blocks, block_size, groups);
+    s.count = static_cast<int>((max_tokens + s.chunk - 1) / s.chunk);
+    // A row of partial results takes 520 bytes, 516 in earlier versions: what filled the array of nvk_decode_attention_paged_static almost
+    // to the end must still fit (127 sequences of 32 / 8 heads, 32768-key tables), in longer chunks.
+    while (part_bytes(part_count(s, batch, num_kv_heads), (num_heads + num_kv_heads - 1) / num_kv_heads) > kStaticScratchBytes &&
+           chunk_scratch_bytes(batch, num_heads, num_kv_heads, kHeadDim, max_blocks, block_size) <= kStaticScratchBytes) {
+        s.chunk *= 2;
+        s.count = static_cast<int>((max_tokens + s.chunk - 1) / s.chunk);
+    }
+    return s;
+}
+
 }  // namespace
 
 // Kernel parameters of a decode call from host-known sizes only, for kernels with `groups` resident groups per SM; returns in
@@ -246,7 +254,7 @@ int decode_plan(const DecodeArgs& a, int groups, dec::DecodeParams* out, int* cl
     p.scale_log2 = a.scale * kLog2e;
     if (a.batch * a.num_heads * kMaxCluster >= (1LL << 31) || a.max_blocks * a.block_size >= (1LL << 31) - kTileTokens * kMaxCluster)
         return fail(NVK_ERR_UNSUPPORTED, "decode attention: batch or block table too large");
-    const Splits s = choose_splits(a.batch, a.num_kv_heads, a.max_blocks, a.block_size, groups, a.workspace != nullptr);
+    const Splits s = choose_splits(a.batch, a.num_heads, a.num_kv_heads, a.max_blocks, a.block_size, groups, a.workspace != nullptr);
     *cluster = s.cluster;
     p.per_seq = s.cluster > 0 ? 1 : 0;
     p.chunk_tokens = s.chunk;
@@ -353,7 +361,7 @@ size_t decode_mma_workspace_bytes(int64_t batch, int num_heads, int num_kv_heads
     if (batch <= 0 || num_heads <= 0 || num_kv_heads <= 0 || max_blocks <= 0 || block_size <= 0) return 0;
     size_t need = chunk_scratch_bytes(batch, num_heads, num_kv_heads, head_dim, max_blocks, block_size);
     for (int groups : {Cache16<__half>::kGroups, Cache8<__half, false>::kGroups}) {
-        const Splits s = choose_splits(batch, num_kv_heads, max_blocks, block_size, groups, true);
+        const Splits s = choose_splits(batch, num_heads, num_kv_heads, max_blocks, block_size, groups, true);
         const size_t n = part_bytes(part_count(s, batch, num_kv_heads), (num_heads + num_kv_heads - 1) / num_kv_heads);
         if (n > need) need = n;
     }

@@ -71,6 +71,13 @@ def test_workspace_size_depends_only_on_host_known_sizes(built):
     assert built.decode_attention_workspace_bytes(0, 32, 8, 128, 32, 256) == 0
 
 
+@pytest.mark.parametrize("batch,block_size,max_blocks", [(127, 256, 128), (101, 256, 160), (253, 16, 1024), (254, 256, 64)])
+def test_what_fits_the_static_scratch_at_516_bytes_a_row_still_does(built, batch, block_size, max_blocks):
+    rows = batch * 32 * (block_size * max_blocks // 2048)               # 32 heads, chunks of 2048 keys
+    assert rows * 516 <= 32 << 20 < rows * 520
+    assert built.decode_attention_workspace_bytes(batch, 32, 8, 128, max_blocks, block_size) <= built.decode_attention_static_scratch_bytes()
+
+
 def test_missing_library_fails_loudly(built, monkeypatch):
     monkeypatch.setattr(built, "_lib", None)
     monkeypatch.setattr(built, "LIB_PATH", os.path.join(ROOT, "does_not_exist", "libnvk.so"))
