@@ -741,7 +741,10 @@ __device__ __forceinline__ bool softmax_row_to_smem(uint32_t t_s, uint32_t t_o, 
 // the chain load -> S -> softmax -> P.V -> store (about 1.5 rounds) every time; here only the first
 // and last item of a block do.  All barrier phases are counted cumulatively over items.
 // =================================================================================================
-constexpr int kTicketSlots = 64;
+// Ticket counters.  Launches that run at the same time must not share one: each would leave out items that the other took.  An eager launch takes
+// the next of 32768, far more launches than streams hold in their queues; a captured one keeps its counter for all replays of its graph,
+// so these have 32768 of their own, which no eager launch meets.
+constexpr int kEagerSlots = 32768, kTicketSlots = 2 * kEagerSlots;
 constexpr int kIssuers5 = 2;        // issuing warps, one per query tile
 constexpr int kThreads5 = 384;      // three warpgroups (register reallocation works on whole warpgroups)
 constexpr int kRegsLow5 = 56;       // registers per thread of the third warpgroup after setmaxnreg.dec
@@ -1241,8 +1244,13 @@ uint32_t make_idesc(bool bf16, bool b_mn_major, int m = kBM) {
 }
 
 
-// Launches that may run at the same time on one device need different ticket counters; 64 of them rotate.
-std::atomic<unsigned int> g_launch_seq{0};
+std::atomic<unsigned int> g_launch_seq{0}, g_capture_seq{0};
+int ticket_slot(cudaStream_t stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) cudaGetLastError();   // (the launch will say what is wrong)
+    return static_cast<int>(status == cudaStreamCaptureStatusNone ? g_launch_seq.fetch_add(1u) % kEagerSlots
+                                                                  : kEagerSlots + g_capture_seq.fetch_add(1u) % (kTicketSlots - kEagerSlots));
+}
 
 // Tensor maps and kernel parameters of a prefill call.
 struct TcLaunch {
@@ -1315,7 +1323,7 @@ int launch_typed(const PrefillArgs& a, bool bf16) {
         pp.pairs = a.num_heads / 2;
         pp.tiles = static_cast<int>(tiles);
         pp.total = static_cast<unsigned int>(pp.pairs) * static_cast<unsigned int>(tiles);
-        pp.slot = static_cast<int>(g_launch_seq.fetch_add(1u) % kTicketSlots);
+        pp.slot = ticket_slot(a.stream);
         const unsigned int blocks = pp.total < static_cast<unsigned int>(sms) ? pp.total : static_cast<unsigned int>(sms);
         const cudaError_t e = launch_pdl(prefill_tc5_kernel<T, false>, dim3(blocks), dim3(kThreads5), kSmemBytes4, a.stream, tq, tk, tv, pp, MixedDecode{});
         if (e != cudaSuccess) return fail(NVK_ERR_CUDA, "prefill_tc5_kernel launch: %s", cudaGetErrorString(e));
@@ -1369,7 +1377,7 @@ int launch_mixed_typed(const PrefillArgs& a, const DecodeArgs& d, int prefill_bl
     pp.pairs = a.num_heads / 2;
     pp.tiles = static_cast<int>(L.tiles);
     pp.total = static_cast<unsigned int>(pp.pairs) * static_cast<unsigned int>(L.tiles);
-    pp.slot = static_cast<int>(g_launch_seq.fetch_add(1u) % kTicketSlots);
+    pp.slot = ticket_slot(a.stream);
     if (prefill_blocks <= 0) {
         // No hint: split the SMs by a crude estimate from host-known sizes -- prefill flops as if all sequences were equally
         // long and had no prefix, at 0.55 PFLOP/s (what the prefill half sustains on a share of the SMs at a few thousand tokens per
