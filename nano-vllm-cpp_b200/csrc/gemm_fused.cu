@@ -902,7 +902,9 @@ int launch_row_linear_push(const char* what, const void* x, const void* weight, 
     p.m = rows; p.n = out_features; p.k = in_features;
     p.addend = addend; p.flags = static_cast<const uint32_t*>(flags); p.rank = rank; p.world = world;
     for (int r = 0; r < world; ++r) {
-        if (!stage_ptrs[r] || !aligned_to(stage_ptrs[r], 16)) return fail(NVK_ERR_INVALID_ARGUMENT, "%s: bad staging area of rank %d", what, r);
+        // (tagged vectors are stored 32 bytes at a time)
+        if (!stage_ptrs[r] || !aligned_to(stage_ptrs[r], 32))
+            return fail(NVK_ERR_INVALID_ARGUMENT, "%s: the staging area of rank %d is missing or not 32-byte aligned", what, r);
         p.stage[r] = static_cast<uint4*>(stage_ptrs[r]);
     }
     return dtype == NVK_BF16 ? launch<__nv_bfloat16, kAllReducePush>(x, weight, p, true, stream, what)

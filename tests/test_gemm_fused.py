@@ -7,6 +7,7 @@
 * ``nvk_tp_row_linear_allreduce_add_rmsnorm`` for 2, 4, 8 ranks on one GPU against torch: per-rank partial products rounded
   to the 16-bit type, summed in fp32 in rank order, rounded once, residual added, fp32 RMSNorm.
 """
+import ctypes
 import importlib
 
 import numpy as np
@@ -133,3 +134,19 @@ def test_gemm_entry_points_refuse_what_they_cannot_run():
     with pytest.raises(ValueError):
         nvk().linear(x.float(), torch.zeros(128, 64, device="cuda"), torch.zeros(4, 128, device="cuda"))
     assert nvk().gemm_status() == 0
+
+
+def test_row_parallel_linear_refuses_staging_areas_off_a_32_byte_boundary():
+    bf, lib, dev = torch.bfloat16, nvk(), "cuda"
+    x, w, buf = torch.zeros(16, 64, device=dev, dtype=bf), torch.zeros(128, 64, device=dev, dtype=bf), torch.zeros(16, 128, device=dev, dtype=bf)
+    size = lib.lib().nvk_tp_allreduce_stage_bytes
+    size.restype, size.argtypes = ctypes.c_size_t, [ctypes.c_int64]
+    nbytes = size(buf.numel())
+    stage, flags = torch.zeros(nbytes + 32, device=dev, dtype=torch.uint8), torch.zeros(256, device=dev, dtype=torch.uint8)
+    p = ctypes.c_void_p
+    tab = (p * 2)(stage.data_ptr(), stage.data_ptr() + 16)
+    rc = lib.lib().nvk_tp_row_linear_allreduce_add_rmsnorm(
+        p(x.data_ptr()), p(w.data_ptr()), ctypes.c_int64(16), ctypes.c_int64(128), ctypes.c_int64(64), p(buf.data_ptr()), p(buf.data_ptr()),
+        p(buf.data_ptr()), tab, ctypes.c_size_t(nbytes), p(flags.data_ptr()), p(buf.data_ptr()), p(w.data_ptr()), ctypes.c_float(1e-6), 0, 2,
+        lib.BF16, None)
+    assert rc == lib.ERR_INVALID_ARGUMENT and b"32-byte" in lib.lib().nvk_last_error()
