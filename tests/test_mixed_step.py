@@ -114,6 +114,58 @@ def test_mixed_step_repeats_with_int64_indices_and_from_a_graph():
     assert lib.prefill_status() == 0
 
 
+def _fp32_rows(q, k, v, scale, seen):
+    """Attention of q [rows, heads, d] over the keys of one sequence in fp32; row r sees the first seen[r] keys."""
+    group = q.shape[1] // k.shape[1]
+    k, v = k.float().repeat_interleave(group, 1), v.float().repeat_interleave(group, 1)
+    s = torch.einsum("qhd,khd->hqk", q.float(), k) * scale
+    s.masked_fill_(torch.arange(k.shape[0], device="cuda")[None, None, :] >= seen[None, :, None], float("-inf"))
+    return torch.einsum("hqk,khd->qhd", s.softmax(-1), v)
+
+
+def test_two_hundred_steps_of_many_items_a_block_are_each_the_two_calls_bit_for_bit():
+    """3 prompts of 500 to 2048 tokens beside 90 decode rows of 500 to 8192 keys, 32 / 8 heads: several items for every block, so that the
+    warps of a block are items apart (an output row staged where a faster warp writes showed in one pass of seven, by up to 7)."""
+    bf, lib, hq, hkv, scale = torch.bfloat16, nvk(), 32, 8, D ** -0.5
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    rng = np.random.default_rng(5)
+    q_lens, ctx_lens = np.array([1210, 500, 2048]), rng.permutation(np.linspace(500, 8192, 90).astype(np.int64))
+    need = [-(-int(n) // BS) for n in (*q_lens, *ctx_lens)]
+    ids, at = rng.permutation(sum(need)), 0
+    pt, dt = np.zeros((3, max(need[:3])), np.int32), np.zeros((90, max(need[3:])), np.int32)
+    for i, n in enumerate(need):
+        (pt[i] if i < 3 else dt[i - 3])[:n] = ids[at:at + n]
+        at += n
+
+    def normal(*shape):
+        return torch.empty(shape, dtype=bf, device="cuda").normal_(generator=gen)
+
+    kc, vc = normal(sum(need), BS, hkv, D), normal(sum(need), BS, hkv, D)
+    pq, dq = normal(int(q_lens.sum()), hq, D), normal(90, hq, D)
+    cu, ctx, pt, dt = (to_dev(a.astype(np.int32)) for a in (np.concatenate([[0], np.cumsum(q_lens)]), ctx_lens, pt, dt))
+    ws = torch.empty(lib.decode_attention_workspace_bytes(90, hq, hkv, D, dt.shape[1], BS), dtype=torch.uint8, device="cuda")
+    want_p, want_d, p_out, d_out = torch.empty_like(pq), torch.empty_like(dq), torch.empty_like(pq), torch.empty_like(dq)
+    lib.launch_prefill_attention_paged(pq, cu, kc, vc, cu, pt, hkv, D, BS, scale, want_p)
+    lib.launch_decode_attention_paged(dq, kc, vc, ctx, dt, hkv, D, BS, scale, want_d, ws)
+    for i in range(3):                                                 # the two calls against fp32
+        n, r0 = int(q_lens[i]), int(q_lens[:i].sum())
+        k, v = (c[pt[i, :need[i]].long()].view(-1, hkv, D)[:n] for c in (kc, vc))
+        ref = _fp32_rows(pq[r0:r0 + n], k, v, scale, torch.arange(1, n + 1, device="cuda"))
+        assert_attention_close(to_np(want_p[r0:r0 + n]), to_np(ref))
+    for i in range(90):
+        n = int(ctx_lens[i])
+        k, v = (c[dt[i, :need[3 + i]].long()].view(-1, hkv, D)[:n] for c in (kc, vc))
+        assert_attention_close(to_np(want_d[i:i + 1]), to_np(_fp32_rows(dq[i:i + 1], k, v, scale, torch.tensor([n], device="cuda"))))
+    wrong = torch.zeros(200, dtype=torch.bool, device="cuda")
+    for i in range(200):
+        p_out.fill_(float("nan"))
+        d_out.fill_(float("nan"))
+        lib.attention_mixed_step(pq, cu, None, None, cu, pt, p_out, dq, ctx, dt, d_out, kc, vc, hkv, D, BS, scale, ws, (0, 0, 0, 1, 60, 148)[i % 6])
+        wrong[i] = (p_out.view(torch.int16) != want_p.view(torch.int16)).any() | (d_out.view(torch.int16) != want_d.view(torch.int16)).any()
+    assert lib.prefill_status() == 0
+    assert not wrong.any(), wrong.nonzero().flatten().tolist()
+
+
 def test_mixed_step_refuses_what_it_cannot_run():
     lib = nvk()
     f32 = torch.float32
