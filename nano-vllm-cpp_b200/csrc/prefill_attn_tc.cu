@@ -1200,9 +1200,6 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kTmemCols2) : "memory");
     }
     if (MIXED && !decode_first) decode_half();
-    // Nothing needs this fence, but grids of several items per block measure faster with it (16 x 2048 tokens 618 -> 603 us, 2 x 8192
-    // 953 -> 946, on every box; the compiled loops are others).  For one item a block it would only add 0.5 us.
-    if (tid == 0 && pp.total > gridDim.x) __threadfence();
 }
 
 // ---- host side ------------------------------------------------------------------------------------------
@@ -1380,8 +1377,10 @@ int launch_mixed_typed(const PrefillArgs& a, const DecodeArgs& d, int prefill_bl
     pp.slot = ticket_slot(a.stream);
     if (prefill_blocks <= 0) {
         // No hint: split the SMs by a crude estimate from host-known sizes -- prefill flops as if all sequences were equally
-        // long and had no prefix, at 0.55 PFLOP/s (what the prefill half sustains on a share of the SMs at a few thousand tokens per
-        // sequence); decode bytes as if every block table were half full, at 6.5 TB/s.
+        // long and had no prefix, at 0.55 PFLOP/s (2048 tokens per sequence; short prompts run slower, long ones faster); decode bytes as if
+        // every block table were half full, at 6.5 TB/s.  Against the best of 17 splits for 19 steps (1 to 6 prompts of 64 to 4000
+        // tokens, 8 to 192 decode rows) it costs 6 % on average and 24 % at most (4 prompts of 800 tokens and 128 rows, 4 / 1 heads).  Other rates,
+        // and a fixed part per item, did no better: what it misses is that items are whole and contexts unknown.
         const double mean_q = static_cast<double>(a.total_q) / static_cast<double>(a.cu_q ? a.num_seqs : 1);
         const double t_prefill = 4.0 * a.num_heads * kHeadDim * static_cast<double>(a.total_q) * (mean_q + 1.0) / 2.0 / 0.55e15;
         const double t_decode = 0.5 * static_cast<double>(d.batch) * d.max_blocks * d.block_size * d.num_kv_heads * kHeadDim * 4.0 / 6.5e12;
