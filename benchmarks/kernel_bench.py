@@ -560,7 +560,7 @@ def bench_linears(nvk, torch, dev, steps, warmup, rows=256, layers=36):
             "config": {"workload": f"QKV projection ({hidden} -> {n_qkv}) + split + q/k RMSNorm + RoPE + KV store as one launch, {rows} rows",
                        "l2": f"time per layer of a replayed CUDA graph over {layers} distinct weight matrices ({layers * n_qkv * hidden * 2 >> 20} MB: beyond L2)"},
             "cases": out, "gemm_status": status,
-            "roofline": {"bound": "hbm", "kernel": "gemm_tc_kernel<T, qkv prologue epilogue>", "achieved": ach, "peak": hbm,
+            "roofline": {"bound": "hbm", "kernel": "gemm_split_kernel<T, qkv prologue epilogue>", "achieved": ach, "peak": hbm,
                          "peak_source": f"{kind} copy bandwidth", "unit": "GB/s", "frac": ach / hbm, "traffic": None},
             "gpu_launches": steps * layers * len(cases), "clocks": clocks}
 

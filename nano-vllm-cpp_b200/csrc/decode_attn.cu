@@ -10,6 +10,7 @@
 //                          whose chunk lies beyond the context exit at once.
 //   decode_merge_kernel    merges the chunks of long contexts; launched only where the table can hold more than one.
 //   decode_cluster_kernel  small steps: a cluster of blocks per (sequence, KV head), merged in the same launch.
+// Which one is taken depends on the table's WIDTH, not on the contexts: one short sequence in a wide table takes chunks and a merge.
 #include "decode_body.cuh"
 
 #include <cooperative_groups.h>
@@ -26,13 +27,13 @@ namespace cg = cooperative_groups;
 constexpr size_t kStaticScratchBytes = 32u << 20;
 constexpr int kMaxCluster = 8;          // portable cluster size
 // Longest range per block (of a full table row) that goes to the cluster kernel: 8 tiles per warp, some 5 us of keys.  Up to there the
-// second launch costs more than chunks of even length give: 1 sequence of 300 keys, 32 / 8 heads, with its prologue, takes 7.1 us a
-// pass (alone, from call to result: 17) where split and merge took 9.4 (41).
+// second launch costs more than chunks of even length give: 1 sequence of 300 keys, 32 / 8 heads, with its prologue, takes 6.7 us a
+// pass in a replayed graph where split and merge took 9.1.
 constexpr int kClusterTokens = 512;
 
 // Sequence number `rank` in order of falling context length, found by every block for itself.  In index order the last blocks to start
 // can be the longest: 100 sequences of 500 to 4096 keys, int8, left half the SMs idle for the last 40 of 106 us; in this order the pass
-// takes 103 us instead of 115.  64 sequences of 100 to 2048 keys, 16-bit: 6 us less.  The order is that of 128 classes of length, and of
+// took 103 us instead of 115 (92 since the keys are the rows of the score MMAs).  64 sequences of 100 to 2048 keys, 16-bit: 6 us less.  The order is that of 128 classes of length, and of
 // the index inside a class: a histogram, one scan and a search through the class.  (Comparing every context with every other one took
 // each block 5 us at 254 sequences: with 4 KV heads and contexts of up to 157 keys 39 us a pass.)
 constexpr int kMaxSorted = 512;

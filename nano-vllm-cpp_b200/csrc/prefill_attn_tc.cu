@@ -1045,7 +1045,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         while (!ok && next.kind) next = take_item();   // a wait gave up: the tickets are still taken to the end
     } else if (warp == 8 || warp == 8 + 2 * (kIssuers5 - 1)) {
         // ------------------------------------------------------------------ MMA issuer(s): with two, warp 8 drives
-        // tile 0 and warp 10 tile 1 (one thread sustains about one MMA per 100 clocks here, the tensor pipe one per 64)
+        // tile 0 and warp 10 tile 1 (a single thread sustained about one MMA per 100 clocks here, the tensor pipe one per 64)
         if (lane == 0) {
             const int t_lo = (kIssuers5 == 2 && warp != 8) ? 1 : 0;
             const int t_hi = (kIssuers5 == 2 && warp == 8) ? 1 : 2;
