@@ -464,8 +464,11 @@ __device__ __forceinline__ void sum_over_cluster(uint32_t at, int splits, float4
 // blockIdx.x = tile column * splits + part of K (= rank in the cluster), blockIdx.y = tile row of MT * 128 rows.  The partial sums go to
 // shared memory as fp32 rows of 132 words (no bank conflicts for the writing threads, each of which has a row); block r adds up and
 // finishes rows r, r + splits, ... of the tile, eight lanes a row.
+// DIRECT: a block with all of K has nothing to add up and takes its tile from TMEM straight to the result (us: 4096 columns, K 128, 128 rows
+// 5.5 -> 4.0); not up to 32 rows, which would leave three of four epilogue warps idle (8 rows 3.2 -> 3.7).  An instantiation of its own: with both
+// ways in one the sums were slower (39 rows through 768 x 4096 and 4096 x 512 in a pass of 25.2 us: 26.4).
 constexpr int kRowWords = kBN + 4;
-template <typename T, int EPI, int MT>
+template <typename T, int EPI, int MT, bool DIRECT>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ GemmParams p, int splits) {
     constexpr int kStageBytes = (MT + 1) * kPanelBytes, kStages = kRingBytes / kStageBytes, kTmemCols = MT * kBN;
@@ -483,9 +486,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     const int rank = static_cast<int>(blockIdx.x) % splits, nt = static_cast<int>(blockIdx.x) / splits;
     const int n0 = nt * kBN, m0 = blockIdx.y * (MT * kBM);
     const int rows = static_cast<int>(min(static_cast<int64_t>(MT * kBM), p.m - m0));   // of the tile that are in C
-    // A block with all of K has nothing to add up: TMEM straight to the result, unless a tile of few rows would leave three of four epilogue
-    // warps idle (us: 4096 columns, K 128, 128 rows 5.5 -> 4.0, 8 rows 3.2 -> 3.7).
-    const bool direct = splits == 1 && rows > 32;
     const int kb_all = static_cast<int>((p.k + kBK - 1) / kBK);
     const int kb0 = kb_all * rank / splits, kb_count = kb_all * (rank + 1) / splits - kb0;
 
@@ -548,7 +548,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         if (lane == 0) ok = mbar_wait(bar_acc, 0, abort_flag, 3);
         ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
         tc_fence_after();
-        if (ok && direct) {
+        if (DIRECT && ok) {
             unsigned char* stage = smem_raw + (smem_base - smem_u32(smem_raw)) + kStageOffset + (warp - 2) * 4096;
 #pragma unroll 1
             for (int t = 0; t < MT; ++t)
@@ -575,7 +575,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     if (warp == 1) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
     }
-    if (direct) return;
+    if (DIRECT) return;
     // ---------------------------------------------------------------------- sum over the cluster and epilogue
     const int sub = lane & 7;
     int q = warp * 4;                      // four rows per warp and trip
@@ -758,6 +758,8 @@ uint32_t make_idesc(bool bf16, int m, int n) {   // kind::f16: D = F32, A / B = 
 // pair's tile is hidden but for the epilogue.  (One fixed part whatever the waves, measured at K 4096 only, took 256-row blocks for
 // 1500 x 4096, K 512: 21.6 us, pairs 12.3.)  One rule for all epilogues, so that they round the same sums: its constants lie between
 // the plain ones (choice within 1 % of the fastest on average, 12 % at most) and those of the slower QKV epilogue (2 %, but 30 % where K is 512).
+// A part of K has four steps at least: with fewer, clusters of 4 that nearly fill the chip gain 0.2 us at most (8 x 4096, K 512, 4.4 us,
+// clusters of 2 4.6).
 struct GemmShape { int mt, splits; };   // mt 1 or 2: gemm_split_kernel; 0: gemm_pair_kernel
 GemmShape choose_gemm(int64_t m, int64_t n, int64_t k) {
     // clusters: what a B200 holds at once (its GPCs have 16 to 20 SMs); rows: per 128 rows of a tile
@@ -769,7 +771,7 @@ GemmShape choose_gemm(int64_t m, int64_t n, int64_t k) {
     double best_time = m > kBM ? static_cast<double>((pair_tiles + 73) / 74) * (static_cast<double>(kb) * 0.31 + 3.0) + 4.7 : 1e30;
     for (const auto& w : kWays) {
         const int64_t tile_rows = w.mt * kBM, tiles = (m + tile_rows - 1) / tile_rows * tiles_n;
-        if ((w.mt == 2 && m <= kBM) || (w.splits > 1 && (kb / w.splits < 2 || tiles > w.clusters))) continue;
+        if ((w.mt == 2 && m <= kBM) || (w.splits > 1 && (kb / w.splits < 4 || tiles > w.clusters))) continue;
         const double rows = static_cast<double>(m < tile_rows ? m : tile_rows) / kBM;
         const double time = static_cast<double>((tiles + w.clusters - 1) / w.clusters) *
                             (static_cast<double>((kb + w.splits - 1) / w.splits) * w.step + w.fixed + w.rows * rows);
@@ -807,7 +809,7 @@ int launch_kernel(void (*kernel)(KArgs...), std::atomic<bool>* attr_done, dim3 g
 
 template <typename T, int EPI>
 int launch(const void* a, const void* b, GemmParams& p, bool bf16, cudaStream_t stream, const char* what) {
-    static std::atomic<bool> done[3][64] = {};
+    static std::atomic<bool> done[5][64] = {};
     CUtensorMap ta, tb;
     const GemmShape g = choose_gemm(p.m, p.n, p.k);
     p.a_rows = g.mt == 1 && p.m < kBM ? static_cast<int>((p.m + 7) / 8 * 8) : kBM;
@@ -823,8 +825,10 @@ int launch(const void* a, const void* b, GemmParams& p, bool bf16, cudaStream_t 
     }
     p.idesc = make_idesc(bf16, kBM, kBN);
     const dim3 grid(static_cast<unsigned>(p.n / kBN * g.splits), static_cast<unsigned>((p.m + g.mt * kBM - 1) / (g.mt * kBM)));
-    return g.mt == 1 ? launch_kernel(gemm_split_kernel<T, EPI, 1>, done[1], grid, kThreads, g.splits, stream, what, ta, tb, p, g.splits)
-                     : launch_kernel(gemm_split_kernel<T, EPI, 2>, done[2], grid, kThreads, g.splits, stream, what, ta, tb, p, g.splits);
+    const bool direct = g.splits == 1 && p.m > 32;
+    auto* kernel = g.mt == 1 ? direct ? gemm_split_kernel<T, EPI, 1, true> : gemm_split_kernel<T, EPI, 1, false>
+                             : direct ? gemm_split_kernel<T, EPI, 2, true> : gemm_split_kernel<T, EPI, 2, false>;
+    return launch_kernel(kernel, done[2 * g.mt - 1 + direct], grid, kThreads, g.splits, stream, what, ta, tb, p, g.splits);
 }
 
 int check_gemm(const char* what, const void* a, const void* b, int64_t m, int64_t n, int64_t k, int dtype) {
