@@ -174,14 +174,17 @@ int cluster_size(int64_t batch, int num_kv_heads, int64_t max_blocks, int block_
 }
 
 // A grid just past a full wave of resident groups: its last blocks run almost alone, and nothing balances equal ones.
-bool just_past_a_wave(int64_t pairs, int groups) { return pairs > kSmCount * groups && 3 * pairs < 4 * kSmCount * groups; }
+bool just_past_a_wave(int64_t pairs, int groups) {
+    return pairs > kSmCount * groups && (groups == 2 ? 4 * pairs < 5 * kSmCount * groups : 3 * pairs < 4 * kSmCount * groups);
+}
 
 // Chunk length in keys (whole cache blocks), from the number of (sequence, KV head) pairs and the table's width; us a call below.
 // Whole contexts: no merge, no second launch.
 //   * Tables of up to 1024 keys: 176 pairs of 1024 keys 19.3, as two chunks 23.7; 264 24.6, 29.1; 432 int8 ones 24.3, 30.5.  But 8-bit
 //     caches with 1.5 to 2 pairs per SM, 264 int8 ones of 1024 keys / of 100 to 1024: 22.3 / 19.6, in two chunks 22.9 / 17.6.
 //   * Tables of up to 4096 keys with a pair for every resident group: 37 sequences of 100 to 2048 keys, 8 KV heads, 2 of 37; but not just past
-//     a wave: 304 / 352 pairs of 4096 keys 116.8 / 123.7, in chunks of 2048 106.1 / 113.5 (384 pairs 126.2, 121.9; 448 137.0, 145.8).
+//     a wave: 304 / 352 pairs of 4096 keys 116.8 / 123.7, in chunks of 2048 106.1 / 113.5; 560 int8 ones 117.4, 105.1 (384 16-bit pairs
+//     126.2, 121.9, but of 97 keys in 2560-key tables 12.3, 13.4; 448 137.0, 145.8).
 // Chunks of 2048 otherwise, halved down to 256 while they leave resident groups without a block.
 //   * A table that 2048 keys cover is cut only below 1.5 (8-bit: 2.5) pairs per SM: 264 pairs of 2048 keys 44.7 whole, 48.5 cut; 432 int8 ones
 //     43.8, 47.5; but 328 int8 ones of 100 to 2048 keys 35.1, 28.7.  What is cut is cut no finer than it takes to have 1.5 blocks per SM
@@ -261,7 +264,7 @@ int decode_plan(const DecodeArgs& a, int groups, dec::DecodeParams* out, int* cl
     p.chunk_tokens = s.chunk;
     p.num_splits = s.count;
     // More than one wave of blocks: the long contexts first, so that the last blocks to start are short.  Contexts in a few chunks as well:
-    // 38 / 48 sequences of 500 / 2000 to 4096 keys, 8 KV heads, 65.4 / 96.6 -> 58.7 / 92.7 us a call (whole 59.8 / 90.4).
+    // 38 / 44 sequences of 500 / 2000 to 4096 keys, 8 KV heads, 65.4 / 90.1 -> 58.7 / 85.9 us a call (whole 59.8 / 84.7).
     p.longest_first = s.cluster == 0 && (s.count == 1 || a.max_blocks * a.block_size <= 4096) && a.batch * a.num_kv_heads > static_cast<int64_t>(kSmCount) * groups &&
                       a.batch <= kMaxSorted && a.max_blocks * a.block_size >= kMinSortedTokens;
     // Contexts shorter than the table leave chunks without keys, whose blocks exit at once.  With sequence after sequence they lie between

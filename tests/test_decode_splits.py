@@ -29,8 +29,8 @@ def _workspace(batch, hq, hkv, blocks, bs):
     (4, 1, 256, (EDGES * 5)[:72], 4),
     (4, 1, 256, (EDGES[:12] * 4)[:40], 2),                  # tables of 512 keys in one block each
     (8, 1, 256, [2047, 2048, 2049, 1, 9000], 80),           # chunks: up to 36 parts of one context
-    (16, 8, 256, EDGES * 3 + [4096, 2500, 2048], 16),       # 4096-key tables just past a wave: chunks, longest first
-    (16, 8, 256, EDGES * 3 + [4096, 2500, 2048, 9, 99], 16),   # and whole contexts
+    (16, 8, 256, EDGES * 3 + [4096, 2500, 2048], 16),       # whole contexts, 4096-key tables
+    (16, 8, 256, EDGES * 2 + [4096, 2500, 2048, 9, 99, 1, 2, 3], 16),   # and just past a wave: chunks, longest first
     (4, 1, 256, (EDGES * 15)[:221] + [2048], 8),            # 2048-key tables, whole
     (4, 1, 256, (EDGES * 15)[:220] + [2048], 8),            # and in two chunks
     (8, 2, 256, [300] * 170 + EDGES * 3 + [1024], 4),       # longest first with most in one class of length
