@@ -1244,7 +1244,10 @@ uint32_t make_idesc(bool bf16, bool b_mn_major, int m = kBM) {
 std::atomic<unsigned int> g_launch_seq{0}, g_capture_seq{0};
 int ticket_slot(cudaStream_t stream) {
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) cudaGetLastError();   // (the launch will say what is wrong)
+    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {   // (status is undefined; the launch will say what is wrong)
+        status = cudaStreamCaptureStatusNone;
+        cudaGetLastError();
+    }
     return static_cast<int>(status == cudaStreamCaptureStatusNone ? g_launch_seq.fetch_add(1u) % kEagerSlots
                                                                   : kEagerSlots + g_capture_seq.fetch_add(1u) % (kTicketSlots - kEagerSlots));
 }
