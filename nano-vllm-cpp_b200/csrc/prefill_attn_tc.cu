@@ -78,6 +78,16 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok;
 }
+// Whether a phase has completed, without waiting for it.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
 // Bounded wait: gives up after kWaitCycles or as soon as another thread of the block gave up.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code) {
     if (mbar_try_wait(bar, parity)) return true;
@@ -127,31 +137,45 @@ __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64
         "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
         ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(acc) : "memory");
 }
-// SS MMA whose descriptors are a base descriptor plus a compile-time offset of the 14-bit start-address field
-// (units of 16 bytes).  The adds sit inside the volatile asm, so the compiler cannot precompute (and then keep in
-// registers, or spill) one descriptor pair per MMA of an unrolled loop: the issuing thread stays small.
-template <int A_OFF16, int B_OFF16>
-__device__ __forceinline__ void umma_ss_off(uint32_t d_tmem, uint64_t a_base, uint64_t b_base, uint32_t idesc, uint32_t acc) {
+// For an issuing warp that stays converged: all lanes run through the same instructions, so that the descriptors live in uniform registers, which
+// is where the MMA wants them, and one lane (`leader` 1) issues.  A single diverged lane has to move every operand there first: 75 to 100
+// clocks an MMA, more than the tensor pipe needs for one.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t leader;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(leader));
+    return leader;
+}
+template <bool ACC>
+__device__ __forceinline__ void umma_ss_by(uint32_t leader, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
-        "add.u64 da, %1, %5;\n\t"
-        "add.u64 db, %2, %6;\n\t"
-        "setp.ne.u32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}\n"
-        :: "r"(d_tmem), "l"(a_base), "l"(b_base), "r"(idesc), "r"(acc), "n"(A_OFF16), "n"(B_OFF16) : "memory");
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %0, 0;\n\tsetp.ne.u32 p, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%1], %2, %3, %4, p;\n\t}\n"
+        :: "r"(leader), "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "n"(ACC ? 1 : 0) : "memory");
 }
-constexpr int kmajor_off16(int step) { return ((step / 4) * kPanelBytes + (step % 4) * 32) / 16; }
+__device__ __forceinline__ void umma_ts_by(uint32_t leader, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %0, 0;\n\tsetp.ne.u32 p, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [%2], %3, %4, p;\n\t}\n"
+        :: "r"(leader), "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(acc) : "memory");
+}
+__device__ __forceinline__ void tc_commit_by(uint32_t leader, uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%1];\n\t}\n" :: "r"(leader), "r"(bar) : "memory");
+}
+constexpr uint64_t kmajor_off16(int step) { return ((step / 4) * kPanelBytes + (step % 4) * 32) / 16; }
 // The 8 K-steps of S = Q K^T (both operands K-major: two 64-element panels, 32 bytes per step inside a panel).
-template <int... KS>
-__device__ __forceinline__ void umma_scores(std::integer_sequence<int, KS...>, uint32_t d_tmem, uint64_t q_base, uint64_t k_base,
-                                            uint32_t idesc) {
-    (umma_ss_off<kmajor_off16(KS), kmajor_off16(KS)>(d_tmem, q_base, k_base, idesc, KS > 0 ? 1u : 0u), ...);
+__device__ __forceinline__ void umma_scores(uint32_t leader, uint32_t d_tmem, uint64_t q_base, uint64_t k_base, uint32_t idesc) {
+    umma_ss_by<false>(leader, d_tmem, q_base, k_base, idesc);
+#pragma unroll
+    for (int ks = 1; ks < 8; ++ks) umma_ss_by<true>(leader, d_tmem, q_base + kmajor_off16(ks), k_base + kmajor_off16(ks), idesc);
 }
-// The 8 K-steps of O += P V (P K-major as above, V MN-major: 2048 bytes per 16 keys).
-template <int... KK>
-__device__ __forceinline__ void umma_pv(std::integer_sequence<int, KK...>, uint32_t d_tmem, uint64_t p_base, uint64_t v_base,
-                                        uint32_t idesc, uint32_t acc_first) {
-    (umma_ss_off<kmajor_off16(KK), KK * 2048 / 16>(d_tmem, p_base, v_base, idesc, KK > 0 ? 1u : acc_first), ...);
+// K-steps FIRST .. FIRST + 3 of O += P V: P in tensor memory (8 columns per 16 keys), V MN-major (2048 bytes per 16 keys).
+template <int FIRST>
+__device__ __forceinline__ void umma_pv(uint32_t leader, uint32_t d_tmem, uint32_t p_tmem, uint64_t v_base, uint32_t idesc, uint32_t acc_first) {
+#pragma unroll
+    for (int kk = FIRST; kk < FIRST + 4; ++kk)
+        umma_ts_by(leader, d_tmem, p_tmem + kk * 8, v_base + kk * 2048 / 16, idesc, kk > FIRST ? 1u : acc_first);
 }
 
 __device__ __forceinline__ void tmem_ld32(uint32_t addr, uint32_t (&r)[32]) {
@@ -183,6 +207,12 @@ __device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&r)[16]
 }
 
 
+// 32 bytes, one sector.
+__device__ __forceinline__ void st_global_32(void* dst, const uint32_t* v) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n"
+                 ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+}
+
 // The TMEM loads are asynchronous: this pins the use of their results after the preceding
 // tcgen05.wait::ld in program order (the compiler may not move register arithmetic across it).
 __device__ __forceinline__ void reg_fence32(uint32_t (&r)[32]) {
@@ -210,6 +240,11 @@ __device__ __forceinline__ void unpack_f32x2(uint64_t v, float& lo, float& hi) {
 __device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
     uint64_t d;
     asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
 __device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
@@ -272,16 +307,11 @@ __device__ __forceinline__ float ex2_ordered(float x) {
     asm volatile("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
     return y;
 }
-template <bool MASK>
-__device__ __forceinline__ void scale_pair(uint32_t (&r)[32], int i, int key_base, int lim, uint64_t scale2, uint64_t neg_m2) {
+__device__ __forceinline__ void scale_pair(uint32_t (&r)[32], int i, uint64_t scale2, uint64_t neg_m2) {
     uint64_t d;
     asm volatile("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(d) : "l"(pack_f32x2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]))), "l"(scale2), "l"(neg_m2));
     float a, b;
     unpack_f32x2(d, a, b);
-    if (MASK) {
-        if (key_base + 2 * i >= lim) a = -INFINITY;
-        if (key_base + 2 * i + 1 >= lim) b = -INFINITY;
-    }
     r[2 * i] = __float_as_uint(a);
     r[2 * i + 1] = __float_as_uint(b);
 }
@@ -295,13 +325,12 @@ __device__ __forceinline__ uint32_t sum_pair(const uint32_t (&r)[32], int i, uin
 // spends most of its time on (two warps of a scheduler need 16 of its clocks per pair of elements), so the other work of a row is
 // issued in their shadow instead of before and after them.  Measured, 2 x 8192 tokens: 1086 -> 1150 TFLOP/s; 16 x 2048: 813 -> 890.
 // (A polynomial for one element in eight on the FMA pipe instead is slower, 1102: the step is not bound by the exponential unit alone.)
-template <typename T, bool MASK, bool NEXT, bool PREV>
-__device__ __forceinline__ void exp_stage(uint32_t (&cur)[32], uint32_t (&next)[32], const uint32_t (&prev)[32], uint32_t (&pk)[16], int next_base, int lim,
-                                          uint64_t scale2, uint64_t neg_m2, uint64_t& acc0, uint64_t& acc1) {
+template <typename T, bool NEXT, bool PREV>
+__device__ __forceinline__ void exp_stage(uint32_t (&cur)[32], uint32_t (&next)[32], const uint32_t (&prev)[32], uint32_t (&pk)[16], uint64_t scale2, uint64_t neg_m2, uint64_t& acc0, uint64_t& acc1) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
         cur[2 * i] = __float_as_uint(ex2_ordered(__uint_as_float(cur[2 * i])));
-        if (NEXT) scale_pair<MASK>(next, i, next_base, lim, scale2, neg_m2);
+        if (NEXT) scale_pair(next, i, scale2, neg_m2);
         cur[2 * i + 1] = __float_as_uint(ex2_ordered(__uint_as_float(cur[2 * i + 1])));
         if (PREV) pk[i] = sum_pair<T>(prev, i, (i & 1) ? acc1 : acc0);
     }
@@ -626,25 +655,59 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 }
 
 // =================================================================================================
-// Head-pair kernel: shared-memory layout and the softmax step.  A block works on the two query heads of a pair
-// that share a KV head (K and V tiles are loaded once for both) with 128-key tiles.  The probabilities go to
-// SHARED memory (canonical K-major 128-byte-swizzled panels, consumed as the A operand of an SS MMA) instead of
-// overwriting the scores in TMEM.  A softmax thread pulls its whole score row into registers first and releases
-// the score columns at once, so S_t(j+1) is computed while softmax_t(j) is still running and a tile's softmax
-// steps follow each other back to back; P.V_t(j) runs under softmax_t(j+1).  K is double buffered, V single
-// buffered, 224 KiB of shared memory and 512 TMEM columns per block.
+// Shared memory of the persistent kernel: two Q tiles and a ring of five 32 KiB stages that K and V tiles go through in the order of
+// their use.  Tensor memory: S0 S1 O0 O1, 128 columns each; a tile's probabilities lie in the first 64 columns of its scores.
 // =================================================================================================
-constexpr int kOff4Q = 0, kOff4K = 2 * kTileBytes, kOff4V = 4 * kTileBytes, kOff4P = 5 * kTileBytes, kOff4Bar = 7 * kTileBytes;
+constexpr int kRing5 = 5;
+constexpr int kOff4Q = 0, kOff4Ring = 2 * kTileBytes, kOff4Bar = (2 + kRing5) * kTileBytes;
 constexpr int kSmemBytes4 = kOff4Bar + 256 + 1024;
 
-// One 128-key online-softmax step of a row.  Scores are read once into registers; `on_scores_read` runs as
-// soon as they are (the caller releases the TMEM columns there); probabilities are written to `p_row`
-// (this row of the two swizzled P panels).  Returns false when a bounded wait gave up.
-template <typename T, typename OnRead>
-__device__ __forceinline__ bool softmax_row_to_smem(uint32_t t_s, uint32_t t_o, unsigned char* p_panels, int row,
-                                                    bool need_mask, int key0, int lim, float scale_log2, bool first,
-                                                    float& m_ref, float& l_run, uint32_t pv_done_bar, uint32_t pv_done_parity,
-                                                    volatile int* abort_flag, OnRead on_scores_read) {
+// Bounded waits of the persistent kernel, by one thread and by a whole warp (the same answer for all its lanes): they give up after 2 to 4 seconds
+// or as soon as another thread of the block gave up.  They are inlined at some twenty places, so that their size counts: the block leaves
+// its first error in shared memory and reports it once, at its end.
+__device__ __forceinline__ uint32_t clock_hi() {   // in units of 2^32 clocks
+    uint32_t c;
+    asm volatile("mov.u32 %0, %%clock_hi;" : "=r"(c));
+    return c;
+}
+template <bool WARP>
+__device__ __forceinline__ bool wait_bar_as(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code) {
+    auto all = [](bool v) { return WARP ? __all_sync(0xffffffffu, v) != 0 : v; };
+    if (all(mbar_try_wait(bar, parity) != 0)) return true;
+    const uint32_t start = clock_hi();
+    while (!all(mbar_try_wait(bar, parity) != 0)) {
+        if (!all(*abort_flag == 0 && clock_hi() - start <= 1u)) {
+            if (*abort_flag == 0) *abort_flag = code;
+            return false;
+        }
+    }
+    return true;
+}
+__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code) {
+    return wait_bar_as<false>(bar, parity, abort_flag, code);
+}
+__device__ __forceinline__ bool wait_bar_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code) {
+    return wait_bar_as<true>(bar, parity, abort_flag, code);
+}
+
+// Raw scores of keys 32 c .. 32 c + 31 of a tile: those from `seen` (keys of the tile that the row sees) on get no weight.  Chunks that the whole warp
+// sees are left alone.
+template <int C>
+__device__ __forceinline__ void hide_chunk(uint32_t (&r)[32], int seen) {
+    if (__all_sync(0xffffffffu, seen >= 32 * C + 32)) return;
+    const int n = min(max(seen - 32 * C, 0), 32);
+    const uint32_t keep = n == 32 ? 0xffffffffu : (1u << n) - 1u;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) r[i] = (keep >> i) & 1u ? r[i] : 0xff800000u;   // -infinity (the scale is positive)
+}
+
+// One online-softmax step of a row: 128 scores (columns of t_s) -> probabilities (16-bit pairs, the first 64 columns of t_s).  All scores are read
+// before the first probability is written.  `seen`: keys of the tile that the row sees; `masked`: some row of the warp does not see
+// all; `half`: no row of the item sees more than 64, the second half of the probabilities is not wanted.  `on_half` runs when the first 64 are
+// written.
+template <typename T, typename OnHalf>
+__device__ __forceinline__ void softmax_row(uint32_t t_s, uint32_t t_o, bool masked, int seen, bool half, float scale_log2, bool first,
+                                            float& m_ref, float& l_run, OnHalf on_half) {
     uint32_t r0[32], r1[32], r2[32], r3[32];
     tmem_ld32(t_s, r0);
     tmem_ld32(t_s + 32, r1);
@@ -652,40 +715,17 @@ __device__ __forceinline__ bool softmax_row_to_smem(uint32_t t_s, uint32_t t_o, 
     tmem_ld32(t_s + 96, r3);
     tc_wait_ld();
     reg_fence32(r0); reg_fence32(r1); reg_fence32(r2); reg_fence32(r3);
-    on_scores_read();
-    uint32_t pk[16], pk2[16];
-    auto store_chunk = [&](int c32, const uint32_t (&v)[16]) {   // 32 keys = four 16-byte pieces of this row
-        unsigned char* panel = p_panels + (c32 >> 1) * kPanelBytes + row * 128;
-#pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
-            const int cc = (c32 & 1) * 4 + q4;   // 16-byte column inside the 128-byte panel row
-            *reinterpret_cast<uint4*>(panel + ((cc ^ (row & 7)) << 4)) =
-                make_uint4(v[q4 * 4], v[q4 * 4 + 1], v[q4 * 4 + 2], v[q4 * 4 + 3]);
-        }
-    };
-    auto row_max = [&]() -> float {
-        float mx;
-        if (need_mask) {
-            mx = fmaxf(fmaxf(chunk_max<true>(r0, key0, lim), chunk_max<true>(r1, key0 + 32, lim)),
-                       fmaxf(chunk_max<true>(r2, key0 + 64, lim), chunk_max<true>(r3, key0 + 96, lim)));
-        } else {
-            mx = fmaxf(fmaxf(chunk_max<false>(r0, 0, 0), chunk_max<false>(r1, 0, 0)),
-                       fmaxf(chunk_max<false>(r2, 0, 0), chunk_max<false>(r3, 0, 0)));
-        }
-        return mx * scale_log2;
-    };
-    // P.V of the previous step must be complete before O is rescaled and before its P is overwritten: wait
-    // as late as that allows (with no rescale, after the first 64 exponentials).
-    bool pv_waited = first;
-    const float mx = row_max();
+    if (masked) {
+        hide_chunk<0>(r0, seen); hide_chunk<1>(r1, seen); hide_chunk<2>(r2, seen); hide_chunk<3>(r3, seen);
+    }
+    const float mx = fmaxf(fmaxf(chunk_max<false>(r0, 0, 0), chunk_max<false>(r1, 0, 0)),
+                           fmaxf(chunk_max<false>(r2, 0, 0), chunk_max<false>(r3, 0, 0))) * scale_log2;
     if (__any_sync(0xffffffffu, mx > m_ref + kRescaleThreshold)) {
-        if (!pv_waited && !warp_mbar_wait(pv_done_bar, pv_done_parity, abort_flag, 42)) return false;
-        pv_waited = true;
         const float m_new = fmaxf(m_ref, mx);
         const float f = (m_new == -INFINITY) ? 1.0f : fast_exp2(m_ref - m_new);
         if (!first) {
-            tc_fence_after();
-#pragma unroll
+            // (the previous P.V was issued before these scores by the same thread: it is complete)
+#pragma unroll 1
             for (int c = 0; c < 4; ++c) {
                 uint32_t r[32];
                 tmem_ld32(t_o + c * 32, r);
@@ -694,7 +734,6 @@ __device__ __forceinline__ bool softmax_row_to_smem(uint32_t t_s, uint32_t t_o, 
                 for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * f);
                 tmem_st32(t_o + c * 32, r);
             }
-            tc_wait_st();
         }
         l_run *= f;
         m_ref = m_new;
@@ -702,50 +741,53 @@ __device__ __forceinline__ bool softmax_row_to_smem(uint32_t t_s, uint32_t t_o, 
     const float m_use = (m_ref == -INFINITY) ? 0.0f : m_ref;
     const uint64_t scale2 = pack_f32x2(scale_log2, scale_log2), neg_m2 = pack_f32x2(-m_use, -m_use);
     uint64_t acc0 = 0ull, acc1 = 0ull;
-    bool ok = true;
-    auto stages = [&](auto mask) {
-        constexpr bool M = decltype(mask)::value;
+    uint32_t pk[16], pk2[16];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) scale_pair<M>(r0, i, key0, lim, scale2, neg_m2);
-        exp_stage<T, M, true, false>(r0, r1, r0, pk, key0 + 32, lim, scale2, neg_m2, acc0, acc1);
-        exp_stage<T, M, true, true>(r1, r2, r0, pk, key0 + 64, lim, scale2, neg_m2, acc0, acc1);
-        // the first 64 probabilities wait in registers: by then the previous P.V has all but always completed
-        if (!pv_waited && !warp_mbar_wait(pv_done_bar, pv_done_parity, abort_flag, 43)) { ok = false; return; }
-        store_chunk(0, pk);
-        exp_stage<T, M, true, true>(r2, r3, r1, pk2, key0 + 96, lim, scale2, neg_m2, acc0, acc1);
-        store_chunk(1, pk2);
-        exp_stage<T, M, false, true>(r3, r3, r2, pk, 0, 0, scale2, neg_m2, acc0, acc1);
-        store_chunk(2, pk);
+    for (int i = 0; i < 16; ++i) scale_pair(r0, i, scale2, neg_m2);
+    exp_stage<T, true, false>(r0, r1, r0, pk, scale2, neg_m2, acc0, acc1);
+    exp_stage<T, true, true>(r1, r2, r0, pk, scale2, neg_m2, acc0, acc1);
+    tmem_st16(t_s, pk);
+    if (half) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) pk2[i] = sum_pair<T>(r1, i, (i & 1) ? acc1 : acc0);
+        tmem_st16(t_s + 16, pk2);
+        on_half();
+    } else {
+        exp_stage<T, true, true>(r2, r3, r1, pk2, scale2, neg_m2, acc0, acc1);
+        tmem_st16(t_s + 16, pk2);
+        on_half();
+        exp_stage<T, false, true>(r3, r3, r2, pk, scale2, neg_m2, acc0, acc1);
+        tmem_st16(t_s + 32, pk);
 #pragma unroll
         for (int i = 0; i < 16; ++i) pk2[i] = sum_pair<T>(r3, i, (i & 1) ? acc1 : acc0);
-        store_chunk(3, pk2);
-    };
-    if (need_mask) stages(std::true_type{}); else stages(std::false_type{});
-    if (!ok) return false;
+        tmem_st16(t_s + 48, pk2);
+    }
     float a0, a1, a2, a3;
     unpack_f32x2(acc0, a0, a1);
     unpack_f32x2(acc1, a2, a3);
     l_run += (a0 + a1) + (a2 + a3);
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // generic-proxy stores -> visible to the MMA
-    return true;
 }
 
-
-
 // =================================================================================================
-// The persistent head-pair kernel.  One block per SM takes (query tile, head pair) items from a
-// ticket counter, heaviest query tiles first, and keeps TMEM, barriers and the three warp roles alive
-// across items: while the softmax warps write one item's output (staged in the P buffer, which the
-// last P.V has finished with), the producer has already fetched the next item's Q and first K tiles and
-// the issuer has its first score MMAs in flight.  A block launched per item pays the fill and drain of
-// the chain load -> S -> softmax -> P.V -> store (about 1.5 rounds) every time; here only the first
-// and last item of a block do.  All barrier phases are counted cumulatively over items.
+// The persistent head-pair kernel.  An item is one stretch of query rows x the heads of two tiles, all of one KV head, so that a K / V tile is loaded
+// once for both.  One block per SM takes items from a ticket counter and keeps TMEM, barriers and the warp roles alive across items.  Per 128-key
+// round and tile: S = Q K^T (SS MMA), softmax by one warpgroup (thread = row), P over the first half of its scores in tensor memory, O += P V (TS MMA).
+//
+// What bounds it is the chain of a tile's round, S -> softmax -> P.V -> next S, with two tiles taking turns: one tile's softmax runs under the other
+// tile's MMAs.  MMAs need 2048 clocks a round and exponentials as many.  What made the chain long was not arithmetic but how fast the code runs
+// (clocks a round, one item alone; us for 2 x 8192 / 16 x 2048 / 32 x 512 / 24 x 310 tokens, 32 / 8 heads):
+//   3600; 958 / 618 / 160 / 89     P through shared memory, one diverged lane issuing the MMAs of a tile, 126 KB of code
+//   4060; 984 / 565 / 114 / 57     P in tensor memory, K and V in a ring of five stages, half of the code (short waits, one mask pass, one copy of
+//                                  each role's body): roles that alternate over more code than the instruction caches hold wait for it, a
+//                                  masked round took 9000 clocks where a steady one took 2600
+//   3043; 832 / 498 / 101 / 50     the issuing warp converged, descriptors in uniform registers (umma_ss_by)
+// Tiles of 128 >> head_shift query rows x 1 << head_shift heads instead of 128 rows of one head lose less on ragged ends and on the diagonal, and an item
+// whose rows see at most half of their last key tile leaves out that tile's second half.  All barrier phases are counted cumulatively over items.
 // =================================================================================================
 // Ticket counters.  Launches that run at the same time must not share one: each would leave out items that the other took.  An eager launch takes
 // the next of 32768, far more launches than streams hold in their queues; a captured one keeps its counter for all replays of its graph,
 // so these have 32768 of their own, which no eager launch meets.
 constexpr int kEagerSlots = 32768, kTicketSlots = 2 * kEagerSlots;
-constexpr int kIssuers5 = 2;        // issuing warps, one per query tile
 constexpr int kThreads5 = 384;      // three warpgroups (register reallocation works on whole warpgroups)
 constexpr int kRegsLow5 = 56;       // registers per thread of the third warpgroup after setmaxnreg.dec
 constexpr int kRegsHigh5 = 224;     // registers per thread of the two softmax warpgroups after setmaxnreg.inc
@@ -755,21 +797,22 @@ __device__ unsigned int g_prefill_ticket[kTicketSlots];
 
 struct Tc5Params {
     TcParams base;
-    int pairs;            // head pairs
+    int head_shift;       // a tile's 128 rows are 128 >> head_shift query rows x 1 << head_shift heads
+    int pairs;            // pairs of tiles that make up all heads
     int tiles;            // upper bound of query tiles over all sequences
     unsigned int total;   // pairs * tiles
     int slot;             // ticket counter of this launch
 };
 
-// One (query tile, head pair), with all that the roles need to know of it, so that none of them reads the sequence bounds again.
+// One (query tile, pair of head sets), with all that the roles need to know of it, so that none of them reads the sequence bounds again.
 struct Tc5Item {
     int kind;             // 1 = work, 0 = no more work
     int seq, pair;
     int q_row, rows;      // first query row and the rows there are
     int lim0, k_len;      // query row r sees keys [0, min(lim0 + r, k_len))
     int num_kt, last_partial;
+    int half;             // no row sees more than 64 keys of the last tile
     int k_row;            // row of the sequence's first key (keys without a block table)
-    int row0, row1;       // rows of its first two key tiles
 };
 
 // Row of key `key0` of a sequence in the K / V tensors; key_rows (past the end: the copy fills zeros) for an invalid block.
@@ -789,15 +832,18 @@ struct Tc5Finder {
     int mine;                  // tiles of the window before this lane's sequence
     int tiles, qb, qe, kb, ke; // of this lane's sequence
 
-    __device__ __forceinline__ void load(const TcParams& p, int lane) {
+    __device__ __forceinline__ void load(const TcParams& p, int tile_rows, int lane) {
         qb = 0; qe = 0; kb = 0; ke = 0;
         if (p.cu_q == nullptr) {
             if (lane == 0) { qe = static_cast<int>(p.total_q); ke = static_cast<int>(p.total_k); }
         } else if (base + lane < p.num_seqs) {
-            qb = static_cast<int>(p.cu_q[base + lane]); qe = static_cast<int>(p.cu_q[base + lane + 1]);
-            kb = static_cast<int>(p.cu_k[base + lane]); ke = static_cast<int>(p.cu_k[base + lane + 1]);
+            // (the low words: the bounds are below 2^31, and both widths take one load without a branch)
+            const int *q = static_cast<const int*>(p.cu_q.ptr) + (static_cast<size_t>(base + lane) << p.cu_q.wide);
+            const int *k = static_cast<const int*>(p.cu_k.ptr) + (static_cast<size_t>(base + lane) << p.cu_k.wide);
+            qb = q[0]; qe = q[1 << p.cu_q.wide];
+            kb = k[0]; ke = k[1 << p.cu_k.wide];
         }
-        tiles = max((qe - qb + kBM - 1) / kBM, 0);
+        tiles = max((qe - qb + tile_rows - 1) / tile_rows, 0);
         int inc = tiles;
 #pragma unroll
         for (int d = 1; d < 32; d *= 2) {
@@ -808,27 +854,31 @@ struct Tc5Finder {
         sum = __shfl_sync(0xffffffffu, inc, 31);
     }
     // Opens on the last window (the first tile asked for is the last one) and returns the number of tiles of all sequences.
-    __device__ __forceinline__ int open(const TcParams& p, int lane) {
-        base = 0; before = 0;
-        load(p, lane);
-        while (p.cu_q != nullptr && base + 32 < p.num_seqs) { before += sum; base += 32; load(p, lane); }
-        return before + sum;
+    __device__ __forceinline__ int open(const TcParams& p, int tile_rows, int lane) {
+        before = 0;
+#pragma unroll 1
+        for (base = 0;; base += 32, before += sum) {
+            load(p, tile_rows, lane);
+            if (p.cu_q == nullptr || base + 32 >= p.num_seqs) return before + sum;
+        }
     }
     // Tile number `want`, in [0, open()): its item, without the pair.
-    __device__ __forceinline__ void find(const TcParams& p, int lane, int want, Tc5Item& it) {
-        while (want < before) { base -= 32; load(p, lane); before -= sum; }
+    __device__ __forceinline__ void find(const TcParams& p, int tile_rows, int lane, int want, Tc5Item& it) {
+#pragma unroll 1
+        while (want < before) { base -= 32; load(p, tile_rows, lane); before -= sum; }
         const int at = 31 - __clz(__ballot_sync(0xffffffffu, before + mine <= want && tiles > 0));
-        const int q0 = (want - before - __shfl_sync(0xffffffffu, mine, at)) * kBM;
+        const int q0 = (want - before - __shfl_sync(0xffffffffu, mine, at)) * tile_rows;
         const int q_begin = __shfl_sync(0xffffffffu, qb, at), q_len = __shfl_sync(0xffffffffu, qe, at) - q_begin;
         it.seq = base + at;
         it.q_row = q_begin + q0;
-        it.rows = min(kBM, q_len - q0);
+        it.rows = min(tile_rows, q_len - q0);
         it.k_row = __shfl_sync(0xffffffffu, kb, at);
         it.k_len = __shfl_sync(0xffffffffu, ke, at) - it.k_row;
         it.lim0 = it.k_len - q_len + q0 + 1;
         const int k_hi = min(it.lim0 + it.rows - 1, it.k_len);
         it.num_kt = k_hi > 0 ? (k_hi + kBN - 1) / kBN : 0;
         it.last_partial = it.num_kt * kBN > it.k_len ? it.num_kt - 1 : -1;
+        it.half = k_hi <= it.num_kt * kBN - kBN / 2 ? 1 : 0;
     }
 };
 
@@ -861,7 +911,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     __shared__ int s_abort;
     __shared__ Tc5Item s_ring[4];
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;   // (uniform, also to the compiler)
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     unsigned char* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
     auto decode_half = [&]() {
@@ -894,26 +944,24 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         __syncthreads();
     }
-    const uint32_t sm_q = smem_base + kOff4Q, sm_k = smem_base + kOff4K, sm_v = smem_base + kOff4V, sm_p = smem_base + kOff4P;
+    const uint32_t sm_q = smem_base + kOff4Q, sm_ring = smem_base + kOff4Ring;
     const uint32_t bars = smem_base + kOff4Bar;
-    const uint32_t bar_qfull = bars, bar_vfix = bars + 8, bar_vfull = bars + 16, bar_vempty = bars + 24, bar_qempty = bars + 144;
-    auto bar_kfull = [&](int s) { return bars + 32 + 8 * s; };
-    auto bar_kempty = [&](int s) { return bars + 48 + 8 * s; };
-    auto bar_sfull = [&](int t) { return bars + 64 + 8 * t; };
-    auto bar_sread = [&](int t) { return bars + 80 + 8 * t; };
-    auto bar_pfull = [&](int t) { return bars + 96 + 8 * t; };
-    auto bar_odone = [&](int t) { return bars + 112 + 8 * t; };
-    auto bar_ofinal = [&](int t) { return bars + 128 + 8 * t; };
-    auto bar_item = [&](int s) { return bars + 152 + 8 * s; };   // ring entry s published
+    const uint32_t bar_qfull = bars, bar_qempty = bars + 8;
+    auto bar_full = [&](int s) { return bars + 16 + 8 * s; };      // ring stage s has landed
+    auto bar_empty = [&](int s) { return bars + 56 + 8 * s; };     // and has been read by both tiles' MMAs
+    auto bar_sfull = [&](int t) { return bars + 96 + 8 * t; };     // scores of a tile (and its P.V before that) complete
+    auto bar_phalf = [&](int t) { return bars + 112 + 8 * t; };    // first 64 keys' probabilities of a tile in tensor memory
+    auto bar_pfull = [&](int t) { return bars + 128 + 8 * t; };    // all of them
+    auto bar_ofinal = [&](int t) { return bars + 144 + 8 * t; };   // an item's last P.V of a tile complete
+    auto bar_item = [&](int s) { return bars + 160 + 8 * s; };     // ring entry s published
     volatile int* abort_flag = &s_abort;
 
     if (tid == 0) {
         s_abort = 0;
-        mbar_init(bar_qfull, 1); mbar_init(bar_qempty, kIssuers5); mbar_init(bar_vfix, 1); mbar_init(bar_vfull, 1); mbar_init(bar_vempty, kIssuers5);
+        mbar_init(bar_qfull, 1); mbar_init(bar_qempty, 1);
+        for (int i = 0; i < kRing5; ++i) { mbar_init(bar_full(i), 1); mbar_init(bar_empty(i), 1); }
         for (int i = 0; i < 2; ++i) {
-            mbar_init(bar_kfull(i), 1); mbar_init(bar_kempty(i), kIssuers5);
-            mbar_init(bar_sfull(i), 1); mbar_init(bar_sread(i), 4); mbar_init(bar_pfull(i), 4);
-            mbar_init(bar_odone(i), 1); mbar_init(bar_ofinal(i), 1);
+            mbar_init(bar_sfull(i), 1); mbar_init(bar_phalf(i), 4); mbar_init(bar_pfull(i), 4); mbar_init(bar_ofinal(i), 1);
         }
         for (int i = 0; i < 4; ++i) mbar_init(bar_item(i), 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -928,7 +976,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = s_tmem_base;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, s_tmem_base, 0);
     const size_t out_stride = static_cast<size_t>(p.num_heads) * kHeadDim;
 
     // Three warpgroups: 0 and 1 are the softmax warps of tile 0 and 1, 2 holds the issuer, the producer and two idle
@@ -940,174 +988,167 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kRegsLow5));
     if (warp == 9) {
         // ------------------------------------------------------------------ ticket taker + TMA producer
-        int n = 0;            // items published so far (all of them carry work)
-        int gk = 0, gv = 0;   // K / V tiles loaded so far, over all items
-        bool ok = true;
-        // The first ticket is taken under the look at the sequence bounds.
+        const int tile_rows = kBM >> pp.head_shift, item_heads = 2 << pp.head_shift;
         unsigned int ticket = 0;
-        bool have_ticket = true;
-        if (lane == 0) ticket = atomicAdd(&g_prefill_ticket[pp.slot], 1u);
+        if (lane == 0) ticket = atomicAdd(&g_prefill_ticket[pp.slot], 1u);   // (the first one under the look at the sequence bounds)
         Tc5Finder find;
-        const int tiles = min(find.open(p, lane), pp.tiles);
+        const int tiles = min(find.open(p, tile_rows, lane), pp.tiles);
         const unsigned int total = static_cast<unsigned int>(tiles) * static_cast<unsigned int>(pp.pairs);
-        // Next item that carries work (whole warp).  Tiles whose rows see no key are zero-filled right here and never published.
-        auto take_item = [&]() -> Tc5Item {
-            Tc5Item it{};
+        int stage = 0, n = -1;   // ring stage of the next K / V tile; the item that is being loaded, -1: none yet
+        uint32_t turn = 0;       // parity of that stage's round through the ring
+        int row = 0, next_row = 0, kvh = 0;
+        bool ok = true;
+        auto load = [&](const CUtensorMap* map, int r) {   // lane 0: the next K or V tile
+            ok = ok && wait_bar(bar_empty(stage), turn ^ 1u, abort_flag, 11);   // (passes at once the first time round)
+            if (!ok) return;
+            const uint32_t dst = sm_ring + stage * kTileBytes, bar = bar_full(stage);
+            mbar_expect_tx(bar, kTileBytes);
+            tma_load_3d(dst, map, 0, kvh, r, bar);
+            tma_load_3d(dst + kPanelBytes, map, 64, kvh, r, bar);
+            if (++stage == kRing5) { stage = 0; turn ^= 1u; }
+        };
+        Tc5Item it{};
+        // Item n is published, its first tiles are under way: take the next ticket under its rounds, then see to the rest of its tiles.  Where a wait
+        // gave up nothing is published any more, but the tickets are still taken to the end.
+        while (true) {
+            Tc5Item next{};
             while (true) {
-                if (!have_ticket && lane == 0) ticket = atomicAdd(&g_prefill_ticket[pp.slot], 1u);
-                have_ticket = false;
                 ticket = __shfl_sync(0xffffffffu, ticket, 0);
                 if (ticket >= total) {
                     if (lane == 0 && ticket == total + gridDim.x - 1) g_prefill_ticket[pp.slot] = 0u;
-                    return it;
+                    break;
                 }
-                it.pair = static_cast<int>(ticket % static_cast<unsigned int>(pp.pairs));
-                find.find(p, lane, tiles - 1 - static_cast<int>(ticket / static_cast<unsigned int>(pp.pairs)), it);
-                if (it.num_kt > 0) break;
-                for (int t = 0; t < 2; ++t) {
-                    T* o0 = static_cast<T*>(p.out) + (static_cast<size_t>(it.q_row) * p.num_heads + 2 * it.pair + t) * kHeadDim;
-                    for (int i = lane; i < it.rows * (kHeadDim / 8); i += 32) {
-                        const int r = i / (kHeadDim / 8), c = i % (kHeadDim / 8);
-                        *reinterpret_cast<uint4*>(o0 + r * out_stride + c * 8) = make_uint4(0u, 0u, 0u, 0u);
-                    }
-                }
+                const unsigned int tile = ticket / static_cast<unsigned int>(pp.pairs);
+                next.pair = static_cast<int>(ticket - tile * static_cast<unsigned int>(pp.pairs));
+                find.find(p, tile_rows, lane, tiles - 1 - static_cast<int>(tile), next);
+                if (next.num_kt > 0) { next.kind = 1; break; }
+                // rows that see no key: zeros, and the next ticket
+                T* o0 = static_cast<T*>(p.out) + (static_cast<size_t>(next.q_row) * p.num_heads + item_heads * next.pair) * kHeadDim;
+#pragma unroll 1
+                for (int r = 0; r < next.rows; ++r)
+#pragma unroll 1
+                    for (int c = lane; c < item_heads * (kHeadDim / 8); c += 32) *reinterpret_cast<uint4*>(o0 + r * out_stride + c * 8) = make_uint4(0u, 0u, 0u, 0u);
+                if (lane == 0) ticket = atomicAdd(&g_prefill_ticket[pp.slot], 1u);
             }
-            it.kind = 1;
-            const int row = lane < 2 && lane < it.num_kt ? tc5_key_row(p, it.seq, it.k_row, lane * kBN) : 0;   // (both trips at once)
-            it.row0 = __shfl_sync(0xffffffffu, row, 0);
-            it.row1 = __shfl_sync(0xffffffffu, row, 1);
-            return it;
-        };
-        Tc5Item next = take_item();
-        while (ok) {
-            const Tc5Item it = next;
-            if (lane == 0) {
-                s_ring[n & 3] = it;
-                mbar_arrive(bar_item(n & 3));   // release: the entry is visible to whoever waits on the barrier
-            }
-            if (!it.kind) break;
-            const int head0 = 2 * it.pair;
-            const int kvh = head0 * p.num_kv_heads / p.num_heads;
-            auto load_k = [&](int j, int r) -> bool {   // lane 0 only
-                const int c = gk + j, s = c & 1;
-                if (c >= 2 && !mbar_wait(bar_kempty(s), ((c >> 1) & 1) ^ 1, abort_flag, 11)) return false;
-                mbar_expect_tx(bar_kfull(s), kTileBytes);
-                tma_load_3d(sm_k + s * kTileBytes, &tm_k, 0, kvh, r, bar_kfull(s));
-                tma_load_3d(sm_k + s * kTileBytes + kPanelBytes, &tm_k, 64, kvh, r, bar_kfull(s));
-                return true;
-            };
-            if (lane == 0) {
-                if (n >= 1) ok = mbar_wait(bar_qempty, (n - 1) & 1, abort_flag, 14);   // previous item's score MMAs are done with Q
-                if (ok) {
-                    mbar_expect_tx(bar_qfull, 2 * kTileBytes);
-                    for (int t = 0; t < 2; ++t) {
-                        tma_load_3d(sm_q + t * kTileBytes, &tm_q, 0, head0 + t, it.q_row, bar_qfull);
-                        tma_load_3d(sm_q + t * kTileBytes + kPanelBytes, &tm_q, 64, head0 + t, it.q_row, bar_qfull);
-                    }
-                    ok = load_k(0, it.row0);
+            int first_row = 0;   // rows of its first two key tiles, both trips at once
+            if (next.kind != 0 && lane < 2 && lane < next.num_kt) first_row = tc5_key_row(p, next.seq, next.k_row, lane * kBN);
+            if (n >= 0 && lane == 0) {
+#pragma unroll 1
+                for (int j = 1; j < it.num_kt; ++j) {
+                    row = next_row;
+                    if (j + 1 < it.num_kt) next_row = tc5_key_row(p, it.seq, it.k_row, (j + 1) * kBN);   // (a block's id is read a round before its copy)
+                    load(&tm_k, row);
+                    load(&tm_v, row);
                 }
             }
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-            int row = it.row0, next_row = it.row1;   // (a block's id is read a round before its copy)
-            for (int j = 0; j < it.num_kt && ok; ++j) {
-                const int cv = gv + j;
-                if (lane == 0) {
-                    if (j + 1 < it.num_kt) ok = load_k(j + 1, next_row);            // K runs one tile ahead of V
-                    if (ok && cv >= 1) ok = mbar_wait(bar_vempty, (cv - 1) & 1, abort_flag, 12);
-                    if (ok) {
-                        mbar_expect_tx(bar_vfull, kTileBytes);
-                        tma_load_3d(sm_v, &tm_v, 0, kvh, row, bar_vfull);
-                        tma_load_3d(sm_v + kPanelBytes, &tm_v, 64, kvh, row, bar_vfull);
-                    }
-                    row = next_row;
-                    if (j + 2 < it.num_kt) next_row = tc5_key_row(p, it.seq, it.k_row, (j + 2) * kBN);
-                }
-                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-                if (ok && j == it.last_partial) {
-                    // rows of V past the sequence may hold anything (0 * NaN = NaN): zero them once landed
-                    ok = warp_mbar_wait(bar_vfull, cv & 1, abort_flag, 13);
-                    if (ok) {
-                        const int first_bad = it.k_len - j * kBN;   // in (0, 128)
-                        for (int i = lane; i < (kBN - first_bad) * 16; i += 32) {
-                            const int r = first_bad + i / 16, c16 = i % 16;
-                            *reinterpret_cast<uint4*>(smem_gen + kOff4V + (c16 >> 3) * kPanelBytes + r * 128 + (c16 & 7) * 16) =
-                                make_uint4(0u, 0u, 0u, 0u);
-                        }
-                        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(bar_vfix);
-                    }
-                }
-                if (ok && j == 0) next = take_item();   // under this item's rounds
+            it = next;
+            ++n;
+            row = first_row;
+            next_row = __shfl_sync(0xffffffffu, first_row, 1);
+            if (lane == 0 && ok) {
+                s_ring[n & 3] = it;
+                mbar_arrive(bar_item(n & 3));   // release: the entry is visible to whoever waits on the barrier
             }
-            gk += it.num_kt; gv += it.num_kt; ++n;
-        }
-        while (!ok && next.kind) next = take_item();   // a wait gave up: the tickets are still taken to the end
-    } else if (warp == 8 || warp == 8 + 2 * (kIssuers5 - 1)) {
-        // ------------------------------------------------------------------ MMA issuer(s): with two, warp 8 drives
-        // tile 0 and warp 10 tile 1 (a single thread sustained about one MMA per 100 clocks here, the tensor pipe one per 64)
-        if (lane == 0) {
-            const int t_lo = (kIssuers5 == 2 && warp != 8) ? 1 : 0;
-            const int t_hi = (kIssuers5 == 2 && warp == 8) ? 1 : 2;
-            int n = 0, G = 0, gk = 0, gv = 0, nf = 0;   // items, rounds, K tiles, V tiles, partial-tile fixes so far
-            bool ok = true;
-            // One base descriptor per operand buffer; a tile-internal offset only moves the 14-bit start-address
-            // field (units of 16 bytes, never carrying out of it), so each MMA's descriptors are one add away and
-            // the issuer needs few registers.
-            const uint64_t dq[2] = {make_smem_desc(sm_q, 16, 1024), make_smem_desc(sm_q + kTileBytes, 16, 1024)};
-            const uint64_t dk[2] = {make_smem_desc(sm_k, 16, 1024), make_smem_desc(sm_k + kTileBytes, 16, 1024)};
-            const uint64_t dp[2] = {make_smem_desc(sm_p, 16, 1024), make_smem_desc(sm_p + kTileBytes, 16, 1024)};
-            const uint64_t dv = make_smem_desc(sm_v, kPanelBytes, 1024);
-            while (ok) {
-                ok = mbar_wait(bar_item(n & 3), (n >> 2) & 1, abort_flag, 28);
-                if (!ok) break;
-                const Tc5Item it = s_ring[n & 3];
-                if (it.kind == 0) break;
-                auto issue_s = [&](int t, int j) {
-                    const int s = (gk + j) & 1;
-                    umma_scores(std::make_integer_sequence<int, 8>{}, tmem_base + t * 128, dq[t], dk[s], p.idesc_s);
-                    tc_commit(bar_sfull(t));
-                };
-                // scores of the item's first key tile: Q and K(0) landed, the previous round's scores were read
-                ok = mbar_wait(bar_qfull, n & 1, abort_flag, 21) && mbar_wait(bar_kfull(gk & 1), (gk >> 1) & 1, abort_flag, 22);
-                for (int t = t_lo; t < t_hi && ok; ++t) {
-                    if (G >= 1) ok = mbar_wait(bar_sread(t), (G - 1) & 1, abort_flag, 29);
-                    if (!ok) break;
-                    tc_fence_after();
-                    issue_s(t, 0);
-                }
-                if (!ok) break;
-                tc_commit(bar_kempty(gk & 1));              // (every issuer arrives)
-                if (it.num_kt == 1) tc_commit(bar_qempty);   // every score MMA of the item has been issued
-                for (int j = 0; j < it.num_kt && ok; ++j) {
-                    if (j + 1 < it.num_kt) {   // next scores as soon as this step's scores have been read
-                        const int c = gk + j + 1;
-                        ok = mbar_wait(bar_kfull(c & 1), (c >> 1) & 1, abort_flag, 26);
-                        for (int t = t_lo; t < t_hi && ok; ++t) {
-                            ok = mbar_wait(bar_sread(t), (G + j) & 1, abort_flag, 27);
-                            if (!ok) break;
-                            tc_fence_after();
-                            issue_s(t, j + 1);
-                        }
-                        if (!ok) break;
-                        tc_commit(bar_kempty(c & 1));
-                        if (j + 2 == it.num_kt) tc_commit(bar_qempty);
+            if (it.kind == 0) break;
+            if (lane == 0) {
+                const int head0 = item_heads * it.pair;
+                kvh = head0 * p.num_kv_heads / p.num_heads;
+                load(&tm_k, row);
+                if (n >= 1) ok = ok && wait_bar(bar_qempty, (n - 1) & 1, abort_flag, 14);   // previous item's score MMAs are done with Q
+                if (ok) {
+                    mbar_expect_tx(bar_qfull, 2 * kTileBytes);
+#pragma unroll 1
+                    for (int t = 0; t < 2; ++t) {
+                        const int head = head0 + (t << pp.head_shift);
+                        tma_load_3d(sm_q + t * kTileBytes, &tm_q, 0, head, it.q_row, bar_qfull);
+                        tma_load_3d(sm_q + t * kTileBytes + kPanelBytes, &tm_q, 64, head, it.q_row, bar_qfull);
                     }
-                    ok = mbar_wait(bar_vfull, (gv + j) & 1, abort_flag, 23);
-                    if (ok && j == it.last_partial) ok = mbar_wait(bar_vfix, nf & 1, abort_flag, 24);
-                    for (int t = t_lo; t < t_hi && ok; ++t) {
-                        // p_full of an item's first round also says that the previous item's output has left TMEM
-                        ok = mbar_wait(bar_pfull(t), (G + j) & 1, abort_flag, 25);
+                }
+                load(&tm_v, row);
+                ticket = atomicAdd(&g_prefill_ticket[pp.slot], 1u);
+            }
+        }
+    } else if (warp == 8) {
+        // ------------------------------------------------------------------ MMA issuer, one for both tiles: P.V of a tile and then
+        // its next scores, then the same of the other tile, so that one tile's softmax runs under the other tile's MMAs.
+        {
+            const uint32_t leader = elect_one();
+            const uint64_t dq0 = make_smem_desc(sm_q, 16, 1024);
+            const uint64_t dk0 = make_smem_desc(sm_ring, 16, 1024), dv0 = make_smem_desc(sm_ring, kPanelBytes, 1024);
+            constexpr uint64_t kTile16 = kTileBytes / 16;   // (only moves the descriptor's start address, never carrying out of it)
+            int ks = 0, vs = 1;           // ring stages of the next K and V tile, parities of their rounds through the ring
+            uint32_t kturn = 0, vturn = 0;
+            auto advance = [](int& s, uint32_t& turn) { s += 2; if (s >= kRing5) { s -= kRing5; turn ^= 1u; } };
+            int n = -1, G = 0;            // the item whose P.V is next, and the rounds before this one; -1: only scores
+            int j = 0, num_kt = 1, half = 0;   // its round, its rounds, whether the last one has keys in its first half only
+            int next_kt = 0, next_half = 0;
+            bool ok = true, more = true;
+            while (ok && more) {
+                const bool last = j + 1 == num_kt;
+                int scores = 0;           // tiles whose scores of the following round are issued
+                bool there = false;       // that round's operands have landed
+                if (n >= 0) ok = wait_bar_warp(bar_full(vs), vturn, abort_flag, 23);
+#pragma unroll 1
+                for (int t = 0; t < 2 && ok; ++t) {
+                    if (n >= 0) {
+                        const uint64_t dv = dv0 + vs * kTile16;
+                        const uint32_t t_s = tmem_base + t * 128, t_o = tmem_base + 256 + t * 128;
+                        // (an item's first round: the probabilities also say that the previous item's output has left tensor memory)
+                        ok = wait_bar_warp(bar_phalf(t), G & 1, abort_flag, 25);
                         if (!ok) break;
                         tc_fence_after();
-                        umma_pv(std::make_integer_sequence<int, 8>{}, tmem_base + 256 + t * 128, dp[t], dv, p.idesc_pv, j > 0 ? 1u : 0u);
-                        tc_commit(bar_odone(t));
-                        if (j == it.num_kt - 1) tc_commit(bar_ofinal(t));
+                        umma_pv<0>(leader, t_o, t_s, dv, p.idesc_pv, j > 0 ? 1u : 0u);
+                        ok = wait_bar_warp(bar_pfull(t), G & 1, abort_flag, 27);
+                        if (!ok) break;
+                        if (!(last && half)) {
+                            tc_fence_after();
+                            umma_pv<4>(leader, t_o, t_s, dv, p.idesc_pv, 1u);
+                        }
+                        if (t == 1) tc_commit_by(leader, bar_empty(vs));
+                        if (last) tc_commit_by(leader, bar_ofinal(t));
                     }
-                    if (ok) tc_commit(bar_vempty);
+                    if (!there && more) {
+                        // The next round's K tile; of the next item also what there is and Q.  Tile 0 does not wait for these: this item's other
+                        // tile comes first then.
+                        const uint32_t item = bar_item((n + 1) & 3), turn_i = ((n + 1) >> 2) & 1;
+                        if (!last) {
+                            ok = wait_bar_warp(bar_full(ks), kturn, abort_flag, 26);
+                        } else {
+                            if (t == 0 && !__all_sync(0xffffffffu, mbar_test(item, turn_i) && mbar_test(bar_qfull, (n + 1) & 1) && mbar_test(bar_full(ks), kturn))) continue;
+                            ok = wait_bar_warp(item, turn_i, abort_flag, 29);
+                            if (!ok) break;
+                            const Tc5Item& it = s_ring[(n + 1) & 3];
+                            more = __shfl_sync(0xffffffffu, it.kind, 0) != 0;
+                            if (!more) continue;
+                            next_kt = __shfl_sync(0xffffffffu, it.num_kt, 0);
+                            next_half = __shfl_sync(0xffffffffu, it.half, 0);
+                            ok = wait_bar_warp(bar_qfull, (n + 1) & 1, abort_flag, 21) && wait_bar_warp(bar_full(ks), kturn, abort_flag, 22);
+                        }
+                        if (!ok) break;
+                        tc_fence_after();
+                        there = true;
+                    }
+                    if (there) {
+#pragma unroll 1
+                        for (; scores <= t; ++scores) {
+                            umma_scores(leader, tmem_base + scores * 128, dq0 + scores * kTile16, dk0 + ks * kTile16, p.idesc_s);
+                            tc_commit_by(leader, bar_sfull(scores));
+                        }
+                    }
                 }
-                G += it.num_kt; gk += it.num_kt; gv += it.num_kt; ++n;
-                if (it.last_partial >= 0) ++nf;
+                if (!ok) break;
+                if (n >= 0) { advance(vs, vturn); ++G; }
+                if (!last) {
+                    ++j;
+                } else {
+                    j = 0; num_kt = next_kt; half = next_half; ++n;
+                }
+                if (there) {
+                    tc_commit_by(leader, bar_empty(ks));
+                    if (j + 1 == num_kt) tc_commit_by(leader, bar_qempty);   // every score MMA of the item has been issued
+                    advance(ks, kturn);
+                }
             }
         }
     }
@@ -1117,85 +1158,92 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         const int t = warp >> 2;
         const int wq = warp & 3;
         const int row = wq * 32 + lane;
+        const int tok = row >> pp.head_shift;   // query row of the item, and the head of it
+        const int sub = (t << pp.head_shift) + (row & ((1 << pp.head_shift) - 1));
         const uint32_t t_s = tmem_base + (static_cast<uint32_t>(wq * 32) << 16) + t * 128;
         const uint32_t t_o = tmem_base + (static_cast<uint32_t>(wq * 32) << 16) + 256 + t * 128;
-        unsigned char* p_panels = smem_gen + kOff4P + t * kTileBytes;
-        const uint32_t sread = bar_sread(t);
         int n = 0, G = 0;
         bool alive = true;
+        auto arrive_p = [&](uint32_t bar) {   // this warp's probabilities so far are in tensor memory
+            tc_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar);
+        };
         while (alive) {
-            alive = warp_mbar_wait(bar_item(n & 3), (n >> 2) & 1, abort_flag, 33);
+            alive = wait_bar_warp(bar_item(n & 3), (n >> 2) & 1, abort_flag, 33);
             if (!alive) break;
-            const Tc5Item it = s_ring[n & 3];
-            if (it.kind == 0) break;
-            const int lim = min(it.lim0 + row, it.k_len);
+            const Tc5Item& it = s_ring[n & 3];
+            const int num_kt = it.kind != 0 ? it.num_kt : 0;
+            if (num_kt == 0) break;
+            const int k_len = it.k_len, lim0 = it.lim0, half = it.half, last_partial = it.last_partial;
+            T* dst = static_cast<T*>(p.out) + (static_cast<size_t>(it.q_row + tok) * p.num_heads + (2 << pp.head_shift) * it.pair + sub) * kHeadDim;
+            const bool mine = tok < it.rows;
+            int seen = min(lim0 + tok, k_len);                                      // keys that the row sees, from the tile's first one on
+            int all_seen = min(lim0 + ((wq * 32) >> pp.head_shift), k_len);         // the warp's first row, which sees least
             float m_ref = -INFINITY, l_run = 0.0f;
-            for (int j = 0; j < it.num_kt; ++j) {
-                alive = warp_mbar_wait(bar_sfull(t), (G + j) & 1, abort_flag, 31);
+#pragma unroll 1
+            for (int j = 0; j < num_kt; ++j, seen -= kBN, all_seen -= kBN) {
+                if (t == 0 && j == last_partial) {
+                    // Rows of V past the sequence may hold anything (0 * NaN = NaN): tile 0's softmax warps, whose P.V comes first, zero them.
+                    const int c = 2 * G + 1, stage = c % kRing5;
+                    alive = wait_bar_warp(bar_full(stage), (c / kRing5) & 1, abort_flag, 13);
+                    if (!alive) break;
+                    if (row >= k_len - j * kBN) {
+                        unsigned char* v_row = smem_gen + kOff4Ring + stage * kTileBytes + row * 128;
+#pragma unroll 4
+                        for (int i = 0; i < 16; ++i)
+                            *reinterpret_cast<uint4*>(v_row + (i >> 3) * kPanelBytes + (((i ^ row) & 7) << 4)) = make_uint4(0u, 0u, 0u, 0u);
+                    }
+                    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                }
+                alive = wait_bar_warp(bar_sfull(t), G & 1, abort_flag, 31);
                 if (!alive) break;
                 tc_fence_after();
-                const int key0 = j * kBN;
-                const bool need_mask = key0 + kBN > min(it.lim0, it.k_len);
-                alive = softmax_row_to_smem<T>(t_s, t_o, p_panels, row, need_mask, key0, lim, p.scale_log2, j == 0, m_ref, l_run,
-                                               bar_odone(t), (G + j - 1) & 1, abort_flag, [&] {
-                                                   tc_fence_before();
-                                                   __syncwarp();
-                                                   if (lane == 0) mbar_arrive(sread);   // the score columns may be overwritten
-                                               });
-                if (!alive) break;
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_pfull(t));
+                softmax_row<T>(t_s, t_o, all_seen < kBN, seen, half != 0 && j + 1 == num_kt, p.scale_log2, j == 0, m_ref, l_run,
+                               [&] { arrive_p(bar_phalf(t)); });
+                arrive_p(bar_pfull(t));
+                ++G;
             }
-            if (alive) alive = warp_mbar_wait(bar_ofinal(t), n & 1, abort_flag, 32);
+            if (alive) alive = wait_bar_warp(bar_ofinal(t), n & 1, abort_flag, 32);
             if (!alive) break;
             tc_fence_after();
             {
-                // The last P.V is complete, so the P buffer is free: stage this warp's 32 output rows there (16-byte
-                // chunks XOR-swizzled by row) and write them out as whole 256-byte rows.  A row is staged where the same row
-                // of P lies in the two panels: a warp that is ahead may already write the next item's P rows, and those must
-                // not be where a slower warp's output still waits to be read.  The next item's Q is already being loaded into
-                // the Q buffer meanwhile.
+                // A thread writes its row straight from its registers, in whole 32-byte sectors, while the next item's first scores are computed.
                 const float inv = l_run > 0.0f ? 1.0f / l_run : 0.0f;
-                auto staged = [&](int r, int chunk) {
-                    return reinterpret_cast<uint4*>(p_panels + (chunk >> 3) * kPanelBytes + r * 128 + (((chunk & 7) ^ (r & 7)) << 4));
-                };
+                const uint64_t inv2 = pack_f32x2(inv, inv);
                 uint32_t o[4][32];   // the whole row at once: one TMEM latency instead of four
 #pragma unroll
                 for (int c = 0; c < 4; ++c) tmem_ld32(t_o + c * 32, o[c]);
                 tc_wait_ld();
+                // O has left TMEM: the arrive on p_half in the next item's first round tells the issuer so
+                uint32_t v[64];
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     reg_fence32(o[c]);
-                    const uint32_t (&r)[32] = o[c];
 #pragma unroll
-                    for (int q4 = 0; q4 < 4; ++q4) {
-                        uint4 v;
-                        v.x = ElemTraits<T>::pack2(__uint_as_float(r[q4 * 8 + 0]) * inv, __uint_as_float(r[q4 * 8 + 1]) * inv);
-                        v.y = ElemTraits<T>::pack2(__uint_as_float(r[q4 * 8 + 2]) * inv, __uint_as_float(r[q4 * 8 + 3]) * inv);
-                        v.z = ElemTraits<T>::pack2(__uint_as_float(r[q4 * 8 + 4]) * inv, __uint_as_float(r[q4 * 8 + 5]) * inv);
-                        v.w = ElemTraits<T>::pack2(__uint_as_float(r[q4 * 8 + 6]) * inv, __uint_as_float(r[q4 * 8 + 7]) * inv);
-                        const int chunk = c * 4 + q4;
-                        *staged(row, chunk) = v;
+                    for (int i = 0; i < 16; ++i) {
+                        float a, b;
+                        unpack_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(o[c][2 * i]), __uint_as_float(o[c][2 * i + 1])), inv2), a, b);
+                        v[c * 16 + i] = ElemTraits<T>::pack2(a, b);
                     }
                 }
-                // O has left TMEM: the arrive on p_full in the next item's first round tells the issuer so
-                __syncwarp();
-                T* o0 = static_cast<T*>(p.out) + (static_cast<size_t>(it.q_row) * p.num_heads + 2 * it.pair + t) * kHeadDim;
-                uint4 v[16];
+                if (mine) {
+                    if ((reinterpret_cast<uintptr_t>(p.out) & 31) == 0) {
 #pragma unroll
-                for (int i = 0; i < 16; ++i) v[i] = *staged(wq * 32 + 2 * i + (lane >> 4), lane & 15);
+                        for (int i = 0; i < 8; ++i) st_global_32(dst + i * 16, v + i * 8);
+                    } else {
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const int r = wq * 32 + 2 * i + (lane >> 4);
-                    if (r < it.rows) *reinterpret_cast<uint4*>(o0 + r * out_stride + (lane & 15) * 8) = v[i];
+                        for (int i = 0; i < 16; ++i) reinterpret_cast<uint4*>(dst)[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                    }
                 }
-                __syncwarp();   // the staging rows are read before the next item's probabilities overwrite them
             }
-            G += it.num_kt; ++n;
+            ++n;
         }
     }
     tc_fence_before();
     __syncthreads();
+    if (tid == 0 && s_abort != 0) atomicCAS(&g_tc_error, 0, s_abort);
     if (warp == 8) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kTmemCols2) : "memory");
     }
@@ -1220,13 +1268,13 @@ EncodeFn encode_fn() {
     return fn;
 }
 
-// [rows, heads, 128] 16-bit tensor -> boxes of `box_rows` rows x 1 head x 64 elements, 128-byte swizzle.
-bool make_map(CUtensorMap* map, const void* base, int64_t rows, int heads, bool bf16, int box_rows = 128) {
+// [rows, heads, 128] 16-bit tensor -> boxes of `box_rows` rows x `box_heads` heads x 64 elements, 128-byte swizzle.
+bool make_map(CUtensorMap* map, const void* base, int64_t rows, int heads, bool bf16, int box_rows = 128, int box_heads = 1) {
     EncodeFn fn = encode_fn();
     if (fn == nullptr || rows <= 0) return false;
     const cuuint64_t dims[3] = {static_cast<cuuint64_t>(kHeadDim), static_cast<cuuint64_t>(heads), static_cast<cuuint64_t>(rows)};
     const cuuint64_t strides[2] = {static_cast<cuuint64_t>(kHeadDim) * 2, static_cast<cuuint64_t>(heads) * kHeadDim * 2};
-    const cuuint32_t box[3] = {64, 1, static_cast<cuuint32_t>(box_rows)};
+    const cuuint32_t box[3] = {64, static_cast<cuuint32_t>(box_heads), static_cast<cuuint32_t>(box_rows)};
     const cuuint32_t elem[3] = {1, 1, 1};
     return fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base),
               dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -1258,10 +1306,10 @@ struct TcLaunch {
     TcParams p;
     int64_t tiles;
 };
-int prepare_tc_launch(const PrefillArgs& a, bool bf16, TcLaunch* out) {
+int prepare_tc_launch(const PrefillArgs& a, bool bf16, int head_shift, TcLaunch* out) {
     const bool paged = a.block_tables != nullptr;
     const int64_t key_rows = paged ? a.num_cache_blocks * a.block_size : a.total_k;
-    if (!make_map(&out->tq, a.q, a.total_q, a.num_heads, bf16) ||
+    if (!make_map(&out->tq, a.q, a.total_q, a.num_heads, bf16, kBM >> head_shift, 1 << head_shift) ||
         !make_map(&out->tk, paged ? a.k_cache : a.k, key_rows, a.num_kv_heads, bf16) ||
         !make_map(&out->tv, paged ? a.v_cache : a.v, key_rows, a.num_kv_heads, bf16))
         return fail(NVK_ERR_CUDA, "prefill attention (tcgen05): cuTensorMapEncodeTiled failed");
@@ -1297,6 +1345,20 @@ int prepare_tc5(int* sms_out) {
     return NVK_OK;
 }
 
+// Heads of one tile of the persistent kernel, as a power of two.  An item takes both tiles from the heads of one KV head; the more heads share
+// the 128 rows of a tile, the fewer query rows it has, and the less is lost on the ragged end of a sequence and beyond the diagonal.
+int tile_head_shift(int group) { return group % 8 == 0 ? 2 : group % 4 == 0 ? 1 : 0; }
+Tc5Params tc5_params(const PrefillArgs& a, const TcParams& p, int head_shift) {
+    Tc5Params pp{};
+    pp.base = p;
+    pp.head_shift = head_shift;
+    pp.pairs = a.num_heads / (2 << head_shift);
+    pp.tiles = static_cast<int>((a.total_q + (kBM >> head_shift) - 1) / (kBM >> head_shift) + (a.cu_q ? a.num_seqs : 0));
+    pp.total = static_cast<unsigned int>(pp.pairs) * static_cast<unsigned int>(pp.tiles);
+    pp.slot = ticket_slot(a.stream);
+    return pp;
+}
+
 template <typename T>
 int launch_typed(const PrefillArgs& a, bool bf16) {
     static std::atomic<bool> attr_done[64] = {};
@@ -1308,22 +1370,17 @@ int launch_typed(const PrefillArgs& a, bool bf16) {
         attr_done[device] = true;
     }
     TcLaunch L;
-    const int rc = prepare_tc_launch(a, bf16, &L);
+    const int group = a.num_heads / a.num_kv_heads, head_shift = tile_head_shift(group);
+    const int rc = prepare_tc_launch(a, bf16, head_shift, &L);
     if (rc != NVK_OK) return rc;
     const CUtensorMap &tq = L.tq, &tk = L.tk, &tv = L.tv;
     const TcParams& p = L.p;
     const int64_t tiles = L.tiles;
-    const int group = a.num_heads / a.num_kv_heads;
     if (group % 2 == 0) {   // pairs of query heads that share a KV head: persistent blocks, one per SM, items from a ticket counter
         int sms = 0;
         const int rc5 = prepare_tc5<T, false>(&sms);
         if (rc5 != NVK_OK) return rc5;
-        Tc5Params pp{};
-        pp.base = p;
-        pp.pairs = a.num_heads / 2;
-        pp.tiles = static_cast<int>(tiles);
-        pp.total = static_cast<unsigned int>(pp.pairs) * static_cast<unsigned int>(tiles);
-        pp.slot = ticket_slot(a.stream);
+        const Tc5Params pp = tc5_params(a, p, head_shift);
         const unsigned int blocks = pp.total < static_cast<unsigned int>(sms) ? pp.total : static_cast<unsigned int>(sms);
         const cudaError_t e = launch_pdl(prefill_tc5_kernel<T, false>, dim3(blocks), dim3(kThreads5), kSmemBytes4, a.stream, tq, tk, tv, pp, MixedDecode{});
         if (e != cudaSuccess) return fail(NVK_ERR_CUDA, "prefill_tc5_kernel launch: %s", cudaGetErrorString(e));
@@ -1343,6 +1400,7 @@ bool prefill_tc_supported(const PrefillArgs& a) {
     if (a.head_dim != kHeadDim) return false;
     if (!aligned_to(a.q, 16) || !aligned_to(a.out, 16)) return false;
     if (a.total_q >= (1LL << 31) || a.num_heads > 65535) return false;
+    if (!(a.scale > 0.0f)) return false;   // a hidden score is minus infinity before it is scaled
     if (a.block_tables) {
         if (a.block_size % kBN != 0) return false;
         if (!aligned_to(a.k_cache, 16) || !aligned_to(a.v_cache, 16)) return false;
@@ -1363,7 +1421,8 @@ namespace {
 template <typename T>
 int launch_mixed_typed(const PrefillArgs& a, const DecodeArgs& d, int prefill_blocks, bool bf16) {
     TcLaunch L;
-    int rc = prepare_tc_launch(a, bf16, &L);
+    const int head_shift = tile_head_shift(a.num_heads / a.num_kv_heads);
+    int rc = prepare_tc_launch(a, bf16, head_shift, &L);
     if (rc != NVK_OK) return rc;
     int sms = 0;
     rc = prepare_tc5<T, true>(&sms);
@@ -1372,20 +1431,15 @@ int launch_mixed_typed(const PrefillArgs& a, const DecodeArgs& d, int prefill_bl
     int cluster = 0;   // the ranges of the cluster kernel are taken one by one here and merged through the workspace
     rc = decode_plan(d, dec::Cache16<T>::kGroups, &md.dp, &cluster);
     if (rc != NVK_OK) return rc;
-    Tc5Params pp{};
-    pp.base = L.p;
-    pp.pairs = a.num_heads / 2;
-    pp.tiles = static_cast<int>(L.tiles);
-    pp.total = static_cast<unsigned int>(pp.pairs) * static_cast<unsigned int>(L.tiles);
-    pp.slot = ticket_slot(a.stream);
+    const Tc5Params pp = tc5_params(a, L.p, head_shift);
     if (prefill_blocks <= 0) {
         // No hint: split the SMs by a crude estimate from host-known sizes -- prefill flops as if all sequences were equally
-        // long and had no prefix, at 0.55 PFLOP/s (2048 tokens per sequence; short prompts run slower, long ones faster); decode bytes as if
-        // every block table were half full, at 6.5 TB/s.  Against the best of 17 splits for 19 steps (1 to 6 prompts of 64 to 4000
-        // tokens, 8 to 192 decode rows) it costs 6 % on average and 24 % at most (4 prompts of 800 tokens and 128 rows, 4 / 1 heads).  Other rates,
-        // and a fixed part per item, did no better: what it misses is that items are whole and contexts unknown.
+        // long and had no prefix, at 0.9 PFLOP/s; decode bytes as if every block table were half full, at 6.5 TB/s.  Against the best of 17
+        // splits for 19 steps (1 to 6 prompts of 64 to 4000 tokens, 8 to 192 decode rows) it costs 4 % on average and 16 % at most.  Too few blocks
+        // cost little, since prefill items are short and all blocks share those that are left; too many a lot, since a block that joins
+        // the decode half late may take a whole long context there (0.7 PFLOP/s: 10 % on average, 55 % at most).
         const double mean_q = static_cast<double>(a.total_q) / static_cast<double>(a.cu_q ? a.num_seqs : 1);
-        const double t_prefill = 4.0 * a.num_heads * kHeadDim * static_cast<double>(a.total_q) * (mean_q + 1.0) / 2.0 / 0.55e15;
+        const double t_prefill = 4.0 * a.num_heads * kHeadDim * static_cast<double>(a.total_q) * (mean_q + 1.0) / 2.0 / 0.9e15;
         const double t_decode = 0.5 * static_cast<double>(d.batch) * d.max_blocks * d.block_size * d.num_kv_heads * kHeadDim * 4.0 / 6.5e12;
         prefill_blocks = static_cast<int>(sms * t_prefill / (t_prefill + t_decode) + 0.5);
     }

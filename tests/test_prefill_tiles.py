@@ -1,0 +1,71 @@
+"""The persistent tensor-core prefill at the edges of its tiles: every way to share a tile's 128 rows between query rows and heads, lengths
+around a tile's query rows and around half and whole key tiles, results that start on a 16-byte boundary only, and whatever lies in the cache
+behind a sequence's last key."""
+import numpy as np
+import pytest
+
+import oracle
+from util import assert_attention_close, nvk, to_dev, to_np, workloads
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def _run(w, hkv, paged, scale, out=None, dtype=torch.bfloat16, tables=None, kc=None, vc=None):
+    lib = nvk()
+    q, cu_q, cu_k = to_dev(w["q"], dtype), to_dev(w["cu_q"]), to_dev(w["cu_k"])
+    if out is None:
+        out = torch.full_like(q, float("nan"))
+    if paged:
+        lib.launch_prefill_attention_paged(q, cu_q, kc if kc is not None else to_dev(w["k_cache"], dtype), vc if vc is not None else to_dev(w["v_cache"], dtype),
+                                           cu_k, to_dev(w["block_tables"]), hkv, 128, 256, scale, out)
+        ref = oracle.prefill_attention_paged(w["q"], w["k_cache"], w["v_cache"], w["cu_q"], w["cu_k"], w["block_tables"], hkv, 128, 256, scale)
+    else:
+        lib.launch_prefill_attention_dense(q, cu_q, to_dev(w["k"], dtype), to_dev(w["v"], dtype), cu_k, hkv, 128, scale, out)
+        ref = oracle.prefill_attention_dense(w["q"], w["k"], w["v"], w["cu_q"], w["cu_k"], hkv, 128, scale)
+    torch.cuda.synchronize()
+    assert lib.prefill_status() == 0
+    return out, ref
+
+
+@pytest.mark.parametrize("hq,hkv", [(2, 1), (4, 1), (6, 1), (8, 1), (16, 1), (24, 2), (4, 2)])
+@pytest.mark.parametrize("q_lens,prefix,paged", [
+    ([1, 15, 16, 17, 31, 32, 33], [0] * 7, False),
+    ([63, 64, 65, 127, 128, 129], [0] * 6, False),
+    ([192, 193, 320, 5], [0, 256, 512, 256], True),
+    ([40, 64, 65], [256, 768, 256], True),
+])
+def test_tiles_of_rows_and_heads(hq, hkv, q_lens, prefix, paged):
+    w = workloads().make_prefill_workload(q_lens, prefix, hq, hkv, 128, 256, seed=hq + len(q_lens), paged=paged)
+    out, ref = _run(w, hkv, paged, w["scale"], dtype=torch.float16 if hq == 8 else torch.bfloat16)
+    assert_attention_close(to_np(out), ref)
+
+
+def test_a_result_on_a_16_byte_boundary():
+    w = workloads().make_prefill_workload([70, 130], [0, 0], 8, 2, 128, 256, seed=3, paged=False)
+    n = w["q"].size
+    room = torch.full((n + 24,), float("nan"), dtype=torch.bfloat16, device="cuda")
+    at = (-(room.data_ptr() // 2) % 16) + 8                                # elements: past a 32-byte boundary by 16 bytes
+    out, ref = _run(w, 2, False, w["scale"], out=room[at:at + n].view(w["q"].shape))
+    assert out.data_ptr() % 32 == 16
+    assert_attention_close(to_np(out), ref)
+    assert torch.isnan(room[:at].float()).all() and torch.isnan(room[at + n:].float()).all()
+
+
+@pytest.mark.parametrize("k_len", [40, 64, 100, 128, 190])
+def test_rows_behind_a_sequence_do_not_matter(k_len):
+    w = workloads().make_prefill_workload([k_len], [0], 8, 2, 128, 256, seed=k_len, paged=True)
+    kc, vc = to_dev(w["k_cache"], torch.bfloat16), to_dev(w["v_cache"], torch.bfloat16)
+    block = int(w["block_tables"][0, 0])
+    kc[block, k_len:] = float("nan")
+    vc[block, k_len:] = float("inf")
+    vc[block, -1] = float("nan")
+    out, ref = _run(w, 2, True, w["scale"], kc=kc, vc=vc)
+    assert_attention_close(to_np(out), ref)
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.05])
+def test_scales_that_are_not_positive(scale):
+    w = workloads().make_prefill_workload([70, 130], [0, 0], 8, 2, 128, 256, seed=11, paged=False)
+    out, ref = _run(w, 2, False, scale)
+    assert_attention_close(to_np(out), ref)
