@@ -207,12 +207,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&r)[16]
 }
 
 
-// 32 bytes, one sector.
-__device__ __forceinline__ void st_global_32(void* dst, const uint32_t* v) {
-    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n"
-                 ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
-}
-
 // The TMEM loads are asynchronous: this pins the use of their results after the preceding
 // tcgen05.wait::ld in program order (the compiler may not move register arithmetic across it).
 __device__ __forceinline__ void reg_fence32(uint32_t (&r)[32]) {
@@ -655,11 +649,11 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 }
 
 // =================================================================================================
-// Shared memory of the persistent kernel: two Q tiles and a ring of five 32 KiB stages that K and V tiles go through in the order of
-// their use.  Tensor memory: S0 S1 O0 O1, 128 columns each; a tile's probabilities lie in the first 64 columns of its scores.
+// Shared memory of the persistent kernel: two Q tiles, a ring of four 32 KiB stages that K and V tiles go through in the order of
+// their use, and 4 KiB for each softmax warp's output.  Tensor memory: S0 S1 O0 O1, 128 columns each; a tile's probabilities lie in the first 64 columns of its scores.
 // =================================================================================================
-constexpr int kRing5 = 5;
-constexpr int kOff4Q = 0, kOff4Ring = 2 * kTileBytes, kOff4Bar = (2 + kRing5) * kTileBytes;
+constexpr int kRing5 = 4;
+constexpr int kOff4Q = 0, kOff4Ring = 2 * kTileBytes, kOff4Out = (2 + kRing5) * kTileBytes, kOff4Bar = kOff4Out + kTileBytes;
 constexpr int kSmemBytes4 = kOff4Bar + 256 + 1024;
 
 // Bounded waits of the persistent kernel, by one thread and by a whole warp (the same answer for all its lanes): they give up after 2 to 4 seconds
@@ -695,10 +689,8 @@ __device__ __forceinline__ bool wait_bar_warp(uint32_t bar, uint32_t parity, vol
 template <int C>
 __device__ __forceinline__ void hide_chunk(uint32_t (&r)[32], int seen) {
     if (__all_sync(0xffffffffu, seen >= 32 * C + 32)) return;
-    const int n = min(max(seen - 32 * C, 0), 32);
-    const uint32_t keep = n == 32 ? 0xffffffffu : (1u << n) - 1u;
 #pragma unroll
-    for (int i = 0; i < 32; ++i) r[i] = (keep >> i) & 1u ? r[i] : 0xff800000u;   // -infinity (the scale is positive)
+    for (int i = 0; i < 32; ++i) r[i] = seen > 32 * C + i ? r[i] : 0xff800000u;   // -infinity (the scale is positive)
 }
 
 // One online-softmax step of a row: 128 scores (columns of t_s) -> probabilities (16-bit pairs, the first 64 columns of t_s).  All scores are read
@@ -716,10 +708,12 @@ __device__ __forceinline__ void softmax_row(uint32_t t_s, uint32_t t_o, bool mas
     tc_wait_ld();
     reg_fence32(r0); reg_fence32(r1); reg_fence32(r2); reg_fence32(r3);
     if (masked) {
-        hide_chunk<0>(r0, seen); hide_chunk<1>(r1, seen); hide_chunk<2>(r2, seen); hide_chunk<3>(r3, seen);
+        hide_chunk<0>(r0, seen); hide_chunk<1>(r1, seen);
+        if (!half) { hide_chunk<2>(r2, seen); hide_chunk<3>(r3, seen); }
     }
-    const float mx = fmaxf(fmaxf(chunk_max<false>(r0, 0, 0), chunk_max<false>(r1, 0, 0)),
-                           fmaxf(chunk_max<false>(r2, 0, 0), chunk_max<false>(r3, 0, 0))) * scale_log2;
+    float mx = fmaxf(chunk_max<false>(r0, 0, 0), chunk_max<false>(r1, 0, 0));
+    if (!half) mx = fmaxf(mx, fmaxf(chunk_max<false>(r2, 0, 0), chunk_max<false>(r3, 0, 0)));
+    mx *= scale_log2;
     if (__any_sync(0xffffffffu, mx > m_ref + kRescaleThreshold)) {
         const float m_new = fmaxf(m_ref, mx);
         const float f = (m_new == -INFINITY) ? 1.0f : fast_exp2(m_ref - m_new);
@@ -781,6 +775,10 @@ __device__ __forceinline__ void softmax_row(uint32_t t_s, uint32_t t_o, bool mas
 //                                  each role's body): roles that alternate over more code than the instruction caches hold wait for it, a
 //                                  masked round took 9000 clocks where a steady one took 2600
 //   3043; 832 / 498 / 101 / 50     the issuing warp converged, descriptors in uniform registers (umma_ss_by)
+//   3002; 805 / 472 / 94 / 47      outputs in whole lines through 32 KB of shared memory (four stages are enough), masks by one compare a score
+// Not here: the first 32 keys' maximum as reference with the row sum as check (no maxima at all, but nothing can be handed to the MMAs before the
+// end: 3307); maxima in the shadow of the exponentials (3427); tickets taken by a warp of its own two items ahead (uneven ends: one prompt of
+// 8192 tokens, 16 / 8 heads, 217 -> 255 us).  Steps of 64 keys would need 2560 clocks of MMAs: at N 64 they are bound by shared memory.
 // Tiles of 128 >> head_shift query rows x 1 << head_shift heads instead of 128 rows of one head lose less on ragged ends and on the diagonal, and an item
 // whose rows see at most half of their last key tile leaves out that tile's second half.  All barrier phases are counted cumulatively over items.
 // =================================================================================================
@@ -832,7 +830,7 @@ struct Tc5Finder {
     int mine;                  // tiles of the window before this lane's sequence
     int tiles, qb, qe, kb, ke; // of this lane's sequence
 
-    __device__ __forceinline__ void load(const TcParams& p, int tile_rows, int lane) {
+    __device__ __forceinline__ void load(const TcParams& p, int head_shift, int lane) {
         qb = 0; qe = 0; kb = 0; ke = 0;
         if (p.cu_q == nullptr) {
             if (lane == 0) { qe = static_cast<int>(p.total_q); ke = static_cast<int>(p.total_k); }
@@ -843,7 +841,7 @@ struct Tc5Finder {
             qb = q[0]; qe = q[1 << p.cu_q.wide];
             kb = k[0]; ke = k[1 << p.cu_k.wide];
         }
-        tiles = max((qe - qb + tile_rows - 1) / tile_rows, 0);
+        tiles = max((qe - qb + (kBM >> head_shift) - 1) >> (7 - head_shift), 0);
         int inc = tiles;
 #pragma unroll
         for (int d = 1; d < 32; d *= 2) {
@@ -854,24 +852,24 @@ struct Tc5Finder {
         sum = __shfl_sync(0xffffffffu, inc, 31);
     }
     // Opens on the last window (the first tile asked for is the last one) and returns the number of tiles of all sequences.
-    __device__ __forceinline__ int open(const TcParams& p, int tile_rows, int lane) {
+    __device__ __forceinline__ int open(const TcParams& p, int head_shift, int lane) {
         before = 0;
 #pragma unroll 1
         for (base = 0;; base += 32, before += sum) {
-            load(p, tile_rows, lane);
+            load(p, head_shift, lane);
             if (p.cu_q == nullptr || base + 32 >= p.num_seqs) return before + sum;
         }
     }
     // Tile number `want`, in [0, open()): its item, without the pair.
-    __device__ __forceinline__ void find(const TcParams& p, int tile_rows, int lane, int want, Tc5Item& it) {
+    __device__ __forceinline__ void find(const TcParams& p, int head_shift, int lane, int want, Tc5Item& it) {
 #pragma unroll 1
-        while (want < before) { base -= 32; load(p, tile_rows, lane); before -= sum; }
+        while (want < before) { base -= 32; load(p, head_shift, lane); before -= sum; }
         const int at = 31 - __clz(__ballot_sync(0xffffffffu, before + mine <= want && tiles > 0));
-        const int q0 = (want - before - __shfl_sync(0xffffffffu, mine, at)) * tile_rows;
+        const int q0 = (want - before - __shfl_sync(0xffffffffu, mine, at)) << (7 - head_shift);
         const int q_begin = __shfl_sync(0xffffffffu, qb, at), q_len = __shfl_sync(0xffffffffu, qe, at) - q_begin;
         it.seq = base + at;
         it.q_row = q_begin + q0;
-        it.rows = min(tile_rows, q_len - q0);
+        it.rows = min(kBM >> head_shift, q_len - q0);
         it.k_row = __shfl_sync(0xffffffffu, kb, at);
         it.k_len = __shfl_sync(0xffffffffu, ke, at) - it.k_row;
         it.lim0 = it.k_len - q_len + q0 + 1;
@@ -988,11 +986,11 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kRegsLow5));
     if (warp == 9) {
         // ------------------------------------------------------------------ ticket taker + TMA producer
-        const int tile_rows = kBM >> pp.head_shift, item_heads = 2 << pp.head_shift;
+        const int item_heads = 2 << pp.head_shift;
         unsigned int ticket = 0;
         if (lane == 0) ticket = atomicAdd(&g_prefill_ticket[pp.slot], 1u);   // (the first one under the look at the sequence bounds)
         Tc5Finder find;
-        const int tiles = min(find.open(p, tile_rows, lane), pp.tiles);
+        const int tiles = min(find.open(p, pp.head_shift, lane), pp.tiles);
         const unsigned int total = static_cast<unsigned int>(tiles) * static_cast<unsigned int>(pp.pairs);
         int stage = 0, n = -1;   // ring stage of the next K / V tile; the item that is being loaded, -1: none yet
         uint32_t turn = 0;       // parity of that stage's round through the ring
@@ -1020,7 +1018,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 }
                 const unsigned int tile = ticket / static_cast<unsigned int>(pp.pairs);
                 next.pair = static_cast<int>(ticket - tile * static_cast<unsigned int>(pp.pairs));
-                find.find(p, tile_rows, lane, tiles - 1 - static_cast<int>(tile), next);
+                find.find(p, pp.head_shift, lane, tiles - 1 - static_cast<int>(tile), next);
                 if (next.num_kt > 0) { next.kind = 1; break; }
                 // rows that see no key: zeros, and the next ticket
                 T* o0 = static_cast<T*>(p.out) + (static_cast<size_t>(next.q_row) * p.num_heads + item_heads * next.pair) * kHeadDim;
@@ -1158,8 +1156,8 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         const int t = warp >> 2;
         const int wq = warp & 3;
         const int row = wq * 32 + lane;
-        const int tok = row >> pp.head_shift;   // query row of the item, and the head of it
-        const int sub = (t << pp.head_shift) + (row & ((1 << pp.head_shift) - 1));
+        const int tok = row >> pp.head_shift;   // query row of the item
+        unsigned char* stage_out = smem_gen + kOff4Out + warp * (kTileBytes / 8);
         const uint32_t t_s = tmem_base + (static_cast<uint32_t>(wq * 32) << 16) + t * 128;
         const uint32_t t_o = tmem_base + (static_cast<uint32_t>(wq * 32) << 16) + 256 + t * 128;
         int n = 0, G = 0;
@@ -1177,8 +1175,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             const int num_kt = it.kind != 0 ? it.num_kt : 0;
             if (num_kt == 0) break;
             const int k_len = it.k_len, lim0 = it.lim0, half = it.half, last_partial = it.last_partial;
-            T* dst = static_cast<T*>(p.out) + (static_cast<size_t>(it.q_row + tok) * p.num_heads + (2 << pp.head_shift) * it.pair + sub) * kHeadDim;
-            const bool mine = tok < it.rows;
+            const int rows = it.rows, q_row = it.q_row, head0 = (2 * it.pair + t) << pp.head_shift;
             int seen = min(lim0 + tok, k_len);                                      // keys that the row sees, from the tile's first one on
             int all_seen = min(lim0 + ((wq * 32) >> pp.head_shift), k_len);         // the warp's first row, which sees least
             float m_ref = -INFINITY, l_run = 0.0f;
@@ -1209,32 +1206,39 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             if (!alive) break;
             tc_fence_after();
             {
-                // A thread writes its row straight from its registers, in whole 32-byte sectors, while the next item's first scores are computed.
+                // Half a row at a time goes through 4 KiB of this warp (16-byte pieces XOR-swizzled by row) and out in whole 128-byte lines, while the
+                // next item's first scores are computed.  (Each thread its own row in 32-byte stores: 32 lines an instruction, 1500 to 1900 clocks an item.)
                 const float inv = l_run > 0.0f ? 1.0f / l_run : 0.0f;
                 const uint64_t inv2 = pack_f32x2(inv, inv);
+                T* dst = static_cast<T*>(p.out) + (static_cast<size_t>(q_row) * p.num_heads + head0) * kHeadDim;   // the tile's first row
                 uint32_t o[4][32];   // the whole row at once: one TMEM latency instead of four
 #pragma unroll
                 for (int c = 0; c < 4; ++c) tmem_ld32(t_o + c * 32, o[c]);
                 tc_wait_ld();
                 // O has left TMEM: the arrive on p_half in the next item's first round tells the issuer so
-                uint32_t v[64];
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    reg_fence32(o[c]);
+                for (int h = 0; h < 2; ++h) {
+                    reg_fence32(o[2 * h]); reg_fence32(o[2 * h + 1]);
+                    __syncwarp();   // the other half has been read
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        float a, b;
-                        unpack_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(o[c][2 * i]), __uint_as_float(o[c][2 * i + 1])), inv2), a, b);
-                        v[c * 16 + i] = ElemTraits<T>::pack2(a, b);
+                    for (int c = 0; c < 8; ++c) {
+                        const uint32_t* r = o[2 * h + (c >> 2)] + (c & 3) * 8;
+                        uint32_t v[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            float a, b;
+                            unpack_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), inv2), a, b);
+                            v[i] = ElemTraits<T>::pack2(a, b);
+                        }
+                        *reinterpret_cast<uint4*>(stage_out + lane * 128 + ((c ^ (lane & 7)) << 4)) = make_uint4(v[0], v[1], v[2], v[3]);
                     }
-                }
-                if (mine) {
-                    if ((reinterpret_cast<uintptr_t>(p.out) & 31) == 0) {
+                    __syncwarp();
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) st_global_32(dst + i * 16, v + i * 8);
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) reinterpret_cast<uint4*>(dst)[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                    for (int i = 0; i < 8; ++i) {
+                        const int r = 4 * i + (lane >> 3), at = wq * 32 + r;   // row of the warp and of the tile
+                        const uint4 v = *reinterpret_cast<const uint4*>(stage_out + r * 128 + (((lane ^ r) & 7) << 4));
+                        if ((at >> pp.head_shift) < rows)
+                            *reinterpret_cast<uint4*>(dst + (at >> pp.head_shift) * static_cast<int>(out_stride) + (at & ((1 << pp.head_shift) - 1)) * kHeadDim + h * 64 + (lane & 7) * 8) = v;
                     }
                 }
             }
