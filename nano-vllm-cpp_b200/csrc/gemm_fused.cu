@@ -22,7 +22,7 @@
 //                       loads half of A and half of B, so an SM moves half the operand bytes of a 128 x 256 tile of its own.  The
 //                       accumulator is double buffered in TMEM: the epilogue of a tile runs under the next tile's MMAs.
 // Before, one block per 128 x 128 tile whatever the size (microseconds in a loop over weights larger than L2; K 4096):
-//   64 x 6144  22 -> 16      64 x 4096  21 -> 12     7440 x 4096  295 -> 175 (1430 TFLOP/s)     7440 x 6144 with QKV epilogue  597 -> 277
+//   64 x 6144  22 -> 16      64 x 4096  21 -> 12 (with MMAs from a converged warp 14.5 and 11.1)     7440 x 4096  295 -> 175 (1430 TFLOP/s)     7440 x 6144 with QKV epilogue  597 -> 277
 // What the fusion removes is the round trip of the result and one or two launches per layer.
 // Every mbarrier wait is bounded; a wait that runs out raises an error word (nvk_gemm_status) and the block leaves.
 #include "nvk_internal.cuh"
@@ -99,6 +99,19 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
         }
     }
 }
+// The same by a converged warp, with the same answer for all its lanes.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity) != 0)) return true;
+    const long long start = clock64();
+    while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity) != 0)) {
+        if (!__all_sync(0xffffffffu, *abort_flag == 0 && clock64() - start <= kWaitCycles)) {
+            if (*abort_flag == 0) atomicCAS(&g_gemm_error, 0, code);
+            *abort_flag = 1;
+            return false;
+        }
+    }
+    return true;
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
@@ -134,14 +147,24 @@ __device__ __forceinline__ float4 ld_cluster(uint32_t addr) {                  /
     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
     return v;
 }
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
+// MMAs and commits of gemm_split_kernel come from a converged warp: all lanes run through the same instructions, so that the operands are uniform registers, which is where
+// the MMA wants them, and one lane (`leader` 1) issues.  A single diverged lane has to move every operand there first, 75 to 100 clocks an
+// MMA; gemm_pair_kernel, whose MMAs take 128, keeps that (its QKV epilogue was 3 % slower beside a whole warp that polls).
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t leader;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(leader));
+    return leader;
 }
-__device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
+__device__ __forceinline__ void tc_commit(uint32_t leader, uint32_t bar) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc) : "memory");
+        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%1];\n\t}\n" ::"r"(leader), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void umma_ss(uint32_t leader, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %0, 0;\n\tsetp.ne.b32 p, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%1], %2, %3, %4, p;\n\t}\n"
+        ::"r"(leader), "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc) : "memory");
 }
 __device__ __forceinline__ void tc_commit_pair(uint32_t bar) {                  // arrives in both blocks of the pair
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
@@ -465,7 +488,7 @@ __device__ __forceinline__ void sum_over_cluster(uint32_t at, int splits, float4
 // shared memory as fp32 rows of 132 words (no bank conflicts for the writing threads, each of which has a row); block r adds up and
 // finishes rows r, r + splits, ... of the tile, eight lanes a row.
 // DIRECT: a block with all of K has nothing to add up and takes its tile from TMEM straight to the result (us: 4096 columns, K 128, 128 rows
-// 5.5 -> 4.0); not up to 32 rows, which would leave three of four epilogue warps idle (8 rows 3.2 -> 3.7).  An instantiation of its own: with both
+// 5.5 -> 4.0); not for the QKV epilogue, which is quicker with eight lanes a row (64 x 3072, K 1024: 10.4, 8.7), nor up to 32 rows, which would leave three of four epilogue warps idle (8 rows 3.2 -> 3.7).  An instantiation of its own: with both
 // ways in one the sums were slower (39 rows through 768 x 4096 and 4096 x 512 in a pass of 25.2 us: 26.4).
 constexpr int kRowWords = kBN + 4;
 template <typename T, int EPI, int MT, bool DIRECT>
@@ -476,7 +499,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     extern __shared__ unsigned char smem_raw[];
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;   // (uniform, also to the compiler)
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t bars = smem_base + kRingBytes;
     auto bar_full = [&](int s) { return bars + 8 * s; };
@@ -504,7 +527,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = s_tmem_base;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, s_tmem_base, 0);
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
@@ -521,26 +544,28 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            bool ok = true;
-            for (int i = 0; i < kb_count && ok; ++i) {
-                const int s = i % kStages;
-                ok = mbar_wait(bar_full(s), (i / kStages) & 1, abort_flag, 2);
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t at = smem_base + s * kStageBytes;
-                const uint64_t db = make_smem_desc(at + MT * kPanelBytes);
+        const uint32_t leader = elect_one();
+        bool ok = true;
+        int s = 0;
+        uint32_t turn = 0;
+#pragma unroll 1
+        for (int i = 0; i < kb_count && ok; ++i) {
+            ok = mbar_wait_warp(bar_full(s), turn, abort_flag, 2);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t at = smem_base + s * kStageBytes;
+            const uint64_t db = make_smem_desc(at + MT * kPanelBytes);
 #pragma unroll
-                for (int t = 0; t < MT; ++t) {
-                    const uint64_t da = make_smem_desc(at + t * kPanelBytes);
+            for (int t = 0; t < MT; ++t) {
+                const uint64_t da = make_smem_desc(at + t * kPanelBytes);
 #pragma unroll
-                    for (int ks = 0; ks < kBK / 16; ++ks)   // 32 bytes further along the 128-byte row per K step: +2 in the address field
-                        umma_ss(tmem_base + t * kBN, da + 2 * ks, db + 2 * ks, p.idesc, (i > 0 || ks > 0) ? 1u : 0u);
-                }
-                tc_commit(bar_empty(s));
+                for (int ks = 0; ks < kBK / 16; ++ks)   // 32 bytes further along the 128-byte row per K step: +2 in the address field
+                    umma_ss(leader, tmem_base + t * kBN, da + 2 * ks, db + 2 * ks, p.idesc, (i > 0 || ks > 0) ? 1u : 0u);
             }
-            if (ok) tc_commit(bar_acc);
+            tc_commit(leader, bar_empty(s));
+            if (++s == kStages) { s = 0; turn ^= 1u; }
         }
+        if (ok) tc_commit(leader, bar_acc);
     } else {
         // ------------------------------------------------------------------ TMEM -> shared memory: thread = row of the tile
         const int wq = warp & 3;                       // TMEM lanes 32 wq .. 32 wq + 31 belong to this warp
@@ -752,23 +777,25 @@ uint32_t make_idesc(bool bf16, int m, int n) {   // kind::f16: D = F32, A / B = 
 }
 
 // Kernel and shape for a size, by what the slowest SM does: waves of blocks times (steps of 64 along K and a fixed part).  The microseconds
-// are fitted to all nine ways at 8 to 7440 rows x 768 to 12288 columns, K 128 to 4096 (replayed graphs over weights larger than L2).  A step
-// costs 32 or 48 KiB out of L2, the bound here, not the tensor pipe (32 KiB per SM for a pair's 256 x 256 tile).  The fixed part (launch, first
+// are fitted to all nine ways at 16 to 3000 rows x 768 to 12288 columns, K 512 to 4096 (replayed graphs over weights larger than L2).  A step
+// costs 32 or 48 KiB out of L2, the bound here, not the tensor pipe (32 KiB per SM for a pair's 256 x 256 tile).  (0.29 and 0.39 us with MMAs from
+// a diverged lane.)  The fixed part (launch, first
 // loads, epilogue; with the sum over the cluster also in proportion to the tile's rows) comes with every wave of blocks, that of a
 // pair's tile is hidden but for the epilogue.  (One fixed part whatever the waves, measured at K 4096 only, took 256-row blocks for
 // 1500 x 4096, K 512: 21.6 us, pairs 12.3.)  One rule for all epilogues, so that they round the same sums: its constants lie between
-// the plain ones (choice within 1 % of the fastest on average, 12 % at most) and those of the slower QKV epilogue (2 %, but 30 % where K is 512).
+// the plain ones (choice 2 % slower than the fastest way on average, 26 % at most: 64 x 6144, K 512, 6.0 us, one block with all of K 4.8) and those of
+// the slower QKV epilogue (1 %, 21 % at most: 128 x 6144, K 512).
 // A part of K has four steps at least: with fewer, clusters of 4 that nearly fill the chip gain 0.2 us at most (8 x 4096, K 512, 4.4 us,
 // clusters of 2 4.6).
 struct GemmShape { int mt, splits; };   // mt 1 or 2: gemm_split_kernel; 0: gemm_pair_kernel
 GemmShape choose_gemm(int64_t m, int64_t n, int64_t k) {
     // clusters: what a B200 holds at once (its GPCs have 16 to 20 SMs); rows: per 128 rows of a tile
     struct { int mt, splits, clusters; double step, fixed, rows; } constexpr kWays[] = {
-        {1, 1, 148, 0.286, 4.1, 0.6}, {1, 2, 74, 0.307, 3.7, 2.5}, {1, 4, 33, 0.35, 3.7, 3.4}, {1, 8, 15, 0.46, 3.3, 4.4},
-        {2, 1, 148, 0.387, 6.1, 0.7}, {2, 2, 74, 0.395, 5.4, 1.9}, {2, 4, 33, 0.42, 7.0, 1.5}, {2, 8, 15, 0.457, 8.0, 2.3}};
+        {1, 1, 148, 0.220, 3.6, 0.7}, {1, 2, 74, 0.231, 3.3, 2.4}, {1, 4, 33, 0.25, 3.4, 3.2}, {1, 8, 15, 0.30, 2.6, 4.2},
+        {2, 1, 148, 0.347, 3.4, 0.3}, {2, 2, 74, 0.343, 4.9, 2.1}, {2, 4, 33, 0.35, 6.3, 1.4}, {2, 8, 15, 0.40, 5.5, 3.0}};
     const int64_t kb = (k + kBK - 1) / kBK, tiles_n = n / kBN, pair_tiles = ((m + 255) / 256) * ((n + 255) / 256);
     GemmShape best{0, 1};
-    double best_time = m > kBM ? static_cast<double>((pair_tiles + 73) / 74) * (static_cast<double>(kb) * 0.31 + 3.0) + 4.7 : 1e30;
+    double best_time = m > kBM ? static_cast<double>((pair_tiles + 73) / 74) * (static_cast<double>(kb) * 0.316 + 1.6) + 3.8 : 1e30;
     for (const auto& w : kWays) {
         const int64_t tile_rows = w.mt * kBM, tiles = (m + tile_rows - 1) / tile_rows * tiles_n;
         if ((w.mt == 2 && m <= kBM) || (w.splits > 1 && (kb / w.splits < 4 || tiles > w.clusters))) continue;
@@ -825,9 +852,10 @@ int launch(const void* a, const void* b, GemmParams& p, bool bf16, cudaStream_t 
     }
     p.idesc = make_idesc(bf16, kBM, kBN);
     const dim3 grid(static_cast<unsigned>(p.n / kBN * g.splits), static_cast<unsigned>((p.m + g.mt * kBM - 1) / (g.mt * kBM)));
-    const bool direct = g.splits == 1 && p.m > 32;
-    auto* kernel = g.mt == 1 ? direct ? gemm_split_kernel<T, EPI, 1, true> : gemm_split_kernel<T, EPI, 1, false>
-                             : direct ? gemm_split_kernel<T, EPI, 2, true> : gemm_split_kernel<T, EPI, 2, false>;
+    constexpr bool kMayDirect = EPI != kQkvPrologue;
+    const bool direct = kMayDirect && g.splits == 1 && p.m > 32;
+    auto* kernel = g.mt == 1 ? direct ? gemm_split_kernel<T, EPI, 1, kMayDirect> : gemm_split_kernel<T, EPI, 1, false>
+                             : direct ? gemm_split_kernel<T, EPI, 2, kMayDirect> : gemm_split_kernel<T, EPI, 2, false>;
     return launch_kernel(kernel, done[2 * g.mt - 1 + direct], grid, kThreads, g.splits, stream, what, ta, tb, p, g.splits);
 }
 
