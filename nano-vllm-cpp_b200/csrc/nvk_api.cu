@@ -32,6 +32,11 @@ namespace {
 bool is_compute_dtype(int dtype) { return dtype == NVK_F16 || dtype == NVK_BF16 || dtype == NVK_F32; }
 bool is_index_dtype(int dtype) { return dtype == NVK_I32 || dtype == NVK_I64; }
 IndexArray index_array(const void* p, int dtype) { return IndexArray(p, dtype == NVK_I64 ? 1 : 0); }
+int launch_prefill(const PrefillArgs& a) {
+    if (prefill_tc_supported(a)) return launch_prefill_tc(a);
+    if (prefill_mma_supported(a)) return launch_prefill_mma(a);
+    return launch_rowwise_prefill(a);
+}
 
 }  // namespace
 }  // namespace nvk
@@ -256,9 +261,7 @@ int nvk_prefill_attention_varlen(const void* query, const void* key, const void*
                   index_array(cu_seqlens_k, cu_seqlens_k_dtype), index_array(block_tables, block_tables_dtype), output, num_seqs,
                   total_q, total_k, max_blocks, num_cache_blocks, max_seqlen_q, num_heads, num_kv_heads, head_dim,
                   block_size, scale, dtype, static_cast<cudaStream_t>(stream)};
-    if (prefill_tc_supported(a)) return launch_prefill_tc(a);
-    if (prefill_mma_supported(a)) return launch_prefill_mma(a);
-    return launch_rowwise_prefill(a);
+    return launch_prefill(a);
 }
 
 int nvk_attention_mixed_step(const void* p_query, const void* p_key, const void* p_value, const void* k_cache, const void* v_cache,
@@ -298,6 +301,10 @@ int nvk_attention_mixed_step(const void* p_query, const void* p_key, const void*
     if (!mixed_step_supported(pa, da))
         return fail(NVK_ERR_UNSUPPORTED, "mixed step: needs F16 / BF16, head_dim 128, an even number of query heads per KV head, at most 8, and "
                                          "paged block sizes that are multiples of 128; call the prefill and decode entry points instead");
+    if (!prefill_tc_supported(pa)) {   // a scale that is not positive: the prefill rows take another kernel
+        const int rc = launch_prefill(pa);
+        return rc != NVK_OK ? rc : launch_decode_mma(da);
+    }
     return launch_mixed_step(pa, da, prefill_blocks);
 }
 

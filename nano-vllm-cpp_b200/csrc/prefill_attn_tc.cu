@@ -1399,12 +1399,11 @@ int launch_typed(const PrefillArgs& a, bool bf16) {
 
 }  // namespace
 
-bool prefill_tc_supported(const PrefillArgs& a) {
+static bool tc_shape_supported(const PrefillArgs& a) {
     if (a.dtype != NVK_F16 && a.dtype != NVK_BF16) return false;
     if (a.head_dim != kHeadDim) return false;
     if (!aligned_to(a.q, 16) || !aligned_to(a.out, 16)) return false;
     if (a.total_q >= (1LL << 31) || a.num_heads > 65535) return false;
-    if (!(a.scale > 0.0f)) return false;   // a hidden score is minus infinity before it is scaled
     if (a.block_tables) {
         if (a.block_size % kBN != 0) return false;
         if (!aligned_to(a.k_cache, 16) || !aligned_to(a.v_cache, 16)) return false;
@@ -1415,6 +1414,9 @@ bool prefill_tc_supported(const PrefillArgs& a) {
     }
     return encode_fn() != nullptr;
 }
+
+// (A hidden score is minus infinity before it is scaled.)
+bool prefill_tc_supported(const PrefillArgs& a) { return a.scale > 0.0f && tc_shape_supported(a); }
 
 int launch_prefill_tc(const PrefillArgs& a) {
     return a.dtype == NVK_BF16 ? launch_typed<__nv_bfloat16>(a, true) : launch_typed<__half>(a, false);
@@ -1463,7 +1465,7 @@ int launch_mixed_typed(const PrefillArgs& a, const DecodeArgs& d, int prefill_bl
 // One launch for a step with prefill and decode sequences: the head-pair prefill kernel and the tensor-core decode kernel
 // must both take their halves, and the decode half needs its split-K workspace.
 bool mixed_step_supported(const PrefillArgs& p, const DecodeArgs& d) {
-    if (!prefill_tc_supported(p) || (p.num_heads / p.num_kv_heads) % 2 != 0) return false;
+    if (!tc_shape_supported(p) || (p.num_heads / p.num_kv_heads) % 2 != 0) return false;
     if (!decode_mma_supported(d) || d.workspace == nullptr) return false;
     if (p.dtype != d.dtype || p.num_heads != d.num_heads || p.num_kv_heads != d.num_kv_heads || p.stream != d.stream) return false;
     if (p.total_q <= 0 || d.batch <= 0) return false;

@@ -64,8 +64,38 @@ def test_rows_behind_a_sequence_do_not_matter(k_len):
     assert_attention_close(to_np(out), ref)
 
 
+def test_rows_that_see_no_key():
+    """More query rows than keys: the first rows see none and are zero."""
+    bf, lib = torch.bfloat16, nvk()
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    q = torch.randn((200, 8, 128), generator=gen, device="cuda").to(bf)
+    k, v = (torch.randn((140, 2, 128), generator=gen, device="cuda").to(bf) for _ in range(2))
+    cu_q, cu_k = (torch.tensor([0, n], dtype=torch.int32, device="cuda") for n in (200, 140))
+    out = torch.full_like(q, float("nan"))
+    lib.launch_prefill_attention_dense(q, cu_q, k, v, cu_k, 2, 128, 0.088, out)
+    torch.cuda.synchronize()
+    ref = oracle.prefill_attention_dense(to_np(q), to_np(k), to_np(v), to_np(cu_q), to_np(cu_k), 2, 128, 0.088)
+    assert bool((out[:60] == 0).all())
+    assert_attention_close(to_np(out), ref)
+
+
 @pytest.mark.parametrize("scale", [0.0, -0.05])
 def test_scales_that_are_not_positive(scale):
     w = workloads().make_prefill_workload([70, 130], [0, 0], 8, 2, 128, 256, seed=11, paged=False)
     out, ref = _run(w, 2, False, scale)
     assert_attention_close(to_np(out), ref)
+
+
+def test_a_mixed_step_takes_scales_that_are_not_positive():
+    bf, lib, hkv = torch.bfloat16, nvk(), 2
+    p = workloads().make_prefill_workload([70, 20], [0, 256], 8, hkv, 128, 256, seed=12, paged=True)
+    kc, vc, pt = to_dev(p["k_cache"], bf), to_dev(p["v_cache"], bf), to_dev(p["block_tables"])
+    pq, cu_q, cu_k, dq = to_dev(p["q"], bf), to_dev(p["cu_q"]), to_dev(p["cu_k"]), to_dev(p["q"][:2], bf)
+    ctx = to_dev(np.array([70, 276], np.int32))
+    ws = torch.empty(max(16, lib.decode_attention_workspace_bytes(2, 8, hkv, 128, pt.shape[1], 256)), dtype=torch.uint8, device="cuda")
+    want_p, want_d, p_out, d_out = torch.empty_like(pq), torch.empty_like(dq), torch.empty_like(pq), torch.empty_like(dq)
+    lib.launch_prefill_attention_paged(pq, cu_q, kc, vc, cu_k, pt, hkv, 128, 256, -0.05, want_p)
+    lib.launch_decode_attention_paged(dq, kc, vc, ctx, pt, hkv, 128, 256, -0.05, want_d, ws)
+    lib.attention_mixed_step(pq, cu_q, None, None, cu_k, pt, p_out, dq, ctx, pt, d_out, kc, vc, hkv, 128, 256, -0.05, ws)
+    torch.cuda.synchronize()
+    assert torch.equal(p_out, want_p) and torch.equal(d_out, want_d)
