@@ -1244,6 +1244,13 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             }
             ++n;
         }
+        if (MIXED && !decode_first) {
+            // Here, where these warps have their 224 registers: behind the roles the code has to make do with the 56 of the other warpgroup,
+            // and a context of 4096 keys took 170 us instead of 90 (1 prompt of 300 tokens, 64 decode rows, 8 blocks: 186 us a step; 3 of 500 to 2048,
+            // 90 rows, 30 blocks: 296).  Both tiles are done with the shared memory when all softmax warps are here.
+            asm volatile("bar.sync 3, %0;\n" ::"n"(2 * kBM) : "memory");
+            decode_half();
+        }
     }
     tc_fence_before();
     __syncthreads();
@@ -1251,7 +1258,6 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     if (warp == 8) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kTmemCols2) : "memory");
     }
-    if (MIXED && !decode_first) decode_half();
 }
 
 // ---- host side ------------------------------------------------------------------------------------------
@@ -1440,12 +1446,11 @@ int launch_mixed_typed(const PrefillArgs& a, const DecodeArgs& d, int prefill_bl
     const Tc5Params pp = tc5_params(a, L.p, head_shift);
     if (prefill_blocks <= 0) {
         // No hint: split the SMs by a crude estimate from host-known sizes -- prefill flops as if all sequences were equally
-        // long and had no prefix, at 0.9 PFLOP/s; decode bytes as if every block table were half full, at 6.5 TB/s.  Against the best of 17
-        // splits for 19 steps (1 to 6 prompts of 64 to 4000 tokens, 8 to 192 decode rows) it costs 4 % on average and 16 % at most.  Too few blocks
-        // cost little, since prefill items are short and all blocks share those that are left; too many a lot, since a block that joins
-        // the decode half late may take a whole long context there (0.7 PFLOP/s: 10 % on average, 55 % at most).
+        // long and had no prefix, at 0.6 PFLOP/s; decode bytes as if every block table were half full, at 6.5 TB/s.  Against the best of 17
+        // splits for 19 steps (1 to 6 prompts of 64 to 4000 tokens, 8 to 192 decode rows) it costs 3 % on average and 11 % at most (0.3 PFLOP/s
+        // 3.5 %, 1.0 4.7 %): it matters little, since every block sees to what is left of the other kind.
         const double mean_q = static_cast<double>(a.total_q) / static_cast<double>(a.cu_q ? a.num_seqs : 1);
-        const double t_prefill = 4.0 * a.num_heads * kHeadDim * static_cast<double>(a.total_q) * (mean_q + 1.0) / 2.0 / 0.9e15;
+        const double t_prefill = 4.0 * a.num_heads * kHeadDim * static_cast<double>(a.total_q) * (mean_q + 1.0) / 2.0 / 0.6e15;
         const double t_decode = 0.5 * static_cast<double>(d.batch) * d.max_blocks * d.block_size * d.num_kv_heads * kHeadDim * 4.0 / 6.5e12;
         prefill_blocks = static_cast<int>(sms * t_prefill / (t_prefill + t_decode) + 0.5);
     }
