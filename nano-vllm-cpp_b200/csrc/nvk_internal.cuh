@@ -49,8 +49,14 @@ struct IndexArray {
         return IndexArray(static_cast<const char*>(ptr) + n * (wide ? 8 : 4), wide);
     }
 #ifdef __CUDACC__
+    // (one of two predicated loads: a branch at every index cost more code than the loads)
     __device__ __forceinline__ int64_t operator[](int64_t i) const {
-        return wide ? static_cast<const int64_t*>(ptr)[i] : static_cast<int64_t>(static_cast<const int32_t*>(ptr)[i]);
+        int64_t v;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\t"
+            "@p ld.global.s64 %0, [%1];\n\t@!p ld.global.s32 %0, [%1];\n\t}\n"
+            : "=l"(v) : "l"(static_cast<const char*>(ptr) + (i << (2 + wide))), "r"(wide));
+        return v;
     }
 #endif
 };
