@@ -170,11 +170,11 @@ __device__ __forceinline__ void umma_scores(uint32_t leader, uint32_t d_tmem, ui
 #pragma unroll
     for (int ks = 1; ks < 8; ++ks) umma_ss_by<true>(leader, d_tmem, q_base + kmajor_off16(ks), k_base + kmajor_off16(ks), idesc);
 }
-// K-steps FIRST .. FIRST + 3 of O += P V: P in tensor memory (8 columns per 16 keys), V MN-major (2048 bytes per 16 keys).
-template <int FIRST>
+// K-steps FIRST .. LAST - 1 of O += P V: P in tensor memory (8 columns per 16 keys), V MN-major (2048 bytes per 16 keys).
+template <int FIRST, int LAST>
 __device__ __forceinline__ void umma_pv(uint32_t leader, uint32_t d_tmem, uint32_t p_tmem, uint64_t v_base, uint32_t idesc, uint32_t acc_first) {
 #pragma unroll
-    for (int kk = FIRST; kk < FIRST + 4; ++kk)
+    for (int kk = FIRST; kk < LAST; ++kk)
         umma_ts_by(leader, d_tmem, p_tmem + kk * 8, v_base + kk * 2048 / 16, idesc, kk > FIRST ? 1u : acc_first);
 }
 
@@ -695,8 +695,8 @@ __device__ __forceinline__ void hide_chunk(uint32_t (&r)[32], int seen) {
 
 // One online-softmax step of a row: 128 scores (columns of t_s) -> probabilities (16-bit pairs, the first 64 columns of t_s).  All scores are read
 // before the first probability is written.  `seen`: keys of the tile that the row sees; `masked`: some row of the warp does not see
-// all; `half`: no row of the item sees more than 64, the second half of the probabilities is not wanted.  `on_half` runs when the first 64 are
-// written.
+// all; `half`: no row of the item sees more than 64, the second half of the probabilities is not wanted.  `on_half` runs when the first 96 are
+// written (64 of a half round): their MMAs run under the last exponentials, and two K-steps are left for the chain.
 template <typename T, typename OnHalf>
 __device__ __forceinline__ void softmax_row(uint32_t t_s, uint32_t t_o, bool masked, int seen, bool half, float scale_log2, bool first,
                                             float& m_ref, float& l_run, OnHalf on_half) {
@@ -749,11 +749,24 @@ __device__ __forceinline__ void softmax_row(uint32_t t_s, uint32_t t_o, bool mas
     } else {
         exp_stage<T, true, true>(r2, r3, r1, pk2, scale2, neg_m2, acc0, acc1);
         tmem_st16(t_s + 16, pk2);
-        on_half();
-        exp_stage<T, false, true>(r3, r3, r2, pk, scale2, neg_m2, acc0, acc1);
-        tmem_st16(t_s + 32, pk);
+        // the last 32: 96 keys' probabilities are handed over before the last 16 exponentials
 #pragma unroll
-        for (int i = 0; i < 16; ++i) pk2[i] = sum_pair<T>(r3, i, (i & 1) ? acc1 : acc0);
+        for (int i = 0; i < 8; ++i) {
+            r3[2 * i] = __float_as_uint(ex2_ordered(__uint_as_float(r3[2 * i])));
+            pk[2 * i] = sum_pair<T>(r2, 2 * i, acc0);
+            r3[2 * i + 1] = __float_as_uint(ex2_ordered(__uint_as_float(r3[2 * i + 1])));
+            pk[2 * i + 1] = sum_pair<T>(r2, 2 * i + 1, acc1);
+        }
+        tmem_st16(t_s + 32, pk);
+        on_half();
+#pragma unroll
+        for (int i = 8; i < 16; ++i) {
+            r3[2 * i] = __float_as_uint(ex2_ordered(__uint_as_float(r3[2 * i])));
+            r3[2 * i + 1] = __float_as_uint(ex2_ordered(__uint_as_float(r3[2 * i + 1])));
+            pk2[i - 8] = sum_pair<T>(r3, i - 8, (i & 1) ? acc1 : acc0);
+        }
+#pragma unroll
+        for (int i = 8; i < 16; ++i) pk2[i] = sum_pair<T>(r3, i, (i & 1) ? acc1 : acc0);
         tmem_st16(t_s + 48, pk2);
     }
     float a0, a1, a2, a3;
@@ -787,8 +800,8 @@ __device__ __forceinline__ void softmax_row(uint32_t t_s, uint32_t t_o, bool mas
 // so these have 32768 of their own, which no eager launch meets.
 constexpr int kEagerSlots = 32768, kTicketSlots = 2 * kEagerSlots;
 constexpr int kThreads5 = 384;      // three warpgroups (register reallocation works on whole warpgroups)
-constexpr int kRegsLow5 = 56;       // registers per thread of the third warpgroup after setmaxnreg.dec
-constexpr int kRegsHigh5 = 224;     // registers per thread of the two softmax warpgroups after setmaxnreg.inc
+constexpr int kRegsLow5 = 88;       // registers per thread of the third warpgroup after setmaxnreg.dec
+constexpr int kRegsHigh5 = 208;     // registers per thread of the two softmax warpgroups after setmaxnreg.inc
 // Ticket counters, zero between launches: every block takes tickets up to its first one past the end (items + blocks in all, whether the first ones
 // come from the counter or are the blocks' numbers), so the launch's last ticket is known, and who holds it sets the counter back.  (A counter of finished blocks is a trip to memory at the end that everything waits for: 1 us.)
 __device__ unsigned int g_prefill_ticket[kTicketSlots];
@@ -948,7 +961,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     auto bar_full = [&](int s) { return bars + 16 + 8 * s; };      // ring stage s has landed
     auto bar_empty = [&](int s) { return bars + 56 + 8 * s; };     // and has been read by both tiles' MMAs
     auto bar_sfull = [&](int t) { return bars + 96 + 8 * t; };     // scores of a tile (and its P.V before that) complete
-    auto bar_phalf = [&](int t) { return bars + 112 + 8 * t; };    // first 64 keys' probabilities of a tile in tensor memory
+    auto bar_phalf = [&](int t) { return bars + 112 + 8 * t; };    // first 96 keys' probabilities of a tile in tensor memory (64 in a half round)
     auto bar_pfull = [&](int t) { return bars + 128 + 8 * t; };    // all of them
     auto bar_ofinal = [&](int t) { return bars + 144 + 8 * t; };   // an item's last P.V of a tile complete
     auto bar_item = [&](int s) { return bars + 160 + 8 * s; };     // ring entry s published
@@ -979,8 +992,8 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 
     // Three warpgroups: 0 and 1 are the softmax warps of tile 0 and 1, 2 holds the issuer, the producer and two idle
     // warps.  The block starts with 168 registers per thread (the cap of 384 threads); the third warpgroup hands
-    // most of its registers back and the softmax warpgroups grow to 224, which holds a whole 128-key score row, its
-    // probabilities and the step's state without spilling.
+    // half of its registers back and the softmax warpgroups grow to 208, which holds a whole 128-key score row, its
+    // probabilities and the step's state without spilling.  (56 and 224 spill in the producer: 24 x 310 tokens 46.4 us, 46.0.)
 
     if (warp >= 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kRegsLow5));
@@ -1100,12 +1113,13 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                         ok = wait_bar_warp(bar_phalf(t), G & 1, abort_flag, 25);
                         if (!ok) break;
                         tc_fence_after();
-                        umma_pv<0>(leader, t_o, t_s, dv, p.idesc_pv, j > 0 ? 1u : 0u);
+                        umma_pv<0, 4>(leader, t_o, t_s, dv, p.idesc_pv, j > 0 ? 1u : 0u);
+                        if (!(last && half)) umma_pv<4, 6>(leader, t_o, t_s, dv, p.idesc_pv, 1u);
                         ok = wait_bar_warp(bar_pfull(t), G & 1, abort_flag, 27);
                         if (!ok) break;
                         if (!(last && half)) {
                             tc_fence_after();
-                            umma_pv<4>(leader, t_o, t_s, dv, p.idesc_pv, 1u);
+                            umma_pv<6, 8>(leader, t_o, t_s, dv, p.idesc_pv, 1u);
                         }
                         if (t == 1) tc_commit_by(leader, bar_empty(vs));
                         if (last) tc_commit_by(leader, bar_ofinal(t));
@@ -1249,7 +1263,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             ++n;
         }
         if (MIXED && !decode_first) {
-            // Here, where these warps have their 224 registers: behind the roles the code has to make do with the 56 of the other warpgroup,
+            // Here, where these warps have their 208 registers: behind the roles the code has to make do with those of the other warpgroup (56 then),
             // and a context of 4096 keys took 170 us instead of 90 (1 prompt of 300 tokens, 64 decode rows, 8 blocks: 186 us a step; 3 of 500 to 2048,
             // 90 rows, 30 blocks: 296).  Both tiles are done with the shared memory when all softmax warps are here.
             asm volatile("bar.sync 3, %0;\n" ::"n"(2 * kBM) : "memory");
