@@ -13,7 +13,7 @@
 //   * every lane group keeps its own running maximum and sum per query head; groups merge by shuffles, warps through shared
 //     memory, blocks through distributed shared memory -- one launch, no workspace.
 // Batch 8, 16 / 8 heads, fp32, context 64 .. 1024, store + decode: 2031 us a pass with one warp per (sequence, head) walking its
-// keys in order, 15.7 us here, of which up to four trips of load, dot product, exponentials and sum follow one another in a warp.
+// keys in order, 15.4 us here (16.5 with branches around the loads of a key and merges written out part by part), of which up to four trips of load, dot product, exponentials and sum follow one another in a warp.
 #include "nvk_internal.cuh"
 
 #include <cooperative_groups.h>
@@ -56,9 +56,22 @@ template <> __device__ __forceinline__ void unpack<__half>(const uint4& w, float
     }
 }
 
-__device__ __forceinline__ uint4 ld_stream16(const void* p) {   // K / V rows are read once
+// K / V rows are read once; zeros, and no read, where there is no row (by a predicate: branches around the loads of each key doubled the loop's code).
+__device__ __forceinline__ uint4 ld_stream16(const void* p, bool there) {
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
+        "@q ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}\n"
+        : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "r"(static_cast<int>(there)));
+    return v;
+}
+
+// A float of this block's shared memory, as block `rank` of the cluster has it.
+__device__ __forceinline__ float ld_block(const float* p, uint32_t rank) {
+    float v;
+    asm volatile(
+        "{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.f32 %0, [a];\n\t}\n"
+        : "=f"(v) : "r"(smem_u32(p)), "r"(rank) : "memory");
     return v;
 }
 
@@ -130,13 +143,8 @@ __global__ void __launch_bounds__(kThreads, HG <= 2 ? 2 : 1) decode_simt_kernel(
             live[u] = row[u] != -2;
 #pragma unroll
             for (int i = 0; i < NV; ++i) {
-                if (row[u] >= 0) {
-                    kv[u][i] = ld_stream16(kc + row[u] * row_elems + i * LANES * VE);
-                    vv[u][i] = ld_stream16(vc + row[u] * row_elems + i * LANES * VE);
-                } else {
-                    kv[u][i] = make_uint4(0u, 0u, 0u, 0u);
-                    vv[u][i] = make_uint4(0u, 0u, 0u, 0u);
-                }
+                kv[u][i] = ld_stream16(kc + row[u] * row_elems + i * LANES * VE, row[u] >= 0);
+                vv[u][i] = ld_stream16(vc + row[u] * row_elems + i * LANES * VE, row[u] >= 0);
             }
         }
 #pragma unroll
@@ -207,15 +215,19 @@ __global__ void __launch_bounds__(kThreads, HG <= 2 ? 2 : 1) decode_simt_kernel(
     // lane groups -> warp
 #pragma unroll
     for (int h = 0; h < HG; ++h) {
+        float mx = m[h];
+#pragma unroll
+        for (int o = LANES; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const float f = m[h] == -INFINITY ? 0.0f : expf(m[h] - mx);
+        m[h] = mx;
+        l[h] *= f;
+#pragma unroll
+        for (int e = 0; e < 16; ++e) acc[h][e] *= f;
 #pragma unroll
         for (int o = LANES; o < 32; o <<= 1) {
-            const float om = __shfl_xor_sync(0xffffffffu, m[h], o), ol = __shfl_xor_sync(0xffffffffu, l[h], o);
-            const float mx = fmaxf(m[h], om);
-            const float f = m[h] == -INFINITY ? 0.0f : expf(m[h] - mx), g = om == -INFINITY ? 0.0f : expf(om - mx);
-            l[h] = l[h] * f + ol * g;
+            l[h] += __shfl_xor_sync(0xffffffffu, l[h], o);
 #pragma unroll
-            for (int e = 0; e < 16; ++e) acc[h][e] = acc[h][e] * f + __shfl_xor_sync(0xffffffffu, acc[h][e], o) * g;
-            m[h] = mx;
+            for (int e = 0; e < 16; ++e) acc[h][e] += __shfl_xor_sync(0xffffffffu, acc[h][e], o);
         }
         if (grp == 0) {
 #pragma unroll
@@ -245,12 +257,28 @@ __global__ void __launch_bounds__(kThreads, HG <= 2 ? 2 : 1) decode_simt_kernel(
     for (int i = rank * kThreads + tid; i < heads * D; i += csize * kThreads) {
         const int h = i / D, d = i % D;
         float mx = -INFINITY, lsum = 0.0f, o = 0.0f;
-        for (int r = 0; r < csize; ++r) mx = fmaxf(mx, *cluster.map_shared_rank(&s_pm[h], r));
-        for (int r = 0; r < csize; ++r) {
-            const float pm = *cluster.map_shared_rank(&s_pm[h], r);
-            const float f = pm == -INFINITY ? 0.0f : expf(pm - mx);
-            lsum += f * *cluster.map_shared_rank(&s_pl[h], r);
-            o += f * *cluster.map_shared_rank(&s_po[h][d], r);
+#pragma unroll 1
+        for (int r0 = 0; r0 < csize; r0 += 4) {   // (four blocks' loads under way at once)
+            float pm[4], pl[4], po[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const uint32_t from = static_cast<uint32_t>(min(r0 + u, csize - 1));
+                pm[u] = ld_block(&s_pm[h], from);
+                pl[u] = ld_block(&s_pl[h], from);
+                po[u] = ld_block(&s_po[h][d], from);
+                if (r0 + u >= csize) pm[u] = -INFINITY;
+            }
+            const float m_new = fmaxf(fmaxf(fmaxf(pm[0], pm[1]), fmaxf(pm[2], pm[3])), mx);
+            const float f = mx == -INFINITY ? 0.0f : expf(mx - m_new);
+            lsum *= f;
+            o *= f;
+            mx = m_new;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const float w = pm[u] == -INFINITY ? 0.0f : expf(pm[u] - mx);
+                lsum += w * pl[u];
+                o += w * po[u];
+            }
         }
         out[i] = ElemTraits<T>::from_float(lsum > 0.0f ? o / lsum : 0.0f);
     }
