@@ -789,6 +789,7 @@ __device__ __forceinline__ void softmax_row(uint32_t t_s, uint32_t t_o, bool mas
 //                                  masked round took 9000 clocks where a steady one took 2600
 //   3043; 832 / 498 / 101 / 50     the issuing warp converged, descriptors in uniform registers (umma_ss_by)
 //   3002; 805 / 472 / 94 / 47      outputs in whole lines through 32 KB of shared memory (four stages are enough), masks by one compare a score
+//   2990; 805 / 470 / 93 / 46      96 of 128 keys' probabilities handed over early, no spills in the third warpgroup
 // Not here: the first 32 keys' maximum as reference with the row sum as check (no maxima at all, but nothing can be handed to the MMAs before the
 // end: 3307); maxima in the shadow of the exponentials (3427); tickets taken by a warp of its own two items ahead (uneven ends: one prompt of
 // 8192 tokens, 16 / 8 heads, 217 -> 255 us).  Steps of 64 keys would need 2560 clocks of MMAs: at N 64 they are bound by shared memory.
