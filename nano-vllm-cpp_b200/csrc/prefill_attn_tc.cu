@@ -644,6 +644,9 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 
 constexpr int kTmemCols2 = 512;   // head-pair kernels: S0 S1 O0 O1
 
+__device__ __forceinline__ void mbar_arrive_if(bool one, uint32_t bar) {   // by a predicate, without a branch
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %1, 0;\n\t@q mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}\n" ::"r"(bar), "r"(static_cast<int>(one)) : "memory");
+}
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
@@ -1185,7 +1188,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             tc_wait_st();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar);
+            mbar_arrive_if(lane == 0, bar);   // (the warp stays converged: more tcgen05.st.sync.aligned follow)
         };
         while (alive) {
             alive = wait_bar_warp(bar_item(n & 3), (n >> 2) & 1, abort_flag, 33);
