@@ -266,7 +266,8 @@ __global__ void __launch_bounds__(kThreads, HG <= 2 ? 2 : 1) decode_simt_kernel(
                 pm[u] = ld_block(&s_pm[h], from);
                 pl[u] = ld_block(&s_pl[h], from);
                 po[u] = ld_block(&s_po[h][d], from);
-                if (r0 + u >= csize) pm[u] = -INFINITY;
+                // (no weight of 0 takes out what a block that is not there would add: the last block's part, read in its place, may be infinite)
+                if (r0 + u >= csize) { pm[u] = -INFINITY; pl[u] = po[u] = 0.0f; }
             }
             const float m_new = fmaxf(fmaxf(fmaxf(pm[0], pm[1]), fmaxf(pm[2], pm[3])), mx);
             const float f = mx == -INFINITY ? 0.0f : expf(mx - m_new);

@@ -48,3 +48,25 @@ def test_decode_simt_matches_a_float64_reference(dtype, head_dim, block_size, nu
     err = np.abs(to_np(out) - _reference(w, num_kv_heads, block_size))
     assert err.max() <= (2e-6 if dtype == "f32" else 1e-2), err.max()
     assert math.isfinite(float(out.float().abs().max()))
+
+
+@pytest.mark.parametrize("dtype,head_dim", [("f32", 128), ("f16", 64)])
+@pytest.mark.parametrize("batch", [1, 6, 10, 20])   # 8 KV heads: clusters of 8, 4, 2 and 1
+def test_infinite_values_stay_infinite(dtype, head_dim, batch):
+    """A visible V row with infinities: these elements of the output are infinite with its sign, all others as without it."""
+    ctx = np.array([(300, 77, 1000, 520, 64)[i % 5] for i in range(batch)], np.int32)
+    w = workloads().make_decode_workload(batch, 16, 8, head_dim, 16, 0, 0, seed=batch, context_lens=ctx, value_scale=0.5)
+    td = torch.float32 if dtype == "f32" else torch.float16
+    for n in ("q", "k_cache", "v_cache"):
+        w[n] = torch.from_numpy(w[n]).to(td).float().numpy()
+    for b in range(batch):
+        for pos, at, value in ((0, 3, np.inf), (int(ctx[b]) - 1, 5, -np.inf), (int(ctx[b]) // 2, head_dim - 1, np.inf)):
+            w["v_cache"][w["block_tables"][b, pos // 16], pos % 16, b % 8, at] = value
+    q = to_dev(w["q"], td)
+    out = torch.full_like(q, float("nan"))
+    nvk().launch_decode_attention_paged(q, to_dev(w["k_cache"], td), to_dev(w["v_cache"], td), to_dev(ctx), to_dev(w["block_tables"]), 8, head_dim, 16,
+                                        w["scale"], out)
+    ref, got = _reference(w, 8, 16), to_np(out)
+    assert np.isinf(ref).sum() == 3 * 2 * batch
+    assert np.array_equal(got[np.isinf(ref)], ref[np.isinf(ref)])
+    assert np.abs(got - ref)[np.isfinite(ref)].max() <= (2e-6 if dtype == "f32" else 1e-2)
