@@ -134,7 +134,10 @@ __device__ __forceinline__ uint32_t in_block(uint32_t addr, uint32_t rank) {   /
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
+// `.aligned` instructions (this barrier, tcgen05.ld and its wait, allocation) want the whole warp at one place.  What lanes do on their own before one
+// -- a branch on a row's slot or position, a single lane's store -- is followed by a warp barrier, a shuffle or a vote.
 __device__ __forceinline__ void cluster_sync_all() {
+    __syncwarp();
     asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
 }
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -210,6 +213,7 @@ __device__ __forceinline__ void st_tagged(uint4* slot, const uint4& v, uint32_t 
 template <typename T>
 __device__ __forceinline__ void load_rounded(uint32_t taddr, float (&v)[32]) {
     uint32_t r[32];
+    __syncwarp();   // (epilogue_row branches on what a row needs, lane by lane)
     tmem_ld32(taddr, r);
     tc_wait_ld();
     reg_fence32(r);

@@ -178,6 +178,9 @@ __device__ __forceinline__ void umma_pv(uint32_t leader, uint32_t d_tmem, uint32
         umma_ts_by(leader, d_tmem, p_tmem + kk * 8, v_base + kk * 2048 / 16, idesc, kk > FIRST ? 1u : acc_first);
 }
 
+// These and the other `.sync.aligned` instructions want the whole warp at one place: what a single lane does before one goes by a predicate
+// (mbar_arrive_if, *_by) or is followed by a warp barrier, a shuffle or a vote.  The waits for a whole warp are such: warp_mbar_wait ends with a shuffle,
+// wait_bar_warp with a vote.
 __device__ __forceinline__ void tmem_ld32(uint32_t addr, uint32_t (&r)[32]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
@@ -1270,6 +1273,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             // Here, where these warps have their 208 registers: behind the roles the code has to make do with those of the other warpgroup (56 then),
             // and a context of 4096 keys took 170 us instead of 90 (1 prompt of 300 tokens, 64 decode rows, 8 blocks: 186 us a step; 3 of 500 to 2048,
             // 90 rows, 30 blocks: 296).  Both tiles are done with the shared memory when all softmax warps are here.
+            __syncwarp();   // (lanes come from the stores of their rows)
             asm volatile("bar.sync 3, %0;\n" ::"n"(2 * kBM) : "memory");
             decode_half();
         }

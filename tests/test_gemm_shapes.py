@@ -78,3 +78,29 @@ def test_qkv_prologue_takes_a_rotary_table_at_any_address(rows, hidden):
     assert nvk().gemm_status() == 0
     for o in got[1:]:
         assert all(torch.equal(a, b) for a, b in zip(o, got[0])) and not any(torch.isnan(a.float()).any() for a in o)
+
+
+@pytest.mark.parametrize("rows,hidden", [(37, 2048), (200, 512), (700, 1024)])     # summed over a cluster, a block each, pairs
+def test_rows_of_a_warp_that_go_different_ways(rows, hidden):
+    """Neighbouring rows with and without a slot, with and without a rotary row: each comes out as in a call where all rows are alike."""
+    bf, d, hq, hkv = torch.bfloat16, 128, 16, 8
+    gen = torch.Generator(device="cuda").manual_seed(rows + 1)
+    x = torch.randn((rows, hidden), generator=gen, device="cuda").to(bf)
+    w = (torch.randn(((hq + 2 * hkv) * d, hidden), generator=gen, device="cuda") / hidden ** 0.5).to(bf)
+    table, norm = to_dev(oracle.build_cos_sin_cache(rows, d, 1e6)), torch.ones(d, dtype=bf, device="cuda")
+    every = torch.arange(rows, dtype=torch.int32, device="cuda")
+
+    def run(pos, slots):
+        q, k, v = (torch.zeros((rows, h, d), dtype=bf, device="cuda") for h in (hq, hkv, hkv))
+        nvk().qkv_linear_norm_rope_store(x, w, pos, norm, norm, 1e-6, table, slots, k, v, hq, hkv, d, q)
+        return q, k, v
+
+    turned, plain = run(every, every), run(torch.full_like(every, rows), every)
+    slot, rope = every % 2 == 0, every % 3 != 0
+    q, k, v = run(torch.where(rope, every, rows + 5), torch.where(slot, every, -1))
+    torch.cuda.synchronize()
+    assert nvk().gemm_status() == 0
+    pick = rope[:, None, None]
+    assert torch.equal(q, torch.where(pick, turned[0], plain[0]))
+    assert torch.equal(k, torch.where(pick, turned[1], plain[1]) * slot[:, None, None])
+    assert torch.equal(v, turned[2] * slot[:, None, None])
