@@ -604,7 +604,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         for (int c = 0; c < 4; ++c) {
             uint32_t r[32];
             tmem_ld32(t_o + c * 32, r);
-            tc_wait_ld();
+            tc_wait_ld(); reg_fence32(r);
 #pragma unroll
             for (int q4 = 0; q4 < 4; ++q4) {
                 uint4 v;
