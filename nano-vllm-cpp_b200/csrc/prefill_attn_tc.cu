@@ -1447,7 +1447,7 @@ static bool tc_shape_supported(const PrefillArgs& a) {
     return encode_fn() != nullptr;
 }
 
-// (A hidden score is minus infinity before it is scaled.)
+// (A hidden score is minus infinity before it is scaled, in softmax_row as in the chunk_max and chunk_probs of odd groups.)
 bool prefill_tc_supported(const PrefillArgs& a) { return a.scale > 0.0f && tc_shape_supported(a); }
 
 int launch_prefill_tc(const PrefillArgs& a) {

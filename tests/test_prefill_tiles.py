@@ -86,6 +86,14 @@ def test_scales_that_are_not_positive(scale):
     assert_attention_close(to_np(out), ref)
 
 
+@pytest.mark.parametrize("scale", [0.0, -0.05])
+def test_odd_groups_with_scales_that_are_not_positive(scale):
+    """Their tensor-core kernel hides scores before it scales them as well."""
+    w = workloads().make_prefill_workload([70, 130], [0, 256], 6, 2, 128, 256, seed=13, paged=True)
+    out, ref = _run(w, 2, True, scale)
+    assert_attention_close(to_np(out), ref)
+
+
 def test_a_mixed_step_takes_scales_that_are_not_positive():
     bf, lib, hkv = torch.bfloat16, nvk(), 2
     p = workloads().make_prefill_workload([70, 20], [0, 256], 8, hkv, 128, 256, seed=12, paged=True)
