@@ -24,7 +24,8 @@
 // Before, one block per 128 x 128 tile whatever the size (microseconds in a loop over weights larger than L2; K 4096):
 //   64 x 6144  22 -> 16      64 x 4096  21 -> 12 (with MMAs from a converged warp 14.5 and 11.1)     7440 x 4096  295 -> 175 (1430 TFLOP/s)     7440 x 6144 with QKV epilogue  597 -> 277
 // What the fusion removes is the round trip of the result and one or two launches per layer.
-// Every mbarrier wait is bounded; a wait that runs out raises an error word (nvk_gemm_status) and the block leaves.
+// Every mbarrier wait is bounded; a wait that runs out raises an error word (nvk_gemm_status), and the block leaves when what it
+// has under way has had time to land.
 #include "nvk_internal.cuh"
 
 #include <cuda.h>
@@ -111,6 +112,13 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
         }
     }
     return true;
+}
+// Where a wait gave up, by the warp that frees the block's tensor memory, before it does (the block is there until all its warps have left): copies into
+// shared memory and MMAs that read it may still be under way, and a wait for each would end with the same limit at the latest.  2 ms.
+__device__ __forceinline__ void settle() {
+    const long long start = clock64();
+    while (clock64() - start < 4000000) {}
+    __syncwarp();
 }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
     asm volatile(
@@ -602,6 +610,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
+        if (*abort_flag) settle();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
     }
     if (DIRECT) return;
@@ -741,6 +750,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     }
     tc_fence_before();
     __syncthreads();
+    if (warp == 1 && *abort_flag) settle();
     cluster_sync_all();   // neither block leaves while the other may still signal its barriers or read its operands
     if (warp == 1) {
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(2 * kPairCols) : "memory");

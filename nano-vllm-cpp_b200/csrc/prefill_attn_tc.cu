@@ -25,7 +25,7 @@
 //     division by the row sum.
 //   * 256 TMEM columns and 96 KiB of shared memory per block: two blocks per SM, so one block's
 //     softmax overlaps the other's MMAs.  Every mbarrier wait is bounded; on a time-out the block
-//     raises an error word, stops waiting, frees its TMEM and returns.
+//     raises an error word, stops waiting, gives what is under way time to land, frees its TMEM and returns.
 //   * No cluster launch and no multicast anywhere.
 #include "decode_body.cuh"
 
@@ -107,6 +107,13 @@ __device__ __forceinline__ bool warp_mbar_wait(uint32_t bar, uint32_t parity, vo
     int ok = 1;
     if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, abort_flag, code) ? 1 : 0;
     return __shfl_sync(0xffffffffu, ok, 0) != 0;
+}
+// Where a wait gave up, by the warp that frees the block's tensor memory, before it does (the block is there until all its warps have left): copies into
+// shared memory and MMAs that read it may still be under way, and a wait for each would end with the same limit at the latest.  2 ms.
+__device__ __forceinline__ void settle() {
+    const long long start = clock64();
+    while (clock64() - start < 4000000) {}
+    __syncwarp();
 }
 __device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
@@ -631,16 +638,9 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             }
         }
     }
-    if (*abort_flag && tid == 0) {
-        // give copies that may still be in flight a bounded chance to land before the block retires
-        for (int j = 0; j < 2; ++j) {
-            const long long start = clock64();
-            while (!mbar_try_wait(bar_k, j) && clock64() - start < 2000000) {}
-            while (!mbar_try_wait(bar_v, j) && clock64() - start < 4000000) {}
-        }
-    }
     __syncwarp();
     if (warp == 0) {
+        if (*abort_flag) settle();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
     }
 }
@@ -1282,6 +1282,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     __syncthreads();
     if (tid == 0 && s_abort != 0) atomicCAS(&g_tc_error, 0, s_abort);
     if (warp == 8) {
+        if (s_abort != 0) settle();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kTmemCols2) : "memory");
     }
 }
