@@ -53,7 +53,7 @@ struct IndexArray {
         return wide ? static_cast<const int64_t*>(ptr)[i] : static_cast<int64_t>(static_cast<const int32_t*>(ptr)[i]);
     }
     // The same as one of two predicated loads, half the code, but no load that the compiler may move: for kernels that look up many indices in a loop
-    // (fp32 decode of 8 sequences 16.4 -> 15.7 us a pass; 1 sequence in the tensor-core kernel 7.2 -> 7.3, which keeps the branch).
+    // (fp32 decode of 8 sequences 16.65 -> 15.9 us a pass; 1 sequence in the tensor-core kernel 7.2 -> 7.3, which keeps the branch).
     __device__ __forceinline__ int64_t load(int64_t i) const {
         int64_t v;
         asm volatile(

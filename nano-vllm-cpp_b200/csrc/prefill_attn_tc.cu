@@ -1474,8 +1474,8 @@ int launch_mixed_typed(const PrefillArgs& a, const DecodeArgs& d, int prefill_bl
     if (prefill_blocks <= 0) {
         // No hint: split the SMs by a crude estimate from host-known sizes -- prefill flops as if all sequences were equally
         // long and had no prefix, at 0.6 PFLOP/s; decode bytes as if every block table were half full, at 6.5 TB/s.  Against the best of 17
-        // splits for 19 steps (1 to 6 prompts of 64 to 4000 tokens, 8 to 192 decode rows) it costs 3 % on average and 11 % at most (0.3 PFLOP/s
-        // 3.5 %, 1.0 4.7 %): it matters little, since every block sees to what is left of the other kind.
+        // splits for 19 steps (1 to 6 prompts of 64 to 4000 tokens, 8 to 192 decode rows) it costs 3 % on average and 11 % at most (with 0.3 PFLOP/s
+        // 3.5 % on average, with 1.0 4.7 %): it matters little, since every block sees to what is left of the other kind.
         const double mean_q = static_cast<double>(a.total_q) / static_cast<double>(a.cu_q ? a.num_seqs : 1);
         const double t_prefill = 4.0 * a.num_heads * kHeadDim * static_cast<double>(a.total_q) * (mean_q + 1.0) / 2.0 / 0.6e15;
         const double t_decode = 0.5 * static_cast<double>(d.batch) * d.max_blocks * d.block_size * d.num_kv_heads * kHeadDim * 4.0 / 6.5e12;
