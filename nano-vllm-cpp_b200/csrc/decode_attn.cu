@@ -13,8 +13,6 @@
 // Which one is taken depends on the table's WIDTH, not on the contexts: one short sequence in a wide table takes chunks and a merge.
 #include "decode_body.cuh"
 
-#include <cooperative_groups.h>
-
 #include <atomic>
 #include <cmath>
 
@@ -22,13 +20,12 @@ namespace nvk {
 namespace {
 
 using namespace dec;
-namespace cg = cooperative_groups;
 
 constexpr size_t kStaticScratchBytes = 32u << 20;
 constexpr int kMaxCluster = 8;          // portable cluster size
 // Longest range per block (of a full table row) that goes to the cluster kernel: 8 tiles per warp, some 5 us of keys.  Up to there the
-// second launch costs more than chunks of even length give: 1 sequence of 300 keys, 32 / 8 heads, with its prologue, takes 6.7 us a
-// pass in a replayed graph where split and merge took 9.1.
+// second launch costs more than chunks of even length give: 1 sequence of 300 keys, 32 / 8 heads, with its prologue, took 6.7 us a
+// pass in a replayed graph where split and merge took 9.1 (5.9 now).
 constexpr int kClusterTokens = 512;
 
 // Sequence number `rank` in order of falling context length, found by every block for itself.  In index order the last blocks to start
@@ -80,6 +77,18 @@ __device__ __forceinline__ int sequence_of_rank(const DecodeParams& p, int rank,
     }
 }
 
+__device__ __forceinline__ uint32_t in_block(uint32_t addr, uint32_t rank) {   // the same place in block `rank` of the cluster
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_cluster4(uint32_t addr, uint32_t rank, const float4& v) {
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"r"(in_block(addr, rank)), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+__device__ __forceinline__ void st_cluster2(uint32_t addr, uint32_t rank, float x, float y) {
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};\n" ::"r"(in_block(addr, rank)), "f"(x), "f"(y) : "memory");
+}
+
 template <class F, typename T>
 __global__ void __launch_bounds__(kGroupThreads, F::kGroups) decode_split_kernel(const __grid_constant__ DecodeParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -90,13 +99,16 @@ __global__ void __launch_bounds__(kGroupThreads, F::kGroups) decode_split_kernel
     run_split<F, T>(p, b, blockIdx.x, split, *reinterpret_cast<GroupSmem<F>*>(smem), threadIdx.x, 1);
 }
 
-// HG > 0: one warp per (sequence, KV head), HG heads at a time, in blocks of kMergeBlockWarps warps, small enough to be resident
+// HG > 0: one warp per (sequence, KV head) and HG of its heads, in blocks of kMergeBlockWarps warps, small enough to be resident
 // beside the blocks of decode_split_kernel.  HG == 0: one block per (sequence, head), where there can be more parts than one warp
 // should add up: 3 sequences of up to 40000 keys left 12 blocks adding up 20 parts each one after the other, 10 us.  These blocks do not
-// fit beside those of decode_split_kernel, so that many of them only queue up behind it.  By warps -> by blocks, us a call: 32 rows of 75
+// fit beside those of decode_split_kernel, so that many of them only queue up behind it.  Between the two, up to 4096 rows that can have more than
+// four parts, HG is 1: 49 sequences of up to 31475 keys, 32 / 8 heads, 494 us a pass with four heads a warp, 486 with one; but 256
+// sequences (8192 rows) of which few have a second part 189 and 192.  By warps -> by blocks, us a call: 32 rows of 75
 // parts 18.3 -> 14.3, 128 rows of 64 157.1 -> 155.4, 256 of 64 160.4 -> 157.1; but 512 rows of which none has a second part 10.5 -> 11.2,
 // 4096 such rows 45.0 -> 50.8, 4096 rows of 2 parts in 32768-key tables 230 -> 244.
 constexpr int kMergeBlockRows = 2 * kSmCount;
+constexpr int kMergeSingleRows = 4096;
 constexpr int kMergeBlockWarps = 2;
 template <typename T, int HG>
 __global__ void __launch_bounds__((HG > 0 ? kMergeBlockWarps : kMergeWarps) * 32) decode_merge_kernel(const __grid_constant__ DecodeParams p) {
@@ -104,8 +116,8 @@ __global__ void __launch_bounds__((HG > 0 ? kMergeBlockWarps : kMergeWarps) * 32
     pdl_wait_then_release();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     auto parts_of = [&](int b, int kvh, int& n) {   // n parts of (b, kvh) and where they are
-        int t0, t1;
-        n = split_range(p, clamped_context(p, b), 0, t0, t1);
+        const int ctx = clamped_context(p, b), len = range_len(p, ctx);
+        n = ctx > 0 ? (ctx + len - 1) / len : 0;
         const size_t part = (static_cast<size_t>(b) * p.num_kv_heads + kvh) * p.num_splits;
         const float* o = p.ws_o + part * p.group * kHeadDim;
         const float2* ml = p.ws_ml + part * p.group;
@@ -114,11 +126,12 @@ __global__ void __launch_bounds__((HG > 0 ? kMergeBlockWarps : kMergeWarps) * 32
     T* out = static_cast<T*>(p.out);
     int n;
     if constexpr (HG > 0) {
-        const int item = blockIdx.x * kMergeBlockWarps + warp;
-        if (item >= p.batch * p.num_kv_heads) return;
-        const int b = item / p.num_kv_heads;
-        const auto get = parts_of(b, item - b * p.num_kv_heads, n);
-        if (n > 1) merge_by_warp<T, HG>(get, n, p.group, out + static_cast<int64_t>(item) * p.group * kHeadDim, lane);
+        const int item = blockIdx.x * kMergeBlockWarps + warp, chunks = (p.group + HG - 1) / HG;
+        const int pair = item / chunks;
+        if (pair >= p.batch * p.num_kv_heads) return;
+        const int b = static_cast<int>(p.by_kv_heads.div(pair));
+        const auto get = parts_of(b, pair - b * p.num_kv_heads, n);
+        if (n > 1) merge_by_warp<T, HG>(get, n, (item - pair * chunks) * HG, p.group, out + static_cast<int64_t>(pair) * p.group * kHeadDim, lane);
     } else {
         const int row = blockIdx.x, b = row / p.num_heads, head = row - b * p.num_heads, kvh = head / p.group;
         const auto get = parts_of(b, kvh, n);
@@ -126,32 +139,61 @@ __global__ void __launch_bounds__((HG > 0 ? kMergeBlockWarps : kMergeWarps) * 32
     }
 }
 
+// A block pushes what it has of the result into the shared memory of the block that finishes it: of 32 quads of a head, block r of the cluster takes
+// 32 / size from r * 32 / size on.  After one cluster barrier everything there is local, and no block has to wait for its peers to have
+// read.  1 sequence of 300 keys, 32 / 8 heads, with its prologue: 7.2 -> 5.85 us a pass with the block ids fetched along with the context and one
+// barrier in a block's merge; from a block's last tile to its end it had been 2.5 us of 4.3.
 template <class F, typename T>
 __global__ void __launch_bounds__(kGroupThreads, F::kGroups) decode_cluster_kernel(const __grid_constant__ DecodeParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ __align__(16) float part_o[kMaxGroup * kHeadDim];
-    __shared__ float2 part_ml[kMaxGroup];
+    __shared__ float4 s_o[kMaxGroup * kHeadDim / 4];           // [block of the cluster][head][quad of this block]
+    __shared__ float2 s_ml[kMaxCluster * kMaxGroup];           // [block of the cluster][head]
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");   // (waited for before the first remote store: every block has started)
     pdl_wait_then_release();
-    cg::cluster_group cluster = cg::this_cluster();
-    const int rank = static_cast<int>(cluster.block_rank());
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int pair = blockIdx.x / p.num_splits;
-    const int kvh = pair % p.num_kv_heads, b = pair / p.num_kv_heads;
-    const int ctx = clamped_context(p, b);
-    int t0, t1;
-    const int n = split_range(p, ctx, rank, t0, t1);
-    if (t0 < t1)
-        attend_range<F>(p, b, kvh, t0, t1, *reinterpret_cast<GroupSmem<F>*>(smem), threadIdx.x, 1,
-                        [&](int h, int d, float o, float m, float l) { write_part(part_o, part_ml, h, d, o, m, l); });
-    cluster.sync();
-    auto get = [&](int i) { return PartRef{cluster.map_shared_rank(part_o, i), cluster.map_shared_rank(part_ml, i)}; };
-    T* out = static_cast<T*>(p.out) + static_cast<int64_t>(pair) * p.group * kHeadDim;
-    for (int h = rank * kGroupWarps + warp; h < p.group; h += p.num_splits * kGroupWarps) {
-        Merged acc[1];
-        sum_parts<1>(get, n, 0, 1, h, p.group, lane, acc);   // (an empty context has no parts: zeros)
-        write_merged<T>(out + h * kHeadDim, acc[0], lane);
+    const int rank = static_cast<int>(blockIdx.x) & (p.num_splits - 1), pair = static_cast<int>(blockIdx.x) >> p.split_shift;
+    const int b = static_cast<int>(p.by_kv_heads.div(pair)), kvh = pair - b * p.num_kv_heads;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const IndexArray::Raw raw_ctx = p.context_lens.raw(b);
+    IndexArray::Raw raw_ids = load_ids(p, b, 0, lane);
+    const int ctx = clamped_context(p, raw_ctx), len = range_len(p, ctx);
+    const int t0 = rank * len, t1 = min(ctx, t0 + len);
+    const int quad_shift = 5 - p.split_shift, quads = 1 << quad_shift;          // quads of a head per block
+    bool waited = false;
+    auto push = [&](int h, int quad, const float4& o, float m, float l) {
+        if (!waited) asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory");
+        waited = true;
+        const uint32_t to = static_cast<uint32_t>(quad >> quad_shift);
+        const int mine = quad & (quads - 1);
+        st_cluster4(smem_u32(s_o + ((rank * p.group + h) << quad_shift) + mine), to, o);
+        if (mine == 0) st_cluster2(smem_u32(s_ml + rank * p.group + h), to, m, l);
+    };
+    if (t0 < t1) {
+        attend_range<F>(p, b, kvh, t0, t1, raw_ids, 0, *reinterpret_cast<GroupSmem<F>*>(smem), tid, 1, push);
+    } else {
+        for (int h = tid >> 5; h < p.group; h += kGroupWarps) push(h, lane, make_float4(0.f, 0.f, 0.f, 0.f), -INFINITY, 0.0f);
     }
-    cluster.sync();   // no block leaves while a peer still reads its shared memory
+    if (!waited) asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory");   // (a warp without a head)
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory");
+    T* out = static_cast<T*>(p.out) + static_cast<int64_t>(pair) * p.group * kHeadDim;
+    for (int i = tid; i < p.group << quad_shift; i += kGroupThreads) {
+        const int h = i >> quad_shift, quad = (rank << quad_shift) + (i & (quads - 1));
+        Merged acc = nothing_merged();
+        for (int r0 = 0; r0 < p.num_splits; r0 += 4) {
+            float4 v[4];
+            float2 ml[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const bool there = r0 + u < p.num_splits;
+                const int r = there ? r0 + u : 0;
+                v[u] = s_o[(r * p.group << quad_shift) + i];
+                ml[u] = s_ml[r * p.group + h];
+                if (!there) { v[u] = make_float4(0.f, 0.f, 0.f, 0.f); ml[u] = make_float2(-INFINITY, 0.0f); }
+            }
+            acc.add(v, ml);
+        }
+        if (ctx == 0) acc = nothing_merged();
+        write_merged<T>(out + h * kHeadDim, acc, quad);
+    }
 }
 
 // ---- host side -----------------------------------------------------------------------------------------------------------
@@ -261,6 +303,9 @@ int decode_plan(const DecodeArgs& a, int groups, dec::DecodeParams* out, int* cl
     const Splits s = choose_splits(a.batch, a.num_heads, a.num_kv_heads, a.max_blocks, a.block_size, groups, a.workspace != nullptr);
     *cluster = s.cluster;
     p.per_seq = s.cluster > 0 ? 1 : 0;
+    while (p.per_seq && (1 << p.split_shift) < s.cluster) ++p.split_shift;
+    p.by_block = FastDiv(static_cast<uint32_t>(a.block_size));
+    p.by_kv_heads = FastDiv(static_cast<uint32_t>(a.num_kv_heads));
     p.chunk_tokens = s.chunk;
     p.num_splits = s.count;
     // More than one wave of blocks: the long contexts first, so that the last blocks to start are short.  Contexts in a few chunks as well:
@@ -290,10 +335,11 @@ int launch_merge_typed(const dec::DecodeParams& p, cudaStream_t stream) {
     if (p.num_splits > kMergeWarps && p.batch * p.num_heads <= kMergeBlockRows) {
         e = launch_pdl(decode_merge_kernel<T, 0>, dim3(p.batch * p.num_heads), dim3(kMergeWarps * 32), 0, stream, p);
     } else {
-        const dim3 grid((p.batch * p.num_kv_heads + kMergeBlockWarps - 1) / kMergeBlockWarps), block(kMergeBlockWarps * 32);
-        e = p.group > 2 ? launch_pdl(decode_merge_kernel<T, 4>, grid, block, 0, stream, p)
-            : p.group == 2 ? launch_pdl(decode_merge_kernel<T, 2>, grid, block, 0, stream, p)
-                           : launch_pdl(decode_merge_kernel<T, 1>, grid, block, 0, stream, p);
+        const int hg = p.group == 1 || (p.num_splits > 4 && p.batch * p.num_heads <= kMergeSingleRows) ? 1 : p.group == 2 ? 2 : 4;
+        const dim3 grid((p.batch * p.num_kv_heads * ((p.group + hg - 1) / hg) + kMergeBlockWarps - 1) / kMergeBlockWarps), block(kMergeBlockWarps * 32);
+        e = hg == 4 ? launch_pdl(decode_merge_kernel<T, 4>, grid, block, 0, stream, p)
+            : hg == 2 ? launch_pdl(decode_merge_kernel<T, 2>, grid, block, 0, stream, p)
+                      : launch_pdl(decode_merge_kernel<T, 1>, grid, block, 0, stream, p);
     }
     if (e != cudaSuccess) return fail(NVK_ERR_CUDA, "decode_merge_kernel launch: %s", cudaGetErrorString(e));
     return check_launch("decode_merge_kernel launch");

@@ -41,21 +41,25 @@ struct DecodeParams {
     int per_seq;                                       // 1: num_splits equal ranges per sequence instead of chunks
     int longest_first;                                 // blocks take the sequences in order of falling context length
     int chunk_major;                                   // decode_split_kernel's grid: all sequences' first chunks, then all second ones, ...
+    int split_shift;                                   // per_seq: log2 of num_splits
+    FastDiv by_block, by_kv_heads;
     float scale_log2;
 };
 
-// context_lens[b], limited to what the block table can address (max_blocks * block_size), and not negative.
-__device__ __forceinline__ int clamped_context(const DecodeParams& p, int b) {
-    const int64_t ctx = p.context_lens[b];
+// A context length, limited to what the block table can address (max_blocks * block_size), and not negative.
+__device__ __forceinline__ int clamped_context(const DecodeParams& p, IndexArray::Raw raw) {
+    const int64_t ctx = p.context_lens.value(raw);
     const int64_t cap = p.max_blocks * p.block_size;
     return static_cast<int>(ctx < 0 ? 0 : ctx < cap ? ctx : cap);
 }
-// Keys of range `split` of a context: [t0, t1), empty where t0 >= t1; returns how many ranges have keys.
-__device__ __forceinline__ int split_range(const DecodeParams& p, int ctx, int split, int& t0, int& t1) {
-    const int len = p.per_seq ? ((ctx + p.num_splits - 1) / p.num_splits + kTileTokens - 1) / kTileTokens * kTileTokens : p.chunk_tokens;
-    t0 = split * len;
-    t1 = min(ctx, t0 + len);
-    return ctx > 0 ? (ctx + len - 1) / len : 0;
+__device__ __forceinline__ int clamped_context(const DecodeParams& p, int b) { return clamped_context(p, p.context_lens.raw(b)); }
+// Range i of a context has keys [i * len, min(ctx, (i + 1) * len)).
+__device__ __forceinline__ int range_len(const DecodeParams& p, int ctx) {
+    return p.per_seq ? (((ctx + p.num_splits - 1) >> p.split_shift) + kTileTokens - 1) / kTileTokens * kTileTokens : p.chunk_tokens;
+}
+// Lane i: entry base + i of a sequence's block table, as loaded.  Entries past the context are loaded and not used.
+__device__ __forceinline__ IndexArray::Raw load_ids(const DecodeParams& p, int b, int base, int lane) {
+    return p.block_tables.raw(b * p.max_blocks + base + lane, base + lane < p.max_blocks);
 }
 
 __device__ __forceinline__ void group_sync(int bar_id, int threads) { asm volatile("bar.sync %0, %1;\n" ::"r"(bar_id), "r"(threads) : "memory"); }
@@ -129,6 +133,7 @@ struct Cache16 {
     static constexpr int kTileBytes = kTileTokens * kRowBytes;
     static constexpr int kStageBytes = 2 * kTileBytes;
     static constexpr int kStages = 3;
+    static constexpr int kPartStride = kHeadDim + 8;
 
     SoftmaxState s;
     uint32_t qa[8][2];   // head g of the 8-column B tile; zero from head G on
@@ -190,9 +195,11 @@ struct Cache16 {
             mma_16816<T>(s.o[mt], a0, a1, a2, a3, pb0, pb1);
         }
     }
-    // Position i = 0..15 of lane group g holds d = dim(g, i) of head 2t + h.
-    __device__ __forceinline__ float value(int h, int i) const { return s.o[i >> 1][(i & 1) * 2 + h]; }
-    static __device__ __forceinline__ int dim(int g, int i) { return (i >> 1) * 16 + (i & 1) * 8 + g; }
+    // The warp's unnormalised output of head 2t + h.
+    __device__ __forceinline__ void write_part(float* row, int h, int g) const {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) row[8 * i + g] = s.o[i >> 1][(i & 1) * 2 + h];
+    }
 };
 
 // Two 8-bit cache elements -> two f16 (MMA operand halves).  int8: the byte glued under the exponent byte of 1024 (the word has
@@ -240,6 +247,7 @@ struct Cache8 {
     static constexpr int kScaleBytes = 2 * kTileTokens * 4;   // one 32-bit word per (K | V, token): the word that holds its fp16 scale
     static constexpr int kStageBytes = 2 * kTileBytes + kScaleBytes;
     static constexpr int kStages = 4;
+    static constexpr int kPartStride = kHeadDim + 4;
     static constexpr float kOffset = FP8 ? 0.0f : 1152.0f;    // 1024 (exponent glue) + 128 (sign flip)
     static constexpr uint32_t kFlip = FP8 ? 0u : 0x80808080u; // int8: sign bits flipped before the glue
 
@@ -349,42 +357,53 @@ struct Cache8 {
         constexpr uint32_t kOnes = 0x3C003C00u;   // {1.0, 1.0}
         if (!FP8) mma_16816<__half>(osum, kOnes, kOnes, kOnes, kOnes, pb0, pb1);
     }
-    __device__ __forceinline__ float value(int h, int i) const { return s.o[i >> 1][(i & 1) * 2 + h] - kOffset * osum[h]; }
-    static __device__ __forceinline__ int dim(int g, int i) { return 16 * g + i; }
+    __device__ __forceinline__ void write_part(float* row, int h, int g) const {
+        const float off = kOffset * osum[h];
+#pragma unroll
+        for (int i = 0; i < 8; i += 2)
+            *reinterpret_cast<float4*>(row + 16 * g + 2 * i) = make_float4(s.o[i][h] - off, s.o[i][2 + h] - off, s.o[i + 1][h] - off, s.o[i + 1][2 + h] - off);
+    }
 };
 
 // ---- a group's range of keys ---------------------------------------------------------------------------------------------
 template <class F>
 struct alignas(128) GroupSmem {
-    union {
-        unsigned char ring[kGroupWarps][F::kStages * F::kStageBytes];
-        struct {                                       // the merge, when the rings are idle
-            float o[kGroupWarps][kMaxGroup][kHeadDim];
-            float2 ml[kGroupWarps][kMaxGroup];
-        } m;
-    };
+    union Warp {
+        unsigned char ring[F::kStages * F::kStageBytes];
+        struct {                                       // what the warp leaves for the merge, when its ring is idle
+            float o[kMaxGroup * F::kPartStride];       // head 2 t + h in row 4 h + t: the lanes of a store hit different banks
+            float2 ml[kMaxGroup];
+        } part;
+    } warps[kGroupWarps];
 };
 
-// Keys [t0, t1) of sequence b (t0 < t1), one KV head.  sink(h, d, o, m, l) takes element d = this thread of head h: unnormalised
-// output, maximum and sum.  `tid`: 0..127 inside the group, `bar_id`: its named barrier; all its threads call it.
+// Keys [t0, t1) of sequence b (t0 < t1), one KV head.  sink(h, quad, o, m, l) takes elements 4 quad .. 4 quad + 3 of head h: unnormalised
+// output, maximum and sum.  `tid`: 0..127 inside the group, `bar_id`: its named barrier; all its threads call it.  `raw_ids`: block
+// table entries `id_base` + lane as loaded.  The four warps' parts come together in one trip over all heads, after one barrier (a warp writes
+// its part over its own ring; before, two barriers and a loop over the heads, a trip each).
 template <class F, class Sink>
-__device__ __forceinline__ void attend_range(const DecodeParams& p, int b, int kvh, int t0, int t1, GroupSmem<F>& sm, int tid, int bar_id, Sink sink) {
+__device__ __forceinline__ void attend_range(const DecodeParams& p, int b, int kvh, int t0, int t1, IndexArray::Raw raw_ids, int id_base, GroupSmem<F>& sm,
+                                             int tid, int bar_id, Sink sink) {
     const int bs = p.block_size, warp = tid >> 5, lane = tid & 31;
-    const uint32_t ring = smem_u32(sm.ring[warp]);
+    const uint32_t ring = smem_u32(sm.warps[warp].ring);
     const int num_tiles = (t1 - t0 + kTileTokens - 1) / kTileTokens;
     const int my_tiles = num_tiles > warp ? (num_tiles - warp + kGroupWarps - 1) / kGroupWarps : 0;
-    const int blocks = (t1 + bs - 1) / bs;
     // The issuing end: this warp's next tile begins at row `off` of table entry `blk`.  Lane i holds the cache block of entry
     // id_base + i (-1: outside the cache, reads as zeros).
     int tok = t0 + warp * kTileTokens;
-    int blk = tok / bs, off = tok - blk * bs, id_base = 0, ids = -1;
-    auto load_ids = [&]() {
-        id_base = blk;
-        int64_t id = -1;
-        if (blk + lane < blocks) id = p.block_tables[b * p.max_blocks + blk + lane];
+    int blk = static_cast<int>(p.by_block.div(tok)), off = tok - blk * bs, ids;
+    auto take_ids = [&](IndexArray::Raw raw) {
+        const int64_t id = p.block_tables.value(raw);
         ids = (id >= 0 && id < p.num_cache_blocks) ? static_cast<int>(id) : -1;
     };
-    load_ids();
+    auto move_window = [&]() {
+        if (blk - id_base >= 32 && tok < t1) {
+            id_base = blk;
+            take_ids(load_ids(p, b, id_base, lane));
+        }
+    };
+    take_ids(raw_ids);
+    move_window();   // (a warp may begin just past what was loaded)
     uint32_t istage = ring;
     auto issue = [&]() {
         if (tok < t1) {
@@ -393,7 +412,7 @@ __device__ __forceinline__ void attend_range(const DecodeParams& p, int b, int k
             istage = istage == ring + (F::kStages - 1) * F::kStageBytes ? ring : istage + F::kStageBytes;
             tok += kGroupWarps * kTileTokens;
             for (off += kGroupWarps * kTileTokens; off >= bs; off -= bs) ++blk;
-            if (blk - id_base >= 32 && tok < t1) load_ids();
+            move_window();
         }
         cp_async_commit();
     };
@@ -414,46 +433,67 @@ __device__ __forceinline__ void attend_range(const DecodeParams& p, int b, int k
         left -= kGroupWarps * kTileTokens;
     }
     cp_async_wait<0>();
-    group_sync(bar_id, kGroupThreads);   // every ring is idle from here on
+    __syncwarp();                              // this warp's ring is idle from here on
     const int g = lane >> 2, t = lane & 3;
+    auto& part = sm.warps[warp].part;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         float l = st.s.l[h];
 #pragma unroll
         for (int x = 4; x < 32; x *= 2) l += __shfl_xor_sync(0xffffffffu, l, x);
-        if (g == 0) sm.m.ml[warp][2 * t + h] = make_float2(st.s.m[h], l);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) sm.m.o[warp][2 * t + h][F::dim(g, i)] = st.value(h, i);
+        if (2 * t + h < p.group) {
+            if (g == 0) part.ml[2 * t + h] = make_float2(st.s.m[h], l);
+            st.write_part(part.o + (4 * h + t) * F::kPartStride, h, g);
+        }
     }
     group_sync(bar_id, kGroupThreads);
-    for (int h = 0; h < p.group; ++h) {
-        float mx = -INFINITY, o = 0.0f, sum = 0.0f;
-#pragma unroll
-        for (int w = 0; w < kGroupWarps; ++w) mx = fmaxf(mx, sm.m.ml[w][h].x);
+    for (int h = warp; h < p.group; h += kGroupWarps) {
+        float4 o[kGroupWarps];
+        float2 ml[kGroupWarps];
 #pragma unroll
         for (int w = 0; w < kGroupWarps; ++w) {
-            const float f = fast_exp2(sm.m.ml[w][h].x - mx);   // 0 for a warp without a tile
-            o += f * sm.m.o[w][h][tid];
-            sum += f * sm.m.ml[w][h].y;
+            const auto& from = sm.warps[w].part;
+            ml[w] = from.ml[h];
+            o[w] = *reinterpret_cast<const float4*>(from.o + (4 * (h & 1) + (h >> 1)) * F::kPartStride + 4 * lane);
         }
-        sink(h, tid, o, mx, sum);
+        float mx = ml[0].x, sum = 0.0f;
+        float4 total = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int w = 1; w < kGroupWarps; ++w) mx = fmaxf(mx, ml[w].x);
+#pragma unroll
+        for (int w = 0; w < kGroupWarps; ++w) {
+            const float f = fast_exp2(ml[w].x - mx);   // 0 for a warp without a tile
+            total.x = fmaf(f, o[w].x, total.x); total.y = fmaf(f, o[w].y, total.y); total.z = fmaf(f, o[w].z, total.z); total.w = fmaf(f, o[w].w, total.w);
+            sum = fmaf(f, ml[w].y, sum);
+        }
+        sink(h, lane, total, mx, sum);
     }
 }
 
-__device__ __forceinline__ void write_part(float* po, float2* pml, int h, int d, float o, float m, float l) {   // [group][128], [group]
-    po[h * kHeadDim + d] = o;
-    if (d == 0) pml[h] = make_float2(m, l);
+template <typename T> __device__ __forceinline__ void write_quad(T* at, const float4& v) {   // four elements of a result
+    *reinterpret_cast<uint2*>(at) = make_uint2(ElemTraits<T>::pack2(v.x, v.y), ElemTraits<T>::pack2(v.z, v.w));
 }
+__device__ __forceinline__ float4 scaled(const float4& v, float f) { return make_float4(v.x * f, v.y * f, v.z * f, v.w * f); }
 
 // Range `split` of (b, kvh): the result if it is all of the context, else a part in the workspace.
 template <class F, typename T>
 __device__ __forceinline__ void run_split(const DecodeParams& p, int b, int kvh, int split, GroupSmem<F>& sm, int tid, int bar_id) {
-    const int ctx = clamped_context(p, b);
-    // A chunk past the context leaves before the divisions of split_range: with tables much wider than the contexts nearly all blocks are
-    // of this kind (128 sequences of 300 keys, 32768-key tables, 16384 blocks: 56.7 -> 50.8 us a call).
+    const int lane = tid & 31;
+    const IndexArray::Raw raw_ctx = p.context_lens.raw(b);
+    // The first range's block ids on their way with the context: a trip to memory less.  Further chunks look whether they have keys first: with tables
+    // much wider than the contexts nearly all blocks are of this kind (256 sequences of 100 to 300 keys, 8 KV heads, 32768-key tables, 32768
+    // blocks: 82 us a pass, 106 with ids for all), and they leave before anything else (128 such sequences: 56.7 -> 50.8 us a call).
+    const bool early = p.per_seq || split == 0;
+    int id_base = 0;
+    IndexArray::Raw raw_ids{0, 0};
+    if (early) raw_ids = load_ids(p, b, 0, lane);
+    const int ctx = clamped_context(p, raw_ctx);
     if (!p.per_seq && split > 0 && static_cast<int64_t>(split) * p.chunk_tokens >= ctx) return;
-    int t0, t1;
-    const int live = split_range(p, ctx, split, t0, t1);
+    const int len = range_len(p, ctx), t0 = split * len, t1 = min(ctx, t0 + len);
+    if (!early) {
+        id_base = static_cast<int>(p.by_block.div(t0));
+        raw_ids = load_ids(p, b, id_base, lane);
+    }
     T* out = static_cast<T*>(p.out) + (static_cast<int64_t>(b) * p.num_heads + kvh * p.group) * kHeadDim;
     if (t0 >= t1) {
         if (ctx == 0 && split == 0) {
@@ -462,9 +502,13 @@ __device__ __forceinline__ void run_split(const DecodeParams& p, int b, int kvh,
         return;
     }
     const size_t part = (static_cast<size_t>(b) * p.num_kv_heads + kvh) * p.num_splits + split;
-    attend_range<F>(p, b, kvh, t0, t1, sm, tid, bar_id, [&](int h, int d, float o, float m, float l) {
-        if (live == 1) out[h * kHeadDim + d] = ElemTraits<T>::from_float(o * (1.0f / l));   // (rounded as write_merged does)
-        else write_part(p.ws_o + part * p.group * kHeadDim, p.ws_ml + part * p.group, h, d, o, m, l);
+    attend_range<F>(p, b, kvh, t0, t1, raw_ids, id_base, sm, tid, bar_id, [&](int h, int quad, const float4& o, float m, float l) {
+        if (ctx <= len) {
+            write_quad(out + h * kHeadDim + 4 * quad, scaled(o, 1.0f / l));   // (rounded as write_merged does)
+        } else {
+            reinterpret_cast<float4*>(p.ws_o + (part * p.group + h) * kHeadDim)[quad] = o;
+            if (quad == 0) p.ws_ml[part * p.group + h] = make_float2(m, l);
+        }
     });
 }
 
@@ -475,20 +519,29 @@ struct PartRef { const float* o; const float2* ml; };   // head 0 of a part
 struct Merged {                                         // elements 4 lane .. 4 lane + 3 of a head's output, maximum and row sum
     float4 o;
     float m, l;
-    __device__ __forceinline__ void add(const float4& v, float vm, float vl) {
-        const float mx = fmaxf(m, vm), f = fast_exp2(m - mx), w = fast_exp2(vm - mx);
-        o.x = o.x * f + w * v.x; o.y = o.y * f + w * v.y; o.z = o.z * f + w * v.z; o.w = o.w * f + w * v.w;
-        l = l * f + w * vl;
+    // Four parts at a time (every merge in the same order, so that who merges makes no difference to a bit); one that is not there: zeros, with a
+    // maximum of minus infinity.
+    __device__ __forceinline__ void add(const float4 (&v)[4], const float2 (&ml)[4]) {
+        const float mx = fmaxf(m, fmaxf(fmaxf(ml[0].x, ml[1].x), fmaxf(ml[2].x, ml[3].x))), f = fast_exp2(m - mx);
+        o = scaled(o, f);
+        l *= f;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const float w = fast_exp2(ml[u].x - mx);
+            o.x = fmaf(w, v[u].x, o.x); o.y = fmaf(w, v[u].y, o.y); o.z = fmaf(w, v[u].z, o.z); o.w = fmaf(w, v[u].w, o.w);
+            l = fmaf(w, ml[u].y, l);
+        }
         m = mx;
     }
 };
+__device__ __forceinline__ Merged nothing_merged() { return Merged{make_float4(0.f, 0.f, 0.f, 0.f), -INFINITY, 0.0f}; }
 
 // Heads h0 .. h0 + HG - 1 (clamped to the group) over parts first, first + stride, ...
 template <int HG, class Get>
 __device__ __forceinline__ void sum_parts(Get get, int n, int first, int stride, int h0, int group, int lane, Merged (&acc)[HG]) {
     constexpr int U = HG == 4 ? 4 : 8;   // parts in flight
 #pragma unroll
-    for (int h = 0; h < HG; ++h) acc[h] = Merged{make_float4(0.f, 0.f, 0.f, 0.f), -INFINITY, 0.0f};
+    for (int h = 0; h < HG; ++h) acc[h] = nothing_merged();
     for (int i0 = first; i0 < n; i0 += U * stride) {
         float2 ml[U][HG];
         float4 v[U][HG];
@@ -503,10 +556,20 @@ __device__ __forceinline__ void sum_parts(Get get, int n, int first, int stride,
             }
         }
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
+        for (int u = 0; u < U; u += 4) {
             if (i0 + u * stride < n) {
 #pragma unroll
-                for (int h = 0; h < HG; ++h) acc[h].add(v[u][h], ml[u][h].x, ml[u][h].y);
+                for (int h = 0; h < HG; ++h) {
+                    float4 four[4];
+                    float2 ml4[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const bool there = i0 + (u + k) * stride < n;
+                        four[k] = there ? v[u + k][h] : make_float4(0.f, 0.f, 0.f, 0.f);
+                        ml4[k] = there ? ml[u + k][h] : make_float2(-INFINITY, 0.0f);
+                    }
+                    acc[h].add(four, ml4);
+                }
             }
         }
     }
@@ -514,18 +577,16 @@ __device__ __forceinline__ void sum_parts(Get get, int n, int first, int stride,
 template <typename T>
 __device__ __forceinline__ void write_merged(T* row, const Merged& a, int lane) {
     const float inv = a.l > 0.0f ? 1.0f / a.l : 0.0f;
-    reinterpret_cast<uint2*>(row)[lane] = make_uint2(ElemTraits<T>::pack2(a.o.x * inv, a.o.y * inv), ElemTraits<T>::pack2(a.o.z * inv, a.o.w * inv));
+    write_quad(row + 4 * lane, scaled(a.o, inv));
 }
-// All heads of the group, rows of `out`, by one warp.
+// Heads h0 .. h0 + HG - 1 of the group, rows of `out`, by one warp.
 template <typename T, int HG, class Get>
-__device__ __forceinline__ void merge_by_warp(Get get, int n, int group, T* out, int lane) {
-    for (int h0 = 0; h0 < group; h0 += HG) {
-        Merged acc[HG];
-        sum_parts<HG>(get, n, 0, 1, h0, group, lane, acc);
+__device__ __forceinline__ void merge_by_warp(Get get, int n, int h0, int group, T* out, int lane) {
+    Merged acc[HG];
+    sum_parts<HG>(get, n, 0, 1, h0, group, lane, acc);
 #pragma unroll
-        for (int h = 0; h < HG; ++h)
-            if (h0 + h < group) write_merged<T>(out + (h0 + h) * kHeadDim, acc[h], lane);
-    }
+    for (int h = 0; h < HG; ++h)
+        if (h0 + h < group) write_merged<T>(out + (h0 + h) * kHeadDim, acc[h], lane);
 }
 // One head, by the whole block; the first kMergeWarps warps work.
 struct MergeScratch { float4 o[kMergeWarps][32]; float2 ml[kMergeWarps]; };
@@ -539,9 +600,10 @@ __device__ __forceinline__ void merge_by_block(Get get, int n, int head, int gro
     }
     __syncthreads();
     if (warp == 0) {
-        Merged a{make_float4(0.f, 0.f, 0.f, 0.f), -INFINITY, 0.0f};
+        Merged a = nothing_merged();
 #pragma unroll
-        for (int w = 0; w < kMergeWarps; ++w) a.add(sm.o[w][lane], sm.ml[w].x, sm.ml[w].y);
+        for (int w = 0; w < kMergeWarps; w += 4)
+            a.add({sm.o[w][lane], sm.o[w + 1][lane], sm.o[w + 2][lane], sm.o[w + 3][lane]}, {sm.ml[w], sm.ml[w + 1], sm.ml[w + 2], sm.ml[w + 3]});
         write_merged<T>(row, a, lane);
     }
     __syncthreads();

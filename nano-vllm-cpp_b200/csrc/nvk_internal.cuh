@@ -62,7 +62,38 @@ struct IndexArray {
             : "=l"(v) : "l"(static_cast<const char*>(ptr) + (i << (2 + wide))), "r"(wide));
         return v;
     }
+    // An index as loaded, both words; value() widens it later, so that other loads can be issued before this one has come back (operator[] waits
+    // for it to extend its sign).
+    struct Raw { int lo, hi; };
+    __device__ __forceinline__ Raw raw(int64_t i, bool there = true) const {   // (0 without a load where there is none)
+        Raw r;
+        asm volatile(
+            "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 q, %4, 0;\n\tsetp.ne.and.s32 p, %3, 0, q;\n\tmov.s32 %0, 0;\n\tmov.s32 %1, 0;\n\t"
+            "@q ld.global.s32 %0, [%2];\n\t@p ld.global.s32 %1, [%2+4];\n\t}\n"
+            : "=r"(r.lo), "=r"(r.hi) : "l"(static_cast<const char*>(ptr) + (i << (2 + wide))), "r"(wide), "r"(static_cast<int>(there)));
+        return r;
+    }
+    __device__ __forceinline__ int64_t value(Raw r) const {
+        const int hi = wide ? r.hi : r.lo >> 31;
+        return static_cast<int64_t>((static_cast<uint64_t>(static_cast<uint32_t>(hi)) << 32) | static_cast<uint32_t>(r.lo));
+    }
 #endif
+};
+
+// Division of 0 <= n < 2^31 by a launch-uniform number: a multiplication and a shift instead of some 25 instructions in a chain.
+struct FastDiv {
+    uint32_t d = 1, mul = 1, shift = 0;
+    FastDiv() = default;
+    explicit FastDiv(uint32_t by) : d(by) {   // 1 <= by < 2^31
+        while ((1ull << shift) < by) ++shift;
+        mul = static_cast<uint32_t>(((1ull << 32) * ((1ull << shift) - by)) / by + 1);
+    }
+#ifdef __CUDACC__
+    __host__ __device__
+#endif
+    uint32_t div(uint32_t n) const {   // (mul * n / 2^32 <= n, so that the sum stays below 2^32)
+        return (static_cast<uint32_t>((static_cast<uint64_t>(n) * mul) >> 32) + n) >> shift;
+    }
 };
 
 constexpr int kSmCount = 148;   // of a B200; grids are sized by it

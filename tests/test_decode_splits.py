@@ -72,3 +72,33 @@ def test_8_bit_caches_do_not_depend_on_how_a_context_is_shared_out(fmt, hq, hkv,
     ref = oracle.decode_attention_paged(w["q"], w["k_cache"], w["v_cache"], w["context_lens"], w["block_tables"], hkv, 128, 256, w["scale"])
     assert float((a.float() - b.float()).abs().max()) <= 1e-2
     assert np.abs(to_np(a) - ref).max() <= (5e-2 if fmt == "int8" else 2.5e-1) and not torch.isnan(b.float()).any()
+
+
+@pytest.mark.parametrize("hq,hkv,bs,lens,table_blocks", [
+    (24, 3, 48, EDGES[:7] + [700], 15),                     # clusters of four, eight heads a group, blocks and heads that are no power of two
+    (3, 3, 48, [300, 47, 48, 49], 7),                       # of eight, one head a group
+    (7, 7, 16, [1024, 513, 16], 64),                        # of four, more table entries than lanes
+    (40, 5, 80, (EDGES * 4)[:45] + [2500, 3999], 50),       # chunks: groups of eight by warps of four heads
+    (16, 8, 256, [9000, 300, 5000] + [40] * 34, 36),        # more than four parts: a warp per head
+    (32, 4, 256, [4000, 2049] + [40] * 127, 33),            # the same as far as it goes (4128 rows: four heads a warp)
+])
+def test_parts_come_together_without_what_is_not_there(hq, hkv, bs, lens, table_blocks):
+    """Every merge form; an infinity in V stays in its column: parts that do not exist add nothing, not even zero times infinity."""
+    w = workloads().make_decode_workload(len(lens), hq, hkv, 128, bs, 0, 0, seed=len(lens) + hq, context_lens=np.array(lens, np.int32),
+                                         pad_blocks_to=table_blocks)
+    bf = torch.bfloat16
+    q, kc, vc, ctx, bt = to_dev(w["q"], bf), to_dev(w["k_cache"], bf), to_dev(w["v_cache"], bf), to_dev(w["context_lens"]), to_dev(w["block_tables"])
+    ref = oracle.decode_attention_paged(w["q"], w["k_cache"], w["v_cache"], w["context_lens"], w["block_tables"], hkv, 128, bs, w["scale"])
+    for ws in (_workspace(len(lens), hq, hkv, bt.shape[1], bs), None):
+        out = torch.full_like(q, float("nan"))
+        nvk().launch_decode_attention_paged(q, kc, vc, ctx, bt, hkv, 128, bs, w["scale"], out, ws)
+        assert_attention_close(to_np(out), ref)
+    last = [int(w["block_tables"][i, (n - 1) // bs]) * bs + (n - 1) % bs for i, n in enumerate(lens) if n]
+    vc.view(-1, hkv, 128)[torch.tensor(last, device="cuda"), :, 5] = float("inf")
+    live = torch.tensor(lens, device="cuda") > 0
+    for ws in (_workspace(len(lens), hq, hkv, bt.shape[1], bs), None):
+        out = torch.full_like(q, float("nan"))
+        nvk().launch_decode_attention_paged(q, kc, vc, ctx, bt, hkv, 128, bs, w["scale"], out, ws)
+        assert bool((out[live][..., 5] == float("inf")).all())
+        rest = torch.cat([out[..., :5], out[..., 6:]], -1)
+        assert_attention_close(to_np(rest), np.concatenate([ref[..., :5], ref[..., 6:]], -1))
