@@ -89,6 +89,25 @@ def test_store_kvcache_large_copies_bit_exact(dtype, row_elems, slot_dtype, n):
     assert np.array_equal(v_cache.cpu().view(torch.uint8).numpy(), vc_ref)
 
 
+@pytest.mark.parametrize("row_elems,n", [(3, 202069), (3, 202070), (1, 1), (1000, 4849), (1000, 4850)])
+@pytest.mark.parametrize("slot_dtype", [torch.int32, torch.int64])
+def test_store_kvcache_around_one_trip_per_thread(row_elems, n, slot_dtype):
+    """2 x n x 3 two-byte vectors and 2 x n x 125 sixteen-byte ones on both sides of 1184 blocks x 1024: two kernels, the same bytes."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    key, value = (torch.randn(n, row_elems, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    rows = n + 77
+    slots = torch.randperm(rows, device="cuda", generator=g)[:n]
+    slots[:: 5] = -1
+    slots[1:: 7] = rows + 3
+    kc, vc = (torch.randn(rows, row_elems, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    want_k, want_v = kc.clone(), vc.clone()
+    live = (slots >= 0) & (slots < rows)
+    want_k[slots[live]], want_v[slots[live]] = key[live], value[live]
+    nvk().store_kvcache(key.view(n, 1, row_elems), value.view(n, 1, row_elems), kc.view(1, rows, 1, row_elems), vc.view(1, rows, 1, row_elems), slots.to(slot_dtype))
+    assert torch.equal(kc, want_k) and torch.equal(vc, want_v)
+
+
 def test_store_kvcache_misaligned_views_and_duplicate_slots():
     rng = np.random.default_rng(5)
     n, row, cache_rows = 64, 24, 128
