@@ -3,38 +3,36 @@
 //
 // Replaces the same reference kernel as decode_attn.cu (src/kernels/attention.cu:313-405).  The op reads each K / V row once
 // and does 4 * G flops per element, so HBM bounds it; what has to be organised is enough bytes in flight from a batch of a
-// few sequences:
-//   * one thread-block cluster per (sequence, KV head, chunk of up to four query heads): cluster size 1, 2, 4 or 8, as large
-//     as keeps the grid within two blocks per SM, so 8 sequences x 8 KV heads already occupy every SM;
-//   * trips of 8 keys (D 128) are dealt round-robin to the cluster's warps; a key is spread over D / 16 lanes, 16 elements
-//     each, so a warp reads whole 128-byte lines and a dot product needs log2(D / 16) shuffles for 32 / (D / 16) keys at
-//     once; a warp's K and V loads of a trip (8 KiB in fp32) are all in flight together, and the rows of the next trip are
-//     looked up in the block table under the current one;
-//   * every lane group keeps its own running maximum and sum per query head; groups merge by shuffles, warps through shared
-//     memory, blocks through distributed shared memory -- one launch, no workspace.
+// few sequences, and little before the first and after the last of them:
+//   * one thread-block cluster per (sequence, KV head, chunk of up to four query heads), blocks of four warps, four (three) to an SM: cluster
+//     size 1, 2, 4 or 8, as large as keeps all blocks resident, so 8 sequences x 8 KV heads already occupy every SM;
+//   * steps of 32 / (D / 16) keys (4 at D 128) are dealt round-robin to the cluster's warps; a key is spread over D / 16 lanes, 16 elements
+//     each, so a warp reads whole 128-byte lines and a dot product needs log2(D / 16) shuffles.  K and V come through a ring in shared
+//     memory by cp.async, 12 KiB a warp: a lane copies what it will read itself, so a step waits for nothing but its own copies;
+//   * every lane group keeps its own running maximum and sum per query head; the groups of a block come together through shared
+//     memory, their sum is pushed to the block of the cluster that finishes those elements, and after one cluster barrier everything is
+//     local -- one launch, no workspace.  The merges run once, and code that runs once is as slow as it is long: with every part unrolled
+//     they took 3 us of a block's 8, now 1.6.
 // Batch 8, 16 / 8 heads, fp32, context 64 .. 1024, store + decode: 2031 us a pass with one warp per (sequence, head) walking its
-// keys in order, 15.7 us here (15.4 to 15.9 over boxes; 16.65 with branches around index and row loads and merges written out part by part), of which up to four trips of load, dot product, exponentials and sum follow one another in a warp.
+// keys in order, 14.7 us with rows in registers (trips of 8 keys in a warp that never overlapped, up to 7.7 us of them, and 3.3 us of merges
+// by shuffles and by fetching peers' parts), 12.5 us here; 1 sequence of 100 keys 7.8 -> 4.7, 7 of 64 to 200 (8 / 4 heads) 9.6 -> 6.0, 8 of 4000 to 4096
+// (32 / 8 heads) 71 -> 64.  Sequences in order of falling context so that long and short blocks share an SM: 13.3 -> 13.7 in an earlier form.
 #include "nvk_internal.cuh"
 
-#include <cooperative_groups.h>
-
+#include <atomic>
 #include <cmath>
 
 namespace nvk {
 namespace {
 
-namespace cg = cooperative_groups;
-
-constexpr int kWarps = 8;
-constexpr int kThreads = kWarps * 32;
-constexpr int kUnroll = 2;       // keys per lane group and trip
 constexpr int kMaxCluster = 8;   // portable cluster size
 
 struct SimtParams {
     const void* q; const void* k; const void* v; void* out;
     IndexArray context_lens, block_tables;
-    int64_t max_blocks, cache_rows;
-    int num_heads, num_kv_heads, group, chunks, block_size;
+    int64_t max_blocks, num_cache_blocks;
+    int batch, num_heads, num_kv_heads, group, chunks, block_size, csize_shift;
+    FastDiv by_block, by_chunks, by_kv_heads;
     float scale;
 };
 
@@ -56,64 +54,113 @@ template <> __device__ __forceinline__ void unpack<__half>(const uint4& w, float
     }
 }
 
-// K / V rows are read once; zeros, and no read, where there is no row (by a predicate: branches around the loads of each key doubled the loop's code).
-__device__ __forceinline__ uint4 ld_stream16(const void* p, bool there) {
+__device__ __forceinline__ uint4 lds16(uint32_t addr) {   // (volatile: stays on its side of the copies that refill the place)
     uint4 v;
-    asm volatile(
-        "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
-        "@q ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}\n"
-        : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "r"(static_cast<int>(there)));
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
     return v;
 }
-
-// A float of this block's shared memory, as block `rank` of the cluster has it.
-__device__ __forceinline__ float ld_block(const float* p, uint32_t rank) {
-    float v;
-    asm volatile(
-        "{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.f32 %0, [a];\n\t}\n"
-        : "=f"(v) : "r"(smem_u32(p)), "r"(rank) : "memory");
-    return v;
+__device__ __forceinline__ uint32_t in_block(const void* p, uint32_t rank) {   // the same place in block `rank` of the cluster
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
+    return r;
 }
 
 // HG: query heads of a chunk (rounded up to 1, 2 or 4; rows past the group are computed on zeros and not written).
-template <typename T, int D, int HG>
-__global__ void __launch_bounds__(kThreads, HG <= 2 ? 2 : 1) decode_simt_kernel(const SimtParams p) {
+// W: warps of a block; 4, of which four (three) fit on an SM, or 8 of 24 KiB each where there are few blocks, one per SM.
+template <int W> constexpr int kWarpRing = W == 4 ? 12 * 1024 : 24 * 1024;
+template <typename T, int D, int HG, int W>
+__global__ void __launch_bounds__(W * 32, W == 8 ? 1 : HG <= 2 ? 4 : 3) decode_simt_kernel(const __grid_constant__ SimtParams p) {
+    constexpr int kWarps = W, kThreads = W * 32, RING = kWarpRing<W>;
     constexpr int LANES = D / 16;                         // lanes per key
-    constexpr int GROUPS = 32 / LANES;                    // keys a warp scores at once
+    constexpr int GROUPS = 32 / LANES;                    // keys of a step
     constexpr int VE = 16 / static_cast<int>(sizeof(T));  // elements per 16-byte vector
     constexpr int NV = 16 / VE;                           // vectors per lane and key
-    constexpr int TRIP = GROUPS * kUnroll;
-    __shared__ __align__(16) float s_q[HG][D];
-    __shared__ float s_o[kWarps][HG][D];
-    __shared__ float s_m[kWarps][HG], s_l[kWarps][HG];
-    __shared__ float s_po[HG][D];                         // this block's merged partial result, read by the whole cluster
-    __shared__ float s_pm[HG], s_pl[HG];
+    constexpr int STAGE = 2 * NV * 512;                   // K and V of a step: NV x 16 bytes of each per lane
+    constexpr int STAGES = RING / STAGE;
+    constexpr int QUADS = HG * D / 4;                     // of the result
+    constexpr int TPQ = kThreads / QUADS < 1 ? 1 : kThreads / QUADS < kWarps ? kThreads / QUADS : kWarps;   // threads of a quad in a block's merge
+    static_assert(GROUPS * HG * D * 4 <= RING, "a warp's parts take its ring's place");
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ __align__(16) float s_q[HG * D];
+    __shared__ float2 s_part[HG][kWarps];                 // (maximum, sum) of every warp
+    __shared__ float4 s_o[QUADS];                         // [block of the cluster][quad that this block finishes]
+    __shared__ float2 s_ml[kMaxCluster][HG];
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");   // (waited for before the first remote store: every block has started)
     pdl_wait_then_release();
-    cg::cluster_group cluster = cg::this_cluster();
-    const int csize = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
+    const int csize = 1 << p.csize_shift, rank = static_cast<int>(blockIdx.x) & (csize - 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int sub = lane % LANES, grp = lane / LANES;
-    const int64_t item = blockIdx.x / csize;
-    const int chunk = static_cast<int>(item % p.chunks);
-    const int kvh = static_cast<int>((item / p.chunks) % p.num_kv_heads);
-    const int64_t b = item / (static_cast<int64_t>(p.chunks) * p.num_kv_heads);
-    const int head0 = kvh * p.group + chunk * HG;
-    const int heads = min(HG, p.group - chunk * HG);
+    const uint32_t item = blockIdx.x >> p.csize_shift;
+    const uint32_t pair = p.by_chunks.div(item);
+    const int chunk = static_cast<int>(item - pair * p.chunks);
+    const int b = static_cast<int>(p.by_kv_heads.div(pair));
+    const int kvh = static_cast<int>(pair) - b * p.num_kv_heads;
     const int64_t cap = p.max_blocks * p.block_size;
-    int64_t ctx = p.context_lens.load(b);
-    if (ctx > cap) ctx = cap;
-    if (ctx < 0) ctx = 0;
-
-    for (int i = tid; i < HG * D; i += kThreads) {
-        const int h = i / D, d = i % D;
-        s_q[h][d] = h < heads ? ElemTraits<T>::to_float(static_cast<const T*>(p.q)[(b * p.num_heads + head0 + h) * D + d]) * p.scale : 0.0f;
-    }
-    __syncthreads();
-
-    const int64_t row_elems = static_cast<int64_t>(p.num_kv_heads) * D;
-    const T* kc = static_cast<const T*>(p.k) + static_cast<int64_t>(kvh) * D + sub * VE;
-    const T* vc = static_cast<const T*>(p.v) + static_cast<int64_t>(kvh) * D + sub * VE;
+    auto clamped = [&](IndexArray::Raw raw) {
+        const int64_t n = p.context_lens.value(raw);
+        return static_cast<int>(n < 0 ? 0 : n < cap ? n : cap);
+    };
+    const int head0 = kvh * p.group + chunk * HG, heads = min(HG, p.group - chunk * HG);
     const IndexArray table = p.block_tables + b * p.max_blocks;
+    const IndexArray::Raw raw_ctx = p.context_lens.raw(b);
+    IndexArray::Raw raw_ids = table.raw(lane, lane < p.max_blocks);
+    float q_in[(HG * D + kThreads - 1) / kThreads];
+#pragma unroll
+    for (int i = 0; i < (HG * D + kThreads - 1) / kThreads; ++i) {
+        const int at = i * kThreads + tid;
+        q_in[i] = at < heads * D ? ElemTraits<T>::to_float(static_cast<const T*>(p.q)[(static_cast<int64_t>(b) * p.num_heads + head0) * D + at]) * p.scale : 0.0f;
+    }
+    const int ctx = clamped(raw_ctx);
+
+    // The copying end: this warp's next step begins at key `tok`.  Lane i holds the cache block of table entry id_base + i (-1: outside the cache, reads
+    // as zeros).
+    const uint32_t ring = smem_u32(smem) + warp * RING + lane * 16;
+    const size_t row_bytes = static_cast<size_t>(p.num_kv_heads) * D * sizeof(T);
+    const size_t lane_at = (static_cast<size_t>(kvh) * D + sub * VE) * sizeof(T);
+    const int first = (rank * kWarps + warp) * GROUPS, stride = kWarps * GROUPS << p.csize_shift;
+    int tok = first, id_base = 0, ids;
+    auto take_ids = [&](IndexArray::Raw raw) {
+        const int64_t id = table.value(raw);
+        ids = id >= 0 && id < p.num_cache_blocks ? static_cast<int>(id) : -1;
+    };
+    take_ids(raw_ids);
+    uint32_t fill = ring;
+    auto issue = [&]() {
+        if (tok < ctx) {
+            const int key = min(tok + grp, ctx - 1), blk = static_cast<int>(p.by_block.div(key));
+            if (static_cast<int>(p.by_block.div(min(tok + GROUPS - 1, ctx - 1))) - id_base >= 32) {   // (warp-uniform; a step's keys lie in fewer blocks)
+                id_base = static_cast<int>(p.by_block.div(tok));
+                take_ids(table.raw(id_base + lane, id_base + lane < p.max_blocks));
+            }
+            const int id = __shfl_sync(0xffffffffu, ids, blk - id_base);
+            const bool there = id >= 0 && tok + grp < ctx;
+            const size_t at = there ? (static_cast<size_t>(id) * p.block_size + (key - blk * p.block_size)) * row_bytes + lane_at : 0;
+#pragma unroll
+            for (int i = 0; i < NV; ++i) {
+                cp_async16(fill + i * 512, static_cast<const char*>(p.k) + at + i * LANES * 16, there ? 16 : 0);
+                cp_async16(fill + (NV + i) * 512, static_cast<const char*>(p.v) + at + i * LANES * 16, there ? 16 : 0);
+            }
+            fill = fill == ring + (STAGES - 1) * STAGE ? ring : fill + STAGE;
+            tok += stride;
+        }
+        cp_async_commit();
+    };
+#pragma unroll 1   // (code that runs once is as slow as it is long)
+    for (int s = 0; s < STAGES - 1; ++s) issue();
+#pragma unroll
+    for (int i = 0; i < (HG * D + kThreads - 1) / kThreads; ++i)
+        if (i * kThreads + tid < HG * D) s_q[i * kThreads + tid] = q_in[i];
+    __syncthreads();
+    constexpr bool kQInRegs = HG <= 2;
+    float qr[kQInRegs ? HG : 1][16];
+    if (kQInRegs) {
+#pragma unroll
+        for (int h = 0; h < HG; ++h) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) qr[h][e] = s_q[h * D + ((e / VE) * LANES + sub) * VE + e % VE];
+        }
+    }
+
     float m[HG], l[HG], acc[HG][16];
 #pragma unroll
     for (int h = 0; h < HG; ++h) {
@@ -121,212 +168,205 @@ __global__ void __launch_bounds__(kThreads, HG <= 2 ? 2 : 1) decode_simt_kernel(
 #pragma unroll
         for (int e = 0; e < 16; ++e) acc[h][e] = 0.0f;
     }
-
-    // cache row of key k, -1 where the block id lies outside the cache (reads as zeros), -2 past the context
-    auto row_of = [&](int64_t k) -> int64_t {
-        if (k >= ctx) return -2;
-        const int ki = static_cast<int>(k);
-        const int blk = ki / p.block_size;
-        const int64_t r = table.load(blk) * p.block_size + (ki - blk * p.block_size);
-        return r >= 0 && r < p.cache_rows ? r : -1;
-    };
-    const int64_t step = static_cast<int64_t>(csize) * kWarps * TRIP;
-    int64_t row[kUnroll];
-    const int64_t first = (static_cast<int64_t>(rank) * kWarps + warp) * TRIP;
+    uint32_t use = ring;
+#pragma unroll 1
+    for (int k0 = first; k0 < ctx; k0 += stride) {
+        issue();
+        cp_async_wait<STAGES - 1>();
+        const bool live = k0 + grp < ctx;
+        float s[HG][4], f[16];
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) row[u] = row_of(first + u * GROUPS + grp);
-    for (int64_t k0 = first; k0 < ctx; k0 += step) {
-        uint4 kv[kUnroll][NV], vv[kUnroll][NV];
-        bool live[kUnroll];
-#pragma unroll
-        for (int u = 0; u < kUnroll; ++u) {
-            live[u] = row[u] != -2;
-#pragma unroll
-            for (int i = 0; i < NV; ++i) {
-                kv[u][i] = ld_stream16(kc + row[u] * row_elems + i * LANES * VE, row[u] >= 0);
-                vv[u][i] = ld_stream16(vc + row[u] * row_elems + i * LANES * VE, row[u] >= 0);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < kUnroll; ++u) row[u] = row_of(k0 + step + u * GROUPS + grp);
-        float s[HG][kUnroll];
+        for (int i = 0; i < NV; ++i) unpack<T>(lds16(use + i * 512), f + i * VE);
 #pragma unroll
         for (int h = 0; h < HG; ++h) {
 #pragma unroll
-            for (int u = 0; u < kUnroll; ++u) s[h][u] = 0.0f;
-        }
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            float kf[kUnroll][VE];
-#pragma unroll
-            for (int u = 0; u < kUnroll; ++u) unpack<T>(kv[u][i], kf[u]);
-#pragma unroll
-            for (int h = 0; h < HG; ++h) {
-#pragma unroll
-                for (int e = 0; e < VE; e += 4) {
-                    const float4 qf = *reinterpret_cast<const float4*>(&s_q[h][(i * LANES + sub) * VE + e]);
-#pragma unroll
-                    for (int u = 0; u < kUnroll; ++u)
-                        s[h][u] = fmaf(qf.w, kf[u][e + 3], fmaf(qf.z, kf[u][e + 2], fmaf(qf.y, kf[u][e + 1], fmaf(qf.x, kf[u][e], s[h][u]))));
-                }
+            for (int e = 0; e < 16; e += 4) {
+                float4 qf;
+                if (kQInRegs) qf = make_float4(qr[h][e], qr[h][e + 1], qr[h][e + 2], qr[h][e + 3]);
+                else qf = *reinterpret_cast<const float4*>(&s_q[h * D + ((e / VE) * LANES + sub) * VE + e % VE]);
+                s[h][0] = e == 0 ? qf.x * f[e] : fmaf(qf.x, f[e], s[h][0]);
+                s[h][1] = e == 0 ? qf.y * f[e + 1] : fmaf(qf.y, f[e + 1], s[h][1]);
+                s[h][2] = e == 0 ? qf.z * f[e + 2] : fmaf(qf.z, f[e + 2], s[h][2]);
+                s[h][3] = e == 0 ? qf.w * f[e + 3] : fmaf(qf.w, f[e + 3], s[h][3]);
             }
+            s[h][0] = (s[h][0] + s[h][1]) + (s[h][2] + s[h][3]);
         }
 #pragma unroll
         for (int o = LANES / 2; o > 0; o >>= 1) {
 #pragma unroll
-            for (int h = 0; h < HG; ++h) {
-#pragma unroll
-                for (int u = 0; u < kUnroll; ++u) s[h][u] += __shfl_xor_sync(0xffffffffu, s[h][u], o);
-            }
+            for (int h = 0; h < HG; ++h) s[h][0] += __shfl_xor_sync(0xffffffffu, s[h][0], o);
         }
 #pragma unroll
-        for (int h = 0; h < HG; ++h) {
-            float m_new = m[h];
+        for (int i = 0; i < NV; ++i) unpack<T>(lds16(use + (NV + i) * 512), f + i * VE);
 #pragma unroll
-            for (int u = 0; u < kUnroll; ++u) if (live[u]) m_new = fmaxf(m_new, s[h][u]);
-            if (m_new > m[h]) {   // (same for all lanes of a group)
-                const float corr = expf(m[h] - m_new);
+        for (int h = 0; h < HG; ++h) {
+            if (live && s[h][0] > m[h]) {   // (same for all lanes of a group)
+                const float corr = expf(m[h] - s[h][0]);
                 l[h] *= corr;
 #pragma unroll
                 for (int e = 0; e < 16; ++e) acc[h][e] *= corr;
-                m[h] = m_new;
+                m[h] = s[h][0];
             }
+            const float w = !live || s[h][0] == -INFINITY ? 0.0f : expf(s[h][0] - m[h]);
+            l[h] += w;
 #pragma unroll
-            for (int u = 0; u < kUnroll; ++u) {
-                s[h][u] = live[u] ? expf(s[h][u] - m[h]) : 0.0f;
-                l[h] += s[h][u];
-            }
+            for (int e = 0; e < 16; ++e) acc[h][e] = fmaf(w, f[e], acc[h][e]);
         }
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-#pragma unroll
-            for (int u = 0; u < kUnroll; ++u) {
-                float vf[VE];
-                unpack<T>(vv[u][i], vf);
-#pragma unroll
-                for (int h = 0; h < HG; ++h) {
-#pragma unroll
-                    for (int e = 0; e < VE; ++e) acc[h][i * VE + e] = fmaf(s[h][u], vf[e], acc[h][i * VE + e]);
-                }
-            }
-        }
+        use = use == ring + (STAGES - 1) * STAGE ? ring : use + STAGE;
     }
 
-    // lane groups -> warp
+    // lane groups -> block: under the warp's maximum every group leaves its part over its warp's ring, TPQ threads add up a quad of the result
+    cp_async_wait<0>();
+    __syncwarp();
+    float* part = reinterpret_cast<float*>(smem + warp * RING) + grp * HG * D;
 #pragma unroll
     for (int h = 0; h < HG; ++h) {
         float mx = m[h];
 #pragma unroll
         for (int o = LANES; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         const float f = m[h] == -INFINITY ? 0.0f : expf(m[h] - mx);
-        m[h] = mx;
-        l[h] *= f;
+        float sum = l[h] * f;
 #pragma unroll
-        for (int e = 0; e < 16; ++e) acc[h][e] *= f;
+        for (int o = LANES; o < 32; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
 #pragma unroll
-        for (int o = LANES; o < 32; o <<= 1) {
-            l[h] += __shfl_xor_sync(0xffffffffu, l[h], o);
-#pragma unroll
-            for (int e = 0; e < 16; ++e) acc[h][e] += __shfl_xor_sync(0xffffffffu, acc[h][e], o);
-        }
-        if (grp == 0) {
-#pragma unroll
-            for (int e = 0; e < 16; ++e) s_o[warp][h][((e / VE) * LANES + sub) * VE + e % VE] = acc[h][e];
-            if (sub == 0) { s_m[warp][h] = m[h]; s_l[warp][h] = l[h]; }
-        }
+        for (int e = 0; e < 16; e += 4)
+            *reinterpret_cast<float4*>(part + h * D + ((e / VE) * LANES + sub) * VE + e % VE) =
+                make_float4(acc[h][e] * f, acc[h][e + 1] * f, acc[h][e + 2] * f, acc[h][e + 3] * f);
+        if (lane == 0) s_part[h][warp] = make_float2(mx, sum);
     }
     __syncthreads();
-    // warps -> block
-    for (int i = tid; i < HG * D; i += kThreads) {
-        const int h = i / D, d = i % D;
-        float mx = -INFINITY, lsum = 0.0f, o = 0.0f;
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) mx = fmaxf(mx, s_m[w][h]);
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
-            const float f = s_m[w][h] == -INFINITY ? 0.0f : expf(s_m[w][h] - mx);
-            lsum += f * s_l[w][h];
-            o += f * s_o[w][h][d];
-        }
-        s_po[h][d] = o;
-        if (d == 0) { s_pm[h] = mx; s_pl[h] = lsum; }
-    }
-    // blocks -> result: every block of the cluster takes its share of the elements
-    cluster.sync();
-    T* out = static_cast<T*>(p.out) + (b * p.num_heads + head0) * D;
-    for (int i = rank * kThreads + tid; i < heads * D; i += csize * kThreads) {
-        const int h = i / D, d = i % D;
-        float mx = -INFINITY, lsum = 0.0f, o = 0.0f;
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    const int quads = QUADS >> p.csize_shift;             // that a block finishes
+    const int split = lane / (32 / TPQ);
 #pragma unroll 1
-        for (int r0 = 0; r0 < csize; r0 += 4) {   // (four blocks' loads under way at once)
-            float pm[4], pl[4], po[4];
+    for (int e = warp * (32 / TPQ) + lane % (32 / TPQ); e < QUADS; e += kThreads / TPQ) {   // (whole warps)
+        const int h = e / (D / 4);
+        float mx = s_part[h][0].x, sum = 0.0f;
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const uint32_t from = static_cast<uint32_t>(min(r0 + u, csize - 1));
-                pm[u] = ld_block(&s_pm[h], from);
-                pl[u] = ld_block(&s_pl[h], from);
-                po[u] = ld_block(&s_po[h][d], from);
-                // (no weight of 0 takes out what a block that is not there would add: the last block's part, read in its place, may be infinite)
-                if (r0 + u >= csize) { pm[u] = -INFINITY; pl[u] = po[u] = 0.0f; }
-            }
-            const float m_new = fmaxf(fmaxf(fmaxf(pm[0], pm[1]), fmaxf(pm[2], pm[3])), mx);
-            const float f = mx == -INFINITY ? 0.0f : expf(mx - m_new);
-            lsum *= f;
-            o *= f;
-            mx = m_new;
+        for (int w = 1; w < kWarps; ++w) mx = fmaxf(mx, s_part[h][w].x);
+        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const float w = pm[u] == -INFINITY ? 0.0f : expf(pm[u] - mx);
-                lsum += w * pl[u];
-                o += w * po[u];
+        for (int i = 0; i < kWarps / TPQ; ++i) {
+            const int w = i * TPQ + split;
+            const float2 ml = s_part[h][w];
+            const float f = ml.x == -INFINITY ? 0.0f : expf(ml.x - mx);
+            const float4* from = reinterpret_cast<const float4*>(smem + w * RING) + e;
+            float4 v = from[0];
+#pragma unroll
+            for (int g = 1; g < GROUPS; ++g) {
+                const float4 u = from[g * QUADS];
+                v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
             }
+            t.x = fmaf(f, v.x, t.x); t.y = fmaf(f, v.y, t.y); t.z = fmaf(f, v.z, t.z); t.w = fmaf(f, v.w, t.w);
+            sum = fmaf(f, ml.y, sum);
         }
-        out[i] = ElemTraits<T>::from_float(lsum > 0.0f ? o / lsum : 0.0f);
+#pragma unroll
+        for (int o = 32 / TPQ; o < 32; o <<= 1) {
+            t.x += __shfl_xor_sync(0xffffffffu, t.x, o); t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
+            t.z += __shfl_xor_sync(0xffffffffu, t.z, o); t.w += __shfl_xor_sync(0xffffffffu, t.w, o);
+            sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        }
+        const int to = e / quads, at = e - to * quads;
+        if (split == 0) {
+            asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};\n"
+                         ::"r"(in_block(s_o + rank * quads + at, to)), "f"(t.x), "f"(t.y), "f"(t.z), "f"(t.w) : "memory");
+            if (at == 0 || e == h * (D / 4))   // (a block may finish quads of several heads, a head may be finished by several blocks)
+                asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};\n" ::"r"(in_block(&s_ml[rank][h], to)), "f"(mx), "f"(sum) : "memory");
+        }
     }
-    cluster.sync();   // no block leaves while a peer still reads its shared memory
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory");
+    // blocks -> result
+    T* out = static_cast<T*>(p.out) + (static_cast<int64_t>(b) * p.num_heads + head0) * D;
+#pragma unroll 1
+    for (int i = tid; i < quads; i += kThreads) {
+        const int e = rank * quads + i, h = e / (D / 4);
+        if (h >= heads) break;
+        float mx = -INFINITY, sum = 0.0f;
+#pragma unroll 4
+        for (int r = 0; r < csize; ++r) mx = fmaxf(mx, s_ml[r][h].x);
+        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+        for (int r = 0; r < csize; ++r) {
+            const float2 ml = s_ml[r][h];
+            const float4 v = s_o[r * quads + i];
+            const float f = ml.x == -INFINITY ? 0.0f : expf(ml.x - mx);
+            t.x = fmaf(f, v.x, t.x); t.y = fmaf(f, v.y, t.y); t.z = fmaf(f, v.z, t.z); t.w = fmaf(f, v.w, t.w);
+            sum = fmaf(f, ml.y, sum);
+        }
+        const bool any = sum > 0.0f;
+        out[4 * e] = ElemTraits<T>::from_float(any ? t.x / sum : 0.0f);
+        out[4 * e + 1] = ElemTraits<T>::from_float(any ? t.y / sum : 0.0f);
+        out[4 * e + 2] = ElemTraits<T>::from_float(any ? t.z / sum : 0.0f);
+        out[4 * e + 3] = ElemTraits<T>::from_float(any ? t.w / sum : 0.0f);
+    }
 }
 
-template <typename T, int D, int HG>
-int launch_simt_typed(const SimtParams& p, int64_t batch, cudaStream_t stream) {
-    const int64_t items = batch * p.num_kv_heads * p.chunks;
-    // Two blocks per SM (one where four heads' accumulators leave no room for two): beyond that a larger cluster only adds
-    // merges.
-    const int64_t resident = static_cast<int64_t>(kSmCount) * (HG <= 2 ? 2 : 1);
-    int csize = 1;
-    while (csize < kMaxCluster && items * csize * 2 <= resident) csize *= 2;
+template <typename T, int D, int HG, int W>
+int launch_simt_blocks(SimtParams& p, int64_t blocks, cudaStream_t stream) {
+    constexpr int kSmemBytes = W * kWarpRing<W>;
+    auto* kernel = decode_simt_kernel<T, D, HG, W>;
+    static std::atomic<bool> attr_done[64] = {};   // per device; the attribute call is idempotent
+    int device = 0;
+    cudaGetDevice(&device);
+    if (device >= 0 && device < 64 && !attr_done[device]) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+        if (e != cudaSuccess) return fail(NVK_ERR_CUDA, "decode_simt_kernel: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+        attr_done[device] = true;
+    }
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(static_cast<unsigned>(items * csize));
-    cfg.blockDim = dim3(kThreads);
+    cfg.gridDim = dim3(static_cast<unsigned>(blocks));
+    cfg.blockDim = dim3(W * 32);
+    cfg.dynamicSmemBytes = kSmemBytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = csize; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    attr[1].val.clusterDim.x = 1u << p.csize_shift; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, decode_simt_kernel<T, D, HG>, p);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
     if (e != cudaSuccess) return fail(NVK_ERR_CUDA, "decode_simt_kernel launch: %s", cudaGetErrorString(e));
     return check_launch("decode_simt_kernel launch");
 }
 
+// Eight warps with twice the ring where no more clusters of 8 than fit at one block per SM (15; a cluster has to fit into one GPC) and tables that
+// give a block some keys: us a pass with four / eight warps: 1 sequence of 4096 keys, 32 / 8 heads, 29.4 / 22.0, 1 of 1600 to 2100, 8 / 2 heads, 15.8 / 13.2,
+// 1 of 500, 16 / 4 heads, 7.8 / 7.3, 1 of 300, 16 / 8 heads, 5.9 / 6.0.  16 to 33 clusters of 4 such blocks: 4 sequences of 4000 keys, 16 / 8 heads, 28.2, clusters
+// of 8 blocks of four warps 26.6.
+constexpr int kWideClusters = 15, kWideTokens = 512;
+template <typename T, int D, int HG>
+int launch_simt_typed(SimtParams& p, cudaStream_t stream) {
+    const int64_t items = static_cast<int64_t>(p.batch) * p.num_kv_heads * p.chunks;
+    // All blocks resident at once: beyond that a larger cluster only adds merges.
+    const bool wide = items <= kWideClusters && p.max_blocks * p.block_size >= kWideTokens;
+    const int64_t resident = static_cast<int64_t>(kSmCount) * (HG <= 2 ? 4 : 3);
+    p.csize_shift = 0;
+    while ((1 << p.csize_shift) < kMaxCluster && (items << (p.csize_shift + 1)) <= resident) ++p.csize_shift;
+    const int64_t blocks = items << p.csize_shift;
+    p.by_block = FastDiv(static_cast<uint32_t>(p.block_size));
+    p.by_chunks = FastDiv(static_cast<uint32_t>(p.chunks));
+    p.by_kv_heads = FastDiv(static_cast<uint32_t>(p.num_kv_heads));
+    return wide ? launch_simt_blocks<T, D, HG, 8>(p, blocks, stream) : launch_simt_blocks<T, D, HG, 4>(p, blocks, stream);
+}
+
 template <typename T, int D>
-int launch_dim(SimtParams& p, int64_t batch, cudaStream_t stream) {
+int launch_dim(SimtParams& p, cudaStream_t stream) {
     const int hg = p.group >= 3 ? 4 : p.group;
     p.chunks = (p.group + hg - 1) / hg;
     switch (hg) {
-        case 1: return launch_simt_typed<T, D, 1>(p, batch, stream);
-        case 2: return launch_simt_typed<T, D, 2>(p, batch, stream);
-        default: return launch_simt_typed<T, D, 4>(p, batch, stream);
+        case 1: return launch_simt_typed<T, D, 1>(p, stream);
+        case 2: return launch_simt_typed<T, D, 2>(p, stream);
+        default: return launch_simt_typed<T, D, 4>(p, stream);
     }
 }
 
 template <typename T>
-int launch_typed(SimtParams& p, int head_dim, int64_t batch, cudaStream_t stream) {
+int launch_typed(SimtParams& p, int head_dim, cudaStream_t stream) {
     switch (head_dim) {
-        case 64: return launch_dim<T, 64>(p, batch, stream);
-        case 128: return launch_dim<T, 128>(p, batch, stream);
-        default: return launch_dim<T, 256>(p, batch, stream);
+        case 64: return launch_dim<T, 64>(p, stream);
+        case 128: return launch_dim<T, 128>(p, stream);
+        default: return launch_dim<T, 256>(p, stream);
     }
 }
 
@@ -335,7 +375,7 @@ int launch_typed(SimtParams& p, int head_dim, int64_t batch, cudaStream_t stream
 bool decode_simt_supported(const DecodeArgs& a) {
     if (a.head_dim != 64 && a.head_dim != 128 && a.head_dim != 256) return false;
     if (!aligned_to(a.k_cache, 16) || !aligned_to(a.v_cache, 16)) return false;
-    if (a.max_blocks * a.block_size >= (1LL << 31)) return false;
+    if (a.max_blocks * a.block_size >= (1LL << 31) - 4096 || a.num_cache_blocks >= (1LL << 31)) return false;
     return a.batch * a.num_heads * kMaxCluster < (1LL << 31);
 }
 
@@ -343,13 +383,13 @@ int launch_decode_simt(const DecodeArgs& a) {
     SimtParams p{};
     p.q = a.q; p.k = a.k_cache; p.v = a.v_cache; p.out = a.out;
     p.context_lens = a.context_lens; p.block_tables = a.block_tables;
-    p.max_blocks = a.max_blocks; p.cache_rows = a.num_cache_blocks * a.block_size;
-    p.num_heads = a.num_heads; p.num_kv_heads = a.num_kv_heads; p.group = a.num_heads / a.num_kv_heads;
+    p.max_blocks = a.max_blocks; p.num_cache_blocks = a.num_cache_blocks;
+    p.batch = static_cast<int>(a.batch); p.num_heads = a.num_heads; p.num_kv_heads = a.num_kv_heads; p.group = a.num_heads / a.num_kv_heads;
     p.block_size = a.block_size; p.scale = a.scale;
     switch (a.dtype) {
-        case NVK_F32: return launch_typed<float>(p, a.head_dim, a.batch, a.stream);
-        case NVK_F16: return launch_typed<__half>(p, a.head_dim, a.batch, a.stream);
-        default: return launch_typed<__nv_bfloat16>(p, a.head_dim, a.batch, a.stream);
+        case NVK_F32: return launch_typed<float>(p, a.head_dim, a.stream);
+        case NVK_F16: return launch_typed<__half>(p, a.head_dim, a.stream);
+        default: return launch_typed<__nv_bfloat16>(p, a.head_dim, a.stream);
     }
 }
 

@@ -70,3 +70,32 @@ def test_infinite_values_stay_infinite(dtype, head_dim, batch):
     assert np.isinf(ref).sum() == 3 * 2 * batch
     assert np.array_equal(got[np.isinf(ref)], ref[np.isinf(ref)])
     assert np.abs(got[np.isfinite(ref)] - ref[np.isfinite(ref)]).max() <= (2e-6 if dtype == "f32" else 1e-2)
+
+
+@pytest.mark.parametrize("dtype,head_dim,block_size", [("f32", 128, 256), ("f32", 64, 48), ("bf16", 256, 16)])
+@pytest.mark.parametrize("num_heads,num_kv_heads,lens,keys", [
+    (8, 2, [511, 3], 511), (8, 2, [512, 1, 0], 512),      # tables on both sides of where few clusters take blocks of eight warps
+    (15, 15, [700], 768), (16, 16, [700], 768),           # as many clusters of those as fit, and one more
+    (3, 1, [5000, 9], 5120),                              # rounds of a ring, more table entries than lanes
+])
+def test_decode_simt_block_sizes_and_keys_without_weight(dtype, head_dim, block_size, num_heads, num_kv_heads, lens, keys):
+    ctx = np.array(lens, np.int32)
+    w = workloads().make_decode_workload(len(lens), num_heads, num_kv_heads, head_dim, block_size, 0, 0, seed=len(lens) + head_dim, context_lens=ctx,
+                                         value_scale=0.5, rounded=dtype != "f32", pad_blocks_to=-(-keys // block_size))
+    td = {"f32": torch.float32, "bf16": torch.bfloat16}[dtype]
+    w["q"] = np.abs(w["q"]) + 0.01 if dtype == "f32" else np.ones_like(w["q"])
+    args = [to_dev(w["q"], td), to_dev(w["k_cache"], td), to_dev(w["v_cache"], td), to_dev(ctx), to_dev(w["block_tables"])]
+    tail = (num_kv_heads, head_dim, block_size, w["scale"])
+    out = torch.full_like(args[0], float("nan"))
+    nvk().launch_decode_attention_paged(*args, *tail, out)
+    err = np.abs(to_np(out) - _reference(w, num_kv_heads, block_size))
+    assert err.max() <= (2e-6 if dtype == "f32" else 1e-2), err.max()
+    # the first and a later key score minus infinity: no weight, nothing else changes
+    for b, n in enumerate(lens):
+        for key in {0, n // 2} if n > 2 else ():
+            row = int(w["block_tables"][b, key // block_size]) * block_size + key % block_size
+            w["k_cache"].reshape(-1, num_kv_heads, head_dim)[row] = -np.inf
+    args[1] = to_dev(w["k_cache"], td)
+    nvk().launch_decode_attention_paged(*args, *tail, out)
+    err = np.abs(to_np(out) - _reference(w, num_kv_heads, block_size))
+    assert err.max() <= (2e-6 if dtype == "f32" else 1e-2), err.max()
