@@ -15,14 +15,14 @@
 //
 // GEMM core: C[M, N] = A[M, K] * B[N, K]^T, both operands K-major as torch linears keep them; TMA (128-byte swizzle) into a ring of
 // shared-memory stages, tcgen05.mma into TMEM.  Two kernels, chosen by size (choose_gemm):
-//   gemm_split_kernel   few rows.  The GEMM streams the weight once and is HBM-bound, so every SM has to stream: a block takes 128 or
-//                       256 rows x 128 columns of C over a part of K, the blocks of a cluster the parts of one tile; they add up
-//                       through distributed shared memory, each for its share of the rows, and run the epilogue on that share.
+//   gemm_split_kernel   few rows.  The GEMM streams the weight once and is HBM-bound, so every SM has to stream: a block takes 128
+//                       rows x 128 columns of C over a part of K (or 256 rows over all of it), the blocks of a cluster the parts of one
+//                       tile; each pushes its sums to the block that finishes a row, which runs the epilogue on its share of the rows.
 //   gemm_pair_kernel    many rows, bound by the tensor pipe.  Persistent pairs of blocks (cta_group::2): 256 x 256 tiles, each block
 //                       loads half of A and half of B, so an SM moves half the operand bytes of a 128 x 256 tile of its own.  The
 //                       accumulator is double buffered in TMEM: the epilogue of a tile runs under the next tile's MMAs.
 // Before, one block per 128 x 128 tile whatever the size (microseconds in a loop over weights larger than L2; K 4096):
-//   64 x 6144  22 -> 16      64 x 4096  21 -> 12 (with MMAs from a converged warp 14.5 and 11.1)     7440 x 4096  295 -> 175 (1430 TFLOP/s)     7440 x 6144 with QKV epilogue  597 -> 277
+//   64 x 6144  22 -> 16      64 x 4096  21 -> 12 (with MMAs from a converged warp 14.5 and 11.1, with pushed sums 13.1 and 10.4)     7440 x 4096  295 -> 175 (1430 TFLOP/s)     7440 x 6144 with QKV epilogue  597 -> 277
 // What the fusion removes is the round trip of the result and one or two launches per layer.
 // Every mbarrier wait is bounded; a wait that runs out raises an error word (nvk_gemm_status), and the block leaves when what it
 // has under way has had time to land.
@@ -39,9 +39,11 @@ namespace {
 constexpr int kBM = 128, kBN = 128, kBK = 64;
 constexpr int kPanelBytes = kBM * kBK * 2;            // 16 KiB: 128 rows x 128 bytes
 constexpr int kRingBytes = 12 * kPanelBytes;          // 192 KiB: 6 stages of 2 panels or 4 of 3
-constexpr int kStageOffset = kRingBytes + 256;        // after the barriers: 4 KiB per epilogue warp of gemm_pair_kernel
-constexpr int kSmemBytes = kStageOffset + 8 * 4096 + 1024;   // + slack for 1024-byte alignment
-constexpr int kThreads = 192;                         // warp 0 TMA, warp 1 MMA + TMEM, warps 2-5 TMEM readers
+constexpr int kEpilogueBytes = 4096;                  // of a warp that takes whole rows from tensor memory
+constexpr int kStageOffset = kRingBytes;              // for the epilogue warps, or what peers push in gemm_split_kernel
+constexpr int kBarOffset = kStageOffset + 8 * kEpilogueBytes;
+constexpr int kSmemBytes = kBarOffset + 256 + 1024;   // + slack for 1024-byte alignment
+constexpr int kThreads = 256;                         // warp 0 TMA, warp 1 MMA + TMEM, warps 2-5 TMEM readers, all for the sums
 constexpr int kPairThreads = 320;                     // the same with warps 2-9 for the epilogue
 constexpr int kMaxSplits = 8;                         // portable cluster size
 constexpr long long kWaitCycles = 4000000000LL;       // ~2 s
@@ -148,6 +150,11 @@ __device__ __forceinline__ void cluster_sync_all() {
     __syncwarp();
     asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
 }
+// `bytes` of this block's shared memory into that of block `rank`, counted on its barrier at `bar`.
+__device__ __forceinline__ void push_bulk(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar, uint32_t rank) {
+    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
+                 ::"r"(in_block(dst, rank)), "r"(src), "r"(bytes), "r"(in_block(bar, rank)) : "memory");
+}
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
     asm("mov.u32 %0, %cluster_ctarank;\n" : "=r"(r));
@@ -228,6 +235,11 @@ __device__ __forceinline__ void load_rounded(uint32_t taddr, float (&v)[32]) {
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = ElemTraits<T>::to_float(ElemTraits<T>::from_float(__uint_as_float(r[i])));
 }
+template <typename T> __device__ __forceinline__ void unpack2(uint32_t w, float& lo, float& hi) {
+    const T* e = reinterpret_cast<const T*>(&w);
+    lo = ElemTraits<T>::to_float(e[0]);
+    hi = ElemTraits<T>::to_float(e[1]);
+}
 template <typename T> __device__ __forceinline__ uint4 pack8(const float* v) {
     return make_uint4(ElemTraits<T>::pack2(v[0], v[1]), ElemTraits<T>::pack2(v[2], v[3]), ElemTraits<T>::pack2(v[4], v[5]), ElemTraits<T>::pack2(v[6], v[7]));
 }
@@ -269,13 +281,18 @@ struct QkvRow {
     const float* table;   // nullptr: no rotation
     bool is_v;
 };
+struct QkvIndex { int pos, slot; bool live; };
+__device__ __forceinline__ QkvIndex qkv_index(const GemmParams& p, int64_t row) {
+    const bool live = row < p.m;
+    return QkvIndex{live ? __ldg(p.positions + row) : 0, live && p.slot_mapping != nullptr ? __ldg(p.slot_mapping + row) : -1, live};
+}
 template <typename T>
-__device__ __forceinline__ QkvRow<T> qkv_row(const GemmParams& p, int head, int64_t row, bool live) {
+__device__ __forceinline__ QkvRow<T> qkv_row(const GemmParams& p, int head, int64_t row, const QkvIndex& at) {
     const bool is_q = head < p.hq, is_k = !is_q && head < p.hq + p.hkv;
-    const int pos = live ? __ldg(p.positions + row) : 0;
-    const int64_t slot = live ? (p.slot_mapping != nullptr ? static_cast<int64_t>(__ldg(p.slot_mapping + row)) : row) : -1;
+    const int pos = at.pos;
+    const int64_t slot = p.slot_mapping != nullptr ? static_cast<int64_t>(at.slot) : row;
     QkvRow<T> x{nullptr, nullptr, nullptr, !is_q && !is_k};
-    if (live) {
+    if (at.live) {
         if (is_q) x.dst = static_cast<T*>(p.q_out) + (row * p.hq + head) * kBN;
         else if (slot >= 0 && slot < p.cache_rows)
             x.dst = static_cast<T*>(is_k ? p.k_cache : p.v_cache) + (slot * p.hkv + (is_k ? head - p.hq : head - p.hq - p.hkv)) * kBN;
@@ -304,9 +321,11 @@ __device__ __forceinline__ PushRow<T> push_row(const GemmParams& p, int64_t row,
 }
 
 // One thread holds the whole row in TMEM columns t_row .. t_row + 127 (warp-collective: every lane runs all of it).  `stage`: 4 KiB of
-// shared memory of this warp.
-template <typename T, int EPI>
-__device__ __forceinline__ void epilogue_row(const GemmParams& p, uint32_t t_row, int64_t row, int nt, unsigned char* stage, int lane) {
+// shared memory of this warp, 8 with WIDE (gemm_pair_kernel has no room for that beside its ring).  `hidden`: other work takes longer than the
+// epilogue, whose instructions cost that work more than its time matters (gemm_pair_kernel, 7440 x 6144, K 4096: 264.5 us, so only behind the last tile 260, one lane a row
+// throughout 262).
+template <typename T, int EPI, bool WIDE>
+__device__ __forceinline__ void epilogue_row(const GemmParams& p, uint32_t t_row, int64_t row, const QkvIndex& at_row, int nt, unsigned char* stage, int lane, bool hidden = false) {
     const bool live = row < p.m;
     const int n0 = nt * kBN;
     if (EPI == kAllReducePush) {
@@ -325,7 +344,7 @@ __device__ __forceinline__ void epilogue_row(const GemmParams& p, uint32_t t_row
         return;
     }
     QkvRow<T> x{};
-    if (EPI == kQkvPrologue) x = qkv_row<T>(p, nt, row, live);
+    if (EPI == kQkvPrologue) x = qkv_row<T>(p, nt, row, at_row);
     if (EPI == kPlain || x.is_v) {             // the rounded GEMM output as it is
         T* dst = EPI == kQkvPrologue ? x.dst : live ? static_cast<T*>(p.out) + row * p.n + n0 : nullptr;
 #pragma unroll 1
@@ -337,52 +356,220 @@ __device__ __forceinline__ void epilogue_row(const GemmParams& p, uint32_t t_row
         }
         return;
     }
-    float inv_rms = 1.0f;
-    if (x.weight != nullptr) {                 // pass 1 over the accumulator: the head's sum of squares
-        float ss = 0.0f;
-#pragma unroll 1
+    // A q or k head.  The thread that has the row takes its sum of squares and leaves the row in shared memory; norm and rotation are done by eight lanes a
+    // row, so that they read table rows and write results in whole 128-byte lines: eight rows a trip, the next trip's table rows under way.  Loads without
+    // branches around them: a branch waits for what was loaded before it, which cost more than the loads.  (Each lane its own table row, 32
+    // lines an instruction, K 512, 1000 rows x 1536 / 3072 columns: pairs 16.3 / 16.0 us, 13.8 / 14.5 now, one block for 128 rows and all of K 8.4, now 6.7 / 12.9;
+    // products alone in pairs 7.9 / 8.7.)
+    if constexpr (WIDE) {
+        const int sub = lane & 7;                  // elements 8 sub .. + 7 of both halves of the head
+        const unsigned long long dst_of = reinterpret_cast<unsigned long long>(x.dst), table_of = reinterpret_cast<unsigned long long>(x.table != nullptr ? x.table : p.cos_sin);
+        const unsigned int rotated = __ballot_sync(0xffffffffu, x.table != nullptr);
+        struct Trig { float4 cs[2], sn[2]; };
+        auto fetch = [&](int at, Trig& g) {        // table row of row `at`
+            const float* from = reinterpret_cast<const float*>(__shfl_sync(0xffffffffu, table_of, at)) + 8 * sub;   // (row 0 where there is none)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) { g.cs[i] = ld_table(p, from + 4 * i); g.sn[i] = ld_table(p, from + 64 + 4 * i); }
+        };
+        Trig now[2], next[2];
+        T w[16];
+        float ss4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
         for (int c = 0; c < 4; ++c) {
             float v[32];
             load_rounded<T>(t_row + c * 32, v);
 #pragma unroll
-            for (int i = 0; i < 32; ++i) ss += v[i] * v[i];
+            for (int i = 0; i < 32; ++i) ss4[i & 3] += v[i] * v[i];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) reinterpret_cast<uint4*>(stage + lane * 256)[(4 * c + q) ^ (lane & 7)] = pack8<T>(v + 8 * q);
         }
-        inv_rms = rsqrtf(ss / static_cast<float>(kBN) + p.eps);
-    }
-#pragma unroll 1
-    for (int c = 0; c < 2; ++c) {              // pass 2: columns [32 c, 32 c + 32) rotate with [64 + 32 c, 64 + 32 c + 32)
-        float lo[32], hi[32];
-        load_rounded<T>(t_row + c * 32, lo);
-        load_rounded<T>(t_row + 64 + c * 32, hi);
         if (x.weight != nullptr) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-                lo[i] = lo[i] * inv_rms * ElemTraits<T>::to_float(x.weight[c * 32 + i]);
-                hi[i] = hi[i] * inv_rms * ElemTraits<T>::to_float(x.weight[64 + c * 32 + i]);
-            }
+            for (int i = 0; i < 16; ++i) w[i] = x.weight[(i >> 3) * 64 + 8 * sub + (i & 7)];
         }
-        if (x.table != nullptr) {              // first half: x cos - partner sin; second half: x cos + partner sin
-            // 16-byte loads: every lane reads its own table row, so an instruction costs 32 cache lines whatever its width
 #pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-                const float4 c4 = ld_table(p, x.table + c * 32 + i), s4 = ld_table(p, x.table + 64 + c * 32 + i);
-                const float cs[4] = {c4.x, c4.y, c4.z, c4.w}, sn[4] = {s4.x, s4.y, s4.z, s4.w};
+        for (int u = 0; u < 2; ++u) fetch(4 * u + (lane >> 3), now[u]);
+        const float ss = (ss4[0] + ss4[1]) + (ss4[2] + ss4[3]);
+        const float inv_rms = rsqrtf(ss / static_cast<float>(kBN) + p.eps);
+        __syncwarp();
+        auto trip = [&](int r, Trig (&now)[2]) {
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const float a = lo[i + u], b = hi[i + u];
-                    lo[i + u] = fmaf(a, cs[u], b * -sn[u]);
-                    hi[i + u] = fmaf(b, cs[u], a * sn[u]);
+            for (int u = 0; u < 2; ++u) {
+                const int at = r + 4 * u + (lane >> 3);
+                const uint4* from = reinterpret_cast<const uint4*>(stage + at * 256);
+                const uint4 lo4 = from[sub ^ (at & 7)], hi4 = from[(8 + sub) ^ (at & 7)];
+                const uint32_t lo_w[4] = {lo4.x, lo4.y, lo4.z, lo4.w}, hi_w[4] = {hi4.x, hi4.y, hi4.z, hi4.w};
+                float lo[8], hi[8];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    unpack2<T>(lo_w[i], lo[2 * i], lo[2 * i + 1]);
+                    unpack2<T>(hi_w[i], hi[2 * i], hi[2 * i + 1]);
+                }
+                if (x.weight != nullptr) {
+                    const float inv = __shfl_sync(0xffffffffu, inv_rms, at);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) { lo[i] = lo[i] * inv * ElemTraits<T>::to_float(w[i]); hi[i] = hi[i] * inv * ElemTraits<T>::to_float(w[8 + i]); }
+                }
+                if ((rotated >> at) & 1u) {        // first half: x cos - partner sin; second half: x cos + partner sin
+                    const float4 (&c4)[2] = now[u].cs, (&s4)[2] = now[u].sn;
+                    const float cs[8] = {c4[0].x, c4[0].y, c4[0].z, c4[0].w, c4[1].x, c4[1].y, c4[1].z, c4[1].w};
+                    const float sn[8] = {s4[0].x, s4[0].y, s4[0].z, s4[0].w, s4[1].x, s4[1].y, s4[1].z, s4[1].w};
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const float a = lo[i], b = hi[i];
+                        lo[i] = fmaf(a, cs[i], b * -sn[i]);
+                        hi[i] = fmaf(b, cs[i], a * sn[i]);
+                    }
+                }
+                T* dst = reinterpret_cast<T*>(__shfl_sync(0xffffffffu, dst_of, at));
+                if (dst != nullptr) {
+                    *reinterpret_cast<uint4*>(dst + 8 * sub) = pack8<T>(lo);
+                    *reinterpret_cast<uint4*>(dst + 64 + 8 * sub) = pack8<T>(hi);
                 }
             }
+        };
+#pragma unroll 1
+        for (int r = 0; r < 32; r += 16) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) fetch(r + 8 + 4 * u + (lane >> 3), next[u]);
+            trip(r, now);
+            if (r < 16) {
+#pragma unroll
+                for (int u = 0; u < 2; ++u) fetch(r + 16 + 4 * u + (lane >> 3), now[u]);
+            }
+            trip(r + 8, next);
         }
-        store_rows<T>(x.dst, c * 32, 64 + c * 32, lo, hi, stage, lane);
+        __syncwarp();                              // the rows have been read
+    } else if (hidden) {
+        // Each lane the row that it has: fewest instructions, and slow.
+        float inv_rms = 1.0f;
+        if (x.weight != nullptr) {                 // pass 1 over the accumulator: the head's sum of squares
+            float ss = 0.0f;
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c) {
+                float v[32];
+                load_rounded<T>(t_row + c * 32, v);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) ss += v[i] * v[i];
+            }
+            inv_rms = rsqrtf(ss / static_cast<float>(kBN) + p.eps);
+        }
+#pragma unroll 1
+        for (int c = 0; c < 2; ++c) {              // pass 2: columns [32 c, 32 c + 32) rotate with [64 + 32 c, 64 + 32 c + 32)
+            float lo[32], hi[32];
+            load_rounded<T>(t_row + c * 32, lo);
+            load_rounded<T>(t_row + 64 + c * 32, hi);
+            if (x.weight != nullptr) {
+#pragma unroll
+                for (int i = 0; i < 32; ++i) {
+                    lo[i] = lo[i] * inv_rms * ElemTraits<T>::to_float(x.weight[c * 32 + i]);
+                    hi[i] = hi[i] * inv_rms * ElemTraits<T>::to_float(x.weight[64 + c * 32 + i]);
+                }
+            }
+            if (x.table != nullptr) {              // first half: x cos - partner sin; second half: x cos + partner sin
+                // 16-byte loads: every lane reads its own table row, so an instruction costs 32 cache lines whatever its width
+#pragma unroll
+                for (int i = 0; i < 32; i += 4) {
+                    const float4 c4 = ld_table(p, x.table + c * 32 + i), s4 = ld_table(p, x.table + 64 + c * 32 + i);
+                    const float cs[4] = {c4.x, c4.y, c4.z, c4.w}, sn[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const float a = lo[i + u], b = hi[i + u];
+                        lo[i + u] = fmaf(a, cs[u], b * -sn[u]);
+                        hi[i + u] = fmaf(b, cs[u], a * sn[u]);
+                    }
+                }
+            }
+            store_rows<T>(x.dst, c * 32, 64 + c * 32, lo, hi, stage, lane);
+        }
+    } else {
+        // With 4 KiB: columns [32 c, 32 c + 32) and their partners [64 + 32 c, ...) at a time, four lanes a row, eight rows a trip.
+        const int sub = lane & 3;                  // elements 8 sub .. + 7 of the columns and of their partners
+        const unsigned long long dst_of = reinterpret_cast<unsigned long long>(x.dst), table_of = reinterpret_cast<unsigned long long>(x.table != nullptr ? x.table : p.cos_sin);
+        const unsigned int rotated = __ballot_sync(0xffffffffu, x.table != nullptr);
+        struct Trig { float4 cs[2], sn[2]; } even, odd;
+        auto fetch = [&](int trip, Trig& g) {      // of eight: four of each c
+            const float* from = reinterpret_cast<const float*>(__shfl_sync(0xffffffffu, table_of, (trip & 3) * 8 + (lane >> 2))) + (trip >> 2) * 32 + 8 * sub;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) { g.cs[i] = ld_table(p, from + 4 * i); g.sn[i] = ld_table(p, from + 64 + 4 * i); }
+        };
+        float ss4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (x.weight != nullptr) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                float v[32];
+                load_rounded<T>(t_row + c * 32, v);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) ss4[i & 3] += v[i] * v[i];
+            }
+        }
+        const float inv_rms = rsqrtf(((ss4[0] + ss4[1]) + (ss4[2] + ss4[3])) / static_cast<float>(kBN) + p.eps);
+        fetch(0, even);
+        fetch(1, odd);
+#pragma unroll 1
+        for (int c = 0; c < 2; ++c) {
+            T w[16];
+            {
+                uint4* row16 = reinterpret_cast<uint4*>(stage + lane * 128);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float v[32];
+                    load_rounded<T>(t_row + c * 32 + h * 64, v);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) row16[(4 * h + q) ^ (lane & 7)] = pack8<T>(v + 8 * q);
+                }
+            }
+            if (x.weight != nullptr) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) w[i] = x.weight[32 * c + (i >> 3) * 64 + 8 * sub + (i & 7)];
+            }
+            __syncwarp();
+            auto trip = [&](int n, Trig& g) {
+                const int at = (n & 3) * 8 + (lane >> 2);
+                const uint4* from = reinterpret_cast<const uint4*>(stage + at * 128);
+                const uint4 lo4 = from[sub ^ (at & 7)], hi4 = from[(4 + sub) ^ (at & 7)];
+                const uint32_t lo_w[4] = {lo4.x, lo4.y, lo4.z, lo4.w}, hi_w[4] = {hi4.x, hi4.y, hi4.z, hi4.w};
+                float lo[8], hi[8];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    unpack2<T>(lo_w[i], lo[2 * i], lo[2 * i + 1]);
+                    unpack2<T>(hi_w[i], hi[2 * i], hi[2 * i + 1]);
+                }
+                if (x.weight != nullptr) {
+                    const float inv = __shfl_sync(0xffffffffu, inv_rms, at);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) { lo[i] = lo[i] * inv * ElemTraits<T>::to_float(w[i]); hi[i] = hi[i] * inv * ElemTraits<T>::to_float(w[8 + i]); }
+                }
+                if ((rotated >> at) & 1u) {
+                    const float cs[8] = {g.cs[0].x, g.cs[0].y, g.cs[0].z, g.cs[0].w, g.cs[1].x, g.cs[1].y, g.cs[1].z, g.cs[1].w};
+                    const float sn[8] = {g.sn[0].x, g.sn[0].y, g.sn[0].z, g.sn[0].w, g.sn[1].x, g.sn[1].y, g.sn[1].z, g.sn[1].w};
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const float a = lo[i], b = hi[i];
+                        lo[i] = fmaf(a, cs[i], b * -sn[i]);
+                        hi[i] = fmaf(b, cs[i], a * sn[i]);
+                    }
+                }
+                fetch((n + 2) & 7, g);
+                T* dst = reinterpret_cast<T*>(__shfl_sync(0xffffffffu, dst_of, at));
+                if (dst != nullptr) {
+                    *reinterpret_cast<uint4*>(dst + 32 * c + 8 * sub) = pack8<T>(lo);
+                    *reinterpret_cast<uint4*>(dst + 64 + 32 * c + 8 * sub) = pack8<T>(hi);
+                }
+            };
+#pragma unroll 1
+            for (int n = 4 * c; n < 4 * c + 4; n += 2) {
+                trip(n, even);
+                trip(n + 1, odd);
+            }
+            __syncwarp();                          // the columns have been read
+        }
     }
 }
 
 // Eight lanes hold a row: lane `sub` elements 32 q + 4 sub .. + 3, q = 0 .. 3 (v[q]), so that the eight read 128 contiguous bytes of the
-// sums at a time -- from another block's shared memory 32-byte pieces 32 bytes apart come in at a quarter of the rate -- and rotation pairs
-// (d, d + 64) meet in a lane.  octet_row fetches what the epilogue of a row needs besides the sums (positions, then table rows: two
-// dependent trips to memory), so that this can be under way before the sums are there.
+// sums at a time and rotation pairs (d, d + 64) meet in a lane.  octet_row fetches what the epilogue of a row needs besides the sums (with the row's
+// position and slot, which come first: two dependent trips to memory), so that this can be under way before the sums are there.
 template <typename T>
 struct OctetRow {
     T* dst;               // kPlain, kQkvPrologue, kAllReducePush (own rows); nullptr: nothing to write there
@@ -392,21 +579,19 @@ struct OctetRow {
     float4 cs[2], sn[2];
 };
 template <typename T, int EPI>
-__device__ __forceinline__ OctetRow<T> octet_row(const GemmParams& p, int64_t row, int nt, int sub) {
+__device__ __forceinline__ OctetRow<T> octet_row(const GemmParams& p, int64_t row, const QkvIndex& at, int nt, int sub) {
     const bool live = row < p.m;
     OctetRow<T> x{};
     if (EPI == kPlain) {
         x.dst = live ? static_cast<T*>(p.out) + row * p.n + nt * kBN : nullptr;
     } else if (EPI == kQkvPrologue) {
-        const QkvRow<T> q = qkv_row<T>(p, nt, row, live);
+        const QkvRow<T> q = qkv_row<T>(p, nt, row, at);
         x.dst = q.dst;
         x.rotate = !q.is_v && q.table != nullptr;
-        if (x.rotate) {
+        if (!q.is_v) {                             // (the same for the whole block; otherwise no branch that waits for what was loaded before it)
+            const float* from = (q.table != nullptr ? q.table : p.cos_sin) + 4 * sub;
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                x.cs[i] = ld_table(p, q.table + 32 * i + 4 * sub);
-                x.sn[i] = ld_table(p, q.table + 64 + 32 * i + 4 * sub);
-            }
+            for (int i = 0; i < 2; ++i) { x.cs[i] = ld_table(p, from + 32 * i); x.sn[i] = ld_table(p, from + 64 + 32 * i); }
         }
     } else {
         const PushRow<T> q = push_row<T>(p, row, live, nt * kBN);
@@ -414,9 +599,17 @@ __device__ __forceinline__ OctetRow<T> octet_row(const GemmParams& p, int64_t ro
     }
     return x;
 }
+// The norm weights of this lane's elements, the same for all rows of the tile.
+template <typename T, int EPI>
+__device__ __forceinline__ void octet_weights(const GemmParams& p, int nt, int sub, T (&w)[16]) {
+    if (EPI != kQkvPrologue || p.q_weight == nullptr || nt >= p.hq + p.hkv) return;
+    const T* weight = static_cast<const T*>(nt < p.hq ? p.q_weight : p.k_weight) + 4 * sub;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) w[i] = weight[32 * (i >> 2) + (i & 3)];
+}
 // Every lane of the warp runs it (shuffles).
 template <typename T, int EPI>
-__device__ __forceinline__ void epilogue_octet(const GemmParams& p, const OctetRow<T>& x, float4 (&v)[4], int nt, int sub) {
+__device__ __forceinline__ void epilogue_octet(const GemmParams& p, const OctetRow<T>& x, float4 (&v)[4], const T (&weight)[16], int nt, int sub) {
     float e[4][4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -426,7 +619,6 @@ __device__ __forceinline__ void epilogue_octet(const GemmParams& p, const OctetR
     }
     if (EPI == kQkvPrologue && nt < p.hq + p.hkv) {   // a q or k head (the same for the whole block)
         if (p.q_weight != nullptr) {
-            const T* weight = static_cast<const T*>(nt < p.hq ? p.q_weight : p.k_weight) + 4 * sub;
             float ss = 0.0f;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -439,7 +631,7 @@ __device__ __forceinline__ void epilogue_octet(const GemmParams& p, const OctetR
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) e[q][i] = e[q][i] * inv_rms * ElemTraits<T>::to_float(weight[32 * q + i]);
+                for (int i = 0; i < 4; ++i) e[q][i] = e[q][i] * inv_rms * ElemTraits<T>::to_float(weight[4 * q + i]);
             }
         }
         if (x.rotate) {
@@ -472,65 +664,54 @@ __device__ __forceinline__ void epilogue_octet(const GemmParams& p, const OctetR
     }
 }
 
-// Sum of one row over the blocks of a cluster, U blocks at a time (loads without branches, so that all of a trip's are in flight).
-template <int U>
-__device__ __forceinline__ void sum_over_cluster(uint32_t at, int splits, float4 (&sum)[4]) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) sum[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int r0 = 0; r0 < splits; r0 += U) {
-        float4 v[U][4];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const uint32_t src = in_block(at, static_cast<uint32_t>(min(r0 + u, splits - 1)));
-#pragma unroll
-            for (int q = 0; q < 4; ++q) v[u][q] = ld_cluster(src + 128 * q);
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (r0 + u < splits) {
-#pragma unroll
-                for (int q = 0; q < 4; ++q) { sum[q].x += v[u][q].x; sum[q].y += v[u][q].y; sum[q].z += v[u][q].z; sum[q].w += v[u][q].w; }
-            }
-        }
-    }
-}
-
 // ---- few rows: blocks of a cluster share K ------------------------------------------------------------------------------------
-// blockIdx.x = tile column * splits + part of K (= rank in the cluster), blockIdx.y = tile row of MT * 128 rows.  The partial sums go to
-// shared memory as fp32 rows of 132 words (no bank conflicts for the writing threads, each of which has a row); block r adds up and
-// finishes rows r, r + splits, ... of the tile, eight lanes a row.
+// blockIdx.x = tile column * splits + part of K (= rank in the cluster), blockIdx.y = tile row of MT * 128 rows.
 // DIRECT: a block with all of K has nothing to add up and takes its tile from TMEM straight to the result (us: 4096 columns, K 128, 128 rows
-// 5.5 -> 4.0); not for the QKV epilogue, which is quicker with eight lanes a row (64 x 3072, K 1024: 10.4, 8.7), nor up to 32 rows, which would leave three of four epilogue warps idle (8 rows 3.2 -> 3.7).  An instantiation of its own: with both
+// 5.5 -> 4.0); not up to 32 rows, which would leave three of four epilogue warps idle (8 rows 3.2 -> 3.7).  An instantiation of its own: with both
 // ways in one the sums were slower (39 rows through 768 x 4096 and 4096 x 512 in a pass of 25.2 us: 26.4).
-constexpr int kRowWords = kBN + 4;
+// Otherwise (MT 1) the partial sums go to shared memory as fp32 rows, and block r adds up and finishes the r-th of `splits` runs of rows: every
+// block pushes each run by one bulk copy into the shared memory of the block that finishes it, where all that follows is local (rows of 512
+// bytes, their 16-byte pieces XOR-swizzled by row: no bank conflicts for the writing threads, each of which has a row, nor for the readers, eight
+// lanes a row).  What peers push has a place of its own, for more than 64 rows the ring's last stage with it.  When the sums were fetched from
+// the peers' shared memory instead, 10 bytes a clock came in: from the last MMA to a block's end 4.0 us for 64 x 6144, K 4096 (15.8 us in all, 13.9
+// now), 3.2 for 64 x 4096 (11.1, 10.4), 5.5 for 128 x 6144 (17.6, 15.8).
 template <typename T, int EPI, int MT, bool DIRECT>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ GemmParams p, int splits) {
+    static_assert(MT == 1 || DIRECT, "sums of 256 rows have no room beside what peers push");
     constexpr int kStageBytes = (MT + 1) * kPanelBytes, kStages = kRingBytes / kStageBytes, kTmemCols = MT * kBN;
-    static_assert(MT * kBM * kRowWords * 4 <= kRingBytes, "the partial sums take the ring's place");
+    constexpr uint32_t kSumBytes = kBN * 4;           // a row of partial sums
     extern __shared__ unsigned char smem_raw[];
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;   // (uniform, also to the compiler)
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t bars = smem_base + kRingBytes;
+    const uint32_t bars = smem_base + kBarOffset;
     auto bar_full = [&](int s) { return bars + 8 * s; };
     auto bar_empty = [&](int s) { return bars + 64 + 8 * s; };
-    const uint32_t bar_acc = bars + 128;
+    const uint32_t bar_acc = bars + 128, bar_recv = bars + 136;
     volatile int* abort_flag = &s_abort;
     const int rank = static_cast<int>(blockIdx.x) % splits, nt = static_cast<int>(blockIdx.x) / splits;
     const int n0 = nt * kBN, m0 = blockIdx.y * (MT * kBM);
     const int rows = static_cast<int>(min(static_cast<int64_t>(MT * kBM), p.m - m0));   // of the tile that are in C
     const int kb_all = static_cast<int>((p.k + kBK - 1) / kBK);
     const int kb0 = kb_all * rank / splits, kb_count = kb_all * (rank + 1) / splits - kb0;
+    // Rows of a run, this block's run, where peers' parts of it come in, and the stages that leaves (a run per block: at most 64 or 128 rows in all)
+    const int run = (rows + splits - 1) / splits, own_rows = min(run, rows - rank * run);
+    const bool narrow = !DIRECT && splits > 1 && rows > kBM / 2;
+    const int stages = narrow ? kStages - 1 : kStages;
+    const uint32_t recv = smem_base + (narrow ? (kStages - 1) * kStageBytes : kStageOffset);
 
     if (tid == 0) {
         s_abort = 0;
         for (int s = 0; s < kStages; ++s) { mbar_init(bar_full(s), 1); mbar_init(bar_empty(s), 1); }
         mbar_init(bar_acc, 1);
+        mbar_init(bar_recv, 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        if (!DIRECT && splits > 1 && own_rows > 0) mbar_expect_tx(bar_recv, (splits - 1) * own_rows * kSumBytes);
     }
     __syncwarp();
+    if (!DIRECT && splits > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");   // (waited for before the push: all barriers are set up)
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&s_tmem_base)), "r"(kTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
@@ -544,14 +725,16 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
         if (lane == 0) {
+            int s = 0;
+            uint32_t turn = 1;
             for (int i = 0; i < kb_count; ++i) {
-                const int s = i % kStages;
-                if (i >= kStages && !mbar_wait(bar_empty(s), ((i / kStages) & 1) ^ 1, abort_flag, 1)) break;
+                if (i >= stages && !mbar_wait(bar_empty(s), turn, abort_flag, 1)) break;
                 mbar_expect_tx(bar_full(s), kPanelBytes + (MT == 1 ? p.a_rows * kBK * 2 : 2 * kPanelBytes));
                 const uint32_t at = smem_base + s * kStageBytes;
                 tma_load_2d(at + MT * kPanelBytes, &tm_b, (kb0 + i) * kBK, n0, bar_full(s));
 #pragma unroll
                 for (int t = 0; t < MT; ++t) tma_load_2d(at + t * kPanelBytes, &tm_a, (kb0 + i) * kBK, m0 + t * kBM, bar_full(s));
+                if (++s == stages) { s = 0; turn ^= 1u; }
             }
         }
     } else if (warp == 1) {
@@ -575,22 +758,25 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
                     umma_ss(leader, tmem_base + t * kBN, da + 2 * ks, db + 2 * ks, p.idesc, (i > 0 || ks > 0) ? 1u : 0u);
             }
             tc_commit(leader, bar_empty(s));
-            if (++s == kStages) { s = 0; turn ^= 1u; }
+            if (++s == stages) { s = 0; turn ^= 1u; }
         }
         if (ok) tc_commit(leader, bar_acc);
-    } else {
+    } else if (warp < 6) {
         // ------------------------------------------------------------------ TMEM -> shared memory: thread = row of the tile
         const int wq = warp & 3;                       // TMEM lanes 32 wq .. 32 wq + 31 belong to this warp
         bool ok = true;
+        QkvIndex index[MT];
+#pragma unroll
+        for (int t = 0; t < MT; ++t) index[t] = DIRECT && EPI == kQkvPrologue ? qkv_index(p, m0 + t * kBM + wq * 32 + lane) : QkvIndex{};
         if (lane == 0) ok = mbar_wait(bar_acc, 0, abort_flag, 3);
         ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
         tc_fence_after();
         if (DIRECT && ok) {
-            unsigned char* stage = smem_raw + (smem_base - smem_u32(smem_raw)) + kStageOffset + (warp - 2) * 4096;
+            unsigned char* stage = smem_raw + (smem_base - smem_u32(smem_raw)) + kStageOffset + (warp - 2) * 2 * kEpilogueBytes;
 #pragma unroll 1
             for (int t = 0; t < MT; ++t)
                 if (t * kBM + wq * 32 < rows)
-                    epilogue_row<T, EPI>(p, tmem_base + (static_cast<uint32_t>(wq * 32) << 16) + t * kBN, m0 + t * kBM + wq * 32 + lane, nt, stage, lane);
+                    epilogue_row<T, EPI, true>(p, tmem_base + (static_cast<uint32_t>(wq * 32) << 16) + t * kBN, m0 + t * kBM + wq * 32 + lane, MT == 2 && t == 1 ? index[MT - 1] : index[0], nt, stage, lane);
         } else if (ok) {
 #pragma unroll 1
             for (int c = 0; c < MT * 4; ++c) {
@@ -600,11 +786,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
                 tmem_ld32(tmem_base + (static_cast<uint32_t>(wq * 32) << 16) + c * 32, r);
                 tc_wait_ld();
                 reg_fence32(r);
-                const uint32_t dst = smem_base + (row_in_tile * kRowWords + (c & 3) * 32) * 4;
+                const uint32_t dst = smem_base + row_in_tile * kSumBytes + (c & 3) * 128;
 #pragma unroll
                 for (int q = 0; q < 8; ++q)
-                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(dst + q * 16), "r"(r[4 * q]), "r"(r[4 * q + 1]), "r"(r[4 * q + 2]), "r"(r[4 * q + 3]) : "memory");
+                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(dst + ((q ^ (row_in_tile & 7)) * 16)), "r"(r[4 * q]), "r"(r[4 * q + 1]), "r"(r[4 * q + 2]), "r"(r[4 * q + 3]) : "memory");
             }
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // (bulk copies read it)
         }
     }
     tc_fence_before();
@@ -616,34 +803,60 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     if (DIRECT) return;
     // ---------------------------------------------------------------------- sum over the cluster and epilogue
     const int sub = lane & 7;
-    int q = warp * 4;                      // four rows per warp and trip
-    auto row_of = [&](int first) { return (first + (lane >> 3)) * splits + rank; };
-    OctetRow<T> x = octet_row<T, EPI>(p, row_of(q) < rows ? m0 + row_of(q) : p.m, nt, sub);
-    if (splits > 1) cluster_sync_all();
-    bool arrived = false;
-    if (!*abort_flag) {
-        for (; q * splits + rank < rows; q += kThreads / 8) {
-            const uint32_t at = smem_base + min(row_of(q), rows - 1) * (kRowWords * 4) + sub * 16;
-            float4 sum[4];
-            if (splits > 2) sum_over_cluster<4>(at, splits, sum);
-            else sum_over_cluster<2>(at, splits, sum);
-            const int next = q + kThreads / 8;
-            if (splits > 1 && next * splits + rank >= rows) {   // this warp's last trip: its peers' memory is not needed any more
-                asm volatile("barrier.cluster.arrive;\n" ::: "memory");
-                arrived = true;
-            }
-            epilogue_octet<T, EPI>(p, x, sum, nt, sub);
-            if (next * splits + rank < rows) x = octet_row<T, EPI>(p, row_of(next) < rows ? m0 + row_of(next) : p.m, nt, sub);
+    const bool summed = *abort_flag == 0;          // (the same for the whole block)
+    if (splits > 1) {
+        __syncwarp();
+        asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+        if (warp == 2 && lane < splits && lane != rank && summed) {
+            const int n = min(run, rows - lane * run);
+            if (n > 0) push_bulk(recv + rank * run * kSumBytes, smem_base + lane * run * kSumBytes, n * kSumBytes, bar_recv, lane);
         }
+        __syncwarp();
     }
-    if (splits > 1) {                      // no block leaves while a peer still reads its shared memory
-        if (!arrived) asm volatile("barrier.cluster.arrive;\n" ::: "memory");
+    constexpr int kTrip = kThreads / 8;            // four rows per warp and trip
+    int l = warp * 4;
+    auto row_of = [&](int first) { return first + (lane >> 3) < own_rows ? m0 + rank * run + first + (lane >> 3) : p.m; };
+    auto index_of = [&](int first) { return EPI == kQkvPrologue && first < own_rows ? qkv_index(p, row_of(first)) : QkvIndex{}; };
+    QkvIndex at = index_of(l), at_next = index_of(l + kTrip);
+    T weights[16];
+    octet_weights<T, EPI>(p, nt, sub, weights);
+    OctetRow<T> x = octet_row<T, EPI>(p, row_of(l), at, nt, sub);
+    bool ok = summed;
+    if (splits > 1) {
+        if (summed && l < own_rows) ok = mbar_wait_warp(bar_recv, 0, abort_flag, 5);
+        asm volatile("barrier.cluster.arrive;\n" ::: "memory");   // what peers pushed here has landed: they need their copies no more
+    }
+#pragma unroll 1
+    for (; ok && l < own_rows; l += kTrip) {
+        // the next trip's table rows and the positions of the one after it are on their way under this one (128 x 6144, K 4096, QKV: 16.0 -> 15.4 us)
+        OctetRow<T> next{};
+        if (l + kTrip < own_rows) next = octet_row<T, EPI>(p, row_of(l + kTrip), at_next, nt, sub);
+        at_next = index_of(l + 2 * kTrip);
+        const int r_own = min(l + (lane >> 3), own_rows - 1), row = rank * run + r_own;
+        float4 sum[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) sum[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+        for (int r = 0; r < splits; ++r) {
+            const unsigned char* from = smem_raw + (r == rank ? smem_base + row * kSumBytes : recv + (r * run + r_own) * kSumBytes) - smem_u32(smem_raw);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float4 v = *reinterpret_cast<const float4*>(from + (8 * q + (sub ^ (row & 7))) * 16);
+                sum[q].x += v.x; sum[q].y += v.y; sum[q].z += v.z; sum[q].w += v.w;
+            }
+        }
+        epilogue_octet<T, EPI>(p, x, sum, weights, nt, sub);
+        x = next;
+    }
+    if (splits > 1) {                              // no block leaves while a peer still reads what it pushed, or may still push
         asm volatile("barrier.cluster.wait;\n" ::: "memory");
+        if (*abort_flag) settle();
     }
 }
 
 // ---- many rows: persistent pairs of blocks ---------------------------------------------------------------------------------------
 constexpr int kPairStages = 6;
+constexpr int kHidingSteps = 48;                      // steps of 64 along K under which a slow epilogue of the tile before disappears: some 9 us
 constexpr int kPairStageBytes = 2 * kPanelBytes;      // this block's halves of A (128 of 256 rows) and B (128 of 256 columns)
 constexpr int kPairCols = 256;                        // accumulator columns of a tile; two of them fill TMEM
 template <typename T, int EPI>
@@ -654,7 +867,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     __shared__ int s_abort;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t bars = smem_base + kRingBytes;
+    const uint32_t bars = smem_base + kBarOffset;
     auto bar_full = [&](int s) { return bars + 8 * s; };         // used in the leader: both blocks' loads of a stage
     auto bar_empty = [&](int s) { return bars + 64 + 8 * s; };   // in each block: the pair's MMAs have read the stage
     auto bar_acc = [&](int b) { return bars + 128 + 8 * b; };    // in each block: accumulator b is complete
@@ -734,15 +947,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         int n = 0;
         for (int tile = first; tile < tiles; tile += step, ++n) {
             const int b = n & 1;
+            const int64_t row = row0_of(tile) + wq * 32 + lane;
+            const QkvIndex index = EPI == kQkvPrologue ? qkv_index(p, row) : QkvIndex{};   // (a trip to memory before the accumulator is there)
             bool ok = true;
             if (lane == 0) ok = mbar_wait(bar_acc(b), (n >> 1) & 1, abort_flag, 3);
             if (__shfl_sync(0xffffffffu, ok ? 1 : 0, 0) == 0) break;
             tc_fence_after();
-            const int64_t row = row0_of(tile) + wq * 32 + lane;
             const uint32_t t_row = tmem_base + b * kPairCols + (static_cast<uint32_t>(wq * 32) << 16);
             const int nt = col0_of(tile) / kBN + half;
-            unsigned char* stage = smem_raw + (smem_base - smem_u32(smem_raw)) + kStageOffset + (warp - 2) * 4096;
-            if (nt * kBN < p.n) epilogue_row<T, EPI>(p, t_row + half * kBN, row, nt, stage, lane);
+            unsigned char* stage = smem_raw + (smem_base - smem_u32(smem_raw)) + kStageOffset + (warp - 2) * kEpilogueBytes;
+            if (nt * kBN < p.n) epilogue_row<T, EPI, false>(p, t_row + half * kBN, row, index, nt, stage, lane, kb_count >= kHidingSteps && tile + step < tiles);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(in_block(bar_free(b), 0));
@@ -791,28 +1005,24 @@ uint32_t make_idesc(bool bf16, int m, int n) {   // kind::f16: D = F32, A / B = 
 }
 
 // Kernel and shape for a size, by what the slowest SM does: waves of blocks times (steps of 64 along K and a fixed part).  The microseconds
-// are fitted to all nine ways at 16 to 3000 rows x 768 to 12288 columns, K 512 to 4096 (replayed graphs over weights larger than L2).  A step
-// costs 32 or 48 KiB out of L2, the bound here, not the tensor pipe (32 KiB per SM for a pair's 256 x 256 tile).  (0.29 and 0.39 us with MMAs from
-// a diverged lane.)  The fixed part (launch, first
-// loads, epilogue; with the sum over the cluster also in proportion to the tile's rows) comes with every wave of blocks, that of a
-// pair's tile is hidden but for the epilogue.  (One fixed part whatever the waves, measured at K 4096 only, took 256-row blocks for
-// 1500 x 4096, K 512: 21.6 us, pairs 12.3.)  One rule for all epilogues, so that they round the same sums: its constants lie between
-// the plain ones (choice 2 % slower than the fastest way on average, 26 % at most: 64 x 6144, K 512, 6.0 us, one block with all of K 4.8) and those of
-// the slower QKV epilogue (1 %, 21 % at most: 128 x 6144, K 512).
-// A part of K has four steps at least: with fewer, clusters of 4 that nearly fill the chip gain 0.2 us at most (8 x 4096, K 512, 4.4 us,
-// clusters of 2 4.6).
+// are fitted to all ways at 1 to 5000 rows x 768 to 8192 columns, K 512 to 4096, with both epilogues (replayed graphs over weights larger than L2).  A
+// step costs 32 or 48 KiB out of L2, the bound here, not the tensor pipe (32 KiB per SM for a pair's 256 x 256 tile).  The fixed part (launch,
+// first loads, epilogue; with the sum over the cluster also in proportion to the tile's rows) comes with every wave of blocks, that of a
+// pair's tile is hidden but for the epilogue.  One rule for all epilogues, so that they round the same sums: for plain products the choice is 0.7 %
+// slower than the fastest way on average and 22 % at most (128 x 1536, K 1024, 7.2 us, one block with all of K 5.9), with the QKV epilogue 1.3 % and
+// 41 % (48 x 8192, K 512, 9.0 us, clusters of 2 6.4).  A part of K has two steps at least.  Blocks of 256 rows that share K in clusters were never the
+// fastest by more than 2 % once peers' sums were pushed (256 x 4096, K 4096: 17.8 us in clusters of 4, 13.9 as two tiles in clusters of 2).
 struct GemmShape { int mt, splits; };   // mt 1 or 2: gemm_split_kernel; 0: gemm_pair_kernel
 GemmShape choose_gemm(int64_t m, int64_t n, int64_t k) {
     // clusters: what a B200 holds at once (its GPCs have 16 to 20 SMs); rows: per 128 rows of a tile
     struct { int mt, splits, clusters; double step, fixed, rows; } constexpr kWays[] = {
-        {1, 1, 148, 0.220, 3.6, 0.7}, {1, 2, 74, 0.231, 3.3, 2.4}, {1, 4, 33, 0.25, 3.4, 3.2}, {1, 8, 15, 0.30, 2.6, 4.2},
-        {2, 1, 148, 0.347, 3.4, 0.3}, {2, 2, 74, 0.343, 4.9, 2.1}, {2, 4, 33, 0.35, 6.3, 1.4}, {2, 8, 15, 0.40, 5.5, 3.0}};
+        {1, 1, 148, 0.207, 3.0, 0.85}, {1, 2, 74, 0.24, 3.3, 2.0}, {1, 4, 33, 0.288, 3.1, 2.3}, {1, 8, 15, 0.333, 3.0, 2.75}, {2, 1, 148, 0.345, 5.3, 0.25}};
     const int64_t kb = (k + kBK - 1) / kBK, tiles_n = n / kBN, pair_tiles = ((m + 255) / 256) * ((n + 255) / 256);
     GemmShape best{0, 1};
-    double best_time = m > kBM ? static_cast<double>((pair_tiles + 73) / 74) * (static_cast<double>(kb) * 0.316 + 1.6) + 3.8 : 1e30;
+    double best_time = m > kBM ? static_cast<double>((pair_tiles + 73) / 74) * (static_cast<double>(kb) * 0.321 + 2.0) + 5.3 : 1e30;
     for (const auto& w : kWays) {
         const int64_t tile_rows = w.mt * kBM, tiles = (m + tile_rows - 1) / tile_rows * tiles_n;
-        if ((w.mt == 2 && m <= kBM) || (w.splits > 1 && (kb / w.splits < 4 || tiles > w.clusters))) continue;
+        if ((w.mt == 2 && m <= kBM) || (w.splits > 1 && (kb / w.splits < 2 || tiles > w.clusters))) continue;
         const double rows = static_cast<double>(m < tile_rows ? m : tile_rows) / kBM;
         const double time = static_cast<double>((tiles + w.clusters - 1) / w.clusters) *
                             (static_cast<double>((kb + w.splits - 1) / w.splits) * w.step + w.fixed + w.rows * rows);
@@ -850,7 +1060,7 @@ int launch_kernel(void (*kernel)(KArgs...), std::atomic<bool>* attr_done, dim3 g
 
 template <typename T, int EPI>
 int launch(const void* a, const void* b, GemmParams& p, bool bf16, cudaStream_t stream, const char* what) {
-    static std::atomic<bool> done[5][64] = {};
+    static std::atomic<bool> done[4][64] = {};
     CUtensorMap ta, tb;
     const GemmShape g = choose_gemm(p.m, p.n, p.k);
     p.a_rows = g.mt == 1 && p.m < kBM ? static_cast<int>((p.m + 7) / 8 * 8) : kBM;
@@ -866,11 +1076,9 @@ int launch(const void* a, const void* b, GemmParams& p, bool bf16, cudaStream_t 
     }
     p.idesc = make_idesc(bf16, kBM, kBN);
     const dim3 grid(static_cast<unsigned>(p.n / kBN * g.splits), static_cast<unsigned>((p.m + g.mt * kBM - 1) / (g.mt * kBM)));
-    constexpr bool kMayDirect = EPI != kQkvPrologue;
-    const bool direct = kMayDirect && g.splits == 1 && p.m > 32;
-    auto* kernel = g.mt == 1 ? direct ? gemm_split_kernel<T, EPI, 1, kMayDirect> : gemm_split_kernel<T, EPI, 1, false>
-                             : direct ? gemm_split_kernel<T, EPI, 2, kMayDirect> : gemm_split_kernel<T, EPI, 2, false>;
-    return launch_kernel(kernel, done[2 * g.mt - 1 + direct], grid, kThreads, g.splits, stream, what, ta, tb, p, g.splits);
+    const bool direct = g.splits == 1 && p.m > 32;
+    auto* kernel = g.mt == 2 ? gemm_split_kernel<T, EPI, 2, true> : direct ? gemm_split_kernel<T, EPI, 1, true> : gemm_split_kernel<T, EPI, 1, false>;
+    return launch_kernel(kernel, done[g.mt == 2 ? 3 : 1 + direct], grid, kThreads, g.splits, stream, what, ta, tb, p, g.splits);
 }
 
 int check_gemm(const char* what, const void* a, const void* b, int64_t m, int64_t n, int64_t k, int dtype) {

@@ -104,3 +104,47 @@ def test_rows_of_a_warp_that_go_different_ways(rows, hidden):
     assert torch.equal(q, torch.where(pick, turned[0], plain[0]))
     assert torch.equal(k, torch.where(pick, turned[1], plain[1]) * slot[:, None, None])
     assert torch.equal(v, turned[2] * slot[:, None, None])
+
+
+@pytest.mark.parametrize("num_q_heads,num_kv_heads,hidden", [(4, 1, 2048), (8, 2, 512), (24, 4, 1024), (32, 8, 640)])   # clusters of 8, 4, 4 and 2
+@pytest.mark.parametrize("rows", [1, 31, 33, 57, 64, 65, 121, 128, 129, 250])                # runs of rows, with and without the ring's last stage
+def test_sums_pushed_through_a_cluster(num_q_heads, num_kv_heads, hidden, rows):
+    """Plain products against fp32, and with norm, rotation and store against the oracle on that product; without norm weights and slots as well."""
+    bf, d, max_pos, heads = torch.bfloat16, 128, 300, num_q_heads + 2 * num_kv_heads
+    gen = torch.Generator(device="cuda").manual_seed(heads * rows)
+    x = torch.randn((rows, hidden), generator=gen, device="cuda").to(bf)
+    w = (torch.randn((heads * d, hidden), generator=gen, device="cuda") / hidden ** 0.5).to(bf)
+    qkv = torch.full((rows, heads * d), float("nan"), dtype=bf, device="cuda")
+    nvk().linear(x, w, qkv)
+    want = x.float() @ w.float().t()
+    err = (qkv.float() - want).abs()                                # half a unit of the result, and the order of the sums
+    assert bool((err <= want.abs().clamp_min(0.05) * 2.0 ** -8 + 1e-3).all()), float(err.max())
+    cache_rows = rows + 10
+    pw = workloads().make_prologue_workload(rows, num_q_heads, num_kv_heads, d, cache_rows, max_pos, seed=rows)
+    pw["slot_mapping"][rows // 2] = -1
+    pw["positions"][rows // 3] = max_pos
+    table = oracle.build_cos_sin_cache(max_pos, d, pw["rope_base"])
+    for normed in (True, False):
+        qw, kw = (pw["q_norm_weight"], pw["k_norm_weight"]) if normed else (None, None)
+        slots = pw["slot_mapping"] if normed else np.arange(rows, dtype=np.int32)
+        kc = torch.zeros(cache_rows, num_kv_heads, d, dtype=bf, device="cuda")
+        vc, q_out = torch.zeros_like(kc), torch.full((rows, num_q_heads, d), float("nan"), dtype=bf, device="cuda")
+        nvk().qkv_linear_norm_rope_store(x, w, to_dev(pw["positions"]), to_dev(qw, bf) if normed else None, to_dev(kw, bf) if normed else None, pw["eps"],
+                                         to_dev(table), to_dev(slots) if normed else None, kc, vc, num_q_heads, num_kv_heads, d, q_out)
+        torch.cuda.synchronize()
+        assert nvk().gemm_status() == 0
+        if normed:
+            kc_ref, vc_ref = np.zeros((cache_rows, num_kv_heads, d), np.float32), np.zeros((cache_rows, num_kv_heads, d), np.float32)
+            q_ref = oracle.fused_split_norm_rope_store(to_np(qkv), pw["positions"], qw, kw, pw["eps"], table, slots, kc_ref, vc_ref, num_q_heads, num_kv_heads, d)
+        else:
+            parts = to_np(qkv).reshape(rows, heads, d)
+            inside = (pw["positions"] >= 0) & (pw["positions"] < max_pos)
+            t = table[np.where(inside, pw["positions"], 0)][:, None]
+            lo, hi, cs, sn = parts[..., :64], parts[..., 64:], t[..., :64], t[..., 64:]
+            turned = np.where(inside[:, None, None], np.concatenate([lo * cs - hi * sn, hi * cs + lo * sn], -1), parts)
+            q_ref = turned[:, :num_q_heads]
+            kc_ref, vc_ref = np.zeros((cache_rows, num_kv_heads, d), np.float32), np.zeros((cache_rows, num_kv_heads, d), np.float32)
+            kc_ref[:rows], vc_ref[:rows] = turned[:, num_q_heads:num_q_heads + num_kv_heads], parts[:, num_q_heads + num_kv_heads:]
+        assert np.array_equal(to_np(vc), vc_ref)
+        for got, ref in ((to_np(q_out), q_ref), (to_np(kc), kc_ref)):
+            assert (np.abs(got - ref) <= np.maximum(np.abs(ref), 1e-3) * 2.0 ** -7 + 2.0 ** -9 * (not normed)).all()   # (cancelling terms of a rotation, 16-bit inputs)
