@@ -312,8 +312,9 @@ int nvk_prefill_attention_varlen(const void* query, const void* key, const void*
  * part and the HBM-bound decode part run one after the other and every SM idles at the boundary.  Here the persistent
  * blocks of the prefill kernel also take the decode kernel's (KV head, split, sequence) items from a second queue:
  * `prefill_blocks` of them start with the prefill items, the rest with the decode items, every block finishes with
- * what is left of the other kind.  (With a scale that is not positive the two parts are launches of their own.)  Results are those of nvk_prefill_attention_varlen on the prefill rows and of
- * nvk_decode_attention_paged (same split policy, so the same bits) on the decode rows.
+ * what is left of the other kind.  (With a scale that is not positive the two parts are launches of their own; so they are
+ * where the prefill part is small by the sizes given, as two kernels that run side by side.)  Results are those of
+ * nvk_prefill_attention_varlen on the prefill rows and of nvk_decode_attention_paged on the decode rows, bit for bit.
  *   prefill part   p_query / p_output [total_q, Hq, D]; keys dense (p_key, p_value [total_k, Hkv, D], p_block_tables
  *                  NULL) or paged through p_block_tables [num_seqs, p_max_blocks]; cu_seqlens_* as in
  *                  nvk_prefill_attention_varlen

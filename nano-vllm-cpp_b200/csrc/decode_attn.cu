@@ -92,11 +92,13 @@ __device__ __forceinline__ void st_cluster2(uint32_t addr, uint32_t rank, float 
 template <class F, typename T>
 __global__ void __launch_bounds__(kGroupThreads, F::kGroups) decode_split_kernel(const __grid_constant__ DecodeParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
-    pdl_wait_then_release();
+    if (p.beside) pdl_start_beside();
+    else pdl_wait_then_release();
     const int rank = p.chunk_major ? blockIdx.y : blockIdx.z, split = p.chunk_major ? blockIdx.z : blockIdx.y;
     const int b = p.longest_first ? sequence_of_rank(p, rank, *reinterpret_cast<SortScratch*>(smem)) : rank;
     if (p.longest_first) __syncthreads();   // (the ring takes the scratch's place)
     run_split<F, T>(p, b, blockIdx.x, split, *reinterpret_cast<GroupSmem<F>*>(smem), threadIdx.x, 1);
+    if (p.beside) pdl_wait_beside();
 }
 
 // HG > 0: one warp per (sequence, KV head) and HG of its heads, in blocks of kMergeBlockWarps warps, small enough to be resident
@@ -149,7 +151,8 @@ __global__ void __launch_bounds__(kGroupThreads, F::kGroups) decode_cluster_kern
     __shared__ float4 s_o[kMaxGroup * kHeadDim / 4];           // [block of the cluster][head][quad of this block]
     __shared__ float2 s_ml[kMaxCluster * kMaxGroup];           // [block of the cluster][head]
     asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");   // (waited for before the first remote store: every block has started)
-    pdl_wait_then_release();
+    if (p.beside) pdl_start_beside();
+    else pdl_wait_then_release();
     const int rank = static_cast<int>(blockIdx.x) & (p.num_splits - 1), pair = static_cast<int>(blockIdx.x) >> p.split_shift;
     const int b = static_cast<int>(p.by_kv_heads.div(pair)), kvh = pair - b * p.num_kv_heads;
     const int tid = threadIdx.x, lane = tid & 31;
@@ -194,6 +197,7 @@ __global__ void __launch_bounds__(kGroupThreads, F::kGroups) decode_cluster_kern
         if (ctx == 0) acc = nothing_merged();
         write_merged<T>(out + h * kHeadDim, acc, quad);
     }
+    if (p.beside) pdl_wait_beside();
 }
 
 // ---- host side -----------------------------------------------------------------------------------------------------------
@@ -298,6 +302,7 @@ int decode_plan(const DecodeArgs& a, int groups, dec::DecodeParams* out, int* cl
     p.num_heads = a.num_heads; p.num_kv_heads = a.num_kv_heads; p.group = a.num_heads / a.num_kv_heads;
     p.block_size = a.block_size;
     p.scale_log2 = a.scale * kLog2e;
+    p.beside = a.beside ? 1 : 0;
     if (a.batch * a.num_heads * kMaxCluster >= (1LL << 31) || a.max_blocks * a.block_size >= (1LL << 31) - kTileTokens * kMaxCluster)
         return fail(NVK_ERR_UNSUPPORTED, "decode attention: batch or block table too large");
     const Splits s = choose_splits(a.batch, a.num_heads, a.num_kv_heads, a.max_blocks, a.block_size, groups, a.workspace != nullptr);

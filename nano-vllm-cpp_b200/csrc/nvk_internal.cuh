@@ -109,6 +109,7 @@ struct DecodeArgs {
     int dtype;
     void* workspace; size_t workspace_bytes;
     cudaStream_t stream;
+    bool beside = false;         // runs beside the kernel launched just before it on the stream, see pdl_wait_beside
 };
 struct DecodeInt8Args {          // 8-bit caches (int8, or e4m3 when fp8 is set) with one fp16 scale per (cache row, KV head)
     DecodeArgs base;
@@ -173,6 +174,8 @@ int launch_store_fp8(const void* key, const void* value, void* k_cache, void* v_
                      int dtype, cudaStream_t stream);
 bool prefill_mma_supported(const PrefillArgs& a);
 int launch_prefill_mma(const PrefillArgs& a);
+double prefill_tiles_save(const PrefillArgs& a);   // microseconds that launch_prefill_mma saves beside launch_prefill_tc, by sizes that the host knows
+int prefill_tile_status(cudaStream_t stream, int* status);
 // tcgen05 / TMEM / TMA path (F16/BF16, head_dim 128, paged block_size % 128 == 0).
 bool prefill_tc_supported(const PrefillArgs& a);
 int launch_prefill_tc(const PrefillArgs& a);
@@ -260,6 +263,12 @@ __device__ __forceinline__ void pdl_wait_then_release() {
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 }
+
+// For a kernel that needs nothing of the one launched just before it, which for its part waited (pdl_wait_then_release) before it let this one start:
+// all that came earlier has completed, and the two run side by side.  It waits at its end instead, in every block, so that whatever follows it in the
+// stream and waits for it has waited for both.
+__device__ __forceinline__ void pdl_start_beside() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait_beside() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
 // <<<grid, block, smem, stream>>> with that attribute.
 template <typename... KArgs, typename... Args>

@@ -1529,5 +1529,5 @@ extern "C" int nvk_prefill_status(void* stream, int* status) {
     }
     if (e != cudaSuccess) return fail(NVK_ERR_CUDA, "prefill status: %s", cudaGetErrorString(e));
     *status = word;
-    return NVK_OK;
+    return word != 0 ? NVK_OK : prefill_tile_status(st, status);
 }

@@ -176,3 +176,41 @@ def test_mixed_step_refuses_what_it_cannot_run():
     with pytest.raises(ValueError):                                    # fp32 takes the general paths: two calls
         lib.attention_mixed_step(q, cu, q, q, cu, None, q.clone(), q[:1], torch.ones(1, device="cuda", dtype=torch.int32),
                                  torch.zeros(1, 1, device="cuda", dtype=torch.int32), q[:1].clone(), kc, kc, 2, 128, 256, 0.1, ws, 0)
+
+
+@pytest.mark.parametrize("batch,longest", [(4, 300), (40, 3000)])   # decode in clusters of blocks, and in chunks with a merge
+def test_a_small_prefill_beside_decode_is_done_when_the_next_kernel_starts(batch, longest):
+    """The two halves run side by side; a kernel queued right behind them sees both results, every time, eager and replayed."""
+    wl, lib, bf = workloads(), nvk(), torch.bfloat16
+    p = wl.make_prefill_workload([300], [0], 4, 1, 128, 256, seed=9, paged=True)
+    ctx = np.linspace(1, longest, batch).astype(np.int32)
+    d = wl.make_decode_workload(batch, 4, 1, 128, 256, 0, 0, seed=10, context_lens=ctx)
+    shift = d["k_cache"].shape[0]
+    kc, vc = (to_dev(np.concatenate([d[n], p[n]]), bf) for n in ("k_cache", "v_cache"))
+    pq, dq, cu_q, cu_k, pt, cl, dt = (to_dev(p["q"], bf), to_dev(d["q"], bf), to_dev(p["cu_q"]), to_dev(p["cu_k"]),
+                                      to_dev((p["block_tables"] + shift).astype(np.int32)), to_dev(ctx), to_dev(d["block_tables"]))
+    ws = torch.empty(max(16, lib.decode_attention_workspace_bytes(batch, 4, 1, 128, dt.shape[1], 256)), dtype=torch.uint8, device="cuda")
+    p_ref, d_ref = torch.empty_like(pq), torch.empty_like(dq)
+    lib.launch_prefill_attention_paged(pq, cu_q, kc, vc, cu_k, pt, 1, 128, 256, p["scale"], p_ref)
+    lib.launch_decode_attention_paged(dq, kc, vc, cl, dt, 1, 128, 256, d["scale"], d_ref, ws)
+    p_out, d_out = torch.empty_like(pq), torch.empty_like(dq)
+    right = torch.ones((), dtype=torch.bool, device="cuda")
+
+    def step():
+        p_out.fill_(float("nan"))
+        d_out.fill_(float("nan"))
+        lib.attention_mixed_step(pq, cu_q, None, None, cu_k, pt, p_out, dq, cl, dt, d_out, kc, vc, 1, 128, 256, p["scale"], ws)
+        right.logical_and_((p_out == p_ref).all())
+        right.logical_and_((d_out == d_ref).all())
+
+    for _ in range(100):
+        step()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        step()
+        step()
+    for _ in range(50):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert lib.prefill_status() == 0 and bool(right)

@@ -107,3 +107,56 @@ def test_a_mixed_step_takes_scales_that_are_not_positive():
     lib.attention_mixed_step(pq, cu_q, None, None, cu_k, pt, p_out, dq, ctx, pt, d_out, kc, vc, hkv, 128, 256, -0.05, ws)
     torch.cuda.synchronize()
     assert torch.equal(p_out, want_p) and torch.equal(d_out, want_d)
+
+
+@pytest.mark.parametrize("index", ["i32", "i64"])
+@pytest.mark.parametrize("hq,hkv,bs,q_lens,prefix,paged", [
+    (8, 1, 256, [8], [256], True), (8, 2, 256, [9, 1], [512, 768], True), (4, 1, 128, [670], [0], True),        # clusters of 8, 8 and 4 (2 rows x 8 heads ...)
+    (32, 8, 256, [77], [512], True), (16, 8, 256, [33], [256], True), (32, 8, 256, [100], [0], True),         # of 4, 8 and single blocks
+    (32, 8, 256, [1] * 40 + [17, 5], [0] * 42, True), (4, 2, 256, [3, 0, 8, 20] * 9, [0] * 36, False),       # more than 32 sequences, empty ones among them
+    (8, 2, 64, [70, 5], [64 * 40, 64 * 37], True), (4, 1, 64, [20], [64 * 70], True),                       # more block ids than lanes
+    (16, 8, 256, [200], [0], False), (6, 3, 256, [65, 64, 63], [0, 256, 0], True),
+])
+def test_small_steps_in_tiles_of_64_rows(index, hq, hkv, bs, q_lens, prefix, paged):
+    w = workloads().make_prefill_workload(q_lens, prefix, hq, hkv, 128, bs, seed=hq + len(q_lens), paged=paged)
+    lib, bf = nvk(), torch.bfloat16
+    it = torch.int32 if index == "i32" else torch.int64
+    q, cu_q, cu_k = to_dev(w["q"], bf), to_dev(w["cu_q"]).to(it), to_dev(w["cu_k"]).to(it)
+    if paged:
+        kc, vc = to_dev(w["k_cache"], bf), to_dev(w["v_cache"], bf)
+        for i, (a, b) in enumerate(zip(q_lens, prefix)):              # what lies behind a sequence's last key does not matter
+            n = a + b
+            if n % bs:
+                last = int(w["block_tables"][i, n // bs])
+                kc[last, n % bs:], vc[last, n % bs:] = float("nan"), float("inf")
+        tables = to_dev(w["block_tables"]).to(it)
+        run = lambda out, scale: lib.launch_prefill_attention_paged(q, cu_q, kc, vc, cu_k, tables, hkv, 128, bs, scale, out)
+        want = lambda scale: oracle.prefill_attention_paged(w["q"], w["k_cache"], w["v_cache"], w["cu_q"], w["cu_k"], w["block_tables"], hkv, 128, bs, scale)
+    else:
+        k, v = to_dev(w["k"], bf), to_dev(w["v"], bf)
+        run = lambda out, scale: lib.launch_prefill_attention_dense(q, cu_q, k, v, cu_k, hkv, 128, scale, out)
+        want = lambda scale: oracle.prefill_attention_dense(w["q"], w["k"], w["v"], w["cu_q"], w["cu_k"], hkv, 128, scale)
+    for scale in (w["scale"], -w["scale"]):
+        out = torch.full_like(q, float("nan"))
+        run(out, scale)
+        torch.cuda.synchronize()
+        assert lib.prefill_status() == 0
+        assert_attention_close(to_np(out), want(scale))
+
+
+def test_small_steps_keep_infinities_in_their_columns_and_rows_without_keys_at_zero():
+    """An infinity in V of the first key: infinite where it is seen, in whatever block's part; rows that see no key give zeros."""
+    w = workloads().make_prefill_workload([40], [512], 32, 8, 128, 256, seed=1, paged=True)
+    lib, bf = nvk(), torch.bfloat16
+    q, kc, vc = to_dev(w["q"], bf), to_dev(w["k_cache"], bf), to_dev(w["v_cache"], bf)
+    vc[int(w["block_tables"][0, 0]), 0, :, 7] = float("inf")
+    out = torch.full_like(q, float("nan"))
+    lib.launch_prefill_attention_paged(q, to_dev(w["cu_q"]), kc, vc, to_dev(w["cu_k"]), to_dev(w["block_tables"]), 8, 128, 256, w["scale"], out)
+    ref = oracle.prefill_attention_paged(w["q"], w["k_cache"], w["v_cache"], w["cu_q"], w["cu_k"], w["block_tables"], 8, 128, 256, w["scale"])
+    assert bool((out[..., 7] == float("inf")).all())
+    keep = [i for i in range(128) if i != 7]
+    assert_attention_close(to_np(out[..., keep]), ref[..., keep])
+    cu_k = torch.tensor([0, 30], dtype=torch.int32, device="cuda")     # 40 rows, 30 keys: the first ten see none
+    lib.launch_prefill_attention_paged(q, to_dev(w["cu_q"]), kc, to_dev(w["v_cache"], bf), cu_k, to_dev(w["block_tables"]), 8, 128, 256, w["scale"], out)
+    torch.cuda.synchronize()
+    assert bool((out[:10] == 0).all()) and bool((out[10:].float().abs().amax((1, 2)) > 0).all())
