@@ -141,14 +141,17 @@ __global__ void __launch_bounds__((HG > 0 ? kMergeBlockWarps : kMergeWarps) * 32
     }
 }
 
-// A block pushes what it has of the result into the shared memory of the block that finishes it: of 32 quads of a head, block r of the cluster takes
-// 32 / size from r * 32 / size on.  After one cluster barrier everything there is local, and no block has to wait for its peers to have
+// A block pushes what it has of the result into the shared memory of the block that finishes it: of 32 quads of a head, block r of n
+// takes 32 / n from r * 32 / n on.  After one cluster barrier everything there is local, and no block has to wait for its peers to have
 // read.  1 sequence of 300 keys, 32 / 8 heads, with its prologue: 7.2 -> 5.85 us a pass with the block ids fetched along with the context and one
 // barrier in a block's merge; from a block's last tile to its end it had been 2.5 us of 4.3.
+// Equal ranges (per_seq): all blocks of the cluster have a part, if an empty one.  Halves of a table row: where a context ends in the first, that block
+// writes the result and the other leaves.
+constexpr int kPartQuads = kMaxGroup * kHeadDim / 4;   // n x 8 heads x 32 / n, for the cluster sizes there are: 1, 2, 4, 8
 template <class F, typename T>
 __global__ void __launch_bounds__(kGroupThreads, F::kGroups) decode_cluster_kernel(const __grid_constant__ DecodeParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ float4 s_o[kMaxGroup * kHeadDim / 4];           // [block of the cluster][head][quad of this block]
+    __shared__ float4 s_o[kPartQuads];                         // [block of the cluster][head][quad of this block]
     __shared__ float2 s_ml[kMaxCluster * kMaxGroup];           // [block of the cluster][head]
     asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");   // (waited for before the first remote store: every block has started)
     if (p.beside) pdl_start_beside();
@@ -156,46 +159,59 @@ __global__ void __launch_bounds__(kGroupThreads, F::kGroups) decode_cluster_kern
     const int rank = static_cast<int>(blockIdx.x) & (p.num_splits - 1), pair = static_cast<int>(blockIdx.x) >> p.split_shift;
     const int b = static_cast<int>(p.by_kv_heads.div(pair)), kvh = pair - b * p.num_kv_heads;
     const int tid = threadIdx.x, lane = tid & 31;
+    const int id_base = p.per_seq ? 0 : static_cast<int>(p.by_block.div(rank * p.chunk_tokens));
     const IndexArray::Raw raw_ctx = p.context_lens.raw(b);
-    IndexArray::Raw raw_ids = load_ids(p, b, 0, lane);
+    IndexArray::Raw raw_ids = load_ids(p, b, id_base, lane);
     const int ctx = clamped_context(p, raw_ctx), len = range_len(p, ctx);
     const int t0 = rank * len, t1 = min(ctx, t0 + len);
-    const int quad_shift = 5 - p.split_shift, quads = 1 << quad_shift;          // quads of a head per block
-    bool waited = false;
-    auto push = [&](int h, int quad, const float4& o, float m, float l) {
-        if (!waited) asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory");
-        waited = true;
-        const uint32_t to = static_cast<uint32_t>(quad >> quad_shift);
-        const int mine = quad & (quads - 1);
-        st_cluster4(smem_u32(s_o + ((rank * p.group + h) << quad_shift) + mine), to, o);
-        if (mine == 0) st_cluster2(smem_u32(s_ml + rank * p.group + h), to, m, l);
-    };
-    if (t0 < t1) {
-        attend_range<F>(p, b, kvh, t0, t1, raw_ids, 0, *reinterpret_cast<GroupSmem<F>*>(smem), tid, 1, push);
-    } else {
-        for (int h = tid >> 5; h < p.group; h += kGroupWarps) push(h, lane, make_float4(0.f, 0.f, 0.f, 0.f), -INFINITY, 0.0f);
-    }
-    if (!waited) asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory");   // (a warp without a head)
-    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory");
-    T* out = static_cast<T*>(p.out) + static_cast<int64_t>(pair) * p.group * kHeadDim;
-    for (int i = tid; i < p.group << quad_shift; i += kGroupThreads) {
-        const int h = i >> quad_shift, quad = (rank << quad_shift) + (i & (quads - 1));
-        Merged acc = nothing_merged();
-        for (int r0 = 0; r0 < p.num_splits; r0 += 4) {
-            float4 v[4];
-            float2 ml[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const bool there = r0 + u < p.num_splits;
-                const int r = there ? r0 + u : 0;
-                v[u] = s_o[(r * p.group << quad_shift) + i];
-                ml[u] = s_ml[r * p.group + h];
-                if (!there) { v[u] = make_float4(0.f, 0.f, 0.f, 0.f); ml[u] = make_float2(-INFINITY, 0.0f); }
+    T* out = static_cast<T*>(p.out) + (static_cast<int64_t>(b) * p.num_kv_heads + kvh) * p.group * kHeadDim;
+    const int n = p.per_seq ? p.num_splits : ctx > len ? 2 : 1;                // blocks with a part (chunks: two)
+    const int quad_shift = n == 1 ? 5 : 5 - p.split_shift, quads = 1 << quad_shift;   // quads of a head that a block finishes
+    if (rank < n) {
+        bool waited = false;
+        auto wait_started = [&]() {
+            if (!waited) asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory");
+            waited = true;
+        };
+        auto push = [&](int h, int quad, const float4& o, float m, float l) {
+            if (n == 1) {
+                write_quad(out + h * kHeadDim + 4 * quad, scaled(o, 1.0f / l));   // (rounded as write_merged does)
+                return;
             }
-            acc.add(v, ml);
+            wait_started();
+            const uint32_t to = static_cast<uint32_t>(quad >> quad_shift);
+            const int mine = quad & (quads - 1);
+            st_cluster4(smem_u32(s_o + ((rank * p.group + h) << quad_shift) + mine), to, o);
+            if (mine == 0) st_cluster2(smem_u32(s_ml + rank * p.group + h), to, m, l);
+        };
+        if (t0 < t1) {
+            attend_range<F>(p, b, kvh, t0, t1, raw_ids, id_base, *reinterpret_cast<GroupSmem<F>*>(smem), tid, 1, push);
+        } else {                                                                  // (alone: an empty context, zeros)
+            for (int h = tid >> 5; h < p.group; h += kGroupWarps) push(h, lane, make_float4(0.f, 0.f, 0.f, 0.f), -INFINITY, n > 1 ? 0.0f : 1.0f);
         }
-        if (ctx == 0) acc = nothing_merged();
-        write_merged<T>(out + h * kHeadDim, acc, quad);
+        if (n > 1) {
+            wait_started();                                                       // (a warp without a head)
+            asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory");
+            for (int i = tid; i < p.group << quad_shift; i += kGroupThreads) {
+                const int h = i >> quad_shift, quad = (rank << quad_shift) + (i & (quads - 1));
+                Merged acc = nothing_merged();
+                for (int r0 = 0; r0 < n; r0 += 4) {
+                    float4 v[4];
+                    float2 ml[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const bool there = r0 + u < n;
+                        const int r = there ? r0 + u : 0;
+                        v[u] = s_o[(r * p.group << quad_shift) + i];
+                        ml[u] = s_ml[r * p.group + h];
+                        if (!there) { v[u] = make_float4(0.f, 0.f, 0.f, 0.f); ml[u] = make_float2(-INFINITY, 0.0f); }
+                    }
+                    acc.add(v, ml);
+                }
+                if (ctx == 0) acc = nothing_merged();
+                write_merged<T>(out + h * kHeadDim, acc, quad);
+            }
+        }
     }
     if (p.beside) pdl_wait_beside();
 }
@@ -208,8 +224,9 @@ __global__ void __launch_bounds__(kGroupThreads, F::kGroups) decode_cluster_kern
 // 8, 300 keys, 32 -> 34 pairs 5.8 -> 9.4 (in one block each 5.7).  Clusters of 2 gain nothing on whole contexts in one block each (80 pairs of
 // 300 / 1024 keys 8.5 / 12.2 us, 6.6 / 11.8), nor do clusters of 4 in tables of up to 512 keys (64 pairs of 300 / 512 keys 7.6 / 8.7, 6.4 / 7.8).
 // Without a workspace there is nothing else, and any cluster that fits is taken.
+struct ClusterWay { int size, resident[2]; };
+constexpr ClusterWay kWays[] = {{8, {33, 48}}, {4, {71, 104}}, {2, {148, 222}}};
 int cluster_size(int64_t batch, int num_kv_heads, int64_t max_blocks, int block_size, int groups, bool have_workspace) {
-    struct { int size, resident[2]; } constexpr kWays[] = {{8, {33, 48}}, {4, {71, 104}}, {2, {148, 222}}};
     const int64_t pairs = batch * num_kv_heads, max_tokens = max_blocks * block_size;
     for (const auto& w : kWays) {
         if (pairs > w.resident[groups == 3]) continue;
@@ -224,25 +241,39 @@ bool just_past_a_wave(int64_t pairs, int groups) {
     return pairs > kSmCount * groups && (groups == 2 ? 4 * pairs < 5 * kSmCount * groups : 3 * pairs < 4 * kSmCount * groups);
 }
 
-// Chunk length in keys (whole cache blocks), from the number of (sequence, KV head) pairs and the table's width; us a call below.
+// Halves of a table row, merged in a cluster of two blocks: where both halves of all contexts find a place at once (a cluster of more than two, or single
+// blocks and a second kernel, were slower on average over contexts that are all as long as the table, down to half of it and down to a twentieth).
+// 16-bit caches, 110 pairs of 0.05 / 0.5 / 1.0 to 2048 keys: 18.2 / 20.9 / 24.4 us a pass, in chunks of 512 19.8 / 26.5 / 29.1; 128 of 4096 30.8 / 37.8 / 47.1,
+// 35.4 / 43.4 / 51.8; 144 of 8192 55.6 / 74.0 / 95.0, 61.8 / 77.1 / 97.9; at 16384 keys nothing is left of it, and few pairs of spread contexts lose (96 of 8192
+// 46 / 52 / 64, 42 / 58 / 74).  8-bit ones: 128 pairs of 2048 17.3 / 18.1 / 18.5, 17.7 / 19.7 / 24.6; 200 of 1536 18.9 / 19.6 / 20.3, 18.9 / 24.6 / 26.4; but 148
+// of 2048 21.3 / 22.3 / 22.7, 18.7 / 24.2 / 26.1, and up to 768 keys whole contexts are as quick.  Fewer pairs than clusters of
+// four hold take those, or more chunks.
+bool halves(int64_t pairs, int64_t max_tokens, int groups) {
+    if (pairs <= kWays[1].resident[groups == 3] || 2 * pairs > static_cast<int64_t>(kSmCount) * groups) return false;
+    return groups == 2 ? max_tokens > 512 && max_tokens <= (pairs < 110 ? 4096 : 8192) : max_tokens > 768 && max_tokens <= (pairs > 130 ? 1536 : 2048);
+}
+
+// Chunk length in keys (whole cache blocks), from the number of (sequence, KV head) pairs and the table's width; us a pass below, for contexts of
+// 0.05 / 0.5 / 1.0 to all of the table.
 // Whole contexts: no merge, no second launch.
-//   * Tables of up to 1024 keys: 176 pairs of 1024 keys 19.3, as two chunks 23.7; 264 24.6, 29.1; 432 int8 ones 24.3, 30.5.  But 8-bit
-//     caches with 1.5 to 2 pairs per SM, 264 int8 ones of 1024 keys / of 100 to 1024: 22.3 / 19.6, in two chunks 22.9 / 17.6.
-//   * Tables of up to 4096 keys with a pair for every resident group: 37 sequences of 100 to 2048 keys, 8 KV heads, 2 of 37; but not just past
-//     a wave: 304 / 352 pairs of 4096 keys 116.8 / 123.7, in chunks of 2048 106.1 / 113.5; 560 int8 ones 117.4, 105.1 (384 16-bit pairs
-//     126.2, 121.9, but of 97 keys in 2560-key tables 12.3, 13.4; 448 137.0, 145.8).
-// Chunks of 2048 otherwise, halved down to 256 while they leave resident groups without a block.
-//   * A table that 2048 keys cover is cut only below 1.5 (8-bit: 2.5) pairs per SM: 264 pairs of 2048 keys 44.7 whole, 48.5 cut; 432 int8 ones
-//     43.8, 47.5; but 328 int8 ones of 100 to 2048 keys 35.1, 28.7.  What is cut is cut no finer than it takes to have 1.5 blocks per SM
-//     (8-bit: 2.25 of 512 keys): 72 pairs of 2048 keys 4 parts 18.2, 8 21.4; 144 2 parts 29.8, 4 32.2; 106 e4m3 ones 4 parts 17.8, 8 22.6.
+//   * Tables of up to 1024 keys: 176 pairs of 1024 keys 19.3 a call, as two chunks 23.7; 264 24.6, 29.1; 432 int8 ones 24.3, 30.5.
+//   * Tables of up to 4096 keys (3072 below 180 pairs) where the halves above have no room: 184 pairs of 2048 keys 25.0 / 29.6 / 34.2, in chunks of 1024 25.7 / 34.4 / 42.7; 264 of
+//     4096 52.7 / 68.7 / 85.3, chunks of 2048 58.6 / 74.7 / 90.7.  But not just past a wave: 304 / 352 pairs, all of 4096 keys, 116.8 / 123.7 a call, in chunks
+//     of 2048 106.1 / 113.5.  8-bit caches up to 1536 keys, 2048 up to 266 pairs (224: 24.5 / 25.5 / 27.2, 25.0 / 26.6 / 34.9; 272 int8 ones 31.4 / 34.5 / 38.7,
+//     28.3 / 35.6 / 37.2), 4096 with a pair for every resident group.
+// Chunks otherwise, of 2048 or, with few pairs and up to 8192 keys, of 1024 (224 pairs of 6144 keys 64.1 / 86.4 / 111.1, 69.7 / 88.2 / 114.5 in chunks of 2048; 8-bit
+// 55.0 / 70.6 / 87.4 for 8192, 60.4 / 73.5 / 89.2), halved down to 256 while they leave resident groups without a block.
+//   * What a table of 2048 keys is cut into is cut no finer than it takes to have 1.5 blocks per SM (8-bit: 2.25 of 512 keys).
 //   * Longer ones need every place filled, since contexts are often shorter than the table (64 pairs of 1000 keys, 4096-key tables: 512-key
 //     chunks 12.0, 1024-key ones 14.9), but 512 keys are not cut for the last few (36 pairs of 4096 keys 19.0, as chunks of 256 21.0).
 // (Whole contexts of 8192-key tables, 256 sequences: 694 us a pass, 689 with chunks.)
 int chunk_tokens(int64_t batch, int num_kv_heads, int64_t max_blocks, int block_size, int groups) {
     const int64_t max_tokens = max_blocks * block_size, pairs = batch * num_kv_heads, resident = static_cast<int64_t>(kSmCount) * groups;
-    if (max_tokens <= 1024 && (groups == 2 || 2 * pairs <= 3 * kSmCount || pairs >= 2 * kSmCount)) return static_cast<int>(max_tokens);
+    if (max_tokens <= 1024) return static_cast<int>(max_tokens);
+    const int64_t whole = groups == 2 ? (pairs < 180 ? 3072 : just_past_a_wave(pairs, groups) ? 2048 : 4096) : 5 * pairs <= 3 * resident ? 2048 : 1536;
+    if (2 * pairs > resident && max_tokens <= whole) return static_cast<int>(max_tokens);
     if (max_tokens <= 4096 && pairs >= resident && !just_past_a_wave(pairs, groups)) return static_cast<int>(max_tokens);
-    int64_t chunk = 2048;
+    int64_t chunk = max_tokens <= 8192 && (groups == 2 ? max_tokens > 4096 && pairs < 2 * resident : 5 * pairs < 4 * resident) ? 1024 : 2048;
     for (; chunk > 256; chunk >>= 1) {
         const int64_t parts = (max_tokens + chunk - 1) / chunk;
         const double blocks_per_sm = groups == 2 ? (max_tokens <= 2048 ? 1.5 : chunk <= 512 ? 1.8 : 2.0)
@@ -269,7 +300,7 @@ size_t chunk_scratch_bytes(int64_t batch, int num_heads, int num_kv_heads, int h
     return (rows * sizeof(float) + 15) / 16 * 16 + rows * static_cast<size_t>(head_dim) * sizeof(float);
 }
 
-struct Splits { int cluster, chunk, count; };
+struct Splits { int cluster, chunk, count; };   // cluster size, 0: single blocks; chunk length, 0: equal ranges; ranges of a table row
 size_t part_bytes(size_t parts, int group) { return parts * group * (kHeadDim * sizeof(float) + sizeof(float2)); }
 size_t part_count(const Splits& s, int64_t batch, int num_kv_heads) {   // (the cluster kernel itself needs none: the mixed step does)
     return s.count > 1 ? static_cast<size_t>(batch) * num_kv_heads * s.count : 0;
@@ -278,6 +309,11 @@ Splits choose_splits(int64_t batch, int num_heads, int num_kv_heads, int64_t max
     Splits s{cluster_size(batch, num_kv_heads, max_blocks, block_size, groups, have_workspace), 0, 0};
     if (s.cluster > 0) { s.count = s.cluster; return s; }
     const int64_t max_tokens = max_blocks * block_size;
+    if (max_blocks > 1 && halves(batch * num_kv_heads, max_tokens, groups)) {
+        s.chunk = static_cast<int>((max_blocks + 1) / 2 * block_size);
+        s.cluster = s.count = 2;
+        return s;
+    }
     s.chunk = chunk_tokens(batch, num_kv_heads, max_blocks, block_size, groups);
     s.count = static_cast<int>((max_tokens + s.chunk - 1) / s.chunk);
     // A row of partial results takes 520 bytes, 516 in earlier versions: what filled the array of nvk_decode_attention_paged_static almost
@@ -307,15 +343,15 @@ int decode_plan(const DecodeArgs& a, int groups, dec::DecodeParams* out, int* cl
         return fail(NVK_ERR_UNSUPPORTED, "decode attention: batch or block table too large");
     const Splits s = choose_splits(a.batch, a.num_heads, a.num_kv_heads, a.max_blocks, a.block_size, groups, a.workspace != nullptr);
     *cluster = s.cluster;
-    p.per_seq = s.cluster > 0 ? 1 : 0;
-    while (p.per_seq && (1 << p.split_shift) < s.cluster) ++p.split_shift;
+    p.per_seq = s.chunk == 0 ? 1 : 0;
+    while ((1 << p.split_shift) < s.cluster) ++p.split_shift;
     p.by_block = FastDiv(static_cast<uint32_t>(a.block_size));
     p.by_kv_heads = FastDiv(static_cast<uint32_t>(a.num_kv_heads));
     p.chunk_tokens = s.chunk;
     p.num_splits = s.count;
     // More than one wave of blocks: the long contexts first, so that the last blocks to start are short.  Contexts in a few chunks as well:
     // 38 / 44 sequences of 500 / 2000 to 4096 keys, 8 KV heads, 65.4 / 90.1 -> 58.7 / 85.9 us a call (whole 59.8 / 84.7).
-    p.longest_first = s.cluster == 0 && (s.count == 1 || a.max_blocks * a.block_size <= 4096) && a.batch * a.num_kv_heads > static_cast<int64_t>(kSmCount) * groups &&
+    p.longest_first = s.chunk > 0 && (s.count == 1 || a.max_blocks * a.block_size <= 4096) && a.batch * a.num_kv_heads > static_cast<int64_t>(kSmCount) * groups &&
                       a.batch <= kMaxSorted && a.max_blocks * a.block_size >= kMinSortedTokens;
     // Contexts shorter than the table leave chunks without keys, whose blocks exit at once.  With sequence after sequence they lie between
     // the blocks with work, and these pile up on the SMs where the empty ones were quickest gone; chunk after chunk the ones with

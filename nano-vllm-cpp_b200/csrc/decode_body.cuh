@@ -41,7 +41,7 @@ struct DecodeParams {
     int per_seq;                                       // 1: num_splits equal ranges per sequence instead of chunks
     int longest_first;                                 // blocks take the sequences in order of falling context length
     int chunk_major;                                   // decode_split_kernel's grid: all sequences' first chunks, then all second ones, ...
-    int split_shift;                                   // per_seq: log2 of num_splits
+    int split_shift;                                   // clusters: log2 of num_splits
     int beside;                                        // waits at its end (pdl_wait_beside)
     FastDiv by_block, by_kv_heads;
     float scale_log2;

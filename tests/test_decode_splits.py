@@ -102,3 +102,33 @@ def test_parts_come_together_without_what_is_not_there(hq, hkv, bs, lens, table_
         assert bool((out[live][..., 5] == float("inf")).all())
         rest = torch.cat([out[..., :5], out[..., 6:]], -1)
         assert_attention_close(to_np(rest), np.concatenate([ref[..., :5], ref[..., 6:]], -1))
+
+
+@pytest.mark.parametrize("kv,hq,hkv,bs,batch,table_blocks", [
+    ("same", 8, 1, 256, 72, 3), ("same", 16, 8, 256, 18, 5), ("same", 6, 2, 48, 37, 43), ("same", 4, 4, 256, 37, 32),     # fewest and most pairs, odd and widest tables
+    ("int8", 8, 1, 256, 105, 5), ("fp8", 4, 2, 64, 111, 24), ("int8", 8, 8, 256, 14, 8),
+])
+def test_halves_of_a_table_in_clusters_of_two(kv, hq, hkv, bs, batch, table_blocks):
+    """Contexts that end in the first half, with it, in the second and with the table, and none."""
+    half, full = (table_blocks + 1) // 2 * bs, table_blocks * bs
+    edges = [0, 1, half - 1, half, half + 1, half + 17, full - 1, full]
+    lens = [min(edges[i % 8], 3000) for i in range(batch)]
+    w = workloads().make_decode_workload(batch, hq, hkv, 128, bs, 0, 0, seed=batch, context_lens=np.array(lens, np.int32), pad_blocks_to=table_blocks)
+    bf, lib = torch.bfloat16, nvk()
+    q, ctx, bt = to_dev(w["q"], bf), to_dev(w["context_lens"]), to_dev(w["block_tables"])
+    kc, vc = to_dev(w["k_cache"], bf), to_dev(w["v_cache"], bf)
+    ws, out = _workspace(batch, hq, hkv, bt.shape[1], bs), torch.full_like(q, float("nan"))
+    if kv == "same":
+        lib.launch_decode_attention_paged(q, kc, vc, ctx, bt, hkv, 128, bs, w["scale"], out, ws)
+        k, v, tol = w["k_cache"], w["v_cache"], None
+    else:
+        store, decode = ((lib.store_kvcache_int8, lib.launch_decode_attention_paged_int8) if kv == "int8" else
+                         (lib.store_kvcache_fp8, lib.launch_decode_attention_paged_fp8))
+        k8, v8 = (torch.empty(kc.shape, dtype=torch.int8 if kv == "int8" else torch.uint8, device="cuda") for _ in range(2))
+        ks, vs = (torch.empty(kc.shape[:-1], dtype=torch.float16, device="cuda") for _ in range(2))
+        store(kc.view(-1, hkv, 128), vc.view(-1, hkv, 128), k8, v8, ks, vs, torch.arange(ks.numel() // hkv, dtype=torch.int32, device="cuda"))
+        decode(q, k8, v8, ks, vs, ctx, bt, hkv, 128, bs, w["scale"], out, ws)
+        plain = (lambda x: x.float()) if kv == "int8" else (lambda x: x.view(torch.float8_e4m3fn).float())
+        k, v = ((plain(x) * s.float()[..., None]).cpu().numpy() for x, s in ((k8, ks), (v8, vs)))   # on the same quantised cache
+    ref = oracle.decode_attention_paged(w["q"], k, v, w["context_lens"], w["block_tables"], hkv, 128, bs, w["scale"])
+    assert_attention_close(to_np(out), ref)
