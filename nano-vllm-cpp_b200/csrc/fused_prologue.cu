@@ -26,6 +26,8 @@ namespace {
 
 constexpr int kWarpsPerBlock = 8;
 constexpr int kSteps = 2;   // head groups per unit
+constexpr int kFewWarps = 4;
+constexpr int kFewUnits = 4 * 16 * kSmCount;   // of one head group: a block of four for each of 16 places on every SM
 
 // Packed fp32 pairs (one 64-bit register pair per two values; Blackwell executes f32x2 mul / fma at one issue slot).
 using F2 = unsigned long long;
@@ -74,6 +76,8 @@ struct PrologueParams {
     int64_t cache_rows, rows;
     int max_positions, hq, hkv;
     float eps;
+    FastDiv by_units;                                       // few rows: units of a row
+    uint32_t few_units;
 };
 
 template <typename T, int D>   // D = head_dim: 64, 128 or 256
@@ -187,10 +191,95 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) fused_prologue_kernel(
     }
 }
 
+// The same for a few rows, where what a call costs is a chain of trips to memory: row's position -> table row.  A warp takes one group of heads of a row, and
+// all loads are under way as soon as their addresses are known, without branches around them (a branch waits for what it merges): clamped heads and
+// positions, and any valid address where there is nothing to load.  us a call in a row of calls, 32 / 8
+// heads: 1 row 2.25 -> 1.6, 64 2.5 -> 1.95, 256 2.95 -> 2.85, 400 4.2 -> 2.9, 700 4.35 -> 4.3.  Above that the kernel before it, whose warps take two groups and
+// fetch weights and table rows late, keeps more rows under way.
 template <typename T, int D>
-int launch_dim(const PrologueParams& p, cudaStream_t stream) {
-    constexpr int GROUPS = 32 / (D / 16);
+__global__ void __launch_bounds__(kFewWarps * 32) fused_prologue_few_rows_kernel(const __grid_constant__ PrologueParams p) {
+    constexpr int LANES = D / 16, GROUPS = 32 / LANES;
+    pdl_wait_then_release();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int sub = lane % LANES, group = lane / LANES;
     const int heads = p.hq + 2 * p.hkv;
+    const uint32_t unit = blockIdx.x * kFewWarps + warp;
+    if (unit >= p.few_units) return;
+    const uint32_t row = p.by_units.div(unit);
+    const int at = static_cast<int>(unit - row * p.by_units.d) * GROUPS + group, head = min(at, heads - 1);
+    const int lo_off = sub * 8, hi_off = D / 2 + sub * 8;
+    const bool normed = p.q_weight != nullptr, is_q = head < p.hq, is_k = !is_q && head < p.hq + p.hkv;
+    const int pos = __ldg(p.positions + row);
+    const int slot_in = __ldg((p.slot_mapping != nullptr ? p.slot_mapping : p.positions) + row);
+    const T* src = static_cast<const T*>(p.qkv) + (static_cast<int64_t>(row) * heads + head) * D;
+    const uint4 lo = ld_stream16(src + lo_off), hi = ld_stream16(src + hi_off);
+    const T* weight = normed ? static_cast<const T*>(is_q ? p.q_weight : p.k_weight) : src;
+    const uint4 w_lo = __ldg(reinterpret_cast<const uint4*>(weight + lo_off)), w_hi = __ldg(reinterpret_cast<const uint4*>(weight + hi_off));
+    const bool rotate = pos >= 0 && pos < p.max_positions;
+    const float* table = p.cos_sin + static_cast<int64_t>(rotate ? pos : 0) * D + lo_off;
+    const float4 c4[2] = {__ldg(reinterpret_cast<const float4*>(table)), __ldg(reinterpret_cast<const float4*>(table + 4))};
+    const float4 s4[2] = {__ldg(reinterpret_cast<const float4*>(table + D / 2)), __ldg(reinterpret_cast<const float4*>(table + D / 2 + 4))};
+    const float2 c[4] = {{c4[0].x, c4[0].y}, {c4[0].z, c4[0].w}, {c4[1].x, c4[1].y}, {c4[1].z, c4[1].w}};
+    const float2 sn[4] = {{s4[0].x, s4[0].y}, {s4[0].z, s4[0].w}, {s4[1].x, s4[1].y}, {s4[1].z, s4[1].w}};
+    float inv_rms = 1.0f;
+    {
+        F2 sq = f2_make(0.0f, 0.0f);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const F2 a = f2_unpack<T>(word(lo, i)), b = f2_unpack<T>(word(hi, i));
+            sq = f2_fma(a, a, sq);
+            sq = f2_fma(b, b, sq);
+        }
+        float s0, s1;
+        f2_split(sq, s0, s1);
+        float ss = s0 + s1;
+#pragma unroll
+        for (int o = LANES / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        inv_rms = rsqrtf(ss / static_cast<float>(D) + p.eps);
+    }
+    const F2 inv2 = f2_make(inv_rms, inv_rms);
+    uint4 out_lo = lo, out_hi = hi;            // v heads: the loaded values as they are
+    if (is_q || is_k) {
+        uint32_t r_lo[4], r_hi[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            F2 a = f2_unpack<T>(word(lo, i)), b = f2_unpack<T>(word(hi, i));
+            if (normed) {
+                a = f2_mul(f2_mul(a, inv2), f2_unpack<T>(word(w_lo, i)));
+                b = f2_mul(f2_mul(b, inv2), f2_unpack<T>(word(w_hi, i)));
+            }
+            if (rotate) {                      // first half: x cos - partner sin; second half: x cos + partner sin
+                const F2 c2 = f2_make(c[i].x, c[i].y), s2 = f2_make(sn[i].x, sn[i].y), n2 = f2_make(-sn[i].x, -sn[i].y);
+                r_lo[i] = f2_pack<T>(f2_fma(a, c2, f2_mul(b, n2)));
+                r_hi[i] = f2_pack<T>(f2_fma(b, c2, f2_mul(a, s2)));
+            } else {                           // positions outside the table leave the value un-rotated
+                r_lo[i] = f2_pack<T>(a);
+                r_hi[i] = f2_pack<T>(b);
+            }
+        }
+        out_lo = make_uint4(r_lo[0], r_lo[1], r_lo[2], r_lo[3]);
+        out_hi = make_uint4(r_hi[0], r_hi[1], r_hi[2], r_hi[3]);
+    }
+    const int64_t slot = p.slot_mapping != nullptr ? static_cast<int64_t>(slot_in) : static_cast<int64_t>(row);
+    if (at >= heads || (!is_q && (slot < 0 || slot >= p.cache_rows))) return;
+    T* dst;
+    if (is_q) dst = static_cast<T*>(p.q_out) + (static_cast<int64_t>(row) * p.hq + head) * D;
+    else dst = static_cast<T*>(is_k ? p.k_cache : p.v_cache) + (slot * p.hkv + (is_k ? head - p.hq : head - p.hq - p.hkv)) * D;
+    *reinterpret_cast<uint4*>(dst + lo_off) = out_lo;
+    *reinterpret_cast<uint4*>(dst + hi_off) = out_hi;
+}
+
+template <typename T, int D>
+int launch_dim(PrologueParams& p, cudaStream_t stream) {
+    constexpr int GROUPS = 32 / (D / 16);
+    const int heads = p.hq + 2 * p.hkv, row_units = (heads + GROUPS - 1) / GROUPS;
+    if (p.rows * row_units <= kFewUnits) {
+        p.few_units = static_cast<uint32_t>(p.rows * row_units);
+        p.by_units = FastDiv(static_cast<uint32_t>(row_units));
+        const cudaError_t e = launch_pdl(fused_prologue_few_rows_kernel<T, D>, dim3((p.few_units + kFewWarps - 1) / kFewWarps), dim3(kFewWarps * 32), 0, stream, p);
+        if (e != cudaSuccess) return fail(NVK_ERR_CUDA, "fused_split_norm_rope_store kernel launch: %s", cudaGetErrorString(e));
+        return check_launch("fused_split_norm_rope_store kernel launch");
+    }
     const int64_t units = p.rows * ((heads + GROUPS * kSteps - 1) / (GROUPS * kSteps));
     const int64_t resident = static_cast<int64_t>(kSmCount) * 4;   // four blocks per SM
     int64_t blocks = (units + kWarpsPerBlock - 1) / kWarpsPerBlock;
@@ -201,7 +290,7 @@ int launch_dim(const PrologueParams& p, cudaStream_t stream) {
 }
 
 template <typename T>
-int launch_typed(const PrologueParams& p, int d, cudaStream_t stream) {
+int launch_typed(PrologueParams& p, int d, cudaStream_t stream) {
     switch (d) {
         case 64: return launch_dim<T, 64>(p, stream);
         case 128: return launch_dim<T, 128>(p, stream);

@@ -413,6 +413,29 @@ def test_fused_split_norm_rope_store_matches_oracle(num_q_heads, num_kv_heads, h
         assert (got == ref).mean() > 0.98
 
 
+@pytest.mark.parametrize("normed,slotted", [(True, True), (False, True), (True, False)])
+@pytest.mark.parametrize("num_q_heads,num_kv_heads,head_dim,few", [(32, 8, 128, 789), (5, 1, 64, 9472), (16, 8, 256, 592), (4, 1, 128, 4736)])
+def test_prologue_of_few_rows_gives_the_bits_of_that_of_many(num_q_heads, num_kv_heads, head_dim, few, normed, slotted):
+    """Two kernels, on both sides of 9472 units of a warp: the same operations in the same order."""
+    rows, max_pos, bf = few + 5, 300, torch.bfloat16
+    w = workloads().make_prologue_workload(rows, num_q_heads, num_kv_heads, head_dim, rows + 64, max_pos, seed=few)
+    w["slot_mapping"][3], w["positions"][5], w["positions"][few - 1] = -1, max_pos + 7, -2
+    table = to_dev(oracle.build_cos_sin_cache(max_pos, head_dim, w["rope_base"]))
+    qkv, pos, slots = to_dev(w["qkv"], bf), to_dev(w["positions"]), to_dev(w["slot_mapping"])
+    qw, kw = (to_dev(w["q_norm_weight"], bf), to_dev(w["k_norm_weight"], bf)) if normed else (None, None)
+    got = []
+    for parts in (((0, rows),), ((0, few), (few, rows))):
+        kc = torch.zeros(rows + 64, num_kv_heads, head_dim, dtype=bf, device="cuda")
+        vc, q_out = torch.zeros_like(kc), torch.full((rows, num_q_heads, head_dim), float("nan"), dtype=bf, device="cuda")
+        for a, b in parts:
+            at = 0 if slotted else a                                  # without slots row i of a call goes to row i of the cache
+            nvk().fused_split_norm_rope_store(qkv[a:b], pos[a:b], qw, kw, w["eps"], table, slots[a:b] if slotted else None, kc[at:], vc[at:],
+                                              num_q_heads, num_kv_heads, head_dim, q_out[a:b])
+        got.append((q_out, kc, vc))
+    assert not torch.isnan(got[0][0].float()).any()
+    assert all(torch.equal(x, y) for x, y in zip(*got))
+
+
 # ------------------------------------------------------- the kernels the library picks by shape
 
 @pytest.mark.parametrize("num_heads,num_kv_heads", [(3, 3), (6, 2), (5, 1)])
