@@ -259,8 +259,8 @@ bool halves(int64_t pairs, int64_t max_tokens, int groups) {
 //   * Tables of up to 1024 keys: 176 pairs of 1024 keys 19.3 a call, as two chunks 23.7; 264 24.6, 29.1; 432 int8 ones 24.3, 30.5.
 //   * Tables of up to 4096 keys (3072 below 180 pairs) where the halves above have no room: 184 pairs of 2048 keys 25.0 / 29.6 / 34.2, in chunks of 1024 25.7 / 34.4 / 42.7; 264 of
 //     4096 52.7 / 68.7 / 85.3, chunks of 2048 58.6 / 74.7 / 90.7.  But not just past a wave: 304 / 352 pairs, all of 4096 keys, 116.8 / 123.7 a call, in chunks
-//     of 2048 106.1 / 113.5.  8-bit caches up to 1536 keys, 2048 up to 266 pairs (224: 24.5 / 25.5 / 27.2, 25.0 / 26.6 / 34.9; 272 int8 ones 31.4 / 34.5 / 38.7,
-//     28.3 / 35.6 / 37.2), 4096 with a pair for every resident group.
+//     of 2048 106.1 / 113.5.  8-bit caches up to 1536 keys (272 pairs 23.7 / 25.5 / 28.4, 23.2 / 26.0 / 30.9; but 256 e4m3 ones of 0.05 to all of 2048 keys 25.9, in
+//     chunks 25.2, and 272 int8 ones 31.4, 28.3), 4096 with a pair for every resident group.
 // Chunks otherwise, of 2048 or, with few pairs and up to 8192 keys, of 1024 (224 pairs of 6144 keys 64.1 / 86.4 / 111.1, 69.7 / 88.2 / 114.5 in chunks of 2048; 8-bit
 // 55.0 / 70.6 / 87.4 for 8192, 60.4 / 73.5 / 89.2), halved down to 256 while they leave resident groups without a block.
 //   * What a table of 2048 keys is cut into is cut no finer than it takes to have 1.5 blocks per SM (8-bit: 2.25 of 512 keys).
@@ -270,7 +270,7 @@ bool halves(int64_t pairs, int64_t max_tokens, int groups) {
 int chunk_tokens(int64_t batch, int num_kv_heads, int64_t max_blocks, int block_size, int groups) {
     const int64_t max_tokens = max_blocks * block_size, pairs = batch * num_kv_heads, resident = static_cast<int64_t>(kSmCount) * groups;
     if (max_tokens <= 1024) return static_cast<int>(max_tokens);
-    const int64_t whole = groups == 2 ? (pairs < 180 ? 3072 : just_past_a_wave(pairs, groups) ? 2048 : 4096) : 5 * pairs <= 3 * resident ? 2048 : 1536;
+    const int64_t whole = groups == 2 ? (pairs < 180 ? 3072 : just_past_a_wave(pairs, groups) ? 2048 : 4096) : 1536;
     if (2 * pairs > resident && max_tokens <= whole) return static_cast<int>(max_tokens);
     if (max_tokens <= 4096 && pairs >= resident && !just_past_a_wave(pairs, groups)) return static_cast<int>(max_tokens);
     int64_t chunk = max_tokens <= 8192 && (groups == 2 ? max_tokens > 4096 && pairs < 2 * resident : 5 * pairs < 4 * resident) ? 1024 : 2048;
