@@ -375,7 +375,8 @@ __global__ void __launch_bounds__(kThreads, 2) prefill_tile_kernel(const __grid_
             sum *= f;
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
-                const bool seen = ml[u].x != -INFINITY;                // (else there may be nothing written)
+                // (No maximum and no sum: there may be nothing written.  A part whose scores are all NaN has no maximum either, but a NaN as its sum.)
+                const bool seen = ml[u].x != -INFINITY || ml[u].y != 0.0f;
                 const float w = fast_exp2(ml[u].x - base);
                 v.x = fmaf(w, seen ? a[u].x : 0.0f, v.x); v.y = fmaf(w, seen ? a[u].y : 0.0f, v.y);
                 v.z = fmaf(w, seen ? a[u].z : 0.0f, v.z); v.w = fmaf(w, seen ? a[u].w : 0.0f, v.w);

@@ -160,3 +160,35 @@ def test_small_steps_keep_infinities_in_their_columns_and_rows_without_keys_at_z
     lib.launch_prefill_attention_paged(q, to_dev(w["cu_q"]), kc, to_dev(w["v_cache"], bf), cu_k, to_dev(w["block_tables"]), 8, 128, 256, w["scale"], out)
     torch.cuda.synchronize()
     assert bool((out[:10] == 0).all()) and bool((out[10:].float().abs().amax((1, 2)) > 0).all())
+
+
+@pytest.mark.parametrize("hq,hkv,q_len,bs", [(16, 8, 20, 256), (32, 8, 77, 256), (32, 8, 130, 64)])   # clusters of 8, 4 and 2 over the keys
+def test_small_steps_keep_nan(hq, hkv, q_len, bs):
+    """A NaN in a query row is in all of that row's results, and NaN keys are in the results of every row that sees them: also where a block's part
+    of a row has nothing but NaN scores, and with them no maximum."""
+    w = workloads().make_prefill_workload([q_len], [512], hq, hkv, 128, bs, seed=q_len, paged=True)
+    lib, bf = nvk(), torch.bfloat16
+    cu_q, cu_k, tables = to_dev(w["cu_q"]), to_dev(w["cu_k"]), to_dev(w["block_tables"])
+    run = lambda q, kc, out: lib.launch_prefill_attention_paged(q, cu_q, kc, vc, cu_k, tables, hkv, 128, bs, w["scale"], out)
+    q, kc, vc = to_dev(w["q"], bf), to_dev(w["k_cache"], bf), to_dev(w["v_cache"], bf)
+    ref = oracle.prefill_attention_paged(w["q"], w["k_cache"], w["v_cache"], w["cu_q"], w["cu_k"], w["block_tables"], hkv, 128, bs, w["scale"])
+    row, head = q_len // 2, hq - 2
+    one = q.clone()
+    one[row, head, 3] = float("nan")
+    out = torch.zeros_like(q)
+    run(one, kc, out)
+    assert bool(torch.isnan(out[row, head].float()).all())
+    rest = torch.ones((q_len, hq), dtype=torch.bool)
+    rest[row, head] = False
+    assert_attention_close(to_np(out)[rest.numpy()], ref[rest.numpy()])
+    bad = kc.clone()
+    for key in range(384):                                           # for one KV head
+        bad[int(w["block_tables"][0, key // bs]), key % bs, 1] = float("nan")
+    out = torch.zeros_like(q)
+    run(q, bad, out)
+    torch.cuda.synchronize()
+    assert lib.prefill_status() == 0
+    group = hq // hkv
+    assert bool(torch.isnan(out[:, group:2 * group].float()).all())
+    others = np.r_[0:group, 2 * group:hq]
+    assert_attention_close(to_np(out)[:, others], ref[:, others])
