@@ -33,7 +33,7 @@ bool is_compute_dtype(int dtype) { return dtype == NVK_F16 || dtype == NVK_BF16 
 bool is_index_dtype(int dtype) { return dtype == NVK_I32 || dtype == NVK_I64; }
 IndexArray index_array(const void* p, int dtype) { return IndexArray(p, dtype == NVK_I64 ? 1 : 0); }
 int launch_prefill(const PrefillArgs& a) {
-    if (prefill_tc_supported(a) && prefill_tiles_save(a) <= 0.0) return launch_prefill_tc(a);
+    if (prefill_tc_supported(a) && !prefill_takes_tiles(a)) return launch_prefill_tc(a);
     if (prefill_mma_supported(a)) return launch_prefill_mma(a);
     return launch_rowwise_prefill(a);
 }
@@ -304,7 +304,7 @@ int nvk_attention_mixed_step(const void* p_query, const void* p_key, const void*
     // A scale that is not positive: the prefill rows take another kernel.  So do few of them, and the decode kernel runs beside that one (us a step as
     // one launch / as these: 1 prompt of 670 tokens, 5 decode rows of 400 keys, 4 / 1 heads, 22.7 / 15.0; 3 of 109 to 136, 9 of up to 1929, 16 / 4
     // heads, 20.1 / 16.2; 1 of 300, 60 of up to 4096, 4 / 1 heads, 31.6 / 27.4).
-    const bool small = prefill_tc_supported(pa) && prefill_tiles_save(pa) > 0.0;
+    const bool small = prefill_tc_supported(pa) && prefill_takes_tiles(pa);
     if (small || !prefill_tc_supported(pa)) {
         const int rc = launch_prefill(pa);
         da.beside = small;

@@ -174,7 +174,7 @@ int launch_store_fp8(const void* key, const void* value, void* k_cache, void* v_
                      int dtype, cudaStream_t stream);
 bool prefill_mma_supported(const PrefillArgs& a);
 int launch_prefill_mma(const PrefillArgs& a);
-double prefill_tiles_save(const PrefillArgs& a);   // microseconds that launch_prefill_mma saves beside launch_prefill_tc, by sizes that the host knows
+bool prefill_takes_tiles(const PrefillArgs& a);   // launch_prefill_mma is quicker than launch_prefill_tc, by sizes that the host knows
 int prefill_tile_status(cudaStream_t stream, int* status);
 // tcgen05 / TMEM / TMA path (F16/BF16, head_dim 128, paged block_size % 128 == 0).
 bool prefill_tc_supported(const PrefillArgs& a);

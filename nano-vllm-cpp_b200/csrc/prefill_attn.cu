@@ -396,37 +396,87 @@ __global__ void __launch_bounds__(kThreads, 2) prefill_tile_kernel(const __grid_
 
 int tile_head_shift(int group) { return group % 8 == 0 ? 3 : group % 4 == 0 ? 2 : group % 2 == 0 ? 1 : 0; }
 
-// What a step takes, in microseconds, from what the host knows: as if all sequences were equally long and, where block tables are wider than
-// these need, had a cached prefix of whole blocks.
-struct Estimate {
-    int64_t q, keys;      // of a sequence
-    explicit Estimate(const PrefillArgs& a) {
-        const int64_t n = a.cu_q ? a.num_seqs : 1;
-        q = (a.total_q + n - 1) / n;
-        keys = (a.total_k + n - 1) / n;
-        if (a.block_tables) {
-            const int64_t before = (a.max_blocks - 1) * a.block_size;
-            keys = q > before ? q : before + (q < a.block_size ? q : a.block_size);
-        }
-        if (keys < 1) keys = 1;
+// What a step takes, in microseconds, from what the host knows: rows and, where the keys are not paged, keys of all sequences together, the block
+// tables' width, maybe the longest sequence's rows.  `count` sequences of q rows that see `keys` keys each.
+struct Alike { int64_t count, q, keys; };
+int64_t sequences(const PrefillArgs& a) { return a.cu_q ? a.num_seqs : 1; }
+int64_t ceil_div(int64_t n, int64_t by) { return (n + by - 1) / by; }
+// All sequences equally long and, where block tables are wider than these need, behind a cached prefix of whole blocks.
+Alike equal_lengths(const PrefillArgs& a) {
+    const int64_t n = sequences(a), q = ceil_div(a.total_q, n);
+    int64_t keys = ceil_div(a.total_k, n);
+    if (a.block_tables) {
+        const int64_t before = (a.max_blocks - 1) * a.block_size;
+        keys = q > before ? q : before + (q < a.block_size ? q : a.block_size);
     }
-};
-// Here a block takes 3.4 us and 1.4 for each of its key tiles, 2.1 where two share an SM, and 2.9 more for the parts of a cluster (32 / 8 heads, with a
-// store of 1.3 us: 77 tokens alone 7.4 us in one block each, 9.7 and 10.5 in clusters of 2 and 4; 8 on a prefix of 256, 5 tiles, 11.4, 9.6 and 8.3
-// in clusters of 2, 4 and 8).  The cluster size that takes least of those that are resident at once.
-double tile_time(const PrefillArgs& a, int* csize_shift) {
-    const Estimate e(a);
+    return {n, q, keys < 1 ? 1 : keys};
+}
+// The other end: sequences as long as any can be (`max_seqlen_q` where it is given; with paged keys none is longer than its table), and the rows that
+// are left on the others.  False: all are of one length.
+bool unequal_lengths(const PrefillArgs& a, Alike (&l)[2]) {
+    const int64_t n = sequences(a), even = ceil_div(a.total_q, n), width = a.block_tables ? a.max_blocks * a.block_size : a.total_q;
+    int64_t q = a.total_q - (n - 1);
+    if (a.max_seqlen_q > 0 && a.max_seqlen_q < q) q = a.max_seqlen_q;
+    if (width < q) q = width;
+    if (n == 1 || q <= even) return false;
+    int64_t count = a.block_tables || a.max_seqlen_q > 0 ? (a.total_q - n) / (q - 1) : 1;
+    if (count < 1) count = 1;
+    if (count > n - 1) count = n - 1;
+    const int64_t left = a.total_q - count * q, rest = left > n - count ? ceil_div(left, n - count) : 1;
+    if (a.block_tables) {
+        const int64_t bs = a.block_size, before = (a.max_blocks - 1) * bs;
+        auto keys = [&](int64_t rows) { return q > before ? rows : before + (rows < bs ? rows : bs); };
+        l[0] = {count, q, keys(q)};
+        l[1] = {n - count, rest, keys(rest)};
+    } else {
+        const int64_t before = a.total_k > a.total_q ? (a.total_k - a.total_q) / n : 0;
+        l[0] = {count, q, before + q};
+        l[1] = {n - count, rest, before + rest};
+    }
+    return true;
+}
+// Items of `rows` rows and `sets` per row range, the rounds of `step` keys that the longest takes, and all of them together.
+struct Load { int64_t items, longest; double rounds; };
+Load load_of(const Alike* l, int n, int64_t rows, int64_t sets, int64_t step) {
+    Load w{0, 1, 0.0};
+    for (int i = 0; i < n; ++i) {
+        const int64_t ranges = ceil_div(l[i].q, rows), longest = ceil_div(l[i].keys, step);
+        w.items += l[i].count * ranges * sets;
+        if (longest > w.longest) w.longest = longest;
+        const double keys = static_cast<double>(l[i].keys - l[i].q) + 0.5 * static_cast<double>((ranges + 1) * rows);   // of an item, on average
+        w.rounds += static_cast<double>(l[i].count * ranges * sets) * (keys / static_cast<double>(step) + 0.5);
+    }
+    return w;
+}
+// Here a block takes 3.4 us and 1.4 for each of its key tiles, 2.1 where two share an SM, 2 more for each further wave of blocks, and 2.9 for the parts
+// of a cluster (32 / 8 heads, with a store of 1.3 us: 77 tokens alone 7.4 us in one block each, 9.7 and 10.5 in clusters of 2 and 4; 8 on a prefix
+// of 256, 5 tiles, 11.4, 9.6 and 8.3 in clusters of 2, 4 and 8).
+double tile_time(const PrefillArgs& a, const Alike* l, int n, int csize_shift) {
     const int head_shift = tile_head_shift(a.num_heads / a.num_kv_heads);
-    const int64_t n = a.cu_q ? a.num_seqs : 1, rows = kBM >> head_shift, sets = a.num_heads >> head_shift;
-    const int64_t grid = ((a.total_q + rows - 1) / rows + (a.cu_q ? n : 0)) * sets, items = n * ((e.q + rows - 1) / rows) * sets, tiles = (e.keys + kBN - 1) / kBN;
-    double best = 1e30;
-    for (int s = 0; s <= 3; ++s) {
-        if (s > 0 && (grid << s) > 2 * kSmCount) break;
-        const int64_t blocks = items << s, waves = (blocks + 2 * kSmCount - 1) / (2 * kSmCount);
-        const double time = 3.4 + static_cast<double>(waves * ((tiles + (1 << s) - 1) >> s)) * (blocks <= kSmCount ? 1.4 : 2.1) + (s > 0 ? 2.9 : 0.0);
-        if (time < best) { best = time; *csize_shift = s; }
-    }
+    const Load w = load_of(l, n, kBM >> head_shift, a.num_heads >> head_shift, kBN);
+    const int64_t blocks = w.items << csize_shift, waves = ceil_div(blocks, 2 * kSmCount), longest = ceil_div(w.longest, 1LL << csize_shift);
+    double rounds = static_cast<double>(n == 1 ? waves * longest : longest);
+    if (n > 1 && w.rounds > rounds * (2 * kSmCount)) rounds = w.rounds / (2 * kSmCount);
+    return 3.4 + rounds * (blocks <= kSmCount ? 1.4 : 2.1) + 2.0 * static_cast<double>(waves - 1) + (csize_shift > 0 ? 2.9 : 0.0);
+}
+// log2 of the cluster size that takes least for equal lengths, of those that are resident at once.
+int best_cluster(const PrefillArgs& a, const Alike& equal) {
+    const int head_shift = tile_head_shift(a.num_heads / a.num_kv_heads);
+    const int64_t rows = kBM >> head_shift, grid = (ceil_div(a.total_q, rows) + (a.cu_q ? a.num_seqs : 0)) * (a.num_heads >> head_shift);
+    int best = 0;
+    for (int s = 1; s <= 3 && (grid << s) <= 2 * kSmCount; ++s)
+        if (tile_time(a, &equal, 1, s) < tile_time(a, &equal, 1, best)) best = s;
     return best;
+}
+// The persistent tcgen05 kernel takes 6.8 us and 1.56 for each round of 128 keys of an item of 256 rows (half a microsecond in doubt).
+double tcgen05_time(const PrefillArgs& a, const Alike* l, int n) {
+    const int group = a.num_heads / a.num_kv_heads, heads = group % 8 == 0 ? 8 : group % 4 == 0 ? 4 : 2;   // of an item
+    const Load w = load_of(l, n, 2 * 128 / heads, a.num_heads / heads, 128);
+    const double waves = n == 1 ? static_cast<double>(ceil_div(w.items, kSmCount)) : static_cast<double>(w.items) / kSmCount;
+    const double more = waves > 1.0 ? 1.5 * (waves - 1.0) : 0.0, longest = 1.56 * static_cast<double>(w.longest);
+    if (n == 1) return 6.3 + waves * longest + more;
+    const double all = 1.56 * w.rounds / kSmCount + more;
+    return 6.3 + (all > longest ? all : longest);
 }
 
 template <typename T>
@@ -453,7 +503,7 @@ int launch_typed(const PrefillArgs& a) {
     p.by_sets = FastDiv(static_cast<uint32_t>(sets));
     p.by_block = FastDiv(static_cast<uint32_t>(p.block_size));
     p.by_group = FastDiv(static_cast<uint32_t>(group));
-    tile_time(a, &p.csize_shift);
+    p.csize_shift = best_cluster(a, equal_lengths(a));
     if (tiles * sets << p.csize_shift > 0x7fffffffLL || tiles > 0x7fffffffLL) return fail(NVK_ERR_UNSUPPORTED, "prefill attention: grid too large");
     p.tiles = static_cast<unsigned int>(tiles);
     cudaLaunchConfig_t cfg{};
@@ -492,18 +542,20 @@ int launch_prefill_mma(const PrefillArgs& a) {
     return a.dtype == NVK_BF16 ? launch_typed<__nv_bfloat16>(a) : launch_typed<__half>(a);
 }
 
-// The persistent tcgen05 kernel takes 6.8 us and 1.56 for each round of 128 keys of an item of 256 rows, and does six times as much at once: where few
-// items leave most SMs idle, or are nearly empty, the smaller tiles above are quicker (us, 32 / 8 heads but where said, tcgen05 / these: 10
-// tokens 8.4 / 5.9, 77 9.5 / 7.4, 150 11.0 / 8.9, 8 on 256 12.0 / 8.3, 77 on 512 16.0 / 14.3, 4 x 8 to 20 on 1024, 4 / 1 heads, 21.5 / 11.2; but 300 tokens
-// 12.7 / 13.7, 12 x 8 on 512 17.7 / 20.3, 11 x 67 to 256, 8 / 2 heads, 12.7 / 13.9).  Returns what these save, in microseconds; 0 or less: nothing.
-double prefill_tiles_save(const PrefillArgs& a) {
-    if ((a.num_heads / a.num_kv_heads) % 2 != 0 || !prefill_mma_supported(a)) return 0.0;   // (odd groups: another tcgen05 kernel)
-    const Estimate e(a);
-    const int group = a.num_heads / a.num_kv_heads, heads = group % 8 == 0 ? 8 : group % 4 == 0 ? 4 : 2;   // of an item there
-    const int64_t n = a.cu_q ? a.num_seqs : 1, rows = 2 * 128 / heads, items = n * ((e.q + rows - 1) / rows) * (a.num_heads / heads);
-    const int64_t waves = (items + kSmCount - 1) / kSmCount, rounds = (e.keys + 127) / 128;
-    int csize_shift = 0;
-    return 6.3 + 1.56 * static_cast<double>(waves * rounds) + 1.5 * static_cast<double>(waves - 1) - tile_time(a, &csize_shift);   // (half a microsecond in doubt)
+// Where few items leave most SMs of the persistent tcgen05 kernel idle, or are nearly empty, the smaller tiles above are quicker, although that does six
+// times as much at once (us, 32 / 8 heads but where said, tcgen05 / these: 10 tokens 8.4 / 5.9, 77 9.5 / 7.4, 150 11.0 / 8.9, 8 on 256 12.0 / 8.3, 77 on
+// 512 16.0 / 14.3, 4 x 8 to 20 on 1024, 4 / 1 heads, 21.5 / 11.2; but 300 tokens 12.7 / 13.7, 12 x 8 on 512 17.7 / 20.3, 11 x 67 to 256, 8 / 2 heads,
+// 12.7 / 13.9).  The host does not know how the rows are shared out, and a block of 64 rows of a long prompt takes as long as the tcgen05 kernel for
+// four times the heads and rows: one of 2000 tokens and 63 of 8 54 / 117, one of 2000 and 31 of 40 (4 / 1 heads) 30 / 55, one of 1500 and 15 of 5 (8 / 2)
+// 24 / 40.  So the tiles have to win for equal lengths and must not lose more than 5 % for the most unequal ones: over 1800 steps of 1 to 64
+// prompts, equal, spread and with one or two long ones, 0.81 of the tcgen05 kernel's time and 1.10 at most (by equal lengths alone 0.80 and 1.98).
+bool prefill_takes_tiles(const PrefillArgs& a) {
+    if ((a.num_heads / a.num_kv_heads) % 2 != 0 || !prefill_mma_supported(a)) return false;   // (odd groups: another tcgen05 kernel)
+    const Alike equal = equal_lengths(a);
+    const int csize_shift = best_cluster(a, equal);
+    if (tile_time(a, &equal, 1, csize_shift) >= tcgen05_time(a, &equal, 1)) return false;
+    Alike unequal[2];
+    return !unequal_lengths(a, unequal) || tile_time(a, unequal, 2, csize_shift) <= 1.05 * tcgen05_time(a, unequal, 2);
 }
 
 // Error word of the waits above; cleared.

@@ -14,6 +14,15 @@ void launch_prefill_attention_paged(const Tensor& query, const Tensor* cu_seqlen
                                     int num_kv_heads, int head_dim, int block_size, float scale, Tensor& output,
                                     cudaStream_t stream = nullptr);
 
+// The same for callers that know the longest sequence's number of new tokens (0: unknown); the choice between the prefill kernels goes by it.
+void launch_prefill_attention_dense(const Tensor& query, const Tensor* cu_seqlens_q, const Tensor& key,
+                                    const Tensor& value, const Tensor* cu_seqlens_k, int num_kv_heads, int head_dim,
+                                    float scale, Tensor& output, cudaStream_t stream, int max_seqlen_q);
+void launch_prefill_attention_paged(const Tensor& query, const Tensor* cu_seqlens_q, const Tensor& k_cache,
+                                    const Tensor& v_cache, const Tensor* cu_seqlens_k, const Tensor& block_tables,
+                                    int num_kv_heads, int head_dim, int block_size, float scale, Tensor& output,
+                                    cudaStream_t stream, int max_seqlen_q);
+
 // No allocator in this signature: split-K scratch comes from the library's built-in array
 // (nvk_decode_attention_paged_static) when the problem fits nvk_decode_attention_static_scratch_bytes(), otherwise the
 // call runs unsplit.  Two rules follow from sharing that array, neither of which the reference's function has:

@@ -112,9 +112,9 @@ Tensor Attention::forward(const Tensor& query, const Tensor& key, const Tensor& 
         if (paged && !is_int8_) {   // an int8 cache is only read by decode: prefill attends over the dense K / V it was given
             if (cu_k == nullptr) throw std::invalid_argument("prefill attention with block_tables requires cu_seqlens_k");
             launch_prefill_attention_paged(query, cu_q, k_cache_, v_cache_, cu_k, ctx.block_tables, num_kv_heads_,
-                                           head_dim_, block_size_, scale_, output, stream);
+                                           head_dim_, block_size_, scale_, output, stream, ctx.max_seqlen_q);
         } else {
-            launch_prefill_attention_dense(query, cu_q, key, value, cu_k, num_kv_heads_, head_dim_, scale_, output, stream);
+            launch_prefill_attention_dense(query, cu_q, key, value, cu_k, num_kv_heads_, head_dim_, scale_, output, stream, ctx.max_seqlen_q);
         }
         return output;
     }

@@ -290,7 +290,7 @@ void launch_decode_attention_paged_int8(const Tensor& query, const Tensor& k_cac
 // ---- prefill ------------------------------------------------------------------------------------------
 void launch_prefill_attention_dense(const Tensor& query, const Tensor* cu_seqlens_q, const Tensor& key,
                                     const Tensor& value, const Tensor* cu_seqlens_k, int num_kv_heads, int head_dim,
-                                    float scale, Tensor& output, cudaStream_t stream) {
+                                    float scale, Tensor& output, cudaStream_t stream, int max_seqlen_q) {
     check_qo(query, output);
     ensure_cuda_tensor("key", key);
     ensure_cuda_tensor("value", value);
@@ -302,15 +302,21 @@ void launch_prefill_attention_dense(const Tensor& query, const Tensor* cu_seqlen
     const int64_t seqs = varlen ? static_cast<int64_t>(cu_seqlens_q->numel()) - 1 : 1;
     throw_on_nvk_status(nvk_prefill_attention_varlen(query.data(), key.data(), value.data(), nullptr, nullptr, cq.ptr,
                                                      cq.dtype, ck.ptr, ck.dtype, nullptr, NVK_I32, seqs, query.sizes()[0],
-                                                     key.sizes()[0], 0, 0, 0,
+                                                     key.sizes()[0], 0, 0, max_seqlen_q,
                                                      static_cast<int>(query.sizes()[1]), num_kv_heads, head_dim, 1, scale,
                                                      output.data(), code(query.dtype()), stream));
+}
+
+void launch_prefill_attention_dense(const Tensor& query, const Tensor* cu_seqlens_q, const Tensor& key,
+                                    const Tensor& value, const Tensor* cu_seqlens_k, int num_kv_heads, int head_dim,
+                                    float scale, Tensor& output, cudaStream_t stream) {
+    launch_prefill_attention_dense(query, cu_seqlens_q, key, value, cu_seqlens_k, num_kv_heads, head_dim, scale, output, stream, 0);
 }
 
 void launch_prefill_attention_paged(const Tensor& query, const Tensor* cu_seqlens_q, const Tensor& k_cache,
                                     const Tensor& v_cache, const Tensor* cu_seqlens_k, const Tensor& block_tables,
                                     int num_kv_heads, int head_dim, int block_size, float scale, Tensor& output,
-                                    cudaStream_t stream) {
+                                    cudaStream_t stream, int max_seqlen_q) {
     if (cu_seqlens_q == nullptr || cu_seqlens_k == nullptr)
         throw std::invalid_argument("paged prefill attention requires cu_seqlens_q and cu_seqlens_k");
     check_qo(query, output);
@@ -324,9 +330,17 @@ void launch_prefill_attention_paged(const Tensor& query, const Tensor* cu_seqlen
     throw_on_nvk_status(nvk_prefill_attention_varlen(
         query.data(), nullptr, nullptr, k_cache.data(), v_cache.data(), cq.ptr, cq.dtype, ck.ptr, ck.dtype, tables.ptr,
         tables.dtype, static_cast<int64_t>(cu_seqlens_q->numel()) - 1,
-        query.sizes()[0], 0, block_tables.sizes()[1], cache_blocks(k_cache, block_size, num_kv_heads, head_dim), 0,
+        query.sizes()[0], 0, block_tables.sizes()[1], cache_blocks(k_cache, block_size, num_kv_heads, head_dim), max_seqlen_q,
         static_cast<int>(query.sizes()[1]), num_kv_heads, head_dim, block_size, scale, output.data(),
         code(query.dtype()), stream));
+}
+
+void launch_prefill_attention_paged(const Tensor& query, const Tensor* cu_seqlens_q, const Tensor& k_cache,
+                                    const Tensor& v_cache, const Tensor* cu_seqlens_k, const Tensor& block_tables,
+                                    int num_kv_heads, int head_dim, int block_size, float scale, Tensor& output,
+                                    cudaStream_t stream) {
+    launch_prefill_attention_paged(query, cu_seqlens_q, k_cache, v_cache, cu_seqlens_k, block_tables, num_kv_heads, head_dim, block_size, scale,
+                                   output, stream, 0);
 }
 
 void throw_if_prefill_error(cudaStream_t stream) {
@@ -340,13 +354,13 @@ void throw_if_prefill_error(cudaStream_t stream) {
 bool flash_attn_available() { return true; }
 
 void flash_attn_varlen_fwd(const Tensor& query, const Tensor& key, const Tensor& value, const Tensor& cu_seqlens_q,
-                           const Tensor& cu_seqlens_k, int /*max_seqlen_q*/, int /*max_seqlen_k*/, float scale,
+                           const Tensor& cu_seqlens_k, int max_seqlen_q, int /*max_seqlen_k*/, float scale,
                            bool is_causal, Tensor& output, DeviceAllocator& /*allocator*/, cudaStream_t stream) {
     if (!is_causal) throw std::invalid_argument("unsupported: non-causal varlen attention");
     const int num_kv_heads = key.defined() && key.dim() == 3 ? static_cast<int>(key.sizes()[1]) : 0;
     const int head_dim = query.defined() && query.dim() == 3 ? static_cast<int>(query.sizes()[2]) : 0;
     launch_prefill_attention_dense(query, &cu_seqlens_q, key, value, &cu_seqlens_k, num_kv_heads, head_dim, scale, output,
-                                   stream);
+                                   stream, max_seqlen_q);
 }
 
 }  // namespace nano_vllm

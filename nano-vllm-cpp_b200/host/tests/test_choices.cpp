@@ -1,0 +1,82 @@
+// Which kernel a call takes, from the sizes that the host knows; no GPU.
+#include "../../csrc/nvk_internal.cuh"
+#include "check.h"
+
+#include <vector>
+
+using namespace nvk;
+
+namespace {
+
+// A causal prefill of prompts of these lengths; behind a prefix of `prefix` keys each with paged keys (tables of the longest's width).
+PrefillArgs prefill(int heads, int kv_heads, const std::vector<int>& lens, bool paged, int prefix = 0, bool longest_known = false) {
+    static char buffer[64] __attribute__((aligned(64)));
+    PrefillArgs a{};
+    a.q = a.k = a.v = a.k_cache = a.v_cache = a.out = buffer;
+    a.cu_q = a.cu_k = IndexArray(buffer, 0);
+    int longest = 0;
+    for (int n : lens) {
+        a.total_q += n;
+        a.total_k += n + prefix;
+        if (n > longest) longest = n;
+    }
+    a.num_seqs = static_cast<int64_t>(lens.size());
+    a.num_heads = heads; a.num_kv_heads = kv_heads; a.head_dim = 128; a.block_size = 256; a.scale = 0.088f; a.dtype = NVK_BF16;
+    a.max_seqlen_q = longest_known ? longest : 0;
+    if (paged) {
+        a.block_tables = IndexArray(buffer, 0);
+        a.max_blocks = (longest + prefix + 255) / 256;
+        a.num_cache_blocks = 4096;
+    }
+    return a;
+}
+std::vector<int> one_and(int longest, int others, int length) {
+    std::vector<int> lens(1 + static_cast<size_t>(others), length);
+    lens[0] = longest;
+    return lens;
+}
+
+}  // namespace
+
+// A long prompt among short ones belongs to the tcgen05 kernel (measured, us: tcgen05 / tiles of 64 rows), whether its length is given or not.
+TEST_CASE(prefill_of_one_long_prompt_among_short_ones) {
+    for (bool known : {false, true}) {
+        CHECK(!prefill_takes_tiles(prefill(32, 8, one_and(2000, 63, 8), false, 0, known)));    // 54 / 117
+        CHECK(!prefill_takes_tiles(prefill(4, 1, one_and(2000, 31, 40), false, 0, known)));    // 30 / 55
+        CHECK(!prefill_takes_tiles(prefill(8, 2, one_and(1500, 15, 5), false, 0, known)));     // 24 / 40
+        CHECK(!prefill_takes_tiles(prefill(8, 4, one_and(1000, 3, 40), false, 0, known)));     // 18 / 23
+        CHECK(!prefill_takes_tiles(prefill(16, 8, one_and(600, 31, 8), true, 0, known)));      // 17 / 21
+        CHECK(!prefill_takes_tiles(prefill(32, 8, one_and(400, 7, 4), false, 0, known)));      // 12 / 15
+        CHECK(!prefill_takes_tiles(prefill(2, 1, one_and(1000, 8, 50), false, 0, known)));     // 18 / 22
+    }
+}
+
+// Small steps stay with the tiles, one prompt or several that are alike.
+TEST_CASE(prefill_of_small_steps) {
+    CHECK(prefill_takes_tiles(prefill(32, 8, {10}, true)));              // 6.6 / 3.9
+    CHECK(prefill_takes_tiles(prefill(32, 8, {77}, true, 512)));         // 13.8 / 12.1
+    CHECK(prefill_takes_tiles(prefill(32, 8, {8}, true, 256)));          // 10.2 / 6.4
+    CHECK(prefill_takes_tiles(prefill(4, 1, {670}, true)));              // 15.1 / 11.1
+    CHECK(prefill_takes_tiles(prefill(4, 1, {8, 12, 16, 20}, true, 1024)));                     // 19.6 / 9.2
+    CHECK(prefill_takes_tiles(prefill(16, 8, std::vector<int>(31, 8), true)));                  // 9.9 / 5.4
+    CHECK(prefill_takes_tiles(prefill(32, 8, std::vector<int>(8, 50), false, 0, true)));
+    CHECK(!prefill_takes_tiles(prefill(32, 8, {512, 1024, 2048}, true)));
+}
+
+// Lengths that do not go together, and the least there can be: the choice is some kernel, not a division by zero.
+TEST_CASE(prefill_of_odd_sizes) {
+    PrefillArgs a = prefill(8, 2, {1}, false);
+    for (int64_t seqs : {1, 2, 3, 1000}) {
+        for (int64_t rows : {1, 2, 3, 999, 1000, 1001}) {
+            for (int longest : {0, 1, 2, 500, 100000}) {
+                a.num_seqs = seqs; a.total_q = rows; a.max_seqlen_q = longest;
+                for (int64_t keys : {int64_t{0}, int64_t{1}, rows, 10 * rows}) { a.total_k = keys; prefill_takes_tiles(a); }
+            }
+        }
+    }
+    a.cu_q = a.cu_k = IndexArray();
+    a.num_seqs = 0; a.total_q = a.total_k = 1;
+    CHECK(prefill_takes_tiles(a));
+}
+
+int main() { return check::run_all(); }

@@ -27,6 +27,12 @@ def test_host_logic_without_a_gpu():
     assert "0 failed" in res.stdout
 
 
+def test_which_kernel_a_call_takes():
+    res = _run("test_choices")
+    assert res.returncode == 0, res.stdout + res.stderr
+    assert "0 failed" in res.stdout
+
+
 @pytest.mark.gpu
 def test_operator_layer_known_answers_on_gpu():
     res = _run("test_host_gpu")
