@@ -386,6 +386,11 @@ int launch_merge_typed(const dec::DecodeParams& p, cudaStream_t stream) {
     return check_launch("decode_merge_kernel launch");
 }
 
+int check_grid(const DecodeArgs& a, const dec::DecodeParams& p) {   // of decode_split_kernel
+    if (a.batch > 65535 || p.num_splits > 65535) return fail(NVK_ERR_UNSUPPORTED, "decode attention: batch or split count exceeds grid limits");
+    return NVK_OK;
+}
+
 template <class F, typename T>
 int launch_typed(const DecodeArgs& a, const void* k_scale, const void* v_scale) {
     constexpr int kSmem = static_cast<int>(sizeof(GroupSmem<F>));
@@ -420,7 +425,7 @@ int launch_typed(const DecodeArgs& a, const void* k_scale, const void* v_scale) 
         if (e != cudaSuccess) return fail(NVK_ERR_CUDA, "decode_cluster_kernel launch: %s", cudaGetErrorString(e));
         return check_launch("decode_cluster_kernel launch");
     }
-    if (a.batch > 65535 || p.num_splits > 65535) return fail(NVK_ERR_UNSUPPORTED, "decode attention: batch or split count exceeds grid limits");
+    if (const int rc1 = check_grid(a, p); rc1 != NVK_OK) return rc1;
     const unsigned batch = static_cast<unsigned>(a.batch), splits = static_cast<unsigned>(p.num_splits);
     const dim3 grid = p.chunk_major ? dim3(a.num_kv_heads, batch, splits) : dim3(a.num_kv_heads, splits, batch);
     const cudaError_t e = launch_pdl(decode_split_kernel<F, T>, grid, dim3(kGroupThreads), kSmem, a.stream, p);
@@ -443,6 +448,14 @@ bool shape_supported(const DecodeArgs& a) {
 // The merge after a mixed step's decode half.
 int launch_decode_merge(const dec::DecodeParams& p, int dtype, cudaStream_t stream) {
     return dtype == NVK_BF16 ? launch_merge_typed<__nv_bfloat16>(p, stream) : launch_merge_typed<__half>(p, stream);
+}
+
+// Whether launch_decode_mma can run a call of this size, for callers that launch something else before it.
+int check_decode_mma(const DecodeArgs& a) {
+    dec::DecodeParams p{};
+    int cluster = 0;
+    const int rc = decode_plan(a, Cache16<__half>::kGroups, &p, &cluster);
+    return rc != NVK_OK || cluster > 0 ? rc : check_grid(a, p);
 }
 
 bool decode_mma_supported(const DecodeArgs& a) { return shape_supported(a) && aligned_to(a.q, 4); }

@@ -304,11 +304,16 @@ int nvk_attention_mixed_step(const void* p_query, const void* p_key, const void*
     // A scale that is not positive: the prefill rows take another kernel.  So do few of them, and the decode kernel runs beside that one (us a step as
     // one launch / as these: 1 prompt of 670 tokens, 5 decode rows of 400 keys, 4 / 1 heads, 22.7 / 15.0; 3 of 109 to 136, 9 of up to 1929, 16 / 4
     // heads, 20.1 / 16.2; 1 of 300, 60 of up to 4096, 4 / 1 heads, 31.6 / 27.4).
-    const bool small = prefill_tc_supported(pa) && prefill_takes_tiles(pa);
-    if (small || !prefill_tc_supported(pa)) {
-        const int rc = launch_prefill(pa);
-        da.beside = small;
-        return rc != NVK_OK ? rc : launch_decode_mma(da);
+    // More decode rows than the decode kernel's grid has room for stay in one launch, or are refused before anything is launched.
+    const bool one_launch = prefill_tc_supported(pa), small = one_launch && prefill_takes_tiles(pa);
+    if (small || !one_launch) {
+        int rc = check_decode_mma(da);
+        if (rc == NVK_OK) {
+            rc = launch_prefill(pa);
+            da.beside = small;
+            return rc != NVK_OK ? rc : launch_decode_mma(da);
+        }
+        if (!one_launch) return rc;
     }
     return launch_mixed_step(pa, da, prefill_blocks);
 }

@@ -146,6 +146,7 @@ int launch_decode_simt(const DecodeArgs& a);
 bool decode_mma_supported(const DecodeArgs& a);
 size_t decode_mma_workspace_bytes(int64_t batch, int num_heads, int num_kv_heads, int head_dim,
                                   int64_t max_blocks, int block_size);
+int check_decode_mma(const DecodeArgs& a);
 int launch_decode_mma(const DecodeArgs& a);
 namespace dec { struct DecodeParams; }
 int decode_plan(const DecodeArgs& a, int groups, dec::DecodeParams* out, int* cluster);

@@ -214,3 +214,26 @@ def test_a_small_prefill_beside_decode_is_done_when_the_next_kernel_starts(batch
         graph.replay()
     torch.cuda.synchronize()
     assert lib.prefill_status() == 0 and bool(right)
+
+
+def test_a_small_prefill_beside_more_decode_rows_than_a_grid_has_room_for():
+    """70000 decode rows of at most one key: one launch, as for any prefill part; with a scale that is not positive refused, and nothing written."""
+    lib, bf, rows = nvk(), torch.bfloat16, 70000
+    p = workloads().make_prefill_workload([10], [0], 2, 1, 128, 256, seed=3, paged=True)
+    kc, vc, pq, cu, pt = to_dev(p["k_cache"], bf), to_dev(p["v_cache"], bf), to_dev(p["q"], bf), to_dev(p["cu_q"]), to_dev(p["block_tables"])
+    dq = torch.ones((rows, 2, 128), dtype=bf, device="cuda")
+    ctx = torch.arange(rows, dtype=torch.int32, device="cuda") % 2
+    dt = torch.full((rows, 1), int(p["block_tables"][0, 0]), dtype=torch.int32, device="cuda")
+    ws = torch.empty(max(16, lib.decode_attention_workspace_bytes(rows, 2, 1, 128, 1, 256)), dtype=torch.uint8, device="cuda")
+    p_out, d_out = torch.full_like(pq, 7.0), torch.full_like(dq, 7.0)
+    with pytest.raises(ValueError):
+        lib.attention_mixed_step(pq, cu, None, None, cu, pt, p_out, dq, ctx, dt, d_out, kc, vc, 1, 128, 256, -p["scale"], ws)
+    torch.cuda.synchronize()
+    assert bool((p_out == 7.0).all()) and bool((d_out == 7.0).all())
+    lib.attention_mixed_step(pq, cu, None, None, cu, pt, p_out, dq, ctx, dt, d_out, kc, vc, 1, 128, 256, p["scale"], ws)
+    torch.cuda.synchronize()
+    assert lib.prefill_status() == 0
+    assert_attention_close(to_np(p_out), oracle.prefill_attention_paged(p["q"], p["k_cache"], p["v_cache"], p["cu_q"], p["cu_k"], p["block_tables"], 1, 128, 256,
+                                                                        p["scale"]))
+    first = vc[int(p["block_tables"][0, 0]), 0]                            # [1, 128]: a row of one key is that key's value
+    assert torch.equal(d_out, (first * ctx[:, None, None].to(bf)).expand_as(d_out))
