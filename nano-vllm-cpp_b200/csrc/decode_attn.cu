@@ -221,9 +221,8 @@ __global__ void __launch_bounds__(kGroupThreads, F::kGroups) decode_cluster_kern
 // Blocks per (sequence, KV head) of the cluster kernel, or 0: chunks.  Only clusters that are all resident at once: a cluster has to fit
 // into one GPC, so that these are fewer than the places for single blocks (the driver's occupancy query for these kernels at two and
 // three blocks per SM).  With one more a second wave follows: clusters of 4, 1024 keys, 70 -> 72 pairs 11.0 -> 15.6 us a call, clusters of
-// 8, 300 keys, 32 -> 34 pairs 5.8 -> 9.4 (in one block each 5.7).  Clusters of 2 gain nothing on whole contexts in one block each (80 pairs of
-// 300 / 1024 keys 8.5 / 12.2 us, 6.6 / 11.8), nor do clusters of 4 in tables of up to 512 keys (64 pairs of 300 / 512 keys 7.6 / 8.7, 6.4 / 7.8).
-// Without a workspace there is nothing else, and any cluster that fits is taken.
+// 8, 300 keys, 32 -> 34 pairs 5.8 -> 9.4 (in one block each 5.7).  Clusters of 4 gain nothing in tables of up to 512 keys (64 pairs of 300 / 512 keys
+// 7.6 / 8.7 us, in one block each 6.4 / 7.8), nor clusters of 2 on equal ranges (their halves of a table's row: see below).  Without a workspace there is nothing else, and any cluster that fits is taken.
 struct ClusterWay { int size, resident[2]; };
 constexpr ClusterWay kWays[] = {{8, {33, 48}}, {4, {71, 104}}, {2, {148, 222}}};
 int cluster_size(int64_t batch, int num_kv_heads, int64_t max_blocks, int block_size, int groups, bool have_workspace) {
@@ -241,39 +240,45 @@ bool just_past_a_wave(int64_t pairs, int groups) {
     return pairs > kSmCount * groups && (groups == 2 ? 4 * pairs < 5 * kSmCount * groups : 3 * pairs < 4 * kSmCount * groups);
 }
 
-// Halves of a table row, merged in a cluster of two blocks: where both halves of all contexts find a place at once (a cluster of more than two, or single
-// blocks and a second kernel, were slower on average over contexts that are all as long as the table, down to half of it and down to a twentieth).
-// 16-bit caches, 110 pairs of 0.05 / 0.5 / 1.0 to 2048 keys: 18.2 / 20.9 / 24.4 us a pass, in chunks of 512 19.8 / 26.5 / 29.1; 128 of 4096 30.8 / 37.8 / 47.1,
-// 35.4 / 43.4 / 51.8; 144 of 8192 55.6 / 74.0 / 95.0, 61.8 / 77.1 / 97.9; at 16384 keys nothing is left of it, and few pairs of spread contexts lose (96 of 8192
-// 46 / 52 / 64, 42 / 58 / 74).  8-bit ones: 128 pairs of 2048 17.3 / 18.1 / 18.5, 17.7 / 19.7 / 24.6; 200 of 1536 18.9 / 19.6 / 20.3, 18.9 / 24.6 / 26.4; but 148
-// of 2048 21.3 / 22.3 / 22.7, 18.7 / 24.2 / 26.1, and up to 768 keys whole contexts are as quick.  Fewer pairs than clusters of
-// four hold take those, or more chunks.
+// How a step beyond the clusters is shared out.  Contexts are rarely as long as the table: a step has one long one among short ones, or a third of them, or
+// an even spread.  Figures are us in a replayed graph with inputs beyond L2, for contexts of which one / a tenth / a third fill the table and the others 1/32
+// or 1/16 of it, and for spreads of 0.05 / 0.5 / 1.0 to all of the table.
+//
+// Halves of a table row, merged in a cluster of two blocks, where both halves of all contexts find a place at once and a half is short enough for one long
+// context not to be what a step waits for.  16-bit caches, 110 pairs of 2048 keys 10.4 / 12.3 / 13.8, 14.3 / 16.9 / 21.3, in chunks of 512 10.1 / 11.8 /
+// 13.3, 16.1 / 22.4 / 24.9; of 3072 14.0 / 16.4 / 18.6, 19.6 / 23.2 / 30.1, in chunks of 1024 13.3 / 15.9 / 17.8, 20.9 / 26.7 / 38.1.  But 90 pairs of 3072
+// 13.8 / 15.7 / 18.2, 18.8 / 20.8 / 26.7, in chunks of 512 8.8 / 10.9 / 13.7, 18.9 / 23.2 / 27.8; and 128 of 4096 17.9 / 20.7 / 23.7, 26.3 / 33.6 / 43.5, in
+// chunks of 512 10.8 / 13.2 / 21.0, 29.0 / 37.7 / 47.3.  8-bit ones: 200 of 1536 10.1 / 13.3 / 16.5, 17.8 / 18.5 / 19.0, in chunks of 512 10.8 / 14.1 / 16.2,
+// 17.0 / 22.1 / 23.8; but 128 of 2048 11.9 / 15.0 / 18.8, 20.4 / 21.1 / 21.4, in chunks of 512 10.2 / 13.8 / 15.8, 16.5 / 17.9 / 21.6.  Fewer pairs than
+// clusters of four hold take those, or more chunks; in tables of up to 512 (8-bit: 768) keys whole contexts are as quick.
 bool halves(int64_t pairs, int64_t max_tokens, int groups) {
     if (pairs <= kWays[1].resident[groups == 3] || 2 * pairs > static_cast<int64_t>(kSmCount) * groups) return false;
-    return groups == 2 ? max_tokens > 512 && max_tokens <= (pairs < 110 ? 4096 : 8192) : max_tokens > 768 && max_tokens <= (pairs > 130 ? 1536 : 2048);
+    return groups == 2 ? max_tokens > 512 && max_tokens <= (pairs < 104 ? 2048 : 3072) : max_tokens > 768 && max_tokens <= 1536;
 }
 
-// Chunk length in keys (whole cache blocks), from the number of (sequence, KV head) pairs and the table's width; us a pass below, for contexts of
-// 0.05 / 0.5 / 1.0 to all of the table.
-// Whole contexts: no merge, no second launch.
-//   * Tables of up to 1024 keys: 176 pairs of 1024 keys 19.3 a call, as two chunks 23.7; 264 24.6, 29.1; 432 int8 ones 24.3, 30.5.
-//   * Tables of up to 4096 keys (3072 below 180 pairs) where the halves above have no room: 184 pairs of 2048 keys 25.0 / 29.6 / 34.2, in chunks of 1024 25.7 / 34.4 / 42.7; 264 of
-//     4096 52.7 / 68.7 / 85.3, chunks of 2048 58.6 / 74.7 / 90.7.  But not just past a wave: 304 / 352 pairs, all of 4096 keys, 116.8 / 123.7 a call, in chunks
-//     of 2048 106.1 / 113.5.  8-bit caches up to 1536 keys (272 pairs 23.7 / 25.5 / 28.4, 23.2 / 26.0 / 30.9; but 256 e4m3 ones of 0.05 to all of 2048 keys 25.9, in
-//     chunks 25.2, and 272 int8 ones 31.4, 28.3), 4096 with a pair for every resident group.
-// Chunks otherwise, of 2048 or, with few pairs and up to 8192 keys, of 1024 (224 pairs of 6144 keys 64.1 / 86.4 / 111.1, 69.7 / 88.2 / 114.5 in chunks of 2048; 8-bit
-// 55.0 / 70.6 / 87.4 for 8192, 60.4 / 73.5 / 89.2), halved down to 256 while they leave resident groups without a block.
+// Chunk length in keys (whole cache blocks), from the number of (sequence, KV head) pairs and the table's width.  Whole contexts (no merge, no second launch)
+// where a block reads one in little time, or where the step has more of them than places:
+//   * 16-bit: tables of up to 1024 keys, 1536 where the halves above have no room (152 pairs 12.8 / 15.0 / 17.5, 16.9 / 18.9 / 21.8, in chunks of 1024 11.8 /
+//     14.7 / 16.8, 17.3 / 20.4 / 25.1).  8-bit: 1024 with few pairs, 768 from 1.5 to an SM on, 1280 from two (320 pairs 13.3 / 18.1 / 23.1, 22.4 / 23.6 /
+//     25.6, in chunks of 1024 14.2 / 18.0 / 23.0, 23.8 / 24.8 / 26.8).
+//   * Tables of up to 4096 keys with a pair for every resident group, but not just past a wave: 304 / 352 16-bit pairs, all of 4096 keys, 116.8 / 123.7 a
+//     call, in chunks of 2048 106.1 / 113.5.
+// Chunks of 512 where the table has up to 4096 keys (8-bit: 1536) and single contexts leave places free: 200 16-bit pairs of 4096 keys 13.0 / 17.5 / 29.6,
+// 40.3 / 54.2 / 68.0, of 2048 20.9 / 26.7 / 30.9, 41.1 / 58.6 / 70.1, whole 30.7 / 35.9 / 40.9, 42.7 / 53.6 / 68.3; 256 int8 pairs of 1536 10.8 / 15.0 /
+// 17.3, 21.2 / 25.1 / 27.4, of 1024 13.8 / 18.2 / 21.1, 23.1 / 24.7 / 29.6, whole 15.2 / 20.4 / 25.6, 24.7 / 26.3 / 28.2.  Chunks of 1024 in tables of up to
+// 8192 keys with few pairs: 224 of 6144 17.2 / 25.1 / 45.3, 60.9 / 83.3 / 107.9, of 2048 22.1 / 30.8 / 46.9, 65.7 / 85.0 / 111.9.  Chunks of 2048 otherwise.
+// All halved down to 256 while they leave resident groups without a block:
 //   * What a table of 2048 keys is cut into is cut no finer than it takes to have 1.5 blocks per SM (8-bit: 2.25 of 512 keys).
-//   * Longer ones need every place filled, since contexts are often shorter than the table (64 pairs of 1000 keys, 4096-key tables: 512-key
-//     chunks 12.0, 1024-key ones 14.9), but 512 keys are not cut for the last few (36 pairs of 4096 keys 19.0, as chunks of 256 21.0).
+//   * Longer ones need every place filled, since contexts are often shorter than the table (64 pairs of 1000 keys, 4096-key tables: 512-key chunks 12.0,
+//     1024-key ones 14.9), but 512 keys are not cut for the last few (36 pairs of 4096 keys 19.0, as chunks of 256 21.0).
 // (Whole contexts of 8192-key tables, 256 sequences: 694 us a pass, 689 with chunks.)
 int chunk_tokens(int64_t batch, int num_kv_heads, int64_t max_blocks, int block_size, int groups) {
     const int64_t max_tokens = max_blocks * block_size, pairs = batch * num_kv_heads, resident = static_cast<int64_t>(kSmCount) * groups;
-    if (max_tokens <= 1024) return static_cast<int>(max_tokens);
-    const int64_t whole = groups == 2 ? (pairs < 180 ? 3072 : just_past_a_wave(pairs, groups) ? 2048 : 4096) : 1536;
-    if (2 * pairs > resident && max_tokens <= whole) return static_cast<int>(max_tokens);
-    if (max_tokens <= 4096 && pairs >= resident && !just_past_a_wave(pairs, groups)) return static_cast<int>(max_tokens);
-    int64_t chunk = max_tokens <= 8192 && (groups == 2 ? max_tokens > 4096 && pairs < 2 * resident : 5 * pairs < 4 * resident) ? 1024 : 2048;
+    const int64_t whole = groups == 2 ? (2 * pairs > resident ? 1536 : 1024) : pairs >= 2 * kSmCount ? 1280 : 2 * pairs <= resident ? 1024 : 768;
+    if (max_tokens <= whole || (max_tokens <= 4096 && pairs >= resident && !just_past_a_wave(pairs, groups))) return static_cast<int>(max_tokens);
+    int64_t chunk = 2048;
+    if (groups == 2 ? max_tokens > 2048 && max_tokens <= 4096 && pairs < resident : max_tokens <= 1536 && pairs < 2 * kSmCount) chunk = 512;
+    else if (groups == 2 ? max_tokens > 4096 && max_tokens <= 8192 && pairs < 2 * resident : max_tokens <= 8192 && 5 * pairs < 4 * resident) chunk = 1024;
     for (; chunk > 256; chunk >>= 1) {
         const int64_t parts = (max_tokens + chunk - 1) / chunk;
         const double blocks_per_sm = groups == 2 ? (max_tokens <= 2048 ? 1.5 : chunk <= 512 ? 1.8 : 2.0)

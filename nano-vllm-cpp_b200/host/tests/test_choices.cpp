@@ -36,6 +36,14 @@ std::vector<int> one_and(int longest, int others, int length) {
     return lens;
 }
 
+// Parts of `tokens` keys each of tables of `table` keys, the cache blocks of 256: what the workspace has to hold.
+size_t parts(int64_t pairs, int64_t table, int64_t tokens, int group) {
+    return static_cast<size_t>(pairs * (table / tokens) * group) * (128 * sizeof(float) + 2 * sizeof(float));
+}
+size_t workspace(int64_t batch, int kv_heads, int64_t table, int group) {
+    return nvk_decode_attention_workspace_bytes(batch, group * kv_heads, kv_heads, 128, table / 256, 256);
+}
+
 }  // namespace
 
 // A long prompt among short ones belongs to the tcgen05 kernel (measured, us: tcgen05 / tiles of 64 rows), whether its length is given or not.
@@ -77,6 +85,17 @@ TEST_CASE(prefill_of_odd_sizes) {
     a.cu_q = a.cu_k = IndexArray();
     a.num_seqs = 0; a.total_q = a.total_k = 1;
     CHECK(prefill_takes_tiles(a));
+}
+
+// One long context among short ones must not be read by one block or two while others have nothing to do (us for 16-bit caches, one context as long
+// as the table and the others 1/32 of it: whole or in halves / in these chunks).
+TEST_CASE(decode_contexts_are_cut_where_one_may_be_long) {
+    CHECK(workspace(200, 1, 4096, 4) >= parts(200, 4096, 512, 4));      // 30.7 / 13.0
+    CHECK(workspace(35, 8, 4096, 4) >= parts(280, 4096, 512, 4));       // 31.4 / 15.6
+    CHECK(workspace(20, 8, 3072, 4) >= parts(160, 3072, 512, 4));       // 23.4 / 10.8
+    CHECK(workspace(128, 1, 4096, 4) >= parts(128, 4096, 512, 4));      // 17.9 / 10.8
+    CHECK(workspace(23, 8, 2048, 4) >= parts(184, 2048, 1024, 4));      // 16.4 / 13.1
+    CHECK(workspace(140, 1, 8192, 4) >= parts(140, 8192, 1024, 4));     // 31.6 / 15.1
 }
 
 int main() { return check::run_all(); }

@@ -132,3 +132,34 @@ def test_halves_of_a_table_in_clusters_of_two(kv, hq, hkv, bs, batch, table_bloc
         k, v = ((plain(x) * s.float()[..., None]).cpu().numpy() for x, s in ((k8, ks), (v8, vs)))   # on the same quantised cache
     ref = oracle.decode_attention_paged(w["q"], k, v, w["context_lens"], w["block_tables"], hkv, 128, bs, w["scale"])
     assert_attention_close(to_np(out), ref)
+
+
+@pytest.mark.parametrize("kv,hq,hkv,bs,batch,table_blocks", [
+    ("same", 4, 1, 256, 149, 7), ("same", 8, 4, 64, 56, 41), ("same", 8, 1, 256, 295, 16), ("same", 4, 2, 256, 52, 12), ("same", 16, 8, 16, 10, 160),   # 1024- and 512-key chunks
+    ("same", 4, 1, 256, 72, 9), ("same", 4, 1, 256, 103, 12), ("same", 6, 3, 48, 34, 43), ("same", 8, 8, 256, 18, 26), ("same", 2, 1, 256, 149, 6),   # beside halves; whole
+    ("same", 6, 2, 48, 37, 41), ("same", 8, 8, 256, 18, 12), ("same", 4, 1, 16, 104, 192),                                                           # halves as far as they go
+    ("int8", 4, 1, 256, 223, 4), ("fp8", 8, 1, 256, 240, 6), ("int8", 8, 8, 64, 30, 20), ("fp8", 4, 4, 256, 74, 5), ("int8", 2, 1, 256, 106, 7), ("fp8", 6, 1, 256, 223, 3),
+])
+def test_contexts_of_unequal_length_in_chunks(kv, hq, hkv, bs, batch, table_blocks):
+    """Contexts that end at the edges of 256-, 512- and 1024-key chunks and with the table, among short and empty ones."""
+    full = table_blocks * bs
+    edges = [min(n, full) for n in (full, 5, 0, 511, 512, 17, 513, full - 1, 40, 1023, 1024, 1, 1025, 255, 257, 3)]
+    lens = [edges[i % 16] for i in range(batch)]
+    w = workloads().make_decode_workload(batch, hq, hkv, 128, bs, 0, 0, seed=batch + 1, context_lens=np.array(lens, np.int32), pad_blocks_to=table_blocks)
+    bf, lib = torch.bfloat16, nvk()
+    q, ctx, bt = to_dev(w["q"], bf), to_dev(w["context_lens"]), to_dev(w["block_tables"])
+    kc, vc = to_dev(w["k_cache"], bf), to_dev(w["v_cache"], bf)
+    ws, out = _workspace(batch, hq, hkv, bt.shape[1], bs), torch.full_like(q, float("nan"))
+    if kv == "same":
+        lib.launch_decode_attention_paged(q, kc, vc, ctx, bt, hkv, 128, bs, w["scale"], out, ws)
+        k, v = w["k_cache"], w["v_cache"]
+    else:
+        store, decode = ((lib.store_kvcache_int8, lib.launch_decode_attention_paged_int8) if kv == "int8" else
+                         (lib.store_kvcache_fp8, lib.launch_decode_attention_paged_fp8))
+        k8, v8 = (torch.empty(kc.shape, dtype=torch.int8 if kv == "int8" else torch.uint8, device="cuda") for _ in range(2))
+        ks, vs = (torch.empty(kc.shape[:-1], dtype=torch.float16, device="cuda") for _ in range(2))
+        store(kc.view(-1, hkv, 128), vc.view(-1, hkv, 128), k8, v8, ks, vs, torch.arange(ks.numel() // hkv, dtype=torch.int32, device="cuda"))
+        decode(q, k8, v8, ks, vs, ctx, bt, hkv, 128, bs, w["scale"], out, ws)
+        plain = (lambda x: x.float()) if kv == "int8" else (lambda x: x.view(torch.float8_e4m3fn).float())
+        k, v = ((plain(x) * s.float()[..., None]).cpu().numpy() for x, s in ((k8, ks), (v8, vs)))   # on the same quantised cache
+    assert_attention_close(to_np(out), oracle.decode_attention_paged(w["q"], k, v, w["context_lens"], w["block_tables"], hkv, 128, bs, w["scale"]))
