@@ -5,7 +5,7 @@
 // the per-tensor attribute look-ups and the stream query took about 14 us, more than the kernels they launch.  Here a call
 // reads the tensors' fields directly and takes well under a microsecond on top of the launches themselves.  Each function
 // takes its arguments by position (the Python wrappers in __init__.py carry names and defaults) and returns how many
-// kernels it launched.
+// kernels it launched (decode: at least).
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -157,9 +157,9 @@ struct Decode {
           bt(cuda("block_tables", bt_)), out(cuda("output", out_)), lens("context_lens", &ctx), tables("block_tables", &bt),
           batch(size(q, 0, "query")), heads(size(q, 1, "query")), max_blocks(size(bt, 1, "block_tables")), hkv(integer(hkv_)), d(integer(d_)),
           bs(integer(bs_)), blocks(cache_blocks(kc, bs, hkv, d)), scale(real(scale_)) {}
+    // At least: contexts of wider tables are always taken in chunks, which a second kernel brings together; narrower ones may be.
     long launches(const at::Tensor* ws) const {
-        return ws != nullptr && nvk_decode_attention_workspace_bytes(batch, static_cast<int>(heads), static_cast<int>(hkv), static_cast<int>(d),
-                                                                     max_blocks, static_cast<int>(bs)) > 0 ? 2 : 1;
+        return ws != nullptr && d == 128 && q.scalar_type() != at::kFloat && heads <= 8 * hkv && bs % 16 == 0 && max_blocks * bs > 4096 ? 2 : 1;
     }
 };
 

@@ -13,6 +13,7 @@
 // Which one is taken depends on the table's WIDTH, not on the contexts: one short sequence in a wide table takes chunks and a merge.
 #include "decode_body.cuh"
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 
@@ -289,6 +290,21 @@ int chunk_tokens(int64_t batch, int num_kv_heads, int64_t max_blocks, int block_
     return static_cast<int>(chunk < max_tokens ? chunk : max_tokens);
 }
 
+// The most parts that a step of up to so many pairs with tables of up to so many keys is shared out into, beyond one for each 2048 keys of a pair (these
+// grow with both): clusters and halves, chunks that were halved to fill the chip, then the lines of chunk_tokens where 16-bit caches begin with 512 and
+// 1024 keys (8-bit caches stay below them).
+int64_t most_parts(int64_t pairs, int64_t max_tokens) {
+    auto up_to = [&](int64_t most_pairs, int64_t most_tokens, int64_t chunk) {
+        return (pairs < most_pairs ? pairs : most_pairs) * (((max_tokens < most_tokens ? max_tokens : most_tokens) + chunk - 1) / chunk);
+    };
+    const int64_t each = (max_tokens + 255) / 256, filling = 2 * 3 * kSmCount;   // (at most 3 blocks per SM before the last halving)
+    int64_t parts = pairs * (each > kMaxCluster ? each : kMaxCluster);
+    if (parts > filling) parts = filling;
+    if (max_tokens > 2048) parts = std::max(parts, up_to(2 * kSmCount - 1, 4096, 512));
+    if (max_tokens > 4096) parts = std::max(parts, up_to(4 * kSmCount - 1, 8192, 1024));
+    return parts;
+}
+
 // Split-K scratch of the chunked split that earlier versions of this library used (chunks of 256 to 2048 keys).  The public
 // workspace size never falls below it, because the limit of nvk_decode_attention_paged_static and what counts as a problem that
 // needs no scratch at all are stated in terms of it.
@@ -465,8 +481,8 @@ int check_decode_mma(const DecodeArgs& a) {
 
 bool decode_mma_supported(const DecodeArgs& a) { return shape_supported(a) && aligned_to(a.q, 4); }
 
-size_t decode_mma_workspace_bytes(int64_t batch, int num_heads, int num_kv_heads, int head_dim,
-                                  int64_t max_blocks, int block_size) {
+size_t decode_mma_workspace_needed(int64_t batch, int num_heads, int num_kv_heads, int head_dim,
+                                   int64_t max_blocks, int block_size) {
     if (batch <= 0 || num_heads <= 0 || num_kv_heads <= 0 || max_blocks <= 0 || block_size <= 0) return 0;
     size_t need = chunk_scratch_bytes(batch, num_heads, num_kv_heads, head_dim, max_blocks, block_size);
     for (int groups : {Cache16<__half>::kGroups, Cache8<__half, false>::kGroups}) {
@@ -475,6 +491,20 @@ size_t decode_mma_workspace_bytes(int64_t batch, int num_heads, int num_kv_heads
         if (n > need) need = n;
     }
     return need;
+}
+
+// The same for every call with no more sequences and no wider tables: a smaller one may be cut into more parts (8 sequences of 1024 keys, 8 KV heads, take
+// clusters of four, 32 whole contexts), and callers keep one workspace for all of them.
+size_t decode_mma_workspace_bytes(int64_t batch, int num_heads, int num_kv_heads, int head_dim,
+                                  int64_t max_blocks, int block_size) {
+    const size_t need = decode_mma_workspace_needed(batch, num_heads, num_kv_heads, head_dim, max_blocks, block_size);
+    if (batch <= 0 || num_heads <= 0 || num_kv_heads <= 0 || max_blocks <= 0 || block_size <= 0) return need;
+    const int group = (num_heads + num_kv_heads - 1) / num_kv_heads;
+    const size_t most = part_bytes(static_cast<size_t>(most_parts(batch * num_kv_heads, max_blocks * block_size)), group);
+    // What fits the static array never needs more than it holds; what fills it but for the last 4 bytes a row of 520 goes on in longer chunks (above), a
+    // slightly smaller one fills it.
+    if (need <= kStaticScratchBytes && (most > kStaticScratchBytes || need + need / 128 > kStaticScratchBytes)) return kStaticScratchBytes;
+    return most > need ? most : need;
 }
 
 bool decode_int8_mma_supported(const DecodeInt8Args& x) {
@@ -550,7 +580,7 @@ extern "C" int nvk_decode_attention_paged_static(const void* query, const void* 
                                                  int num_heads, int num_kv_heads, int head_dim, int block_size,
                                                  float scale, void* output, int dtype, void* stream) {
     using namespace nvk;
-    const size_t need = nvk_decode_attention_workspace_bytes(batch, num_heads, num_kv_heads, head_dim, max_blocks, block_size);
+    const size_t need = decode_mma_workspace_needed(batch, num_heads, num_kv_heads, head_dim, max_blocks, block_size);
     if (need > kStaticScratchBytes)
         return fail(NVK_ERR_INVALID_ARGUMENT,
                     "decode attention (static scratch): this problem needs %zu bytes of split-K scratch but the built-in "

@@ -114,7 +114,7 @@ int nvk_decode_attention_paged(const void* query, const void* k_cache, const voi
                  static_cast<cudaStream_t>(stream)};
     if (decode_mma_supported(a)) {
         if (workspace != nullptr) {
-            const size_t need = decode_mma_workspace_bytes(batch, num_heads, num_kv_heads, head_dim, max_blocks, block_size);
+            const size_t need = decode_mma_workspace_needed(batch, num_heads, num_kv_heads, head_dim, max_blocks, block_size);
             if (workspace_bytes < need)
                 return fail(NVK_ERR_INVALID_ARGUMENT, "decode attention: workspace of %zu bytes given, %zu needed",
                             workspace_bytes, need);
@@ -167,7 +167,7 @@ int nvk_decode_attention_paged_int8(const void* query, const void* k_cache, cons
                      k_scale, v_scale};
     if (decode_int8_mma_supported(a)) {
         if (workspace != nullptr) {
-            const size_t need = decode_mma_workspace_bytes(batch, num_heads, num_kv_heads, head_dim, max_blocks, block_size);
+            const size_t need = decode_mma_workspace_needed(batch, num_heads, num_kv_heads, head_dim, max_blocks, block_size);
             if (workspace_bytes < need)
                 return fail(NVK_ERR_INVALID_ARGUMENT, "decode attention (int8): workspace of %zu bytes given, %zu needed",
                             workspace_bytes, need);
@@ -219,7 +219,7 @@ int nvk_decode_attention_paged_fp8(const void* query, const void* k_cache, const
         return fail(NVK_ERR_UNSUPPORTED, "decode attention (fp8): F16 / BF16 queries, head_dim 128, at most 8 query heads per KV head, "
                                          "block_size a multiple of 16");
     if (workspace != nullptr) {
-        const size_t need = decode_mma_workspace_bytes(batch, num_heads, num_kv_heads, head_dim, max_blocks, block_size);
+        const size_t need = decode_mma_workspace_needed(batch, num_heads, num_kv_heads, head_dim, max_blocks, block_size);
         if (workspace_bytes < need)
             return fail(NVK_ERR_INVALID_ARGUMENT, "decode attention (fp8): workspace of %zu bytes given, %zu needed", workspace_bytes, need);
         if (!aligned_to(workspace, 16)) return fail(NVK_ERR_INVALID_ARGUMENT, "decode attention (fp8): workspace must be 16-byte aligned");
@@ -295,7 +295,7 @@ int nvk_attention_mixed_step(const void* p_query, const void* p_key, const void*
     DecodeArgs da{d_query, k_cache, v_cache, index_array(context_lens, context_lens_dtype), index_array(d_block_tables, d_block_tables_dtype),
                   d_output, batch, d_max_blocks, num_cache_blocks, num_heads, num_kv_heads, head_dim, block_size, scale, dtype, workspace,
                   workspace_bytes, st};
-    const size_t need = decode_mma_workspace_bytes(batch, num_heads, num_kv_heads, head_dim, d_max_blocks, block_size);
+    const size_t need = decode_mma_workspace_needed(batch, num_heads, num_kv_heads, head_dim, d_max_blocks, block_size);
     if (workspace == nullptr || workspace_bytes < need || !aligned_to(workspace, 16))
         return fail(NVK_ERR_INVALID_ARGUMENT, "mixed step: a 16-byte aligned workspace of %zu bytes is needed (nvk_decode_attention_workspace_bytes)", need);
     if (!mixed_step_supported(pa, da))

@@ -13,6 +13,7 @@
 #include <utility>
 
 #include "../../include/nvk.h"
+#include "decode_sizes.h"
 
 namespace nvk {
 

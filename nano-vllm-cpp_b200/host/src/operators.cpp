@@ -10,6 +10,8 @@
 
 #include "nvk.h"
 
+#include "../../csrc/decode_sizes.h"
+
 #include <stdexcept>
 #include <string>
 
@@ -210,7 +212,7 @@ void decode_common(const Tensor& query, const Tensor& k_cache, const Tensor& v_c
     const int64_t max_blocks = block_tables.sizes()[1];
     const int64_t blocks = cache_blocks(k_cache, block_size, num_kv_heads, head_dim);
     if (allocator != nullptr) {
-        const size_t need = nvk_decode_attention_workspace_bytes(batch, heads, num_kv_heads, head_dim, max_blocks, block_size);
+        const size_t need = nvk::decode_mma_workspace_needed(batch, heads, num_kv_heads, head_dim, max_blocks, block_size);
         Memory::Ptr scratch = need > 0 ? allocator->allocate(need, query.device()) : nullptr;
         throw_on_nvk_status(nvk_decode_attention_paged(query.data(), k_cache.data(), v_cache.data(), lens.ptr, lens.dtype,
                                                        tables.ptr, tables.dtype, batch, max_blocks, blocks, heads,
@@ -218,7 +220,7 @@ void decode_common(const Tensor& query, const Tensor& k_cache, const Tensor& v_c
                                                        code(query.dtype()), scratch ? scratch->data() : nullptr, need, stream));
         return;   // the scratch block returns to the allocator's cache; stream order keeps it valid for this launch
     }
-    const size_t need = nvk_decode_attention_workspace_bytes(batch, heads, num_kv_heads, head_dim, max_blocks, block_size);
+    const size_t need = nvk::decode_mma_workspace_needed(batch, heads, num_kv_heads, head_dim, max_blocks, block_size);
     if (need > 0 && need <= nvk_decode_attention_static_scratch_bytes()) {
         throw_on_nvk_status(nvk_decode_attention_paged_static(query.data(), k_cache.data(), v_cache.data(), lens.ptr,
                                                               lens.dtype, tables.ptr, tables.dtype, batch, max_blocks,

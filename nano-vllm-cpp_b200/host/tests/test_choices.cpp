@@ -41,7 +41,7 @@ size_t parts(int64_t pairs, int64_t table, int64_t tokens, int group) {
     return static_cast<size_t>(pairs * (table / tokens) * group) * (128 * sizeof(float) + 2 * sizeof(float));
 }
 size_t workspace(int64_t batch, int kv_heads, int64_t table, int group) {
-    return nvk_decode_attention_workspace_bytes(batch, group * kv_heads, kv_heads, 128, table / 256, 256);
+    return decode_mma_workspace_needed(batch, group * kv_heads, kv_heads, 128, table / 256, 256);
 }
 
 }  // namespace
@@ -96,6 +96,32 @@ TEST_CASE(decode_contexts_are_cut_where_one_may_be_long) {
     CHECK(workspace(128, 1, 4096, 4) >= parts(128, 4096, 512, 4));      // 17.9 / 10.8
     CHECK(workspace(23, 8, 2048, 4) >= parts(184, 2048, 1024, 4));      // 16.4 / 13.1
     CHECK(workspace(140, 1, 8192, 4) >= parts(140, 8192, 1024, 4));     // 31.6 / 15.1
+}
+
+// A workspace sized for the most sequences and the widest table is enough for every call with fewer sequences and narrower tables.
+TEST_CASE(decode_workspace_of_the_largest_call_is_enough_for_smaller_ones) {
+    constexpr size_t kStatic = 32u << 20;
+    for (int kv_heads : {1, 3, 8}) {
+        for (int group : {1, 4, 8}) {
+            for (int block_size : {16, 48, 256}) {
+                std::vector<size_t> widest(static_cast<size_t>(900 / kv_heads) + 1, 0);   // the largest need of so many sequences in narrower tables
+                for (int64_t tokens : {256, 512, 768, 1000, 1024, 1280, 1536, 2048, 2304, 3072, 4096, 5000, 6144, 8192, 10240, 16384, 30720, 32768, 40960}) {
+                    const int64_t blocks = tokens / block_size;
+                    size_t least = 0;                                                     // and of fewer sequences
+                    int wrong = 0;
+                    for (size_t batch = 1; batch < widest.size(); ++batch) {
+                        const size_t need = decode_mma_workspace_needed(static_cast<int64_t>(batch), kv_heads * group, kv_heads, 128, blocks, block_size);
+                        const size_t given = nvk_decode_attention_workspace_bytes(static_cast<int64_t>(batch), kv_heads * group, kv_heads, 128, blocks, block_size);
+                        if (need > widest[batch]) widest[batch] = need;
+                        if (widest[batch] > least) least = widest[batch];
+                        if (given < need || (given < least && !(need <= kStatic && least > kStatic))) ++wrong;
+                        if (need <= kStatic && given > kStatic) ++wrong;                  // what fits the static array still does
+                    }
+                    CHECK(wrong == 0);
+                }
+            }
+        }
+    }
 }
 
 int main() { return check::run_all(); }
