@@ -444,15 +444,15 @@ __device__ __forceinline__ void epilogue_row(const GemmParams& p, uint32_t t_row
         // Each lane the row that it has: fewest instructions, and slow.
         float inv_rms = 1.0f;
         if (x.weight != nullptr) {                 // pass 1 over the accumulator: the head's sum of squares
-            float ss = 0.0f;
+            float ss4[4] = {0.0f, 0.0f, 0.0f, 0.0f};   // (the order of the other forms: a row's bits do not depend on its tile's place)
 #pragma unroll 1
             for (int c = 0; c < 4; ++c) {
                 float v[32];
                 load_rounded<T>(t_row + c * 32, v);
 #pragma unroll
-                for (int i = 0; i < 32; ++i) ss += v[i] * v[i];
+                for (int i = 0; i < 32; ++i) ss4[i & 3] += v[i] * v[i];
             }
-            inv_rms = rsqrtf(ss / static_cast<float>(kBN) + p.eps);
+            inv_rms = rsqrtf(((ss4[0] + ss4[1]) + (ss4[2] + ss4[3])) / static_cast<float>(kBN) + p.eps);
         }
 #pragma unroll 1
         for (int c = 0; c < 2; ++c) {              // pass 2: columns [32 c, 32 c + 32) rotate with [64 + 32 c, 64 + 32 c + 32)

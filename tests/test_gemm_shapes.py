@@ -148,3 +148,50 @@ def test_sums_pushed_through_a_cluster(num_q_heads, num_kv_heads, hidden, rows):
         assert np.array_equal(to_np(vc), vc_ref)
         for got, ref in ((to_np(q_out), q_ref), (to_np(kc), kc_ref)):
             assert (np.abs(got - ref) <= np.maximum(np.abs(ref), 1e-3) * 2.0 ** -7 + 2.0 ** -9 * (not normed)).all()   # (cancelling terms of a rotation, 16-bit inputs)
+
+
+@pytest.mark.parametrize("normed", [True, False])
+@pytest.mark.parametrize("num_q_heads,num_kv_heads,hidden", [(32, 8, 4096), (32, 8, 3080), (16, 8, 4096)])   # pairs with several tiles each, and one or two
+def test_qkv_prologue_of_many_rows_does_not_depend_on_the_place_of_a_row(num_q_heads, num_kv_heads, hidden, normed):
+    """Large K: a pair's tiles but the last finish under the next one's MMAs, in a form of their own.  Equal rows have equal bits in all tiles, and the
+    first ones are what the oracle makes of the product."""
+    dt, d, max_pos, heads, rows, period = torch.float16, 128, 300, num_q_heads + 2 * num_kv_heads, 1900, 256
+    gen = torch.Generator(device="cuda").manual_seed(heads + hidden)
+    at = torch.arange(rows, device="cuda") % period
+    x = torch.randn((period, hidden), generator=gen, device="cuda").to(dt)[at].contiguous()
+    w = (torch.randn((heads * d, hidden), generator=gen, device="cuda") / hidden ** 0.5).to(dt)
+    pw = workloads().make_prologue_workload(rows, num_q_heads, num_kv_heads, d, rows, max_pos, seed=hidden)
+    table = oracle.build_cos_sin_cache(max_pos, d, pw["rope_base"])
+    pos, slots = np.arange(rows) % period + 20, np.arange(rows)[::-1].copy()
+    pos[7::period], slots[rows // 2] = max_pos, -1                       # outside the table; not stored
+    pos, slots = pos.astype(np.int32), slots.astype(np.int32)
+    qw, kw = ((1 + 0.1 * torch.randn(d, generator=gen, device="cuda")).to(dt) for _ in range(2))
+    q = torch.full((rows, num_q_heads, d), float("nan"), dtype=dt, device="cuda")
+    kc, vc = (torch.zeros((rows, num_kv_heads, d), dtype=dt, device="cuda") for _ in range(2))
+    nvk().qkv_linear_norm_rope_store(x, w, to_dev(pos), qw if normed else None, kw if normed else None, pw["eps"], to_dev(table), to_dev(slots), kc, vc,
+                                     num_q_heads, num_kv_heads, d, q)
+    qkv = torch.empty((rows, heads * d), dtype=dt, device="cuda")
+    nvk().linear(x, w, qkv)
+    torch.cuda.synchronize()
+    assert nvk().gemm_status() == 0
+    k, v = kc.flip(0), vc.flip(0)                                        # in the order of the rows
+    stored = torch.ones(rows, dtype=torch.bool, device="cuda")
+    stored[rows // 2] = False
+    assert bool((k[rows // 2] == 0).all()) and bool((v[rows // 2] == 0).all())
+    assert torch.equal(q, q[at]) and torch.equal(k[stored], k[at][stored]) and torch.equal(v[stored], v[at][stored])
+    n = period
+    if normed:
+        kc_ref, vc_ref = np.zeros((n, num_kv_heads, d), np.float32), np.zeros((n, num_kv_heads, d), np.float32)
+        q_ref = oracle.fused_split_norm_rope_store(to_np(qkv[:n]), pos[:n], to_np(qw), to_np(kw), pw["eps"], table, np.arange(n, dtype=np.int32), kc_ref, vc_ref,
+                                                   num_q_heads, num_kv_heads, d, oracle.ROUND_NONE)
+    else:
+        parts = to_np(qkv[:n]).reshape(n, heads, d)
+        inside = pos[:n] < max_pos
+        t = table[np.where(inside, pos[:n], 0)][:, None]
+        lo, hi, cs, sn = parts[..., :64], parts[..., 64:], t[..., :64], t[..., 64:]
+        turned = np.where(inside[:, None, None], np.concatenate([lo * cs - hi * sn, hi * cs + lo * sn], -1), parts)
+        q_ref, kc_ref, vc_ref = turned[:, :num_q_heads], turned[:, num_q_heads:num_q_heads + num_kv_heads], parts[:, num_q_heads + num_kv_heads:]
+    assert np.array_equal(to_np(v[:n]), vc_ref)
+    for got, ref in ((to_np(q[:n]), q_ref), (to_np(k[:n]), kc_ref)):
+        # half a unit of an fp16 result and the fp32 steps before it; where a rotation's terms cancel, those of the terms (at most some 6)
+        assert (np.abs(got - ref) <= np.abs(ref) * 2.0 ** -10 + 2.0 ** -18).all(), np.abs(got - ref).max()
