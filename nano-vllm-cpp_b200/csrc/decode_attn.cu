@@ -78,11 +78,6 @@ __device__ __forceinline__ int sequence_of_rank(const DecodeParams& p, int rank,
     }
 }
 
-__device__ __forceinline__ uint32_t in_block(uint32_t addr, uint32_t rank) {   // the same place in block `rank` of the cluster
-    uint32_t r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
 __device__ __forceinline__ void st_cluster4(uint32_t addr, uint32_t rank, const float4& v) {
     asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"r"(in_block(addr, rank)), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }

@@ -59,11 +59,6 @@ __device__ __forceinline__ uint4 lds16(uint32_t addr) {   // (volatile: stays on
     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
     return v;
 }
-__device__ __forceinline__ uint32_t in_block(const void* p, uint32_t rank) {   // the same place in block `rank` of the cluster
-    uint32_t r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
-    return r;
-}
 
 // HG: query heads of a chunk (rounded up to 1, 2 or 4; rows past the group are computed on zeros and not written).
 // W: warps of a block; 4, of which four (three) fit on an SM, or 8 of 24 KiB each where there are few blocks, one per SM.
@@ -269,9 +264,9 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 1 : HG <= 2 ? 4 : 3) decode_s
         const int to = e / quads, at = e - to * quads;
         if (split == 0) {
             asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};\n"
-                         ::"r"(in_block(s_o + rank * quads + at, to)), "f"(t.x), "f"(t.y), "f"(t.z), "f"(t.w) : "memory");
+                         ::"r"(in_block(smem_u32(s_o + rank * quads + at), to)), "f"(t.x), "f"(t.y), "f"(t.z), "f"(t.w) : "memory");
             if (at == 0 || e == h * (D / 4))   // (a block may finish quads of several heads, a head may be finished by several blocks)
-                asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};\n" ::"r"(in_block(&s_ml[rank][h], to)), "f"(mx), "f"(sum) : "memory");
+                asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};\n" ::"r"(in_block(smem_u32(&s_ml[rank][h]), to)), "f"(mx), "f"(sum) : "memory");
         }
     }
     asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory");

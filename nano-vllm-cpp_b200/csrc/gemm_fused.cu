@@ -45,7 +45,6 @@ constexpr int kBarOffset = kStageOffset + 8 * kEpilogueBytes;
 constexpr int kSmemBytes = kBarOffset + 256 + 1024;   // + slack for 1024-byte alignment
 constexpr int kThreads = 256;                         // warp 0 TMA, warp 1 MMA + TMEM, warps 2-5 TMEM readers, all for the sums
 constexpr int kPairThreads = 320;                     // the same with warps 2-9 for the epilogue
-constexpr int kMaxSplits = 8;                         // portable cluster size
 constexpr long long kWaitCycles = 4000000000LL;       // ~2 s
 constexpr int kMaxRanks = NVK_TP_MAX_RANKS;
 
@@ -136,11 +135,6 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
         ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(bar) : "memory");
 }
-__device__ __forceinline__ uint32_t in_block(uint32_t addr, uint32_t rank) {   // the same place in block `rank` of the cluster
-    uint32_t r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
@@ -150,20 +144,10 @@ __device__ __forceinline__ void cluster_sync_all() {
     __syncwarp();
     asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
 }
-// `bytes` of this block's shared memory into that of block `rank`, counted on its barrier at `bar`.
-__device__ __forceinline__ void push_bulk(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar, uint32_t rank) {
-    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
-                 ::"r"(in_block(dst, rank)), "r"(src), "r"(bytes), "r"(in_block(bar, rank)) : "memory");
-}
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
     asm("mov.u32 %0, %cluster_ctarank;\n" : "=r"(r));
     return r;
-}
-__device__ __forceinline__ float4 ld_cluster(uint32_t addr) {                  // shared::cluster address
-    float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
-    return v;
 }
 // MMAs and commits of gemm_split_kernel come from a converged warp: all lanes run through the same instructions, so that the operands are uniform registers, which is where
 // the MMA wants them, and one lane (`leader` 1) issues.  A single diverged lane has to move every operand there first, 75 to 100 clocks an

@@ -53,16 +53,6 @@ struct IndexArray {
     __device__ __forceinline__ int64_t operator[](int64_t i) const {
         return wide ? static_cast<const int64_t*>(ptr)[i] : static_cast<int64_t>(static_cast<const int32_t*>(ptr)[i]);
     }
-    // The same as one of two predicated loads, half the code, but no load that the compiler may move: for kernels that look up many indices in a loop
-    // (fp32 decode of 8 sequences 16.65 -> 15.9 us a pass; 1 sequence in the tensor-core kernel 7.2 -> 7.3, which keeps the branch).
-    __device__ __forceinline__ int64_t load(int64_t i) const {
-        int64_t v;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\t"
-            "@p ld.global.s64 %0, [%1];\n\t@!p ld.global.s32 %0, [%1];\n\t}\n"
-            : "=l"(v) : "l"(static_cast<const char*>(ptr) + (i << (2 + wide))), "r"(wide));
-        return v;
-    }
     // An index as loaded, both words; value() widens it later, so that other loads can be issued before this one has come back (operator[] waits
     // for it to extend its sign).
     struct Raw { int lo, hi; };
@@ -81,7 +71,8 @@ struct IndexArray {
 #endif
 };
 
-// Division of 0 <= n < 2^31 by a launch-uniform number: a multiplication and a shift instead of some 25 instructions in a chain.
+// Division of 0 <= n < 2^31 by a launch-uniform number: a multiplication and a shift instead of some 25 instructions in a chain (the rounded-up
+// reciprocal of Granlund and Montgomery, Division by Invariant Integers using Multiplication, 1994).
 struct FastDiv {
     uint32_t d = 1, mul = 1, shift = 0;
     FastDiv() = default;
@@ -264,6 +255,18 @@ constexpr float kLog2e = 1.4426950408889634f;
 __device__ __forceinline__ void pdl_wait_then_release() {
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
+// The same place of shared memory in block `rank` of the cluster.
+__device__ __forceinline__ uint32_t in_block(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+// `bytes` of this block's shared memory into that of block `rank`, counted on its barrier at `bar`.
+__device__ __forceinline__ void push_bulk(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar, uint32_t rank) {
+    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
+                 ::"r"(in_block(dst, rank)), "r"(src), "r"(bytes), "r"(in_block(bar, rank)) : "memory");
 }
 
 // For a kernel that needs nothing of the one launched just before it, which for its part waited (pdl_wait_then_release) before it let this one start:

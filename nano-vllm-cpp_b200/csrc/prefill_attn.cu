@@ -54,16 +54,6 @@ struct PrefillParams {
 __device__ __forceinline__ uint32_t swz(int row, int chunk) {
     return static_cast<uint32_t>(row * kRowBytes + ((chunk ^ (row & 7)) << 4));
 }
-__device__ __forceinline__ uint32_t in_block(uint32_t addr, uint32_t rank) {   // the same place in block `rank` of the cluster
-    uint32_t r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-// `bytes` of this block's shared memory into that of block `rank`, counted on its barrier at `bar`.
-__device__ __forceinline__ void push_bulk(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar, uint32_t rank) {
-    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
-                 ::"r"(in_block(dst, rank)), "r"(src), "r"(bytes), "r"(in_block(bar, rank)) : "memory");
-}
 __device__ int g_prefill_error = 0;
 
 template <typename T>
@@ -464,7 +454,7 @@ int best_cluster(const PrefillArgs& a, const Alike& equal) {
     const int head_shift = tile_head_shift(a.num_heads / a.num_kv_heads);
     const int64_t rows = kBM >> head_shift, grid = (ceil_div(a.total_q, rows) + (a.cu_q ? a.num_seqs : 0)) * (a.num_heads >> head_shift);
     int best = 0;
-    for (int s = 1; s <= 3 && (grid << s) <= 2 * kSmCount; ++s)
+    for (int s = 1; (1 << s) <= kMaxCluster && (grid << s) <= 2 * kSmCount; ++s)
         if (tile_time(a, &equal, 1, s) < tile_time(a, &equal, 1, best)) best = s;
     return best;
 }
