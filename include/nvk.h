@@ -90,7 +90,8 @@ int nvk_fused_split_norm_rope_store(const void* qkv, const int32_t* positions,
 /*
  * Scratch size for nvk_decode_attention_paged (split-K partial results).  Depends only on
  * host-known sizes, never on context_lens, so the value is stable across graph replays.  Enough for
- * every call with no more sequences and no wider block tables.
+ * every call with no more sequences and no wider block tables.  0: a call of these sizes has no use for
+ * scratch (smaller ones may have: they run without it when workspace is NULL).
  */
 size_t nvk_decode_attention_workspace_bytes(int64_t batch, int num_heads, int num_kv_heads,
                                             int head_dim, int64_t max_blocks, int block_size);

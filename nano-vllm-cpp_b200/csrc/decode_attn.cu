@@ -493,9 +493,12 @@ size_t decode_mma_workspace_needed(int64_t batch, int num_heads, int num_kv_head
 size_t decode_mma_workspace_bytes(int64_t batch, int num_heads, int num_kv_heads, int head_dim,
                                   int64_t max_blocks, int block_size) {
     const size_t need = decode_mma_workspace_needed(batch, num_heads, num_kv_heads, head_dim, max_blocks, block_size);
-    if (batch <= 0 || num_heads <= 0 || num_kv_heads <= 0 || max_blocks <= 0 || block_size <= 0) return need;
+    // Whole contexts in narrow tables: none, and a caller without scratch passes none to smaller calls either.  (But with 1.5 to 2.5 pairs to an SM,
+    // where 8-bit caches were once cut in two, the one workspace has always been enough for fewer sequences.)
+    const int64_t pairs = batch * num_kv_heads;
+    if (need == 0 && (2 * pairs <= 3 * kSmCount || 2 * pairs >= 5 * kSmCount)) return 0;
     const int group = (num_heads + num_kv_heads - 1) / num_kv_heads;
-    const size_t most = part_bytes(static_cast<size_t>(most_parts(batch * num_kv_heads, max_blocks * block_size)), group);
+    const size_t most = part_bytes(static_cast<size_t>(most_parts(pairs, max_blocks * block_size)), group);
     // What fits the static array never needs more than it holds; what fills it but for the last 4 bytes a row of 520 goes on in longer chunks (above), a
     // slightly smaller one fills it.
     if (need <= kStaticScratchBytes && (most > kStaticScratchBytes || need + need / 128 > kStaticScratchBytes)) return kStaticScratchBytes;
