@@ -4,12 +4,13 @@
 // reference: one warp per (sequence, query head), every KV row re-read by each query head of its group, 8 dependent shuffles per
 // key) and the FlashAttention-2 call it can dlopen (src/kernels/flash_attn.cpp:302-431).
 //
-// The op is HBM-bound; decode_body.cuh has the arithmetic and the two ways to share out the keys.  What each kernel here adds:
+// The op is HBM-bound; decode_body.cuh has the arithmetic and the ways to share out the keys.  What each kernel here adds:
 //   decode_split_kernel    one four-warp block per (KV head, chunk, sequence), two per SM (three for 8-bit caches).  The grid is fixed
 //                          from host-known sizes: nothing depends on host knowledge of context_lens (CUDA-graph safe); blocks
 //                          whose chunk lies beyond the context exit at once.
 //   decode_merge_kernel    merges the chunks of long contexts; launched only where the table can hold more than one.
-//   decode_cluster_kernel  small steps: a cluster of blocks per (sequence, KV head), merged in the same launch.
+//   decode_cluster_kernel  small steps: a cluster of blocks per (sequence, KV head) takes equal ranges of the context, beyond them two blocks the halves
+//                          of the table's row; merged in the same launch.
 // Which one is taken depends on the table's WIDTH, not on the contexts: one short sequence in a wide table takes chunks and a merge.
 #include "decode_body.cuh"
 

@@ -6,11 +6,12 @@
 // per KV head.  Each warp streams every fourth tile of 16 keys through a private ring of cp.async stages (no barrier in the main
 // loop); at the end the four warps merge through shared memory.
 //
-// Two ways to share a sequence out, by the sizes the host knows:
+// Three ways to share a sequence out, by the sizes the host knows:
 //   chunks     ranges of `chunk_tokens` keys; where a context is longer than one, the ranges leave partial results (maximum, sum,
 //              unnormalised output) in the workspace and a second kernel merges them;
 //   per_seq    num_splits equal ranges of every sequence in one thread-block cluster, merged through distributed shared memory in
-//              the same launch, without a workspace: for small steps.
+//              the same launch, without a workspace: for small steps;
+//   halves     two chunks, each half of the table's row, in one cluster: a context that ends in the first is one block's alone.
 //
 // Cutting the whole batch's keys into equal runs that ignore sequence boundaries (each block sums up the contexts, warps or groups
 // walk on from one sequence to the next with their rings full, a quarter of the work handed out dynamically) was built and measured:

@@ -14,9 +14,9 @@
 //     local -- one launch, no workspace.  The merges run once, and code that runs once is as slow as it is long: with every part unrolled
 //     they took 3 us of a block's 8, now 1.6.
 // Batch 8, 16 / 8 heads, fp32, context 64 .. 1024, store + decode: 2031 us a pass with one warp per (sequence, head) walking its
-// keys in order, 14.7 us with rows in registers (trips of 8 keys in a warp that never overlapped, up to 7.7 us of them, and 3.3 us of merges
-// by shuffles and by fetching peers' parts), 12.5 us here; 1 sequence of 100 keys 7.8 -> 4.7, 7 of 64 to 200 (8 / 4 heads) 9.6 -> 6.0, 8 of 4000 to 4096
-// (32 / 8 heads) 71 -> 64.  Sequences in order of falling context so that long and short blocks share an SM: 13.3 -> 13.7 in an earlier form.
+// keys in order, 15.2 us with rows in registers (trips of 8 keys in a warp that never overlapped, up to 7.7 us of them, and 3.3 us of merges
+// by shuffles and by fetching peers' parts), 12.4 us here; 1 sequence of 100 keys 8.1 -> 4.7, 7 of 64 to 200 (8 / 4 heads) 10.0 -> 6.0, 8 of 4000 to 4096
+// (32 / 8 heads) 71.5 -> 64.  Sequences in order of falling context so that long and short blocks share an SM: 13.3 -> 13.7 in an earlier form.
 #include "nvk_internal.cuh"
 
 #include <atomic>

@@ -22,7 +22,7 @@
 //                       loads half of A and half of B, so an SM moves half the operand bytes of a 128 x 256 tile of its own.  The
 //                       accumulator is double buffered in TMEM: the epilogue of a tile runs under the next tile's MMAs.
 // Before, one block per 128 x 128 tile whatever the size (microseconds in a loop over weights larger than L2; K 4096):
-//   64 x 6144  22 -> 16      64 x 4096  21 -> 12 (with MMAs from a converged warp 14.5 and 11.1, with pushed sums 13.1 and 10.4)     7440 x 4096  295 -> 175 (1430 TFLOP/s)     7440 x 6144 with QKV epilogue  597 -> 277
+//   64 x 6144  22 -> 16      64 x 4096  21 -> 12 (with MMAs from a converged warp 14.5 and 11.1, with pushed sums 13.3 and 10.0)     7440 x 4096  295 -> 175 (1430 TFLOP/s)     7440 x 6144 with QKV epilogue  597 -> 277
 // What the fusion removes is the round trip of the result and one or two launches per layer.
 // Every mbarrier wait is bounded; a wait that runs out raises an error word (nvk_gemm_status), and the block leaves when what it
 // has under way has had time to land.
@@ -657,8 +657,8 @@ __device__ __forceinline__ void epilogue_octet(const GemmParams& p, const OctetR
 // block pushes each run by one bulk copy into the shared memory of the block that finishes it, where all that follows is local (rows of 512
 // bytes, their 16-byte pieces XOR-swizzled by row: no bank conflicts for the writing threads, each of which has a row, nor for the readers, eight
 // lanes a row).  What peers push has a place of its own, for more than 64 rows the ring's last stage with it.  When the sums were fetched from
-// the peers' shared memory instead, 10 bytes a clock came in: from the last MMA to a block's end 4.0 us for 64 x 6144, K 4096 (15.8 us in all, 13.9
-// now), 3.2 for 64 x 4096 (11.1, 10.4), 5.5 for 128 x 6144 (17.6, 15.8).
+// the peers' shared memory instead, 10 bytes a clock came in: from the last MMA to a block's end 4.0 us for 64 x 6144, K 4096 with the QKV epilogue (15.8
+// us in all, 14.0 now), 3.2 for 64 x 4096 (11.1, 10.0), 5.5 for QKV 128 x 6144 (17.6, 15.7).
 template <typename T, int EPI, int MT, bool DIRECT>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ GemmParams p, int splits) {
@@ -812,7 +812,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     }
 #pragma unroll 1
     for (; ok && l < own_rows; l += kTrip) {
-        // the next trip's table rows and the positions of the one after it are on their way under this one (128 x 6144, K 4096, QKV: 16.0 -> 15.4 us)
+        // the next trip's table rows and the positions of the one after it are on their way under this one (128 x 6144, K 4096, QKV: 0.6 us)
         OctetRow<T> next{};
         if (l + kTrip < own_rows) next = octet_row<T, EPI>(p, row_of(l + kTrip), at_next, nt, sub);
         at_next = index_of(l + 2 * kTrip);

@@ -2,8 +2,8 @@
 // F16 / BF16, head_dim 128, dense or paged keys (block_size a multiple of 128).
 //
 // Replaces the same reference code as prefill_attn.cu (src/kernels/attention.cu:114-302,
-// src/kernels/flash_attn.cpp:203-300); prefill_attn.cu (mma.sync) remains the path for shapes this
-// kernel does not take.
+// src/kernels/flash_attn.cpp:203-300); prefill_attn.cu (mma.sync) takes small steps and what
+// these kernels do not (cache blocks that are no multiple of 128, scales that are not positive).
 //
 // Two kernels live here, chosen by shape: the single-tile kernel described next (odd GQA group sizes) and the
 // persistent head-pair kernel further down (even group sizes: the two query heads of a pair share their K / V tiles).
