@@ -4,8 +4,8 @@
 // Replaces the same reference kernel as decode_attn.cu (src/kernels/attention.cu:313-405).  The op reads each K / V row once
 // and does 4 * G flops per element, so HBM bounds it; what has to be organised is enough bytes in flight from a batch of a
 // few sequences, and little before the first and after the last of them:
-//   * one thread-block cluster per (sequence, KV head, chunk of up to four query heads), blocks of four warps, four (three) to an SM: cluster
-//     size 1, 2, 4 or 8, as large as keeps all blocks resident, so 8 sequences x 8 KV heads already occupy every SM;
+//   * one thread-block cluster per (sequence, KV head, chunk of up to four query heads), blocks of four or eight warps, sixteen (twelve, eight) warps to an
+//     SM: cluster size 1, 2, 4 or 8, so 8 sequences x 8 KV heads already occupy every SM;
 //   * steps of 32 / (D / 16) keys (4 at D 128) are dealt round-robin to the cluster's warps; a key is spread over D / 16 lanes, 16 elements
 //     each, so a warp reads whole 128-byte lines and a dot product needs log2(D / 16) shuffles.  K and V come through a ring in shared
 //     memory by cp.async, 12 KiB a warp: a lane copies what it will read itself, so a step waits for nothing but its own copies;
@@ -61,11 +61,14 @@ __device__ __forceinline__ uint4 lds16(uint32_t addr) {   // (volatile: stays on
 }
 
 // HG: query heads of a chunk (rounded up to 1, 2 or 4; rows past the group are computed on zeros and not written).
-// W: warps of a block; 4, of which four (three) fit on an SM, or 8 of 24 KiB each where there are few blocks, one per SM.
-template <int W> constexpr int kWarpRing = W == 4 ? 12 * 1024 : 24 * 1024;
+// W: warps of a block; 4, of which four (HG 4: three) fit on an SM, or 8, of which two (one) do.
+template <int HG, int W> constexpr int kBlocksPerSm = W == 4 ? (HG <= 2 ? 4 : 3) : HG <= 2 ? 2 : 1;
+template <int HG, int W> constexpr int kWarpRing = W == 8 && HG == 4 ? 24 * 1024 : 12 * 1024;
 template <typename T, int D, int HG, int W>
-__global__ void __launch_bounds__(W * 32, W == 8 ? 1 : HG <= 2 ? 4 : 3) decode_simt_kernel(const __grid_constant__ SimtParams p) {
-    constexpr int kWarps = W, kThreads = W * 32, RING = kWarpRing<W>;
+__global__ void __launch_bounds__(W * 32, kBlocksPerSm<HG, W>) decode_simt_kernel(const __grid_constant__ SimtParams p) {
+    constexpr int kWarps = W, kThreads = W * 32, RING = kWarpRing<HG, W>;
+    // Steps in one trip of the loop: a step is a serial chain (dot product, shuffles, exponential, sum), which two warps per scheduler do not hide.
+    constexpr int U = W == 8 && HG == 4 ? 2 : 1;
     constexpr int LANES = D / 16;                         // lanes per key
     constexpr int GROUPS = 32 / LANES;                    // keys of a step
     constexpr int VE = 16 / static_cast<int>(sizeof(T));  // elements per 16-byte vector
@@ -141,7 +144,7 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 1 : HG <= 2 ? 4 : 3) decode_s
         cp_async_commit();
     };
 #pragma unroll 1   // (code that runs once is as slow as it is long)
-    for (int s = 0; s < STAGES - 1; ++s) issue();
+    for (int s = 0; s < STAGES - U; ++s) issue();
 #pragma unroll
     for (int i = 0; i < (HG * D + kThreads - 1) / kThreads; ++i)
         if (i * kThreads + tid < HG * D) s_q[i * kThreads + tid] = q_in[i];
@@ -164,50 +167,82 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 1 : HG <= 2 ? 4 : 3) decode_s
         for (int e = 0; e < 16; ++e) acc[h][e] = 0.0f;
     }
     uint32_t use = ring;
+    auto next = [&](uint32_t at) { return at == ring + (STAGES - 1) * STAGE ? ring : at + STAGE; };
 #pragma unroll 1
-    for (int k0 = first; k0 < ctx; k0 += stride) {
-        issue();
-        cp_async_wait<STAGES - 1>();
-        const bool live = k0 + grp < ctx;
-        float s[HG][4], f[16];
+    for (int k0 = first; k0 < ctx; k0 += U * stride) {
 #pragma unroll
-        for (int i = 0; i < NV; ++i) unpack<T>(lds16(use + i * 512), f + i * VE);
+        for (int u = 0; u < U; ++u) issue();
+        cp_async_wait<STAGES - U>();
+        float sc[U][HG], fv[16];                 // scores, then weights; V (the first step's on its way under the exponentials)
+        bool live[U];
+        uint32_t at = use;
 #pragma unroll
-        for (int h = 0; h < HG; ++h) {
+        for (int u = 0; u < U; ++u) {
+            float f[16];
+            live[u] = k0 + u * stride + grp < ctx;
 #pragma unroll
-            for (int e = 0; e < 16; e += 4) {
-                float4 qf;
-                if (kQInRegs) qf = make_float4(qr[h][e], qr[h][e + 1], qr[h][e + 2], qr[h][e + 3]);
-                else qf = *reinterpret_cast<const float4*>(&s_q[h * D + ((e / VE) * LANES + sub) * VE + e % VE]);
-                s[h][0] = e == 0 ? qf.x * f[e] : fmaf(qf.x, f[e], s[h][0]);
-                s[h][1] = e == 0 ? qf.y * f[e + 1] : fmaf(qf.y, f[e + 1], s[h][1]);
-                s[h][2] = e == 0 ? qf.z * f[e + 2] : fmaf(qf.z, f[e + 2], s[h][2]);
-                s[h][3] = e == 0 ? qf.w * f[e + 3] : fmaf(qf.w, f[e + 3], s[h][3]);
+            for (int i = 0; i < NV; ++i) unpack<T>(lds16(at + i * 512), f + i * VE);
+#pragma unroll
+            for (int h = 0; h < HG; ++h) {
+                float s[4];
+#pragma unroll
+                for (int e = 0; e < 16; e += 4) {
+                    float4 qf;
+                    if (kQInRegs) qf = make_float4(qr[h][e], qr[h][e + 1], qr[h][e + 2], qr[h][e + 3]);
+                    else qf = *reinterpret_cast<const float4*>(&s_q[h * D + ((e / VE) * LANES + sub) * VE + e % VE]);
+                    s[0] = e == 0 ? qf.x * f[e] : fmaf(qf.x, f[e], s[0]);
+                    s[1] = e == 0 ? qf.y * f[e + 1] : fmaf(qf.y, f[e + 1], s[1]);
+                    s[2] = e == 0 ? qf.z * f[e + 2] : fmaf(qf.z, f[e + 2], s[2]);
+                    s[3] = e == 0 ? qf.w * f[e + 3] : fmaf(qf.w, f[e + 3], s[3]);
+                }
+                sc[u][h] = (s[0] + s[1]) + (s[2] + s[3]);
             }
-            s[h][0] = (s[h][0] + s[h][1]) + (s[h][2] + s[h][3]);
+            at = next(at);
         }
 #pragma unroll
         for (int o = LANES / 2; o > 0; o >>= 1) {
 #pragma unroll
-            for (int h = 0; h < HG; ++h) s[h][0] += __shfl_xor_sync(0xffffffffu, s[h][0], o);
+            for (int u = 0; u < U; ++u) {
+#pragma unroll
+                for (int h = 0; h < HG; ++h) sc[u][h] += __shfl_xor_sync(0xffffffffu, sc[u][h], o);
+            }
         }
 #pragma unroll
-        for (int i = 0; i < NV; ++i) unpack<T>(lds16(use + (NV + i) * 512), f + i * VE);
+        for (int i = 0; i < NV; ++i) unpack<T>(lds16(use + (NV + i) * 512), fv + i * VE);
 #pragma unroll
         for (int h = 0; h < HG; ++h) {
-            if (live && s[h][0] > m[h]) {   // (same for all lanes of a group)
-                const float corr = expf(m[h] - s[h][0]);
+            float top = m[h];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (live[u] && sc[u][h] > top) top = sc[u][h];
+            if (top > m[h]) {   // (same for all lanes of a group)
+                const float corr = expf(m[h] - top);
                 l[h] *= corr;
 #pragma unroll
                 for (int e = 0; e < 16; ++e) acc[h][e] *= corr;
-                m[h] = s[h][0];
+                m[h] = top;
             }
-            const float w = !live || s[h][0] == -INFINITY ? 0.0f : expf(s[h][0] - m[h]);
-            l[h] += w;
 #pragma unroll
-            for (int e = 0; e < 16; ++e) acc[h][e] = fmaf(w, f[e], acc[h][e]);
+            for (int u = 0; u < U; ++u) {
+                sc[u][h] = !live[u] || sc[u][h] == -INFINITY ? 0.0f : expf(sc[u][h] - m[h]);
+                l[h] += sc[u][h];
+            }
         }
-        use = use == ring + (STAGES - 1) * STAGE ? ring : use + STAGE;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (u == 0 || k0 + u * stride < ctx) {   // (what was not copied for there is not read: nothing times a weight of 0 but what is finite)
+                if (u > 0) {
+#pragma unroll
+                    for (int i = 0; i < NV; ++i) unpack<T>(lds16(use + (NV + i) * 512), fv + i * VE);
+                }
+#pragma unroll
+                for (int h = 0; h < HG; ++h) {
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) acc[h][e] = fmaf(sc[u][h], fv[e], acc[h][e]);
+                }
+            }
+            use = next(use);
+        }
     }
 
     // lane groups -> block: under the warp's maximum every group leaves its part over its warp's ring, TPQ threads add up a quad of the result
@@ -298,7 +333,7 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 1 : HG <= 2 ? 4 : 3) decode_s
 
 template <typename T, int D, int HG, int W>
 int launch_simt_blocks(SimtParams& p, int64_t blocks, cudaStream_t stream) {
-    constexpr int kSmemBytes = W * kWarpRing<W>;
+    constexpr int kSmemBytes = W * kWarpRing<HG, W>;
     auto* kernel = decode_simt_kernel<T, D, HG, W>;
     static std::atomic<bool> attr_done[64] = {};   // per device; the attribute call is idempotent
     int device = 0;
@@ -325,24 +360,43 @@ int launch_simt_blocks(SimtParams& p, int64_t blocks, cudaStream_t stream) {
     return check_launch("decode_simt_kernel launch");
 }
 
-// Eight warps with twice the ring where no more clusters of 8 than fit at one block per SM (15; a cluster has to fit into one GPC) and tables that
-// give a block some keys: us a pass with four / eight warps: 1 sequence of 4096 keys, 32 / 8 heads, 29.4 / 22.0, 1 of 1600 to 2100, 8 / 2 heads, 15.8 / 13.2,
-// 1 of 500, 16 / 4 heads, 7.8 / 7.3, 1 of 300, 16 / 8 heads, 5.9 / 6.0.  16 to 33 clusters of 4 such blocks: 4 sequences of 4000 keys, 16 / 8 heads, 28.2, clusters
-// of 8 blocks of four warps 26.6.
-constexpr int kWideClusters = 15, kWideTokens = 512;
+// log2 of the cluster size and warps of a block, for so many items and keys of a table row.  Blocks of four warps: as large a cluster as keeps all blocks
+// resident; beyond that a larger one only adds merges.  Blocks of eight where that gives an item more warps (with four heads, whose trips then take two steps: as
+// many), because one long context is what a step waits for: with few items, and with so many that each gets one block.  us a call, four / eight warps,
+// fp32, head_dim 128, contexts of 2600 keys: 1 sequence of 8 / 1 heads 19.8 / 13.9; 4 of 16 / 8, of which one is that long and the others have 80, 13.3 / 11.8; 8 of 32 / 8, from 130
+// keys on, 41.2 / 36.4; 48 of 16 / 8, one long, 73.2 / 45.2, from 130 on 101 / 88, all 165 / 160; 120 of 8 / 1, one long, 124 / 76, all 182 / 140; but 200 of 8 / 1,
+// all, 185 / 210 (one long 125 / 70), 24 of 16 / 8 from 130 on 53.8 / 56.7, and 300 of 300 keys, 16 / 8 heads of 64, 67 / 77.  (With blocks of four warps alone 120 sequences of 8 / 1
+// heads of 256, 16-bit, one of 2600 keys, took 279 us; in an earlier form of eight warps with rows in registers 151, now 148.)
+struct Shape { int csize_shift, warps; };
+Shape choose_shape(int64_t items, int64_t tokens, int head_dim, int elem_bytes, int heads) {
+    const int64_t resident = static_cast<int64_t>(kSmCount) * (heads <= 2 ? 4 : 3);
+    const bool slow = heads == 4 && head_dim == 256 && elem_bytes == 2;   // the longest steps for their bytes
+    int four = 0;
+    while ((1 << four) < kMaxCluster && (items << (four + 1)) <= resident) ++four;
+    if (four == 0) {
+        if (tokens <= 512) return {0, items <= (heads <= 2 || head_dim == 256 ? 3 : 2) * kSmCount ? 8 : 4};
+        return {0, heads <= 2 || head_dim == 256 || items <= 8 * kSmCount ? 8 : 4};
+    }
+    if (tokens <= 512 && head_dim < 256) return {four, 4};
+    if (heads <= 2) return items <= 33 ? Shape{3, 8} : Shape{four, 4};
+    // Eight warps, one block to an SM.  A cluster has to fit into one GPC: 15 of eight blocks, 33 of four, 74 of two are resident at once; three of eight blocks more
+    // are quicker than smaller ones where a single context is long.
+    if (items <= 15 || (items <= 18 && tokens > 2048 && head_dim > 64)) return {3, 8};
+    if (items > 18 && items <= 33) return {2, 8};
+    if (items > 55 && items <= 74) return {1, 8};
+    if (items > 111 && (items <= kSmCount || slow)) return {0, 8};
+    return {four, 4};
+}
 template <typename T, int D, int HG>
 int launch_simt_typed(SimtParams& p, cudaStream_t stream) {
     const int64_t items = static_cast<int64_t>(p.batch) * p.num_kv_heads * p.chunks;
-    // All blocks resident at once: beyond that a larger cluster only adds merges.
-    const bool wide = items <= kWideClusters && p.max_blocks * p.block_size >= kWideTokens;
-    const int64_t resident = static_cast<int64_t>(kSmCount) * (HG <= 2 ? 4 : 3);
-    p.csize_shift = 0;
-    while ((1 << p.csize_shift) < kMaxCluster && (items << (p.csize_shift + 1)) <= resident) ++p.csize_shift;
+    const Shape shape = choose_shape(items, p.max_blocks * p.block_size, D, sizeof(T), HG);
+    p.csize_shift = shape.csize_shift;
     const int64_t blocks = items << p.csize_shift;
     p.by_block = FastDiv(static_cast<uint32_t>(p.block_size));
     p.by_chunks = FastDiv(static_cast<uint32_t>(p.chunks));
     p.by_kv_heads = FastDiv(static_cast<uint32_t>(p.num_kv_heads));
-    return wide ? launch_simt_blocks<T, D, HG, 8>(p, blocks, stream) : launch_simt_blocks<T, D, HG, 4>(p, blocks, stream);
+    return shape.warps == 8 ? launch_simt_blocks<T, D, HG, 8>(p, blocks, stream) : launch_simt_blocks<T, D, HG, 4>(p, blocks, stream);
 }
 
 template <typename T, int D>

@@ -99,3 +99,28 @@ def test_decode_simt_block_sizes_and_keys_without_weight(dtype, head_dim, block_
     nvk().launch_decode_attention_paged(*args, *tail, out)
     err = np.abs(to_np(out) - _reference(w, num_kv_heads, block_size))
     assert err.max() <= (2e-6 if dtype == "f32" else 1e-2), err.max()
+
+
+@pytest.mark.parametrize("dtype,head_dim", [("f32", 128), ("f32", 64), ("bf16", 256)])
+@pytest.mark.parametrize("num_heads,num_kv_heads,batch,keys", [
+    (4, 1, 15, 1024), (4, 1, 16, 1024), (4, 1, 18, 2304), (8, 1, 16, 1024), (4, 1, 34, 768), (4, 1, 55, 768), (4, 1, 56, 768), (4, 1, 75, 768), (4, 1, 112, 768),
+    (3, 1, 149, 768), (4, 1, 223, 512), (4, 1, 223, 768), (4, 1, 297, 512), (4, 1, 1185, 768),                    # four heads: clusters of 8, 4, 2 and 1, of both kinds of blocks
+    (2, 1, 33, 768), (2, 1, 34, 768), (1, 1, 297, 768), (2, 1, 297, 512), (2, 1, 445, 512),                      # one and two
+])
+def test_decode_simt_blocks_of_four_and_of_eight_warps(dtype, head_dim, num_heads, num_kv_heads, batch, keys):
+    """Both sides of the lines between them; contexts around one and two steps of a block's warps, a few of them long; what was left in shared memory by
+    others (infinities) does not matter."""
+    per = 8 * 512 // head_dim                                            # keys of a step of eight warps
+    ctx = np.array(([1, 0, per // 2, per - 1, per, per + 1, 2 * per - 1, 2 * per, 2 * per + 1, 3 * per, 5] * (batch // 11 + 1))[:batch], np.int32)
+    ctx[0], ctx[-1] = keys, keys - 1
+    w = workloads().make_decode_workload(batch, num_heads, num_kv_heads, head_dim, 256, 0, 0, seed=batch + head_dim, context_lens=ctx,
+                                         value_scale=0.5, rounded=dtype != "f32")
+    td = {"f32": torch.float32, "bf16": torch.bfloat16}[dtype]
+    q, kc, vc, lens, bt = to_dev(w["q"], td), to_dev(w["k_cache"], td), to_dev(w["v_cache"], td), to_dev(ctx), to_dev(w["block_tables"])
+    out = torch.full_like(q, float("nan"))
+    inf = torch.full_like(vc, float("inf"))
+    nvk().launch_decode_attention_paged(q, kc, inf, lens, bt, num_kv_heads, head_dim, 256, w["scale"], out)
+    out.fill_(float("nan"))
+    nvk().launch_decode_attention_paged(q, kc, vc, lens, bt, num_kv_heads, head_dim, 256, w["scale"], out)
+    err = np.abs(to_np(out) - _reference(w, num_kv_heads, 256))
+    assert err.max() <= (2e-6 if dtype == "f32" else 1e-2), err.max()
